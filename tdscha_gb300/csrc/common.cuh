@@ -71,6 +71,10 @@ struct MixedStore {
 
 }  // namespace tdscha
 
+namespace tdscha {
+struct DigitStore;   // perturb_digits.cu
+}
+
 struct tdscha_ctx {
     int device = 0;
     int M = 0, N = 0, S = 0;
@@ -142,6 +146,7 @@ struct tdscha_ctx {
     double *host_pinned = nullptr;
     int nblk_dot = 0;
     tdscha::MixedStore mx;
+    tdscha::DigitStore *dg = nullptr;   // float64 averages by digit products (null: CUDA cores)
     // diagnostics: CUDA-event pairs per kernel id while profiling is on
     int prof = 0;
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> prof_ev[8];
@@ -192,6 +197,11 @@ namespace tdscha {
 // perturb_fp64.cu
 int perturb_fp64(tdscha_ctx *c, int apply_d4, cudaStream_t st);
 int alloc_fp64_scratch(tdscha_ctx *c);
+// perturb_digits.cu: the float64 averages by exact digit products on the tensor cores
+int digits_prepare(tdscha_ctx *c);
+void digits_release(tdscha_ctx *c);
+int digits_check_error(tdscha_ctx *c);
+int perturb_digits(tdscha_ctx *c, int apply_d4, cudaStream_t st);
 // perturb_mixed.cu
 int mixed_prepare(tdscha_ctx *c);
 int mixed_release(tdscha_ctx *c);
@@ -233,6 +243,11 @@ int psi_perturbation64(tdscha_ctx *c, cudaStream_t st);
 // j*jstride + a*lda + b] and force partials fpart[(j*nfchunk + chunk)*M + m]
 int psi_finalize64(tdscha_ctx *c, const double *gpart, int nsplit, long sstride, long jstride,
                    long lda, const double *fpart, int nfchunk, cudaStream_t st);
+// the two halves of psi_finalize64: hs and fs of images j0 .. j0 + nj - 1 (the
+// partials of image j0 first), then f and d2v from all of them
+int psi_hsum64(tdscha_ctx *c, const double *gpart, int nsplit, long sstride, long jstride, long lda,
+               const double *fpart, int nfchunk, int j0, int nj, cudaStream_t st);
+int psi_reduce64(tdscha_ctx *c, cudaStream_t st);
 int psi_finalize32(tdscha_ctx *c, const float *gpart, int nsplit, long sstride, long jstride,
                    long lda, const float *fpart, int nfchunk, double *f_out, double *d2v_out,
                    cudaStream_t st);

@@ -233,6 +233,7 @@ static void ctx_free(tdscha_ctx *c) {
     if (!c) return;
     prof_clear(c);
     mixed_release(c);
+    digits_release(c);
     double *bufs[] = {c->w, c->fY, c->fpsi, c->rho, c->Yw, c->ReAw, c->D, c->F, c->pc,
                       c->R1, c->Y1, c->f, c->d2v, c->qp_part, c->alpha, c->beta, c->c1,
                       c->c2, c->gpart, c->fpart, c->Lq, c->pL, c->rk, c->sk, c->mask,
@@ -407,7 +408,6 @@ images_done:
 
     TRYC(dev_alloc(&c->R1, M)); TRYC(dev_alloc(&c->Y1, (size_t)M * M));
     TRYC(dev_alloc(&c->f, M)); TRYC(dev_alloc(&c->d2v, (size_t)M * M));
-    TRYC(alloc_fp64_scratch(c));
     TRYC(dev_alloc(&c->Lq, c->P)); TRYC(dev_alloc(&c->pL, c->P));
     TRYC(dev_alloc(&c->rk, c->P)); TRYC(dev_alloc(&c->sk, c->P));
     TRYC(dev_alloc(&c->mask, c->P)); TRYC(dev_alloc(&c->pc, 12 * c->H + 4 * (size_t)M));
@@ -422,6 +422,8 @@ images_done:
     CUC(cudaMemset(c->scal, 0, sizeof(double) * 64));
     CUC(cudaMallocHost((void **)&c->host_pinned, sizeof(double) * 64));
     TRYC(build_pair_coeffs(c));
+    if (with_mixed != 2) TRYC(digits_prepare(c));
+    if (!c->dg) TRYC(alloc_fp64_scratch(c));
     if (with_mixed) TRYC(mixed_prepare(c));
     CUC(cudaDeviceSynchronize());
     if (with_mixed == 2) {

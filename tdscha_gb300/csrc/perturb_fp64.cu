@@ -1,4 +1,6 @@
-// Float64 perturbation averages on the CUDA cores.
+// Float64 perturbation averages on the CUDA cores: the contexts whose digit
+// operands (perturb_digits.cu, 20 times the rate at M=573, N=50000) would not
+// fit the device, and the entry point that allocates nothing (noalloc.cu).
 //
 // The three reference loops (get_f_average_from_Y_pert_sym_fast,
 // get_d2v_dR2_from_R_pert_sym_fast, get_d2v_dR2_from_Y_pert_sym_fast,
@@ -397,6 +399,7 @@ static int perturb_fp64_img(tdscha_ctx *c, int apply_d4, cudaStream_t st) {
 }
 
 int perturb_fp64(tdscha_ctx *c, int apply_d4, cudaStream_t st) {
+    if (c->dg) return perturb_digits(c, apply_d4, st);
     if (c->J > 1) return perturb_fp64_img(c, apply_d4, st);
     int M = c->M;
     long R = c->R;

@@ -412,18 +412,25 @@ int psi_perturbation64(tdscha_ctx *c, cudaStream_t st) {
     return TDSCHA_OK;
 }
 
-template <typename T>
-static int psi_finalize(tdscha_ctx *c, const T *gpart, int nsplit, long sstride, long jstride,
-                        long lda, const T *fpart, int nfchunk, cudaStream_t st) {
+int psi_hsum64(tdscha_ctx *c, const double *gpart, int nsplit, long sstride, long jstride, long lda,
+               const double *fpart, int nfchunk, int j0, int nj, cudaStream_t st) {
+    const int M = c->M, J = c->J;
+    const size_t MM = (size_t)M * M;
+    double *hs = c->hs, *fs = hs + 2 * J * MM;
+    ProfScope ps(c, 4, st);
+    const int nt = ceil_div(M, 32);
+    dim3 gt(nt * (nt + 1) / 2, nj);
+    k_psi_hsum<double><<<gt, 256, 0, st>>>(gpart, nsplit, sstride, jstride, lda, fpart, nfchunk, M,
+                                           hs + j0 * MM, fs + (size_t)j0 * M);
+    TDS_CHECK_LAUNCH();
+    return TDSCHA_OK;
+}
+
+int psi_reduce64(tdscha_ctx *c, cudaStream_t st) {
     const int M = c->M, J = c->J;
     const size_t JMM = (size_t)J * M * M, JM = (size_t)J * M;
     double *hs = c->hs, *tj = hs + JMM, *fs = tj + JMM, *tf = fs + JM;
     ProfScope ps(c, 4, st);
-    const int nt = ceil_div(M, 32);
-    dim3 gt(nt * (nt + 1) / 2, J);
-    k_psi_hsum<T><<<gt, 256, 0, st>>>(gpart, nsplit, sstride, jstride, lda, fpart, nfchunk, M, hs,
-                                      fs);
-    TDS_CHECK_LAUNCH();
     k_psi_sandwich<<<grid_for((long)JMM), 256, 0, st>>>(c->sr_idx, c->sr_val, hs, fs, J, M,
                                                         c->maxdeg, tj, tf);
     TDS_CHECK_LAUNCH();
@@ -435,7 +442,8 @@ static int psi_finalize(tdscha_ctx *c, const T *gpart, int nsplit, long sstride,
 
 int psi_finalize64(tdscha_ctx *c, const double *gpart, int nsplit, long sstride, long jstride,
                    long lda, const double *fpart, int nfchunk, cudaStream_t st) {
-    return psi_finalize<double>(c, gpart, nsplit, sstride, jstride, lda, fpart, nfchunk, st);
+    TDS_TRY(psi_hsum64(c, gpart, nsplit, sstride, jstride, lda, fpart, nfchunk, 0, c->J, st));
+    return psi_reduce64(c, st);
 }
 
 int psi_finalize32(tdscha_ctx *c, const float *gpart, int nsplit, long sstride, long jstride,
