@@ -17,10 +17,17 @@
 // Digits: 7 of the resident operand (55 bits under the largest element of its
 // row), 8 of the operand made per call (62 bits), products of order 0..7 (35 of
 // 56).  What is left out is below 2^-64 of the product of the two row maxima;
-// the float64 sums this replaces round every partial sum at 2^-53.  An
-// accumulation covers three K blocks (192 elements): 5 * 192 products of
-// 2^14 stay below 2^24, which keeps orders 0..4 exact for any input; orders
-// 5..7 could only round if every digit were at its limit, at 2^-64 of the sum.
+// the float64 sums this replaces round every partial sum at 2^-53.
+//
+// Length of an accumulation: three K blocks (192 elements) keep orders 0..4 exact
+// for any input (5 * 192 products of 2^14 stay below 2^24).  The digits of real
+// numbers are far from their limits, so the longest accumulation is chosen per
+// ensemble by a bound that holds for every perturbation: by Cauchy and Schwarz the
+// order-o sum is at most sum_i |d_i| 128 sqrt(K) with |d_i| the largest 2-norm of
+// digit i over K elements of any row, measured when the context is made
+// (digits_flush).  Gaussian displacements allow five to seven blocks.  Orders 5..7
+// could round, by 2^-53 of the row maxima's product or less, only where the
+// digits of two rows agree in sign and size over a whole accumulation.
 //
 // Error (2-norm, against 113-bit arithmetic) of f and d2v, these kernels | those
 // of perturb_fp64.cu: M=573 N=2000 6.9e-16 7.0e-16 | 1.3e-15 1.2e-15; with Y1 over
@@ -60,7 +67,9 @@ constexpr int kGK = 64;         // K block: one 128-byte swizzle row of fp16
 constexpr int kRes = 7;         // digits of the resident operand
 constexpr int kCall = 8;        // digits of the operand made per call
 constexpr int kOrders = 8;      // orders kept: 8 x 64 accumulator columns fill the TMEM
-constexpr int kFlush = 3;       // K blocks per exact accumulation
+constexpr int kFlushMin = 3;    // K blocks per accumulation, exact for any input
+constexpr int kFlushMax = 9;
+constexpr int kFlushes = kFlushMax - kFlushMin + 1;
 constexpr int kUnit = -69;      // one unit of the order-7 accumulator: 2^(-7-6-56)
 constexpr int kBadExp = 1 << 20;   // exponent of a row with a non-finite element
 constexpr uint32_t kGA = kGM * kGK * 2;   // bytes of one digit of an A block
@@ -137,32 +146,32 @@ __device__ __forceinline__ uint32_t sw_place(int row, int c) {
     return (uint32_t)row * 128u + (uint32_t)((c ^ (row & 7)) << 4);
 }
 
-// (hi 2^32 + lo) 2^e rounded to float64, |hi| < 2^62.  Whole-number operations:
-// a conversion of a 64-bit integer occupies the float64 pipe.
+// (hi 2^32 + lo) 2^e as float64, |hi| < 2^62, rounded to nearest to within 2^-60
+// of itself or one unit of lo.  About 25 whole-number operations: a conversion of
+// a 64-bit integer, like every float64 operation, runs at two per cycle per SM.
 __device__ __forceinline__ double fixed_to_double(long long hi, long long lo, int e) {
-    const long long h = hi + (lo >> 32);      // floor: what remains is in [0, 2^32)
-    const uint32_t l = (uint32_t)lo;
-    const bool neg = h < 0;
-    unsigned long long mh = neg ? ~(unsigned long long)h + (l == 0u) : (unsigned long long)h;
-    const uint32_t ml = neg ? 0u - l : l;
-    // the leading 64 bits of the magnitude
-    int z;
-    unsigned long long top;
-    if (mh) {
-        z = __clzll((long long)mh);
-        top = (mh << z) | (((unsigned long long)ml << 32) >> (64 - z));     // z >= 1
-    } else {
-        if (ml == 0u) return e >= kBadExp / 2 ? __longlong_as_double(0x7ff8000000000000LL) : 0.0;
-        z = 64 + __clz((int)ml);
-        top = (unsigned long long)ml << (z - 32);
+    const long long h = hi + (lo >> 32);      // what remains of lo is in [0, 2^32)
+    const uint32_t sgn = (uint32_t)(h >> 63);
+    // magnitude, three words (of a negative number one unit too small)
+    const uint32_t w2 = (uint32_t)((unsigned long long)h >> 32) ^ sgn, w1 = (uint32_t)h ^ sgn,
+                   w0 = (uint32_t)lo ^ sgn;
+    const bool k0 = w2 != 0u, k1 = w1 != 0u;
+    const uint32_t a = k0 ? w2 : k1 ? w1 : w0, b = k0 ? w1 : k1 ? w0 : 0u, c = k0 ? w0 : 0u;
+    const int z = __clz((int)a);
+    // the leading 64 bits, then 53 of them
+    const uint32_t th = __funnelshift_l(b, a, z), tl = __funnelshift_l(c, b, z);
+    const uint64_t m = (((uint64_t)th << 32 | tl) >> 11) + ((tl >> 10) & 1u);
+    // one less than the exponent field: the leading bit of m adds one
+    const int E = 1074 + 43 + e - z - (k0 ? 0 : k1 ? 32 : 64);
+    uint64_t bits = ((uint64_t)(uint32_t)E << 52) + m;
+    if (a == 0u || (uint32_t)E >= 2046u) {
+        bits = 0u;
+        if (e >= kBadExp / 2)
+            bits = 0x7ff8000000000000ULL;
+        else if (a != 0u && E >= 2046)
+            bits = 0x7ff0000000000000ULL;
     }
-    const unsigned long long m = (top >> 11) + ((top >> 10) & 1ULL);   // 2^52 <= m <= 2^53
-    const int E = 1074 + 43 - z + e;          // one less than the exponent field: m adds one
-    if (E >= 2046) return __longlong_as_double(e >= kBadExp / 2 ? 0x7ff8000000000000LL
-                                               : neg ? 0xfff0000000000000ULL : 0x7ff0000000000000LL);
-    if (E < 0) return 0.0;
-    const unsigned long long bits = ((unsigned long long)E << 52) + m;
-    return __longlong_as_double((long long)(bits | (neg ? 1ULL << 63 : 0ULL)));
+    return __longlong_as_double((long long)(bits | ((uint64_t)(sgn & 0x80000000u) << 32)));
 }
 
 // 2^e for the exponents of finite float64 rows
@@ -249,11 +258,54 @@ __global__ void k_dg_rowexp(const double *__restrict__ dt, const int *__restrict
     }
 }
 
+// Sums of the squares of each digit over the 64 elements of a block's row, from
+// the eight lanes that hold it: nrm[digit * rows + row].
+__device__ __forceinline__ void digit_norms(const uint4 (&w)[kRes], int c, float *__restrict__ nrm,
+                                            int rows, int row) {
+#pragma unroll
+    for (int d = 0; d < kRes; ++d) {
+        const uint32_t v[4] = {w[d].x, w[d].y, w[d].z, w[d].w};
+        float s = 0.f;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&v[k]));
+            s = fmaf(f.x, f.x, fmaf(f.y, f.y, s));
+        }
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (c == 0) nrm[d * rows + row] = s;
+    }
+}
+
+// out[L - 3][digit]: largest norm (squared) over the accumulations of L = 3 +
+// blockIdx.y blocks of any row; nrm[tile][block][digit][rows], thread = row.
+__global__ void k_dg_windows(const float *__restrict__ nrm, int nkb, float *__restrict__ out) {
+    const float *p = nrm + blockIdx.x * (long)nkb * kRes * blockDim.x + threadIdx.x;
+    const int L = kFlushMin + blockIdx.y;
+    float mx[kRes] = {};
+    for (int kb = 0; kb < nkb; kb += L) {
+        float s[kRes] = {};
+        for (int k = kb; k < min(nkb, kb + L); ++k)
+#pragma unroll
+            for (int d = 0; d < kRes; ++d) s[d] += p[((long)k * kRes + d) * blockDim.x];
+#pragma unroll
+        for (int d = 0; d < kRes; ++d) mx[d] = fmaxf(mx[d], s[d]);
+    }
+#pragma unroll
+    for (int d = 0; d < kRes; ++d) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) mx[d] = fmaxf(mx[d], __shfl_xor_sync(0xffffffffu, mx[d], o));
+        // non-negative floats order like their bit patterns
+        if ((threadIdx.x & 31) == 0)
+            atomicMax(reinterpret_cast<int *>(out + blockIdx.y * kRes + d), __float_as_int(mx[d]));
+    }
+}
+
 // xa: thread = (row, eight modes); xb: thread = (mode, eight rows)
 __global__ void __launch_bounds__(256) k_dg_xa(const double *__restrict__ D,
                                                const int *__restrict__ ec,
                                                const int *__restrict__ er, long R, int M, int nkb,
-                                               __half *__restrict__ xa) {
+                                               __half *__restrict__ xa, float *__restrict__ nrm) {
     const long rt = blockIdx.x;
     const int kb = blockIdx.y, c = threadIdx.x & 7;
     uint8_t *out = reinterpret_cast<uint8_t *>(xa) + (rt * nkb + kb) * (long)kRes * kGA;
@@ -271,12 +323,13 @@ __global__ void __launch_bounds__(256) k_dg_xa(const double *__restrict__ D,
 #pragma unroll
         for (int d = 0; d < kRes; ++d)
             *reinterpret_cast<uint4 *>(out + d * kGA + sw_place(row, c)) = w[d];
+        digit_norms(w, c, nrm + (rt * nkb + kb) * kRes * kGM, kGM, row);
     }
 }
 
 __global__ void __launch_bounds__(256) k_dg_xb(const double *__restrict__ dt,
                                                const int *__restrict__ ec, int Mp, long nkb,
-                                               __half *__restrict__ xb) {
+                                               __half *__restrict__ xb, float *__restrict__ nrm) {
     const long kb = blockIdx.x;
     const int at = blockIdx.y, c = threadIdx.x & 7;
     uint8_t *out = reinterpret_cast<uint8_t *>(xb) + (at * nkb + kb) * kRes * (long)kGB;
@@ -292,6 +345,7 @@ __global__ void __launch_bounds__(256) k_dg_xb(const double *__restrict__ dt,
 #pragma unroll
         for (int d = 0; d < kRes; ++d)
             *reinterpret_cast<uint4 *>(out + d * kGB + sw_place(row, c)) = w[d];
+        digit_norms(w, c, nrm + (at * nkb + kb) * kRes * kGN, kGN, row);
     }
 }
 
@@ -468,7 +522,7 @@ __global__ void __launch_bounds__(256) k_dg_wbuild(
 }
 
 // -------------------------------------------------------- the contraction
-// Persistent, one CTA per SM, 320 threads, one 128 x 64 output tile at a time;
+// Persistent, one CTA per SM, 512 threads, one 128 x 64 output tile at a time;
 // its accumulators, eight orders of 64 columns, fill the TMEM.
 //   warp 8  copies: B blocks (all digits of 64 rows) into two buffers, A digits
 //           (128 rows each) into a ring
@@ -476,6 +530,7 @@ __global__ void __launch_bounds__(256) k_dg_wbuild(
 //           lie behind one another in shared memory as their accumulators do in
 //           TMEM, so one instruction covers up to four orders (N = 256).  i
 //           runs downwards: the light high orders come first.
+//   warps 12-15  (stage A) s and t
 //   warps 0-7  every three K blocks the accumulators are read, order 7 first,
 //           and added to two 64-bit integers an element (warp w: lanes 32 (w % 4),
 //           columns 32 (w / 4) of every order).  Each order has its own
@@ -487,6 +542,7 @@ struct DgArgs {
     const __half *a, *b;
     int nkb;               // K blocks of an operand row
     int kbps;              // K blocks per work item (stage A: nkb)
+    int flush;             // K blocks per accumulation
     int nat, nbt;          // A and B tiles
     long nitems;
     int Mp;
@@ -499,12 +555,16 @@ struct DgArgs {
     long R;
     int nct;               // column tiles of one image
     // stage B
-    const double *fY;
     const int *ec, *ew;
-    double *gpart;         // [split][A rows][Mp]
-    int M;
+    double *gpart;         // [split][A rows][Mp]: H[b][a]
+    int M;                 // both stages
     long rows_b;           // rows (image, mode) in use
 };
+
+// 512 threads of 128 registers; the epilogue's two warpgroups take 192 of each
+// thread, the other two 64: 256 * 192 + 256 * 64 = 512 * 128.
+constexpr int kGThreads = 512, kGRegsEpi = 192, kGRegsRest = 64;
+static_assert(256 * kGRegsEpi + 256 * kGRegsRest == kGThreads * 128, "register shares");
 
 template <bool kStageA>
 struct DgShape {
@@ -513,8 +573,8 @@ struct DgShape {
     static constexpr uint32_t bbytes = SB * kGB;
     static constexpr int bars = 2 * slots + 4 + 1 + kOrders + 1;
     static constexpr size_t ring = 2 * (size_t)bbytes + slots * (size_t)kGA;
-    static constexpr size_t smem = 1024 + ring + 2 * 4 * 128 * sizeof(double) +
-                                   2 * kGN * (2 * sizeof(double) + sizeof(int)) + 8 * bars + 16;
+    static constexpr size_t smem = 1024 + ring + 2 * 2 * 128 * sizeof(double) +
+                                   2 * kGN * sizeof(int) + 8 * bars + 16;
 };
 static_assert(DgShape<true>::smem <= 232448 && DgShape<false>::smem <= 232448,
               "shared memory above the per-block limit");
@@ -534,16 +594,15 @@ __device__ __forceinline__ bool dg_sync_or(bool pred) {
 }
 
 template <bool kStageA>
-__global__ void __launch_bounds__(320, 1) k_dg_gemm(const DgArgs args) {
+__global__ void __launch_bounds__(kGThreads, 1) k_dg_gemm(const DgArgs args) {
     using Sh = DgShape<kStageA>;
     constexpr int SA = Sh::SA, SB = Sh::SB, slots = Sh::slots;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>(
         (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t *ring = smem + 2 * Sh::bbytes;
-    double *red = reinterpret_cast<double *>(smem + Sh::ring);        // [2][4][128]
-    double *colv = red + 2 * 4 * 128;                                  // [2][2][64]
-    int *cole = reinterpret_cast<int *>(colv + 2 * 2 * kGN);           // [2][64]
+    double *red = reinterpret_cast<double *>(smem + Sh::ring);        // [2][2][128]
+    int *cole = reinterpret_cast<int *>(red + 2 * 2 * 128);            // [2][64]
     uint64_t *bars = reinterpret_cast<uint64_t *>(cole + 2 * kGN);
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + Sh::bars);
     volatile int *abort = reinterpret_cast<volatile int *>(tmem_slot + 1);
@@ -552,9 +611,6 @@ __global__ void __launch_bounds__(320, 1) k_dg_gemm(const DgArgs args) {
                    done = tempty + 8 * kOrders;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long long budget = args.budget;
-    const long G = gridDim.x;
-    const long nloc = args.nitems > (long)blockIdx.x ? (args.nitems - 1 - blockIdx.x) / G + 1 : 0;
-    const int tiles = args.nat * args.nbt;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < slots; ++s) {
@@ -580,50 +636,86 @@ __global__ void __launch_bounds__(320, 1) k_dg_gemm(const DgArgs args) {
     pdl_enter();
     int fail_code = 0;
 
-    // work item i of this CTA: neighbouring CTAs take neighbouring B tiles of
-    // one A tile (stage A) or of one split (stage B) and share it in L2
-    auto item = [&](long i, int &at, int &bt, int &kb0, int &nkb) {
-        const long w = blockIdx.x + i * G;
-        const int split = (int)(w / tiles), tile = (int)(w % tiles);
-        at = tile / args.nbt;
-        bt = tile % args.nbt;
-        kb0 = split * args.kbps;
-        nkb = min(args.kbps, args.nkb - kb0);
+    // Work items blockIdx.x, blockIdx.x + gridDim.x, ...: neighbouring CTAs take
+    // neighbouring B tiles of one A tile (stage A) or of one split (stage B) and
+    // share it in L2.  Stepped, not divided: 64-bit divisions between two blocks
+    // held the issue thread up for longer than its MMAs run.
+    struct Item {
+        int at, bt, split, left;
+        int step_at, step_bt, step_split, nat, nbt;
+        __device__ Item(const DgArgs &a) {
+            const int w = (int)blockIdx.x, g = (int)gridDim.x;
+            nat = a.nat;
+            nbt = a.nbt;
+            bt = w % nbt;
+            at = w / nbt % nat;
+            split = w / nbt / nat;
+            step_bt = g % nbt;
+            step_at = g / nbt % nat;
+            step_split = g / nbt / nat;
+            left = a.nitems > w ? (int)((a.nitems - 1 - w) / g) + 1 : 0;
+        }
+        __device__ void next() {
+            bt += step_bt;
+            at += step_at;
+            split += step_split;
+            if (bt >= nbt) {
+                bt -= nbt;
+                ++at;
+            }
+            if (at >= nat) {
+                at -= nat;
+                ++split;
+            }
+            --left;
+        }
+    };
+    // a ring's slot and the parity of its use
+    struct Cursor {
+        int s = 0;
+        uint32_t ph = 0;
+        __device__ void next(int n) {
+            if (++s == n) {
+                s = 0;
+                ph ^= 1;
+            }
+        }
     };
 
+    if (warp >= 8) {
+    regs_dec<kGRegsRest>();
     if (warp == 8) {
         if (lane == 0) {
-            long ga = 0, gb = 0;
-            for (long i = 0; i < nloc && !fail_code; ++i) {
-                int at, bt, kb0, nkb;
-                item(i, at, bt, kb0, nkb);
+            Cursor ca, cb;
+            long ga = 0, gb = 0;             // copies issued
+            for (Item w(args); w.left > 0 && !fail_code; w.next()) {
+                const int kb0 = w.split * args.kbps, nkb = min(args.kbps, args.nkb - kb0);
                 const uint8_t *pa = reinterpret_cast<const uint8_t *>(args.a) +
-                                    ((long)at * args.nkb + kb0) * SA * (long)kGA;
+                                    ((long)w.at * args.nkb + kb0) * SA * (long)kGA;
                 const uint8_t *pb = reinterpret_cast<const uint8_t *>(args.b) +
-                                    ((long)bt * args.nkb + kb0) * SB * (long)kGB;
+                                    ((long)w.bt * args.nkb + kb0) * SB * (long)kGB;
                 for (int kb = 0; kb < nkb && !fail_code; ++kb) {
-                    const int sb = (int)(gb & 1);
-                    if (gb >= 2 && !mbar_wait_ab(bempty + 8 * sb, ((uint32_t)(gb >> 1) & 1) ^ 1,
-                                                 budget, abort)) {
+                    if (gb >= 2 && !mbar_wait_ab(bempty + 8 * cb.s, cb.ph ^ 1, budget, abort)) {
                         fail_code = 1;
                         break;
                     }
-                    mbar_expect_tx(bfull + 8 * sb, Sh::bbytes);
+                    mbar_expect_tx(bfull + 8 * cb.s, Sh::bbytes);
 #pragma unroll
                     for (int d = 0; d < SB; ++d)
-                        bulk_load(smem_u32(smem + sb * Sh::bbytes + d * kGB), pb + d * kGB, kGB,
-                                  bfull + 8 * sb);
+                        bulk_load(smem_u32(smem + cb.s * Sh::bbytes + d * kGB), pb + d * kGB, kGB,
+                                  bfull + 8 * cb.s);
                     pb += SB * (long)kGB;
+                    cb.next(2);
                     ++gb;
                     for (int d = SA - 1; d >= 0; --d, ++ga) {
-                        const int s = (int)(ga % slots);
-                        const uint32_t n = (uint32_t)(ga / slots);
-                        if (ga >= slots && !mbar_wait_ab(aempty + 8 * s, (n & 1) ^ 1, budget, abort)) {
+                        if (ga >= slots && !mbar_wait_ab(aempty + 8 * ca.s, ca.ph ^ 1, budget, abort)) {
                             fail_code = 1;
                             break;
                         }
-                        mbar_expect_tx(afull + 8 * s, kGA);
-                        bulk_load(smem_u32(ring + s * kGA), pa + d * (long)kGA, kGA, afull + 8 * s);
+                        mbar_expect_tx(afull + 8 * ca.s, kGA);
+                        bulk_load(smem_u32(ring + ca.s * kGA), pa + d * (long)kGA, kGA,
+                                  afull + 8 * ca.s);
+                        ca.next(slots);
                     }
                     pa += SA * (long)kGA;
                 }
@@ -638,154 +730,230 @@ __global__ void __launch_bounds__(320, 1) k_dg_gemm(const DgArgs args) {
             }
         }
     } else if (warp == 9) {
-        if (lane == 0) {
-            long ga = 0, gb = 0, nch = 0;    // A digits, B blocks, accumulations so far
-            for (long i = 0; i < nloc && !fail_code; ++i) {
-                int at, bt, kb0, nkb;
-                item(i, at, bt, kb0, nkb);
-                for (int kb = 0; kb < nkb && !fail_code; ++kb, ++gb) {
-                    const bool first = kb % kFlush == 0;
-                    const int sb = (int)(gb & 1);
-                    if (!mbar_wait_ab(bfull + 8 * sb, (uint32_t)(gb >> 1) & 1, budget, abort)) {
+        {
+            // the whole warp runs the loop, one lane issues
+            const uint32_t one = elect_one();
+            Cursor ca, cb;
+            uint32_t nch = 0;                // accumulations so far
+            bool ready = false;              // the next A digit was seen to have landed
+            for (Item w(args); w.left > 0 && !fail_code; w.next()) {
+                const int kb0 = w.split * args.kbps, nkb = min(args.kbps, args.nkb - kb0);
+                int in = 0;                  // K blocks in this accumulation
+                for (int kb = 0; kb < nkb && !fail_code; ++kb) {
+                    const bool first = in == 0;
+                    const int sb = cb.s;
+                    if (!__all_sync(0xffffffffu, mbar_wait_ab(bfull + 8 * sb, cb.ph, budget, abort))) {
                         fail_code = 2;
                         break;
                     }
-                    const uint32_t bbase = smem_u32(smem + sb * Sh::bbytes);
+                    cb.next(2);
+                    const uint64_t db0 = sdesc_sw128(smem_u32(smem + sb * Sh::bbytes));
 #pragma unroll
                     for (int d = SA - 1; d >= 0; --d) {
                         constexpr int kTop = SA - 1;
-                        const int cnt = SB < kOrders - d ? SB : kOrders - d;   // orders d .. d + cnt - 1
-                        const int s = (int)(ga % slots);
-                        bool ok = mbar_wait_ab(afull + 8 * s, (uint32_t)(ga / slots) & 1, budget, abort);
+                        const int cnt = min(SB, kOrders - d);       // orders d .. d + cnt - 1
+                        const int s = ca.s;
+                        bool ok = ready || __all_sync(0xffffffffu, mbar_wait_ab(afull + 8 * s, ca.ph, budget, abort));
                         if (first && nch > 0) {
                             // the orders that this digit writes first: d, and at the
                             // top digit all of its orders
-                            const uint32_t par = (uint32_t)(nch - 1) & 1;
+                            const uint32_t par = (nch - 1) & 1;
                             for (int o = d; o < (d == kTop ? d + cnt : d + 1); ++o)
-                                ok = ok && mbar_wait_ab(tempty + 8 * o, par, budget, abort);
+                                ok = __all_sync(0xffffffffu, mbar_wait_ab(tempty + 8 * o, par, budget, abort)) && ok;
                         }
                         if (!ok) {
                             fail_code = 2;
                             break;
                         }
+                        ca.next(slots);
+                        // the next digit's barrier is read while this digit's MMAs
+                        // go out (a wait between two digits idled the tensor core
+                        // for about 100 cycles)
+                        ready = __all_sync(0xffffffffu, mbar_test(afull + 8 * ca.s, ca.ph));
                         tc_fence_after();
-                        const uint32_t abase = smem_u32(ring + s * kGA);
+                        const uint64_t da0 = sdesc_sw128(smem_u32(ring + s * kGA));
+                        const uint32_t col = tmem + kGN * d;
+                        // at most four orders (N = 256) an instruction
+                        const int n1 = cnt > 4 ? (cnt + 1) / 2 : cnt;
 #pragma unroll
                         for (int kk = 0; kk < kGK / 16; ++kk) {
-                            const uint64_t da = sdesc_sw128(abase + kk * 32);
-                            const uint32_t col = tmem + kGN * d;
+                            // descriptor addresses count 16 bytes; the digits of B
+                            // lie kGB apart
                             auto span = [&](int j0, int n, uint32_t acc) {
-                                mma_f16(col + kGN * j0, da, sdesc_sw128(bbase + j0 * kGB + kk * 32),
-                                        idesc_f16(kGM, kGN * n), acc);
+                                mma_f16_one(one, col + kGN * j0, da0 + 2 * kk,
+                                        db0 + j0 * (kGB / 16) + 2 * kk, idesc_f16(kGM, kGN * n), acc);
                             };
-                            const int n1 = cnt > 4 ? (cnt + 1) / 2 : cnt;
-                            if (first && kk == 0 && d < kTop) {
-                                // order d starts here, the higher ones go on
-                                span(0, 1, 0u);
-                                if (cnt > 5) {
-                                    span(1, 4, 1u);
-                                    span(5, cnt - 5, 1u);
-                                } else if (cnt > 1) {
-                                    span(1, cnt - 1, 1u);
+                            if (kk == 0 && first) {
+                                // order d starts here, the higher ones go on; at the
+                                // top digit (at most two orders) all of them start
+                                if (d == kTop) {
+                                    span(0, cnt, 0u);
+                                } else {
+                                    span(0, 1, 0u);
+                                    span(1, min(4, cnt - 1), 1u);
+                                    if (cnt > 5) span(5, cnt - 5, 1u);
                                 }
                             } else {
-                                const uint32_t acc = (kk == 0 && first) ? 0u : 1u;
-                                span(0, n1, acc);
-                                if (cnt > n1) span(n1, cnt - n1, acc);
+                                span(0, n1, 1u);
+                                if (cnt > n1) span(n1, cnt - n1, 1u);
                             }
                         }
-                        mma_commit(aempty + 8 * s);
-                        ++ga;
+                        mma_commit_one(one, aempty + 8 * s);
                     }
                     if (fail_code) break;
-                    mma_commit(bempty + 8 * sb);
-                    if (kb % kFlush == kFlush - 1 || kb == nkb - 1) {
-                        mma_commit(tfull);
+                    mma_commit_one(one, bempty + 8 * sb);
+                    if (++in == args.flush || kb == nkb - 1) {
+                        mma_commit_one(one, tfull);
                         ++nch;
+                        in = 0;
                     }
                 }
             }
             if (fail_code) *abort = 1;
-            mma_commit(done);
+            mma_commit_one(one, done);
         }
+    } else if (warp >= 12) {
+        if (kStageA) {
+            // thread = row: its partial s and t over the tile's 64 modes, beside
+            // the matrix work (in the epilogue these two products an element kept
+            // the float64 pipe for longer than the tile's MMAs run)
+            const int row = (warp - 12) * 32 + lane;
+            for (Item w(args); w.left > 0; w.next()) {
+                const int at = w.at, bt = w.bt;
+                const long tile = ((long)at * args.Mp + (long)(bt % args.nct) * kGN) * 128 + row;
+                const double *pd = args.dt + tile, *pg = args.gt + tile;
+                const double *vs = args.vs + (long)bt * kGN, *vt = args.vt + (long)bt * kGN;
+                double s = 0, t = 0;
+#pragma unroll 1
+                for (int c = 0; c < kGN; c += 8) {
+                    double d[8], g[8];
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        d[e] = pd[(c + e) * 128];
+                        g[e] = pg[(c + e) * 128];
+                    }
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        s = fma(vs[c + e], d[e], s);
+                        t = fma(vt[c + e], g[e], t);
+                    }
+                }
+                const long r = (long)at * kGM + row;
+                if (r < args.R) {
+                    double *o = args.qp + (long)bt * 4 * args.R + r;
+                    o[2 * args.R] = s;
+                    o[3 * args.R] = t;
+                }
+            }
+        }
+    }
     } else {
+        regs_inc<kGRegsEpi>();
         const int quad = warp & 3, half = warp >> 2;
         const int row = quad * 32 + lane;
         const uint32_t base = tmem + ((uint32_t)(quad * 32) << 16) + 32 * half;
-        long nch = 0;
-        for (long i = 0; i < nloc; ++i) {
-            int at, bt, kb0, nkb;
-            item(i, at, bt, kb0, nkb);
-            double *cv = colv + (i & 1) * 2 * kGN;
+        uint32_t nch = 0;
+        bool bad = false;            // a wait of this warp gave up
+        int i = 0;
+        for (Item w(args); w.left > 0; w.next(), ++i) {
+            const int at = w.at, bt = w.bt;
+            const int nkb = min(args.kbps, args.nkb - w.split * args.kbps);
             int *ce = cole + (i & 1) * kGN;
             if (threadIdx.x < kGN) {
                 const long c = (long)bt * kGN + threadIdx.x;
-                if (kStageA) {
-                    cv[threadIdx.x] = args.vs[c];
-                    cv[kGN + threadIdx.x] = args.vt[c];
-                    ce[threadIdx.x] = args.et[c] + kUnit;
-                } else {
-                    cv[threadIdx.x] = c < args.M ? args.fY[c] : 0.0;
-                    ce[threadIdx.x] = args.ec[c] + kUnit;
-                }
+                ce[threadIdx.x] = (kStageA ? args.et[c] : args.ec[c]) + kUnit;
             }
+            const int nacc = (nkb + args.flush - 1) / args.flush;
+            // An accumulator |a| <= 2^22 becomes a whole number by adding 1.5 2^23:
+            // the bits of the sum are kMagic + a.  Their weighted sums are taken
+            // modulo 2^64 from minus what the kMagic terms add up to.  (Conversions
+            // run at an eighth of this rate and took as long as an accumulation's
+            // read may take.)
+            constexpr uint32_t kMagic = 0x4B400000u;
             long long hi[32], lo[32];
+            const long long start = -(long long)nacc * (long long)((uint64_t)kMagic * 0x01010101u);
 #pragma unroll
-            for (int e = 0; e < 32; ++e) hi[e] = lo[e] = 0;
-            const int nacc = (nkb + kFlush - 1) / kFlush;
+            for (int e = 0; e < 32; ++e) hi[e] = lo[e] = start;
             for (int c = 0; c < nacc; ++c, ++nch) {
-                const bool ok = mbar_wait_ab(tfull, (uint32_t)nch & 1, budget, abort);
-                __syncwarp();
-                if (dg_sync_or(!ok)) {     // also publishes cv and ce
-                    fail_code = 3;
-                    break;
+                if (!bad && !__all_sync(0xffffffffu, mbar_wait_ab(tfull, nch & 1, budget, abort))) {
+                    bad = true;
+                    *abort = 1;
                 }
+                if (bad) continue;
                 tc_fence_after();
+                // Half an order (16 columns) at a time, the next half's read on its
+                // way while one is added.  Rolled: a small call runs this code once.
+                uint32_t v[2][16];
+                tmem_ld16(base + kGN * (kOrders - 1), v[0]);
+                auto add = [&](const uint32_t(&x)[16], uint32_t w, long long *acc) {
+                    uint32_t b[16], over = 0;
 #pragma unroll
-                for (int o = kOrders - 1; o >= 0; --o) {
-                    const int k = 8 * ((kOrders - 1 - o) & 3);
-#pragma unroll
-                    for (int e0 = 0; e0 < 32; e0 += 16) {
-                        uint32_t v[16];
-                        tmem_ld16(base + kGN * o + e0, v);
-                        tmem_wait_ld();
-                        if (e0) {
-                            tc_fence_before();
-                            __syncwarp();
-                            if (lane == 0) mbar_arrive(tempty + 8 * o);
-                        }
-#pragma unroll
-                        for (int e = 0; e < 16; ++e) {
-                            const long long t = (long long)__float2int_rn(__uint_as_float(v[e]));
-                            if (o >= 4)
-                                lo[e0 + e] += t * (1LL << k);
-                            else
-                                hi[e0 + e] += t * (1LL << k);
-                        }
+                    for (int e = 0; e < 16; ++e) {
+                        b[e] = __float_as_uint(__uint_as_float(x[e]) + 12582912.f);
+                        over |= b[e] ^ 0x4B000000u;
                     }
-                }
+                    if (__any_sync(0xffffffffu, over >> 23)) {
+#pragma unroll
+                        for (int e = 0; e < 16; ++e)
+                            b[e] = kMagic + (uint32_t)__float2int_rn(__uint_as_float(x[e]));
+                    }
+#pragma unroll
+                    for (int e = 0; e < 16; ++e) acc[e] += (long long)((uint64_t)b[e] * w);
+                };
+                auto order = [&](int o, uint32_t w, long long(&acc)[32]) {
+                    tmem_wait_ld();
+                    tmem_ld16(base + kGN * o + 16, v[1]);
+                    add(v[0], w, acc);
+                    tmem_wait_ld();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(tempty + 8 * o);
+                    if (o > 0) tmem_ld16(base + kGN * (o - 1), v[0]);
+                    add(v[1], w, acc + 16);
+                };
+#pragma unroll 1
+                for (int k = 0; k < 4; ++k) order(7 - k, 1u << (8 * k), lo);
+#pragma unroll 1
+                for (int k = 0; k < 4; ++k) order(3 - k, 1u << (8 * k), hi);
             }
-            if (fail_code) break;
+            // the other warps' column scales and failures
+            if (dg_sync_or(bad)) {
+                fail_code = 3;
+                break;
+            }
             const int c0 = half * 32;
             if (kStageA) {
                 const long tile = ((long)at * args.Mp + (long)(bt % args.nct) * kGN + c0) * 128 + row;
                 const double *pd = args.dt + tile, *pg = args.gt + tile;
-                double q = 0, p = 0, s = 0, t = 0;
+                // eight modes' x and g on the way while the eight before are used
+                double q = 0, p = 0, d[8], g[8];
 #pragma unroll
-                for (int e = 0; e < 32; ++e) {
-                    const double d = pd[e * 128], g = pg[e * 128];
-                    const double v = fixed_to_double(hi[e], lo[e], ce[c0 + e]);
-                    q = fma(d, v, q);
-                    p = fma(g, v, p);
-                    s = fma(cv[c0 + e], d, s);
-                    t = fma(cv[kGN + c0 + e], g, t);
+                for (int e = 0; e < 8; ++e) {
+                    d[e] = pd[e * 128];
+                    g[e] = pg[e * 128];
                 }
-                double *rb = red + (i & 1) * 4 * 128 + row;
+                const int ncol = args.M - (bt % args.nct) * kGN - c0;    // the rest is padding
+#pragma unroll
+                for (int e0 = 0; e0 < 32; e0 += 8) {
+                    if (e0 >= ncol) break;
+                    double v[8];
+#pragma unroll
+                    for (int e = 0; e < 8; ++e)
+                        v[e] = fixed_to_double(hi[e0 + e], lo[e0 + e], ce[c0 + e0 + e]);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        q = fma(d[e], v[e], q);
+                        p = fma(g[e], v[e], p);
+                        if (e0 < 24) {
+                            d[e] = pd[(e0 + 8 + e) * 128];
+                            g[e] = pg[(e0 + 8 + e) * 128];
+                        }
+                    }
+                }
+                double *rb = red + (i & 1) * 2 * 128 + row;
                 if (half) {
                     rb[0] = q;
                     rb[128] = p;
-                    rb[256] = s;
-                    rb[384] = t;
                 }
                 asm volatile("bar.sync 1, 256;" ::: "memory");
                 const long r = (long)at * kGM + row;
@@ -793,25 +961,22 @@ __global__ void __launch_bounds__(320, 1) k_dg_gemm(const DgArgs args) {
                     double *o = args.qp + (long)bt * 4 * args.R + r;
                     o[0] = q + rb[0];
                     o[args.R] = p + rb[128];
-                    o[2 * args.R] = s + rb[256];
-                    o[3 * args.R] = t + rb[384];
                 }
             } else {
                 const long grow = (long)at * kGM + row;
                 const int b = (int)(grow % args.Mp);
                 const bool live = grow < args.rows_b && b < args.M;
                 if (live) {
-                    const long w = blockIdx.x + i * G;
-                    const double fb = args.fY[b];
                     const int eb = args.ew[grow];
-                    double *o = args.gpart + ((w / tiles) * args.nat * kGM + grow) * args.Mp +
+                    double *o = args.gpart + ((long)w.split * args.nat * kGM + grow) * args.Mp +
                                 (long)bt * kGN + c0;
+                    const int ncol = args.M - bt * kGN - c0;
 #pragma unroll
                     for (int e = 0; e < 32; e += 2) {
+                        if (e >= ncol) break;
                         double2 x;
-                        x.x = fixed_to_double(hi[e], lo[e], ce[c0 + e] + eb) * (fb * cv[c0 + e]);
-                        x.y = fixed_to_double(hi[e + 1], lo[e + 1], ce[c0 + e + 1] + eb) *
-                              (fb * cv[c0 + e + 1]);
+                        x.x = fixed_to_double(hi[e], lo[e], ce[c0 + e] + eb);
+                        x.y = fixed_to_double(hi[e + 1], lo[e + 1], ce[c0 + e + 1] + eb);
                         *reinterpret_cast<double2 *>(o + e) = x;
                     }
                 }
@@ -845,13 +1010,14 @@ __device__ __forceinline__ double dg_split_sum(const double *__restrict__ p, int
     return acc;
 }
 
-// d2v = -(G + G^T) / norm and f = sum fpart / norm of the image blockIdx.y (no
+// d2v = -f_Y,a f_Y,b (H + H^T) / norm and f = sum fpart / norm of the image blockIdx.y (no
 // symmetry images): one block per 8-row slab of a pair (A, B), A <= B, of
 // 32 x 32 tiles, each element summed over the splits once.
 __global__ void __launch_bounds__(256) k_dg_final(const double *__restrict__ gpart, int nsplit,
                                                   long stride, int M, int Mp,
                                                   const double *__restrict__ fpart, int nfc,
-                                                  double norm, double *__restrict__ f,
+                                                  const double *__restrict__ fY, double norm,
+                                                  double *__restrict__ f,
                                                   double *__restrict__ d2v) {
     pdl_enter();
     gpart += blockIdx.y * (long)Mp * Mp;
@@ -877,7 +1043,8 @@ __global__ void __launch_bounds__(256) k_dg_final(const double *__restrict__ gpa
     {
         const int a = a0 + ty, b = b0 + tx;
         if (a < M && b < M) {
-            const double v = -(dg_split_sum(gpart + (long)a * Mp + b, nsplit, stride) + tr[tx][ty]) * inv;
+            const double h = dg_split_sum(gpart + (long)a * Mp + b, nsplit, stride) + tr[tx][ty];
+            const double v = -(h * fY[a]) * fY[b] * inv;
             d2v[(long)a * M + b] = v;
             if (A != B) d2v[(long)b * M + a] = v;
         }
@@ -902,6 +1069,7 @@ struct DigitStore {
     long Rp = 0, nkbR = 0;
     int cap = 1;                 // images that the per-call buffers hold
     int per = 1, nfc = 1;        // K blocks of one W block, force partials an image
+    int flushA = kFlushMin, flushB = kFlushMin;   // K blocks per accumulation of the stages
     void *slab = nullptr;
     double *dt = nullptr, *gt = nullptr, *vs = nullptr, *vt = nullptr, *qp = nullptr,
            *gpart = nullptr, *fpart = nullptr;
@@ -925,7 +1093,7 @@ static int dg_blocks_per_split(const DigitStore *x, int nat) {
     for (long n = 1; n <= std::min<long>(nkb, 96); ++n) {
         long kb = (nkb + n - 1) / n;
         // whole accumulations where a split has several
-        if (kb > kFlush) kb = (kb + kFlush - 1) / kFlush * kFlush;
+        if (kb > x->flushB) kb = (kb + x->flushB - 1) / x->flushB * x->flushB;
         const long ns = (nkb + kb - 1) / kb;
         if (kb > 16384) continue;             // 64-bit sums of the orders
         const double cost = (double)((tiles * ns + x->nsm - 1) / x->nsm) * (kb * 4900.0 + 8000.0) +
@@ -936,6 +1104,24 @@ static int dg_blocks_per_split(const DigitStore *x, int nat) {
         }
     }
     return kb_best;
+}
+
+// The longest accumulation (K blocks) that keeps orders 0..4 below 2^24 for any
+// per-call operand: mx[L - 3][i] is the largest squared norm of digit i over L
+// blocks.  The other operand's digits are at most 64 (the first) and 128.
+static int digits_flush(const float *mx) {
+    for (int L = kFlushMax; L > kFlushMin; --L) {
+        bool fits = true;
+        for (int o = 0; o <= 4 && fits; ++o) {
+            double sum = 0;
+            for (int i = 0; i <= o; ++i)
+                sum += std::sqrt((double)mx[(L - kFlushMin) * kRes + i] * kGK * L) *
+                       (i == o ? 64.0 : 128.0);
+            fits = sum <= 16777216.0;
+        }
+        if (fits) return L;
+    }
+    return kFlushMin;
 }
 
 void digits_release(tdscha_ctx *c) {
@@ -973,10 +1159,14 @@ int digits_prepare(tdscha_ctx *c) {
     x->per = (int)std::max<long>(1, std::min<long>(16, x->nkbR * nat / (152L * 8)));
     x->nfc = ceil_div(x->nkbR, x->per);
     size_t gbytes = 0;
-    for (int n = 1; n <= cap; ++n) {
-        const int na = ceil_div((long)n * Mp, kGM), kb = dg_blocks_per_split(x, na);
-        gbytes = std::max(gbytes, (size_t)ceil_div(x->nkbR, kb) * na * kGM * Mp * sizeof(double));
+    for (x->flushB = kFlushMax; ; --x->flushB) {      // ends at kFlushMin, its value until measured
+        for (int n = 1; n <= cap; ++n) {
+            const int na = ceil_div((long)n * Mp, kGM), kb = dg_blocks_per_split(x, na);
+            gbytes = std::max(gbytes, (size_t)ceil_div(x->nkbR, kb) * na * kGM * Mp * sizeof(double));
+        }
+        if (x->flushB == kFlushMin) break;
     }
+    float *fl = nullptr;         // largest digit norms of xa and of xb
     struct Part {
         void **p;
         size_t bytes;
@@ -1002,6 +1192,7 @@ int digits_prepare(tdscha_ctx *c) {
         {(void **)&x->vt, d * cap * Mp, true},
         {(void **)&x->et, i4 * cap * Mp, true},
         {(void **)&x->ew, i4 * (size_t)nat * kGM, true},
+        {(void **)&fl, sizeof(float) * 2 * kFlushes * kRes, true},
         {(void **)&x->yb, 2 * kCall * (size_t)cap * Mp * Mp, true},
         {(void **)&x->wa, 2 * kCall * (size_t)nat * kGM * x->Rp, true},
     };
@@ -1043,10 +1234,22 @@ int digits_prepare(tdscha_ctx *c) {
     TDS_CHECK_LAUNCH();
     k_dg_rowexp<<<(unsigned)nrt, dim3(128, 8)>>>(x->dt, x->ec, M, Mp, x->er);
     TDS_CHECK_LAUNCH();
-    k_dg_xa<<<dim3((unsigned)nrt, x->nkbM), 256>>>(c->D, x->ec, x->er, R, M, x->nkbM, x->xa);
+    // the digit norms pass through the W digits' space, which is zeroed again
+    float *nrm = reinterpret_cast<float *>(x->wa);
+    k_dg_xa<<<dim3((unsigned)nrt, x->nkbM), 256>>>(c->D, x->ec, x->er, R, M, x->nkbM, x->xa, nrm);
     TDS_CHECK_LAUNCH();
-    k_dg_xb<<<dim3((unsigned)x->nkbR, x->nct), 256>>>(x->dt, x->ec, Mp, x->nkbR, x->xb);
+    k_dg_windows<<<dim3((unsigned)nrt, kFlushes), kGM>>>(nrm, x->nkbM, fl);
     TDS_CHECK_LAUNCH();
+    k_dg_xb<<<dim3((unsigned)x->nkbR, x->nct), 256>>>(x->dt, x->ec, Mp, x->nkbR, x->xb, nrm);
+    TDS_CHECK_LAUNCH();
+    k_dg_windows<<<dim3(x->nct, kFlushes), kGN>>>(nrm, (int)x->nkbR, fl + kFlushes * kRes);
+    TDS_CHECK_LAUNCH();
+    TDS_CUDA(cudaMemsetAsync(nrm, 0, sizeof(float) * kRes * (elems / kGK), 0));
+    float h_fl[2 * kFlushes * kRes];
+    TDS_CUDA(cudaMemcpy(h_fl, fl, sizeof(h_fl), cudaMemcpyDeviceToHost));
+    x->flushA = digits_flush(h_fl);
+    x->flushB = digits_flush(h_fl + kFlushes * kRes);
+    if (const char *e = getenv("DBG_FLUSH")) printf("flush %d %d of %d %ld\n", x->flushA, x->flushB, x->nkbM, x->nkbR);
     TDS_CUDA(cudaFuncSetAttribute(k_dg_gemm<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)DgShape<true>::smem));
     TDS_CUDA(cudaFuncSetAttribute(k_dg_gemm<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1080,6 +1283,7 @@ static int digits_contract(tdscha_ctx *c, int nimg, const double *Y1, const doub
     ga.a = x->xa;
     ga.b = x->yb;
     ga.nkb = ga.kbps = x->nkbM;
+    ga.flush = x->flushA;
     ga.nat = (int)(x->Rp / kGM);
     ga.nbt = nimg * x->nct;
     ga.nitems = (long)ga.nat * ga.nbt;
@@ -1094,9 +1298,10 @@ static int digits_contract(tdscha_ctx *c, int nimg, const double *Y1, const doub
     ga.qp = x->qp;
     ga.R = R;
     ga.nct = x->nct;
+    ga.M = M;
     {
         ProfScope ps(c, 0, st);
-        TDS_CUDA(launch_pdl(k_dg_gemm<true>, (int)std::min<long>(ga.nitems, x->nsm), 320,
+        TDS_CUDA(launch_pdl(k_dg_gemm<true>, (int)std::min<long>(ga.nitems, x->nsm), kGThreads,
                             DgShape<true>::smem, st, ga));
     }
     {
@@ -1121,6 +1326,7 @@ static int digits_contract(tdscha_ctx *c, int nimg, const double *Y1, const doub
     gb.b = x->xb;
     gb.nkb = (int)x->nkbR;
     gb.kbps = dg_blocks_per_split(x, nat);
+    gb.flush = x->flushB;
     gb.nat = nat;
     gb.nbt = x->nct;
     *nsplit = ceil_div(x->nkbR, gb.kbps);
@@ -1128,14 +1334,13 @@ static int digits_contract(tdscha_ctx *c, int nimg, const double *Y1, const doub
     gb.Mp = Mp;
     gb.err = x->err;
     gb.budget = x->budget;
-    gb.fY = c->fY;
     gb.ec = x->ec;
     gb.ew = x->ew;
     gb.gpart = x->gpart;
     gb.M = M;
     gb.rows_b = (long)nimg * Mp;
     ProfScope ps(c, 3, st);
-    TDS_CUDA(launch_pdl(k_dg_gemm<false>, (int)std::min<long>(gb.nitems, x->nsm), 320,
+    TDS_CUDA(launch_pdl(k_dg_gemm<false>, (int)std::min<long>(gb.nitems, x->nsm), kGThreads,
                         DgShape<false>::smem, st, gb));
     return TDSCHA_OK;
 }
@@ -1151,7 +1356,8 @@ int perturb_digits(tdscha_ctx *c, int apply_d4, cudaStream_t st) {
         const int nt = ceil_div(M, 32), nat = ceil_div((long)Mp, kGM);
         TDS_CUDA(launch_pdl(k_dg_final, dim3(4 * (nt * (nt + 1) / 2), 1), 256, 0, st,
                             (const double *)x->gpart, ns, (long)nat * kGM * Mp, M, Mp,
-                            (const double *)x->fpart, x->nfc, c->sum_rho * c->S, c->f, c->d2v));
+                            (const double *)x->fpart, x->nfc, (const double *)c->fY,
+                            c->sum_rho * c->S, c->f, c->d2v));
         return TDSCHA_OK;
     }
     TDS_TRY(psi_perturbation64(c, st));
@@ -1161,7 +1367,7 @@ int perturb_digits(tdscha_ctx *c, int apply_d4, cudaStream_t st) {
                                 c->vsv + (size_t)(J + j0) * M, 0, apply_d4, &ns, st));
         const int nat = ceil_div((long)nj * Mp, kGM);
         TDS_TRY(psi_hsum64(c, x->gpart, ns, (long)nat * kGM * Mp, (long)Mp * Mp, Mp, x->fpart,
-                           x->nfc, j0, nj, st));
+                           x->nfc, c->fY, j0, nj, st));
     }
     return psi_reduce64(c, st);
 }

@@ -95,11 +95,11 @@ __device__ __forceinline__ double split_sum(const T *__restrict__ p, int n, long
 // into shared memory, and both halves of the symmetric result written along
 // rows.  Blocks of the first tile pair row also form
 // fs[j][m] = sum_ch fpart[(j*nfc + ch)*M + m] for their columns.
-template <typename T>
-__global__ void __launch_bounds__(256) k_psi_hsum(const T *__restrict__ g, int nsplit, long ss,
-                                                  long js, long lda, const T *__restrict__ fpart,
-                                                  int nfc, int M, double *__restrict__ hs,
-                                                  double *__restrict__ fs) {
+__global__ void __launch_bounds__(256) k_psi_hsum(const double *__restrict__ g, int nsplit, long ss,
+                                                  long js, long lda,
+                                                  const double *__restrict__ fpart, int nfc,
+                                                  const double *__restrict__ fY, int M,
+                                                  double *__restrict__ hs, double *__restrict__ fs) {
     __shared__ double t1[32][33], t2[32][33];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;    // 32 x 8
     const int nt = (M + 31) / 32;
@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(256) k_psi_hsum(const T *__restrict__ g, int n
     const int L = K + rem;
     const int k0 = K * 32, l0 = L * 32;
     const long j = blockIdx.y;
-    const T *base = g + j * js;
+    const double *base = g + j * js;
     for (int r = ty; r < 32; r += 8) {
         int k = k0 + r, l = l0 + tx;
         t1[r][tx] = (k < M && l < M) ? split_sum(base + (long)k * lda + l, nsplit, ss) : 0.0;
@@ -125,10 +125,16 @@ __global__ void __launch_bounds__(256) k_psi_hsum(const T *__restrict__ g, int n
     double *H = hs + j * (long)M * M;
     for (int r = ty; r < 32; r += 8) {
         int k = k0 + r, l = l0 + tx;        // rows of tile (K, L)
-        if (k < M && l < M) H[(long)k * M + l] = t1[r][tx] + m2[tx][r];
+        if (k < M && l < M) {
+            const double h = t1[r][tx] + m2[tx][r];
+            H[(long)k * M + l] = fY ? (h * fY[k]) * fY[l] : h;
+        }
         if (K != L) {
             int l2 = l0 + r, k2 = k0 + tx;  // rows of the mirror tile (L, K)
-            if (l2 < M && k2 < M) H[(long)l2 * M + k2] = t1[tx][r] + m2[r][tx];
+            if (l2 < M && k2 < M) {
+                const double h = t1[tx][r] + m2[r][tx];
+                H[(long)l2 * M + k2] = fY ? (h * fY[k2]) * fY[l2] : h;
+            }
         }
     }
     if (K == 0 && ty == 0) {
@@ -413,15 +419,16 @@ int psi_perturbation64(tdscha_ctx *c, cudaStream_t st) {
 }
 
 int psi_hsum64(tdscha_ctx *c, const double *gpart, int nsplit, long sstride, long jstride, long lda,
-               const double *fpart, int nfchunk, int j0, int nj, cudaStream_t st) {
+               const double *fpart, int nfchunk, const double *fY, int j0, int nj,
+               cudaStream_t st) {
     const int M = c->M, J = c->J;
     const size_t MM = (size_t)M * M;
     double *hs = c->hs, *fs = hs + 2 * J * MM;
     ProfScope ps(c, 4, st);
     const int nt = ceil_div(M, 32);
     dim3 gt(nt * (nt + 1) / 2, nj);
-    k_psi_hsum<double><<<gt, 256, 0, st>>>(gpart, nsplit, sstride, jstride, lda, fpart, nfchunk, M,
-                                           hs + j0 * MM, fs + (size_t)j0 * M);
+    k_psi_hsum<<<gt, 256, 0, st>>>(gpart, nsplit, sstride, jstride, lda, fpart, nfchunk, fY, M,
+                                   hs + j0 * MM, fs + (size_t)j0 * M);
     TDS_CHECK_LAUNCH();
     return TDSCHA_OK;
 }
@@ -442,7 +449,8 @@ int psi_reduce64(tdscha_ctx *c, cudaStream_t st) {
 
 int psi_finalize64(tdscha_ctx *c, const double *gpart, int nsplit, long sstride, long jstride,
                    long lda, const double *fpart, int nfchunk, cudaStream_t st) {
-    TDS_TRY(psi_hsum64(c, gpart, nsplit, sstride, jstride, lda, fpart, nfchunk, 0, c->J, st));
+    TDS_TRY(psi_hsum64(c, gpart, nsplit, sstride, jstride, lda, fpart, nfchunk, nullptr, 0,
+                       c->J, st));
     return psi_reduce64(c, st);
 }
 

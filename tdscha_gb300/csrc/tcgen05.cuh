@@ -36,6 +36,19 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
     return ok != 0;
 }
 
+// Whether the phase of the given parity is complete (does not suspend the thread).
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+
 // Wait for the phase of the given parity; false when the budget runs out.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, long long budget) {
     long long t0 = clock64();
@@ -93,6 +106,37 @@ __device__ __forceinline__ void mma_f16(uint32_t tmem, uint64_t a, uint64_t b, u
         : "memory");
 }
 
+// The same for a whole warp that runs the issue loop: the lane with `one` set
+// issues.  With the loop inside `if (lane == 0)` its operands pass from vector to
+// uniform registers before each instruction, which took about 140 cycles an MMA.
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t one;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(one));
+    return one;
+}
+__device__ __forceinline__ void mma_f16_one(uint32_t one, uint32_t tmem, uint64_t a, uint64_t b,
+                                            uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
+        "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(one)
+        : "memory");
+}
+__device__ __forceinline__ void mma_commit_one(uint32_t one, uint32_t bar) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "setp.ne.b32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar),
+        "r"(one)
+        : "memory");
+}
+
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
     asm volatile(
         "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
@@ -134,6 +178,17 @@ __device__ __forceinline__ void tmem_wait_ld() {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+// Registers a thread of the executing warps from here on (all warps of a
+// warpgroup execute it; the shares add up to what the block was launched with).
+template <int N>
+__device__ __forceinline__ void regs_inc() {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
+}
+template <int N>
+__device__ __forceinline__ void regs_dec() {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
+}
+
 template <int NCOLS>
 __device__ __forceinline__ void tmem_alloc(uint32_t slot) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot),
@@ -151,7 +206,10 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr) {
 // Bounded wait that also gives up once another role has raised `abort`.
 __device__ __forceinline__ bool mbar_wait_ab(uint32_t bar, uint32_t parity, long long budget,
                                              volatile int *abort) {
-    long long t0 = clock64();
+    // the clock only where there is something to wait for: reading it first cost
+    // the MMA issue thread 16 cycles a barrier
+    if (mbar_try(bar, parity)) return true;
+    const long long t0 = clock64();
     uint32_t spins = 0;
     while (!mbar_try(bar, parity)) {
         if ((++spins & 31u) == 0 && *abort) return false;
