@@ -33,8 +33,8 @@
 // of perturb_fp64.cu: M=573 N=2000 6.9e-16 7.0e-16 | 1.3e-15 1.2e-15; with Y1 over
 // six decades 7.9e-16 7.7e-16 | 1.4e-15 1.2e-15; M=192 N=3000 1.5e-15 1.5e-15 |
 // 1.7e-15 1.6e-15; M=24 N=400 48 images 1.3e-15 5.3e-16 | 3.1e-15 5.6e-16.
-// One call: M=573 N=50000 57.1 -> 2.55 ms; M=189 N=10000 48 images 62.8 -> 3.69 ms;
-// M=97 N=4999 554 -> 99 us; M=21 N=1000 245 -> 73 us.
+// One call: M=573 N=50000 57.1 -> 1.77 ms; M=189 N=10000 48 images 62.8 -> 2.68 ms;
+// M=97 N=4999 554 -> 86 us; M=21 N=1000 245 -> 61 us.
 //
 // Form of the contractions, with g = y / f_Y (= f_psi y) so that both operands
 // of the second stage come from x and g alone (u = f_Y x, y = f_Y g):
@@ -538,6 +538,15 @@ __global__ void __launch_bounds__(256) k_dg_wbuild(
 //           lower ones are still read.  At the end of a tile the sums become
 //           float64: row dots (stage A) or a partial tile (stage B).
 // Bounded waits and the abort flag as in perturb_mixed.cu.
+//
+// What it takes at M=573, N=50000 (1.95 GHz): stage A 700 us, stage B 774 us; the
+// 35 products alone are 0.93 and 1.04 million cycles an SM, 480 and 530 us.  The
+// same loop on one thread (`if (lane == 0)`) took 794 and 928 us, with 64-bit
+// divisions for the ring slots 1165 and 1098.  Reading an accumulation back takes
+// the epilogue 8000 cycles, of which 1200 stand before the next MMAs; a tile's end
+// 12000 (stage A: two float64 products an element on the float64 pipe).  With 48
+// images stage A (976 us at M=189, N=10000) is bound by that pipe and the epilogue.
+// The copies (176 KB a K block) take 3700 cycles of a block's 4500 and do not show.
 struct DgArgs {
     const __half *a, *b;
     int nkb;               // K blocks of an operand row
@@ -735,14 +744,15 @@ __global__ void __launch_bounds__(kGThreads, 1) k_dg_gemm(const DgArgs args) {
             const uint32_t one = elect_one();
             Cursor ca, cb;
             uint32_t nch = 0;                // accumulations so far
-            bool ready = false;              // the next A digit was seen to have landed
+            // the next A digit, the next B block were seen to have landed
+            bool ready = false, readyb = false;
             for (Item w(args); w.left > 0 && !fail_code; w.next()) {
                 const int kb0 = w.split * args.kbps, nkb = min(args.kbps, args.nkb - kb0);
                 int in = 0;                  // K blocks in this accumulation
                 for (int kb = 0; kb < nkb && !fail_code; ++kb) {
                     const bool first = in == 0;
                     const int sb = cb.s;
-                    if (!__all_sync(0xffffffffu, mbar_wait_ab(bfull + 8 * sb, cb.ph, budget, abort))) {
+                    if (!readyb && !__all_sync(0xffffffffu, mbar_wait_ab(bfull + 8 * sb, cb.ph, budget, abort))) {
                         fail_code = 2;
                         break;
                     }
@@ -770,7 +780,8 @@ __global__ void __launch_bounds__(kGThreads, 1) k_dg_gemm(const DgArgs args) {
                         // go out (a wait between two digits idled the tensor core
                         // for about 100 cycles)
                         ready = __all_sync(0xffffffffu, mbar_test(afull + 8 * ca.s, ca.ph));
-                        tc_fence_after();
+                        if (d == 0) readyb = __all_sync(0xffffffffu, mbar_test(bfull + 8 * cb.s, cb.ph));
+                        if (first) tc_fence_after();
                         const uint64_t da0 = sdesc_sw128(smem_u32(ring + s * kGA));
                         const uint32_t col = tmem + kGN * d;
                         // at most four orders (N = 256) an instruction
@@ -1249,7 +1260,6 @@ int digits_prepare(tdscha_ctx *c) {
     TDS_CUDA(cudaMemcpy(h_fl, fl, sizeof(h_fl), cudaMemcpyDeviceToHost));
     x->flushA = digits_flush(h_fl);
     x->flushB = digits_flush(h_fl + kFlushes * kRes);
-    if (const char *e = getenv("DBG_FLUSH")) printf("flush %d %d of %d %ld\n", x->flushA, x->flushB, x->nkbM, x->nkbR);
     TDS_CUDA(cudaFuncSetAttribute(k_dg_gemm<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)DgShape<true>::smem));
     TDS_CUDA(cudaFuncSetAttribute(k_dg_gemm<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
