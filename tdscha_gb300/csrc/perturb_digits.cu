@@ -752,7 +752,7 @@ __global__ void __launch_bounds__(kGThreads, 1) k_dg_gemm(const DgArgs args) {
                 for (int kb = 0; kb < nkb && !fail_code; ++kb) {
                     const bool first = in == 0;
                     const int sb = cb.s;
-                    if (!readyb && !__all_sync(0xffffffffu, mbar_wait_ab(bfull + 8 * sb, cb.ph, budget, abort))) {
+                    if (!readyb && !mbar_all(bfull + 8 * sb, cb.ph, budget, abort)) {
                         fail_code = 2;
                         break;
                     }
@@ -763,13 +763,13 @@ __global__ void __launch_bounds__(kGThreads, 1) k_dg_gemm(const DgArgs args) {
                         constexpr int kTop = SA - 1;
                         const int cnt = min(SB, kOrders - d);       // orders d .. d + cnt - 1
                         const int s = ca.s;
-                        bool ok = ready || __all_sync(0xffffffffu, mbar_wait_ab(afull + 8 * s, ca.ph, budget, abort));
+                        bool ok = ready || mbar_all(afull + 8 * s, ca.ph, budget, abort);
                         if (first && nch > 0) {
                             // the orders that this digit writes first: d, and at the
                             // top digit all of its orders
                             const uint32_t par = (nch - 1) & 1;
                             for (int o = d; o < (d == kTop ? d + cnt : d + 1); ++o)
-                                ok = __all_sync(0xffffffffu, mbar_wait_ab(tempty + 8 * o, par, budget, abort)) && ok;
+                                ok = mbar_all(tempty + 8 * o, par, budget, abort) && ok;
                         }
                         if (!ok) {
                             fail_code = 2;
@@ -886,7 +886,7 @@ __global__ void __launch_bounds__(kGThreads, 1) k_dg_gemm(const DgArgs args) {
 #pragma unroll
             for (int e = 0; e < 32; ++e) hi[e] = lo[e] = start;
             for (int c = 0; c < nacc; ++c, ++nch) {
-                if (!bad && !__all_sync(0xffffffffu, mbar_wait_ab(tfull, nch & 1, budget, abort))) {
+                if (!bad && !mbar_all(tfull, nch & 1, budget, abort)) {
                     bad = true;
                     *abort = 1;
                 }

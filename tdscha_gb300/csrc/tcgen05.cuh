@@ -218,6 +218,12 @@ __device__ __forceinline__ bool mbar_wait_ab(uint32_t bar, uint32_t parity, long
     return true;
 }
 
+// The same by a whole warp: true where every lane saw the phase complete.
+__device__ __forceinline__ bool mbar_all(uint32_t bar, uint32_t parity, long long budget,
+                                         volatile int *abort) {
+    return __all_sync(0xffffffffu, mbar_wait_ab(bar, parity, budget, abort));
+}
+
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
