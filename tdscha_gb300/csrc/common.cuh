@@ -202,6 +202,22 @@ int digits_prepare(tdscha_ctx *c);
 void digits_release(tdscha_ctx *c);
 int digits_check_error(tdscha_ctx *c);
 int perturb_digits(tdscha_ctx *c, int apply_d4, cudaStream_t st);
+// Without symmetry images (digits_single): straight from and to the caller's
+// device arrays (Y1 need not be symmetric); from psi into c->f, c->d2v (factors
+// ca, cb of the transposed or the Wigner layout, null in the plain one); from the
+// pair of a bi-Lanczos step, or nvec <= digits_batch(c) static vectors, into
+// consecutive f and d2v of the store
+bool digits_single(const tdscha_ctx *c);
+int digits_batch(const tdscha_ctx *c);
+int digits_from_matrix(tdscha_ctx *c, int apply_d4, const double *R1, const double *Y1, double *f,
+                       double *d2v, cudaStream_t st);
+int digits_from_psi(tdscha_ctx *c, int apply_d4, const double *psi, const double *ca,
+                    const double *cb, cudaStream_t st);
+int digits_from_pair(tdscha_ctx *c, int apply_d4, const double *q, const double *p,
+                     const double *ca, const double *cb, double **f, double **d2v,
+                     cudaStream_t st);
+int digits_from_static(tdscha_ctx *c, int apply_d4, int nvec, const double *psi, double **f,
+                       double **d2v, cudaStream_t st);
 // perturb_mixed.cu
 int mixed_prepare(tdscha_ctx *c);
 int mixed_release(tdscha_ctx *c);

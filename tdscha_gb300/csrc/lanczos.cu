@@ -287,6 +287,11 @@ int apply_full_L_dev(tdscha_ctx *c, const double *psi_in, double *psi_out, int t
             TDS_TRY(perturb_mixed_psi(c, c->ignore_v4 ? 0 : 1, psi_in,
                                       transpose ? c->pc + PC_TY * H : nullptr,
                                       transpose ? c->pc + PC_TRA * H : nullptr, st));
+        } else if (precision == TDSCHA_PREC_FP64 && digits_single(c)) {
+            const bool w = c->use_wigner, t = transpose != 0;
+            TDS_TRY(digits_from_psi(c, c->ignore_v4 ? 0 : 1, psi_in,
+                                    w ? c->pc + PC_UA * H : t ? c->pc + PC_TY * H : nullptr,
+                                    w ? c->pc + PC_UB * H : t ? c->pc + PC_TRA * H : nullptr, st));
         } else {
             dim3 gu(ceil_div(M, 256), std::min(M, 65535));
             TDS_CUDA(launch_pdl(k_unpack, gu, 256, 0, st, psi_in, c->pc, M, H, c->use_wigner,
@@ -313,12 +318,12 @@ int apply_full_L_dev(tdscha_ctx *c, const double *psi_in, double *psi_out, int t
     return TDSCHA_OK;
 }
 
-// L q and L^T p of a bi-Lanczos step.  On the tensor-core path (normal
+// L q and L^T p of a bi-Lanczos step.  On the tensor-core paths (normal
 // representation, anharmonic part on, no translation projection) both
-// perturbation averages run as one two-perturbation call (perturb_mixed_pair:
-// the ensemble read once, one launch per kernel for both) and give the bits of
-// two separate applications; otherwise, or with TDSCHA_PAIR_APPLY=0 in the
-// environment, two applications.
+// perturbation averages run as one two-perturbation call (perturb_mixed_pair,
+// which gives the bits of two separate applications, or digits_from_pair: the
+// ensemble read once, one launch per kernel for both); otherwise, or with
+// TDSCHA_PAIR_APPLY=0 in the environment, two applications.
 static bool pair_apply_enabled() {
     const char *e = getenv("TDSCHA_PAIR_APPLY");
     return !(e && atoi(e) == 0);
@@ -326,25 +331,37 @@ static bool pair_apply_enabled() {
 
 int apply_full_L_pair_dev(tdscha_ctx *c, const double *q, const double *p, double *Lq,
                           double *pL, int precision, cudaStream_t st) {
-    const bool pair = pair_apply_enabled() && precision == TDSCHA_PREC_MIXED && c->with_mixed &&
-                      !c->use_wigner && !c->ignore_v3 && c->tr_ntrans == 0 && c->f2;
-    if (!pair) {
+    const bool both = pair_apply_enabled() && !c->use_wigner && !c->ignore_v3 && c->tr_ntrans == 0;
+    const bool mixed = precision == TDSCHA_PREC_MIXED && c->with_mixed && c->f2;
+    const bool digits = precision == TDSCHA_PREC_FP64 && digits_batch(c) >= 2;
+    if (!both || !(mixed || digits)) {
         TDS_TRY(apply_full_L_dev(c, q, Lq, 0, precision, st));
         return apply_full_L_dev(c, p, pL, 1, precision, st);
     }
     const long H = c->H;
     const int M = c->M;
-    TDS_TRY(perturb_mixed_pair(c, c->ignore_v4 ? 0 : 1, q, p, c->pc + PC_TY * H,
-                               c->pc + PC_TRA * H, st));
+    const double *f = c->f, *d2v = c->d2v, *f2 = c->f2, *d2v2 = c->d2v2;
+    if (digits) {
+        double *fo, *d2vo;
+        TDS_TRY(digits_from_pair(c, c->ignore_v4 ? 0 : 1, q, p, c->pc + PC_TY * H,
+                                 c->pc + PC_TRA * H, &fo, &d2vo, st));
+        f = fo;
+        f2 = fo + M;
+        d2v = d2vo;
+        d2v2 = d2vo + (long)M * M;
+    } else {
+        TDS_TRY(perturb_mixed_pair(c, c->ignore_v4 ? 0 : 1, q, p, c->pc + PC_TY * H,
+                                   c->pc + PC_TRA * H, st));
+    }
     const int nb = std::max(1, std::min(ceil_div(M + H, 256), 4096));
     const dim3 g(nb, 2);
     if (c->reverse_L)
-        TDS_CUDA(launch_pdl(k_assemble_pair<true>, g, 256, 0, st, q, c->f, c->d2v, Lq, p, c->f2,
-                            c->d2v2, pL, c->pc, c->tri, c->w, c->Yw, c->Ywinv, c->ReAw, M, H,
+        TDS_CUDA(launch_pdl(k_assemble_pair<true>, g, 256, 0, st, q, f, d2v, Lq, p, f2,
+                            d2v2, pL, c->pc, c->tri, c->w, c->Yw, c->Ywinv, c->ReAw, M, H,
                             c->ignore_harmonic, c->shift));
     else
-        TDS_CUDA(launch_pdl(k_assemble_pair<false>, g, 256, 0, st, q, c->f, c->d2v, Lq, p, c->f2,
-                            c->d2v2, pL, c->pc, c->tri, c->w, c->Yw, c->Ywinv, c->ReAw, M, H,
+        TDS_CUDA(launch_pdl(k_assemble_pair<false>, g, 256, 0, st, q, f, d2v, Lq, p, f2,
+                            d2v2, pL, c->pc, c->tri, c->w, c->Yw, c->Ywinv, c->ReAw, M, H,
                             c->ignore_harmonic, c->shift));
     return TDSCHA_OK;
 }

@@ -350,25 +350,65 @@ __global__ void __launch_bounds__(256) k_dg_xb(const double *__restrict__ dt,
 }
 
 // ------------------------------------------------- once per call
+// Where a call's Y1 and R1 come from: matrices, or psi unpacked on the way
+// (Modules/DynamicalLanczos.py:2773-2948, :3009-3053, :3369-3430), so that no
+// Y1 is written and read again.  Image i of a source starts i strides further on.
+enum { DG_MATRIX = 0,     // symmetric as it is
+       DG_AVERAGE,        // (Y1 + Y1^T) / 2
+       DG_PSI,            // plain layout
+       DG_PSI_T,          // transposed layout, per-pair factors ca, cb
+       DG_PSI_WIGNER,     // ca a' - cb b'
+       DG_STATIC };       // -2 Upsilon W Upsilon, Upsilon = ca
+struct DgSource {
+    int kind;
+    const double *Y, *R;
+    long ystride, rstride;
+    const double *S;          // the vector of s, or null: f_Y R
+    const double *ca, *cb;
+    long H;
+    int no_r;                 // R1 = 0
+};
+// images 0 .. n - 2 are sources 0 .. n - 2, the others follow source n - 1
+struct DgSources {
+    DgSource s[2];
+    int n;
+};
+
+__device__ __forceinline__ double dg_y1(const DgSource &c, const double *__restrict__ Y, int M,
+                                        int n, int m) {
+    if (c.kind == DG_MATRIX) return Y[(long)n * M + m];
+    if (c.kind == DG_AVERAGE)
+        return n == m ? Y[(long)n * M + n] : 0.5 * (Y[(long)n * M + m] + Y[(long)m * M + n]);
+    const int i = min(n, m), j = max(n, m);
+    const long k = (long)i * M - (long)i * (i - 1) / 2 + (j - i);
+    const double y = Y[M + k];
+    if (c.kind == DG_PSI) return y;
+    if (c.kind == DG_PSI_T) return y * c.ca[k] + Y[M + c.H + k] * c.cb[k];
+    if (c.kind == DG_PSI_WIGNER) return c.ca[k] * y - c.cb[k] * Y[M + c.H + k];
+    // both orders of the product, as the average of the matrix and its transpose
+    const double a = -2 * ((y * c.ca[n]) * c.ca[m]), b = -2 * ((y * c.ca[m]) * c.ca[n]);
+    return n == m ? a : 0.5 * (a + b);
+}
+
 // Row n of image blockIdx.y of Y1 (symmetric): digits of y 2^(ec - et) with et
 // the exponent above the row's maximum, and the two vectors of the row scalars.
 // Also clears the image's maxima of alpha and beta.
-__global__ void __launch_bounds__(128) k_dg_y1(const double *__restrict__ Y1,
-                                               const double *__restrict__ svec,
-                                               const double *__restrict__ tvec, int s_times_fy,
-                                               const double *__restrict__ fY,
+__global__ void __launch_bounds__(128) k_dg_y1(const DgSources src, const double *__restrict__ fY,
                                                const int *__restrict__ ec, int M, int Mp,
                                                __half *__restrict__ yb, int *__restrict__ et,
                                                double *__restrict__ vs, double *__restrict__ vt,
                                                unsigned long long *__restrict__ absmax) {
     pdl_enter();
+    extern __shared__ double yrow[];     // M
     __shared__ int sh[4];
-    const int n = blockIdx.x;
-    const long img = blockIdx.y;
-    const double *y = Y1 + (img * M + n) * M;
+    const int n = blockIdx.x, is = min((int)blockIdx.y, src.n - 1);
+    const long img = blockIdx.y, rel = img - is;
+    const DgSource &c = src.s[is];
+    const double *Y = c.Y + rel * c.ystride;
     int e = INT_MIN;
     for (int m = threadIdx.x; m < M; m += blockDim.x) {
-        const double v = y[m];
+        const double v = dg_y1(c, Y, M, n, m);
+        yrow[m] = v;
         if (v != 0) e = max(e, isfinite(v) ? exp_above(v) + ec[m] : kBadExp);
     }
 #pragma unroll
@@ -381,24 +421,24 @@ __global__ void __launch_bounds__(128) k_dg_y1(const double *__restrict__ Y1,
     const int nkb = Mp / kGK, row = n % kGN;
     uint8_t *out = reinterpret_cast<uint8_t *>(yb) + (img * (Mp / kGN) + n / kGN) * nkb * (long)kCall * kGB;
     for (int ch = threadIdx.x; ch < Mp / 8; ch += blockDim.x) {
-        const int kb = ch >> 3, c = ch & 7;
+        const int kb = ch >> 3, c8 = ch & 7;
         long long q[8];
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             const int m = ch * 8 + k;
-            q[k] = (m < M && !bad) ? fixed_point(y[m], 62 + ec[m] - e) : 0;
+            q[k] = (m < M && !bad) ? fixed_point(yrow[m], 62 + ec[m] - e) : 0;
         }
         uint4 w[kCall];
         digits8<kCall>(q, w);
 #pragma unroll
         for (int d = 0; d < kCall; ++d)
-            *reinterpret_cast<uint4 *>(out + (kb * (long)kCall + d) * kGB + sw_place(row, c)) = w[d];
+            *reinterpret_cast<uint4 *>(out + (kb * (long)kCall + d) * kGB + sw_place(row, c8)) = w[d];
     }
     if (threadIdx.x == 0) {
         et[img * Mp + n] = e;
-        const double s = svec[img * M + n];
-        vs[img * Mp + n] = s_times_fy ? fY[n] * s : s;
-        vt[img * Mp + n] = fY[n] * tvec[img * M + n];
+        const double r = c.no_r ? 0.0 : c.R[rel * c.rstride + n];
+        vs[img * Mp + n] = c.S ? c.S[rel * c.rstride + n] : fY[n] * r;
+        vt[img * Mp + n] = fY[n] * r;
         if (n == 0) absmax[2 * img] = absmax[2 * img + 1] = 0ULL;
     }
 }
@@ -1083,7 +1123,7 @@ struct DigitStore {
     int flushA = kFlushMin, flushB = kFlushMin;   // K blocks per accumulation of the stages
     void *slab = nullptr;
     double *dt = nullptr, *gt = nullptr, *vs = nullptr, *vt = nullptr, *qp = nullptr,
-           *gpart = nullptr, *fpart = nullptr;
+           *gpart = nullptr, *fpart = nullptr, *fo = nullptr, *d2vo = nullptr;
     RowScalars *abcc = nullptr;
     unsigned long long *dmax = nullptr, *gmax = nullptr, *absmax = nullptr;
     __half *xa = nullptr, *xb = nullptr, *yb = nullptr, *wa = nullptr;
@@ -1150,6 +1190,7 @@ int digits_prepare(tdscha_ctx *c) {
         if (atoi(e) == 0) return TDSCHA_OK;
     const int M = c->M;
     const long R = c->Nrows;
+    if (sizeof(double) * M > 200 * 1024) return TDSCHA_OK;   // k_dg_y1 keeps a row on chip
     DigitStore *x = new DigitStore();
     x->Mp = ceil_div(M, kGN) * kGN;
     x->nkbM = x->nct = x->Mp / kGK;
@@ -1163,8 +1204,16 @@ int digits_prepare(tdscha_ctx *c) {
     if (const char *b = getenv("TDSCHA_WAIT_BUDGET_CYCLES")) x->budget = atoll(b);
     const int Mp = x->Mp;
     const size_t elems = (size_t)Mp * x->Rp;
-    // images of one pass over W: all of them within 6 GB of W digits
-    x->cap = (int)std::max<size_t>(1, std::min<size_t>(c->J, (size_t(6) << 30) / (elems * 2 * kCall)));
+    // Images of one pass: the context's symmetry images within 6 GB of W digits; or,
+    // without images, perturbations given together (the two of a bi-Lanczos step,
+    // static vectors), two within 6 GB and up to 32 within 256 MB.
+    const size_t per_img = elems * 2 * kCall;
+    const size_t most = std::max<size_t>(1, (size_t(6) << 30) / per_img);
+    if (c->J > 1)
+        x->cap = (int)std::min<size_t>(c->J, most);
+    else
+        x->cap = (int)std::max(std::min<size_t>(2, most),
+                               std::min<size_t>(32, (size_t(256) << 20) / per_img));
     const int cap = x->cap, nat = ceil_div((long)cap * Mp, kGM);
     // about eight W blocks per SM, at most 16 K blocks each
     x->per = (int)std::max<long>(1, std::min<long>(16, x->nkbR * nat / (152L * 8)));
@@ -1194,6 +1243,8 @@ int digits_prepare(tdscha_ctx *c) {
         {(void **)&x->abcc, sizeof(RowScalars) * (size_t)cap * x->Rp, false},
         {(void **)&x->gpart, gbytes, false},
         {(void **)&x->fpart, d * (size_t)cap * x->nfc * M, false},
+        {(void **)&x->fo, c->J == 1 ? d * cap * M : 0, false},
+        {(void **)&x->d2vo, c->J == 1 ? d * (size_t)cap * M * M : 0, false},
         {(void **)&x->ec, i4 * Mp, false},
         // zero from the start: maxima, and the rows of padding modes
         {(void **)&x->dmax, u8 * Mp, true},
@@ -1260,6 +1311,7 @@ int digits_prepare(tdscha_ctx *c) {
     TDS_CUDA(cudaMemcpy(h_fl, fl, sizeof(h_fl), cudaMemcpyDeviceToHost));
     x->flushA = digits_flush(h_fl);
     x->flushB = digits_flush(h_fl + kFlushes * kRes);
+    TDS_CUDA(cudaFuncSetAttribute(k_dg_y1, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     TDS_CUDA(cudaFuncSetAttribute(k_dg_gemm<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)DgShape<true>::smem));
     TDS_CUDA(cudaFuncSetAttribute(k_dg_gemm<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1275,19 +1327,18 @@ int digits_check_error(tdscha_ctx *c) {
     return TDSCHA_ERR_TIMEOUT;
 }
 
-// Stages A and B for nimg symmetric matrices Y1 (M x M each) with their two row
-// vectors (M each): split-K partials of every image's H in x->gpart, force
-// partials in x->fpart.
-static int digits_contract(tdscha_ctx *c, int nimg, const double *Y1, const double *svec,
-                           const double *tvec, int s_times_fy, int apply_d4, int *nsplit,
-                           cudaStream_t st) {
+// Stages A and B for nimg perturbations: split-K partials of every image's H in
+// x->gpart, force partials in x->fpart.
+static int digits_contract(tdscha_ctx *c, int nimg, const DgSources &src, int apply_d4,
+                           int *nsplit, cudaStream_t st) {
     DigitStore *x = c->dg;
     const int M = c->M, Mp = x->Mp;
     const long R = c->Nrows;
     {
         ProfScope ps(c, 5, st);
-        TDS_CUDA(launch_pdl(k_dg_y1, dim3(M, nimg), 128, 0, st, Y1, svec, tvec, s_times_fy, c->fY,
-                            x->ec, M, Mp, x->yb, x->et, x->vs, x->vt, x->absmax));
+        TDS_CUDA(launch_pdl(k_dg_y1, dim3(M, nimg), 128, sizeof(double) * M, st, src,
+                            (const double *)c->fY, (const int *)x->ec, M, Mp, x->yb, x->et, x->vs,
+                            x->vt, x->absmax));
     }
     DgArgs ga{};
     ga.a = x->xa;
@@ -1355,31 +1406,84 @@ static int digits_contract(tdscha_ctx *c, int nimg, const double *Y1, const doub
     return TDSCHA_OK;
 }
 
+static DgSource dg_matrix(int kind, const double *Y, const double *R, long ystride) {
+    return DgSource{kind, Y, R, ystride, 0, nullptr, nullptr, nullptr, 0, 0};
+}
+
+// The averages of nimg <= cap perturbations, one context image each (J = 1), into
+// f (M each) and d2v (M x M each).
+static int digits_averages(tdscha_ctx *c, int nimg, const DgSources &src, int apply_d4, double *f,
+                           double *d2v, cudaStream_t st) {
+    DigitStore *x = c->dg;
+    const int M = c->M, Mp = x->Mp;
+    int ns = 0;
+    TDS_TRY(digits_contract(c, nimg, src, apply_d4, &ns, st));
+    ProfScope ps(c, 4, st);
+    const int nt = ceil_div(M, 32), nat = ceil_div((long)nimg * Mp, kGM);
+    TDS_CUDA(launch_pdl(k_dg_final, dim3(4 * (nt * (nt + 1) / 2), nimg), 256, 0, st,
+                        (const double *)x->gpart, ns, (long)nat * kGM * Mp, M, Mp,
+                        (const double *)x->fpart, x->nfc, (const double *)c->fY,
+                        c->sum_rho * c->S, f, d2v));
+    return TDSCHA_OK;
+}
+
+bool digits_single(const tdscha_ctx *c) { return c->dg && c->J == 1; }
+int digits_batch(const tdscha_ctx *c) { return digits_single(c) ? c->dg->cap : 0; }
+
 // The averages of c->Y1 (symmetric), c->R1 into c->f, c->d2v.
 int perturb_digits(tdscha_ctx *c, int apply_d4, cudaStream_t st) {
     DigitStore *x = c->dg;
     const int M = c->M, Mp = x->Mp, J = c->J;
-    int ns = 0;
-    if (J == 1) {
-        TDS_TRY(digits_contract(c, 1, c->Y1, c->R1, c->R1, 1, apply_d4, &ns, st));
-        ProfScope ps(c, 4, st);
-        const int nt = ceil_div(M, 32), nat = ceil_div((long)Mp, kGM);
-        TDS_CUDA(launch_pdl(k_dg_final, dim3(4 * (nt * (nt + 1) / 2), 1), 256, 0, st,
-                            (const double *)x->gpart, ns, (long)nat * kGM * Mp, M, Mp,
-                            (const double *)x->fpart, x->nfc, (const double *)c->fY,
-                            c->sum_rho * c->S, c->f, c->d2v));
-        return TDSCHA_OK;
-    }
+    if (J == 1)
+        return digits_averages(c, 1, {{dg_matrix(DG_MATRIX, c->Y1, c->R1, 0)}, 1}, apply_d4, c->f,
+                               c->d2v, st);
     TDS_TRY(psi_perturbation64(c, st));
+    const long MM = (long)M * M;
     for (int j0 = 0; j0 < J; j0 += x->cap) {
         const int nj = std::min(x->cap, J - j0);
-        TDS_TRY(digits_contract(c, nj, c->Y1all + (size_t)j0 * M * M, c->vsv + (size_t)j0 * M,
-                                c->vsv + (size_t)(J + j0) * M, 0, apply_d4, &ns, st));
+        int ns = 0;
+        DgSource s = dg_matrix(DG_MATRIX, c->Y1all + j0 * MM, c->vsv + (long)(J + j0) * M, MM);
+        s.rstride = M;
+        s.S = c->vsv + (long)j0 * M;
+        TDS_TRY(digits_contract(c, nj, {{s}, 1}, apply_d4, &ns, st));
         const int nat = ceil_div((long)nj * Mp, kGM);
         TDS_TRY(psi_hsum64(c, x->gpart, ns, (long)nat * kGM * Mp, (long)Mp * Mp, Mp, x->fpart,
                            x->nfc, c->fY, j0, nj, st));
     }
     return psi_reduce64(c, st);
+}
+
+int digits_from_matrix(tdscha_ctx *c, int apply_d4, const double *R1, const double *Y1, double *f,
+                       double *d2v, cudaStream_t st) {
+    return digits_averages(c, 1, {{dg_matrix(DG_AVERAGE, Y1, R1, 0)}, 1}, apply_d4, f, d2v, st);
+}
+
+static DgSource dg_psi(const tdscha_ctx *c, const double *psi, const double *ca, const double *cb) {
+    const int kind = c->use_wigner ? DG_PSI_WIGNER : ca ? DG_PSI_T : DG_PSI;
+    return DgSource{kind, psi, psi, 0, 0, nullptr, ca, cb, c->H, c->ignore_v3};
+}
+
+int digits_from_psi(tdscha_ctx *c, int apply_d4, const double *psi, const double *ca,
+                    const double *cb, cudaStream_t st) {
+    return digits_averages(c, 1, {{dg_psi(c, psi, ca, cb)}, 1}, apply_d4, c->f, c->d2v, st);
+}
+
+int digits_from_pair(tdscha_ctx *c, int apply_d4, const double *q, const double *p,
+                     const double *ca, const double *cb, double **f, double **d2v,
+                     cudaStream_t st) {
+    *f = c->dg->fo;
+    *d2v = c->dg->d2vo;
+    return digits_averages(c, 2, {{dg_psi(c, q, nullptr, nullptr), dg_psi(c, p, ca, cb)}, 2},
+                           apply_d4, *f, *d2v, st);
+}
+
+int digits_from_static(tdscha_ctx *c, int apply_d4, int nvec, const double *psi, double **f,
+                       double **d2v, cudaStream_t st) {
+    const long Ps = c->M + c->H;
+    *f = c->dg->fo;
+    *d2v = c->dg->d2vo;
+    const DgSource s{DG_STATIC, psi, psi, Ps, Ps, nullptr, c->Yw, nullptr, c->H, 0};
+    return digits_averages(c, nvec, {{s}, 1}, apply_d4, *f, *d2v, st);
 }
 
 }  // namespace tdscha

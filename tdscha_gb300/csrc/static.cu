@@ -8,6 +8,7 @@
 // Y1_ab = -2 psi_W(ab) Upsilon_a Upsilon_b (Upsilon = 2w/(2n+1)); its output is
 // [-f | d2v upper triangle].  The harmonic part is diagonal: psi_R w^(2p) and
 // psi_W / Lambda^p with the pair factor Lambda of apply_L1_static.
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -82,6 +83,11 @@ __global__ void k_assemble_static(const double *__restrict__ psi, const double *
                                   const double *__restrict__ lam, const int *__restrict__ tri,
                                   int M, long H, int harm, int anh, double power,
                                   double *__restrict__ out) {
+    // vector blockIdx.y of a batch
+    psi += blockIdx.y * (M + H);
+    out += blockIdx.y * (M + H);
+    f += blockIdx.y * (long)M;
+    d2v += blockIdx.y * (long)M * M;
     for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < M + H; e += (long)gridDim.x * blockDim.x) {
         double o = 0;
         if (e < M) {
@@ -190,6 +196,19 @@ extern "C" int tdscha_static_L(tdscha_ctx *ctx, int nvec, const double *psi_in, 
     const int harm = what & 1, anh = (what >> 1) & 1;
     const int nbu = std::max(1, std::min(ceil_div((long)M * M, 256), 4096));
     const int nba = std::max(1, std::min(ceil_div(Ps, 256), 4096));
+    const int batch = anh && precision == TDSCHA_PREC_FP64 ? digits_batch(ctx) : 0;
+    // float64 averages of many vectors together: one launch per kernel for all
+    for (int v = 0; batch > 0 && v < nvec; v += batch) {
+        const int n = std::min(batch, nvec - v);
+        double *f, *d2v;
+        TDS_TRY(digits_from_static(ctx, ctx->ignore_v4 ? 0 : 1, n, psi_in + (long)v * Ps, &f, &d2v,
+                                   st));
+        k_assemble_static<<<dim3(nba, n), 256, 0, st>>>(psi_in + (long)v * Ps, f, d2v, ctx->w,
+                                                        ctx->lam_static, ctx->tri, M, H, harm, anh,
+                                                        power, psi_out + (long)v * Ps);
+        TDS_CHECK_LAUNCH();
+    }
+    if (batch > 0) return TDSCHA_OK;
     for (int v = 0; v < nvec; ++v) {
         const double *in = psi_in + (long)v * Ps;
         double *out = psi_out + (long)v * Ps;
