@@ -222,6 +222,9 @@ int digits_from_static(tdscha_ctx *c, int apply_d4, int nvec, const double *psi,
 int mixed_prepare(tdscha_ctx *c);
 int mixed_release(tdscha_ctx *c);
 int perturb_mixed(tdscha_ctx *c, int apply_d4, cudaStream_t st);
+// straight from and to the caller's device arrays (Y1 need not be symmetric)
+int perturb_mixed_from_matrix(tdscha_ctx *c, int apply_d4, const double *R1, const double *Y1,
+                              double *f, double *d2v, cudaStream_t st);
 // the same with Y1 and R1 unpacked from psi inside the operand preparation
 // (plain layout, or the transposed one with its per-pair factors cty / ctra)
 int perturb_mixed_psi(tdscha_ctx *c, int apply_d4, const double *psi, const double *cty,

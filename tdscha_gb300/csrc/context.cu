@@ -529,10 +529,12 @@ extern "C" int tdscha_perturb_averages(tdscha_ctx *ctx, const double *R1, const 
         for (long k = 0; k < (long)M * M; ++k)
             if (!std::isfinite(Y1[k])) { set_error("perturb_averages: non-finite Y1"); return TDSCHA_ERR_NAN; }
     }
-    // the digit path reads and writes device arrays in place: R1 and Y1 are read
-    // by its first kernel, f_out and d2v_out written by its last
+    // the tensor-core paths read and write device arrays in place: R1 and Y1 are
+    // read by their first kernels, f_out and d2v_out written by their last
     if (device_ptrs && precision == TDSCHA_PREC_FP64 && digits_single(ctx))
         return digits_from_matrix(ctx, apply_D4, R1, Y1, f_out, d2v_out, st);
+    if (device_ptrs && precision == TDSCHA_PREC_MIXED && ctx->with_mixed)
+        return perturb_mixed_from_matrix(ctx, apply_D4, R1, Y1, f_out, d2v_out, st);
     TDS_CUDA(cudaMemcpyAsync(ctx->R1, R1, sizeof(double) * M, in, st));
     TDS_CUDA(cudaMemcpyAsync(ctx->Y1, Y1, sizeof(double) * M * M, in, st));
     TDS_TRY(run_perturb(ctx, apply_D4, precision, st));

@@ -1072,7 +1072,11 @@ __global__ void k_prep_cols(const double *__restrict__ D, const double *__restri
 struct Y1FromBuffers {
     const double *Y1, *R1;
     int M;
-    __device__ double y(int n, int m) const { return Y1[(long)n * M + m]; }
+    int average;     // take (Y1 + Y1^T) / 2
+    __device__ double y(int n, int m) const {
+        const double v = Y1[(long)n * M + m];
+        return average && n != m ? 0.5 * (v + Y1[(long)m * M + n]) : v;
+    }
     __device__ double r(int n) const { return R1[n]; }
 };
 struct Y1FromPsi {
@@ -1959,23 +1963,30 @@ int mixed_check_error(tdscha_ctx *c) {
 }
 
 static int perturb_mixed_src(tdscha_ctx *c, int apply_d4, const Y1FromPsi *psrc, int nsrc,
-                             cudaStream_t st);
+                             const Y1FromBuffers &bsrc, double *f, double *d2v, cudaStream_t st);
 
 int perturb_mixed(tdscha_ctx *c, int apply_d4, cudaStream_t st) {
-    return perturb_mixed_src(c, apply_d4, nullptr, 1, st);
+    const Y1FromBuffers b{c->Y1, c->R1, c->M, 0};
+    return perturb_mixed_src(c, apply_d4, nullptr, 1, b, c->f, c->d2v, st);
+}
+
+int perturb_mixed_from_matrix(tdscha_ctx *c, int apply_d4, const double *R1, const double *Y1,
+                              double *f, double *d2v, cudaStream_t st) {
+    const Y1FromBuffers b{Y1, R1, c->M, 1};
+    return perturb_mixed_src(c, apply_d4, nullptr, 1, b, f, d2v, st);
 }
 
 int perturb_mixed_psi(tdscha_ctx *c, int apply_d4, const double *psi, const double *cty,
                       const double *ctra, cudaStream_t st) {
     Y1FromPsi src{psi, cty, ctra, c->M, c->H, c->ignore_v3};
-    return perturb_mixed_src(c, apply_d4, &src, 1, st);
+    return perturb_mixed_src(c, apply_d4, &src, 1, {}, c->f, c->d2v, st);
 }
 
 int perturb_mixed_pair(tdscha_ctx *c, int apply_d4, const double *psi_a, const double *psi_b,
                        const double *cty, const double *ctra, cudaStream_t st) {
     Y1FromPsi src[2] = {{psi_a, nullptr, nullptr, c->M, c->H, c->ignore_v3},
                         {psi_b, cty, ctra, c->M, c->H, c->ignore_v3}};
-    return perturb_mixed_src(c, apply_d4, src, 2, st);
+    return perturb_mixed_src(c, apply_d4, src, 2, {}, c->f, c->d2v, st);
 }
 
 // One tensor-core call for nsrc perturbations (1, or 2: the L and L^T
@@ -1984,9 +1995,10 @@ int perturb_mixed_pair(tdscha_ctx *c, int apply_d4, const double *psi_a, const d
 // reads the ensemble once for all of them and every other kernel runs once over
 // all images.  Each image has its own W scales, so the results of a
 // two-perturbation call are those of two one-perturbation calls, bit for bit.
-// psrc == nullptr: one perturbation from the Y1 and R1 buffers.
+// psrc == nullptr: one perturbation from the matrices of bsrc.  The first
+// perturbation's results go to f and d2v, the second's to f2 and d2v2.
 static int perturb_mixed_src(tdscha_ctx *c, int apply_d4, const Y1FromPsi *psrc, int nsrc,
-                             cudaStream_t st) {
+                             const Y1FromBuffers &bsrc, double *f, double *d2v, cudaStream_t st) {
     MixedStore &mx = c->mx;
     MixedExtra *x = extra(c);
     if (!x) { set_error("mixed store not prepared"); return TDSCHA_ERR_STATE; }
@@ -2012,7 +2024,7 @@ static int perturb_mixed_src(tdscha_ctx *c, int apply_d4, const Y1FromPsi *psrc,
                                     c->maxdeg, c->fY, c->fpsi, x->sd, M, Mp, mx.y1_hi, mx.y1_lo,
                                     x->tcol, x->vs, x->vt, x->absmax));
             } else {
-                const Y1FromBuffers b1{c->Y1, c->R1, M};
+                const Y1FromBuffers &b1 = bsrc;
                 const SrcPair<Y1FromBuffers> sp{{b1, b1}};
                 TDS_CUDA(launch_pdl(k_y1_df<Y1FromBuffers>, gy, 256, 0, st, sp, M, x->y1df));
                 TDS_CUDA(launch_pdl(k_prep_y1_img<Y1FromBuffers>, gi, 256, sm, st, sp,
@@ -2027,7 +2039,7 @@ static int perturb_mixed_src(tdscha_ctx *c, int apply_d4, const Y1FromPsi *psrc,
                 TDS_CUDA(launch_pdl(k_prep_y1<Y1FromPsi>, g, 256, 0, st, sp, c->fY, c->fpsi, x->sd,
                                     M, Mp, mx.y1_hi, mx.y1_lo, x->tcol, x->vs, x->vt, x->absmax));
             } else {
-                const Y1FromBuffers b1{c->Y1, c->R1, M};
+                const Y1FromBuffers &b1 = bsrc;
                 const SrcPair<Y1FromBuffers> sp{{b1, b1}};
                 TDS_CUDA(launch_pdl(k_prep_y1<Y1FromBuffers>, g, 256, 0, st, sp, c->fY, c->fpsi,
                                     x->sd, M, Mp, mx.y1_hi, mx.y1_lo, x->tcol, x->vs, x->vt,
@@ -2102,7 +2114,7 @@ static int perturb_mixed_src(tdscha_ctx *c, int apply_d4, const Y1FromPsi *psrc,
             const long io = (long)sidx * J;
             TDS_TRY(psi_finalize32(c, mx.gpart + io * Mp, mx.nsplit, sstride, Mp, ldGb,
                                    x->fpart + io * x->nfchunk * M, x->nfchunk,
-                                   sidx ? c->f2 : c->f, sidx ? c->d2v2 : c->d2v, st));
+                                   sidx ? c->f2 : f, sidx ? c->d2v2 : d2v, st));
         }
     } else {
         // both perturbations' split-K sums and (f, d2v) in one launch
@@ -2110,7 +2122,7 @@ static int perturb_mixed_src(tdscha_ctx *c, int apply_d4, const Y1FromPsi *psrc,
         const int nt = ceil_div(M, 32);
         TDS_CUDA(launch_pdl(k_gfinal, dim3(4 * (nt * (nt + 1) / 2), nsrc), 256, 0, st, mx.gpart,
                             mx.nsplit, (long)ldGb, sstride, M, Mp, x->fpart, x->nfchunk,
-                            c->sum_rho * c->S, c->f, c->d2v, c->f2, c->d2v2));
+                            c->sum_rho * c->S, f, d2v, c->f2, c->d2v2));
     }
     return TDSCHA_OK;
 }

@@ -11,12 +11,16 @@
 //     f   <- P_t f,  P_t = mean_R pols^T P_R pols
 //     d2v <- pols^T [ mean_R Perm_R(pols d2v pols^T) ] pols
 //   Perm_R(D)[r][s] = D[perm_R[r]][perm_R[s]] (Cartesian index permutations).
-// All float64 (complex double2 for the Bloch projection) on the CUDA cores:
-// one-off or O(M^3) per application, no tensor-core variant.
+// The mode projection of an ensemble, N x n_cart x M, runs as exact digit products
+// on the tensor cores (perturb_digits.cu explains them); the others, O(M^3) per
+// application or small, in float64 (complex double2 for the Bloch projection) on
+// the CUDA cores.
+#include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <vector>
 
-#include "common.cuh"
+#include "digits.cuh"
 
 namespace tdscha {
 
@@ -120,6 +124,174 @@ __global__ void k_prologue(const double *__restrict__ a, long n, int K, int widt
     }
 }
 
+// Digits of the rows a' of k_prologue (real data), one warp per row, and the
+// exponent above each row's maximum.  Rows past n (of the last tile) are zero.
+__global__ void __launch_bounds__(256) k_dg_slice_rows(const double *__restrict__ a, long n, int K,
+                                                       int nkb, double s,
+                                                       const double *__restrict__ sub,
+                                                       const double *__restrict__ mul,
+                                                       __half *__restrict__ out,
+                                                       int *__restrict__ er) {
+    const long r = blockIdx.x * 8L + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
+    const double *p = a + r * K;
+    auto value = [&](int k) {
+        double v = p[k] * s;
+        if (sub) v -= sub[k];
+        return v * mul[k];
+    };
+    int e = INT_MIN;
+    if (r < n)
+        for (int k = lane; k < K; k += 32) {
+            const double v = value(k);
+            if (v != 0) e = max(e, isfinite(v) ? exp_above(v) : kBadExp);
+        }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, o));
+    if (e == INT_MIN) e = 0;
+    const bool bad = e >= kBadExp / 2 || r >= n;
+    if (lane == 0) er[r] = e;
+    uint8_t *blk = reinterpret_cast<uint8_t *>(out) + (r / kGM) * nkb * kRes * (long)kGA;
+    const int row = (int)(r % kGM);
+    for (int ch = lane; ch < nkb * 8; ch += 32) {
+        long long q[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const int m = ch * 8 + k;
+            q[k] = m < K && !bad ? fixed_point(value(m), 55 - e) : 0;
+        }
+        uint4 w[kRes];
+        digits8<kRes>(q, w);
+#pragma unroll
+        for (int d = 0; d < kRes; ++d)
+            *reinterpret_cast<uint4 *>(blk + ((ch >> 3) * (long)kRes + d) * kGA +
+                                       sw_place(row, ch & 7)) = w[d];
+    }
+}
+
+// Digits of the columns of b (K x n): block = column (up to a multiple of 64, the
+// padding zero)
+__global__ void __launch_bounds__(128) k_dg_slice_cols(const double *__restrict__ b, int K, int n,
+                                                       int nkb, __half *__restrict__ out,
+                                                       int *__restrict__ et) {
+    __shared__ int sh[4];
+    const int c = blockIdx.x;
+    int e = INT_MIN;
+    if (c < n)
+        for (int k = threadIdx.x; k < K; k += blockDim.x) {
+            const double v = b[(long)k * n + c];
+            if (v != 0) e = max(e, isfinite(v) ? exp_above(v) : kBadExp);
+        }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, o));
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = e;
+    __syncthreads();
+    e = max(max(sh[0], sh[1]), max(sh[2], sh[3]));
+    if (e == INT_MIN) e = 0;
+    const bool bad = e >= kBadExp / 2 || c >= n;
+    if (threadIdx.x == 0) et[c] = e;
+    uint8_t *blk = reinterpret_cast<uint8_t *>(out) + (c / kGN) * nkb * (long)kCall * kGB;
+    for (int ch = threadIdx.x; ch < nkb * 8; ch += blockDim.x) {
+        long long q[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const int m = ch * 8 + k;
+            q[k] = m < K && !bad ? fixed_point(b[(long)m * n + c], 62 - e) : 0;
+        }
+        uint4 w[kCall];
+        digits8<kCall>(q, w);
+#pragma unroll
+        for (int d = 0; d < kCall; ++d)
+            *reinterpret_cast<uint4 *>(blk + ((ch >> 3) * (long)kCall + d) * kGB +
+                                       sw_place(c % kGN, ch & 7)) = w[d];
+    }
+}
+
+// C (rows x n) = A' B by digit products: A' the rows of k_prologue, B K x n.  The
+// digits of 2^16 rows at a time (14 bytes an element) beside those of B.
+struct DigitProduct {
+    void *slab = nullptr;
+    __half *a = nullptr, *b = nullptr;
+    int *er = nullptr, *et = nullptr, *err = nullptr;
+    int K = 0, n = 0, nkb = 0, nbt = 0, nsm = 1;
+    long chunk = 0;
+    long long budget = kDefaultBudget;
+    ~DigitProduct() { cached_free(slab); }
+
+    // false: the digits do not fit (the caller takes the CUDA-core product)
+    bool init(long rows, int K_, int n_) {
+        if (const char *e = getenv("TDSCHA_FP64_DIGITS"))
+            if (atoi(e) == 0) return false;
+        if (const char *e = getenv("TDSCHA_WAIT_BUDGET_CYCLES")) budget = atoll(e);
+        K = K_;
+        n = n_;
+        nkb = ceil_div(K, kGK);
+        nbt = ceil_div(n, kGN);
+        chunk = std::min<long>(65536, (rows + kGM - 1) / kGM * kGM);
+        int dev = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+        auto pad = [](size_t x) { return (x + 1023) & ~size_t(1023); };
+        const size_t ba = (size_t)chunk * nkb * kGK * 2 * kRes, bb = (size_t)nbt * nkb * kCall * kGB,
+                     be = pad(sizeof(int) * chunk), bt = pad(sizeof(int) * nbt * kGN);
+        if (cached_malloc(&slab, ba + bb + be + bt + 1024) != cudaSuccess) {
+            cudaGetLastError();
+            slab = nullptr;
+            return false;
+        }
+        uint8_t *p = reinterpret_cast<uint8_t *>(slab);
+        a = reinterpret_cast<__half *>(p);
+        b = reinterpret_cast<__half *>(p + ba);
+        er = reinterpret_cast<int *>(p + ba + bb);
+        et = reinterpret_cast<int *>(p + ba + bb + be);
+        err = reinterpret_cast<int *>(p + ba + bb + be + bt);
+        return true;
+    }
+
+    int set_b(const double *B) {
+        TDS_CUDA(cudaMemsetAsync(err, 0, sizeof(int), 0));
+        TDS_CUDA(cudaFuncSetAttribute(k_dg_gemm<DG_STORE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)DgShape<DG_STORE>::smem));
+        k_dg_slice_cols<<<nbt * kGN, 128>>>(B, K, n, nkb, b, et);
+        TDS_CHECK_LAUNCH();
+        return TDSCHA_OK;
+    }
+
+    int product(const double *A, long rows, double s, const double *sub, const double *mul, double *C) {
+        for (long r0 = 0; r0 < rows; r0 += chunk) {
+            const long nr = std::min(chunk, rows - r0), nrp = (nr + kGM - 1) / kGM * kGM;
+            k_dg_slice_rows<<<(unsigned)(nrp / 8), 256>>>(A + r0 * K, nr, K, nkb, s, sub, mul, a, er);
+            TDS_CHECK_LAUNCH();
+            DgArgs g{};
+            g.a = a;
+            g.b = b;
+            g.nkb = g.kbps = nkb;
+            g.flush = kFlushMin;
+            g.nat = (int)(nrp / kGM);
+            g.nbt = nbt;
+            g.nitems = (long)g.nat * nbt;
+            g.err = err;
+            g.budget = budget;
+            g.et = et;
+            g.er = er;
+            g.R = nr;
+            g.M = n;
+            g.out = C + r0 * n;
+            TDS_CUDA(launch_pdl(k_dg_gemm<DG_STORE>, (int)std::min<long>(g.nitems, nsm), kGThreads,
+                                DgShape<DG_STORE>::smem, (cudaStream_t)0, g));
+        }
+        return TDSCHA_OK;
+    }
+
+    int status() {
+        int v = 0;
+        TDS_CUDA(cudaMemcpy(&v, err, sizeof(int), cudaMemcpyDeviceToHost));
+        if (!v) return TDSCHA_OK;
+        set_error("tensor-core pipeline: a bounded wait expired (code %d)", v);
+        return TDSCHA_ERR_TIMEOUT;
+    }
+};
+
 // Perm-average: out[r][s] = mean_R D[perm_R[r]][perm_R[s]]
 __global__ void k_perm_average(const double *__restrict__ D, const int *__restrict__ perms,
                                int n_trans, int n, double *__restrict__ out) {
@@ -222,34 +394,44 @@ extern "C" int tdscha_project_modes(int N, int n_cart, int M, const double *u, c
     }
     size_t nu = (size_t)N * n_cart, nx = (size_t)N * M;
     double *d_in = nullptr, *d_tmp = nullptr, *d_pols = nullptr, *d_out = nullptr, *d_vec = nullptr;
+    // blocks of the process-wide cache: five cudaMalloc and cudaFree of an
+    // ensemble's size cost as much as the product
     auto done = [&](int rc) {
+        if (rc != TDSCHA_OK) cudaDeviceSynchronize();
         double *b[] = {d_in, d_tmp, d_pols, d_out, d_vec};
-        for (double *p : b) if (p) cudaFree(p);
+        for (double *p : b) cached_free(p);
         return rc;
     };
 #define PCU(x) do { cudaError_t _e = (x); if (_e != cudaSuccess) { set_error("%s: %s", #x, cudaGetErrorString(_e)); return done(TDSCHA_ERR_CUDA); } } while (0)
-    PCU(cudaMalloc(&d_in, sizeof(double) * nu));
-    PCU(cudaMalloc(&d_tmp, sizeof(double) * nu));
-    PCU(cudaMalloc(&d_pols, sizeof(double) * (size_t)n_cart * M));
-    PCU(cudaMalloc(&d_out, sizeof(double) * nx));
-    PCU(cudaMalloc(&d_vec, sizeof(double) * 3 * n_cart));
+    DigitProduct dg;
+    const bool digits = dg.init(N, n_cart, M);
+    PCU(cached_malloc(&d_in, sizeof(double) * nu));
+    if (!digits) PCU(cached_malloc(&d_tmp, sizeof(double) * nu));
+    PCU(cached_malloc(&d_pols, sizeof(double) * (size_t)n_cart * M));
+    PCU(cached_malloc(&d_out, sizeof(double) * nx));
+    PCU(cached_malloc(&d_vec, sizeof(double) * 3 * n_cart));
     PCU(cudaMemcpy(d_pols, pols, sizeof(double) * (size_t)n_cart * M, cudaMemcpyHostToDevice));
     PCU(cudaMemcpy(d_vec, sq.data(), sizeof(double) * n_cart, cudaMemcpyHostToDevice));
     PCU(cudaMemcpy(d_vec + n_cart, isq.data(), sizeof(double) * n_cart, cudaMemcpyHostToDevice));
     if (f_mean) PCU(cudaMemcpy(d_vec + 2 * n_cart, sub.data(), sizeof(double) * n_cart, cudaMemcpyHostToDevice));
-    int nb = std::max(1, std::min(ceil_div((long)nu, 256), 152 * 8));
+    int nb = std::max(1, std::min(ceil_div((long)nu, 256), 152 * 8)), rc = TDSCHA_OK;
+    if (digits && (rc = dg.set_b(d_pols)) != TDSCHA_OK) return done(rc);
     for (int pass = 0; pass < 2; ++pass) {
         PCU(cudaMemcpy(d_in, pass == 0 ? u : f, sizeof(double) * nu, cudaMemcpyHostToDevice));
-        if (pass == 0)
-            k_prologue<<<nb, 256>>>(d_in, N, n_cart, 1, u_scale, nullptr, d_vec, d_tmp);
-        else
-            k_prologue<<<nb, 256>>>(d_in, N, n_cart, 1, f_scale, f_mean ? d_vec + 2 * n_cart : nullptr,
-                                    d_vec + n_cart, d_tmp);
-        PCU(cudaGetLastError());
-        int rc = gemm<RealOps>(d_tmp, d_pols, d_out, N, M, n_cart, n_cart, 1, M, 1, M, 0);
+        const double scale = pass == 0 ? u_scale : f_scale;
+        const double *sub = pass == 1 && f_mean ? d_vec + 2 * n_cart : nullptr;
+        const double *mul = pass == 0 ? d_vec : d_vec + n_cart;
+        if (digits) {
+            rc = dg.product(d_in, N, scale, sub, mul, d_out);
+        } else {
+            k_prologue<<<nb, 256>>>(d_in, N, n_cart, 1, scale, sub, mul, d_tmp);
+            PCU(cudaGetLastError());
+            rc = gemm<RealOps>(d_tmp, d_pols, d_out, N, M, n_cart, n_cart, 1, M, 1, M, 0);
+        }
         if (rc != TDSCHA_OK) return done(rc);
         PCU(cudaMemcpy(pass == 0 ? X_out : Y_out, d_out, sizeof(double) * nx, cudaMemcpyDeviceToHost));
     }
+    if (digits && (rc = dg.status()) != TDSCHA_OK) return done(rc);
 #undef PCU
     return done(TDSCHA_OK);
 }

@@ -157,3 +157,22 @@ def test_bounded_wait_reports_timeout(gpu_lib, monkeypatch):
     f_ref, d_ref = oracle.perturb_averages(ens["X"], ens["Y"], ens["w"], ens["rho"], R1, Y1,
                                            ens["T"], 1, *_tables(ens, M))
     assert _rel(f, f_ref) <= TOL and _rel(d2v, d_ref) <= TOL
+
+
+@pytest.mark.parametrize("N,n,M", [(1, 3, 1), (127, 63, 60), (128, 64, 64), (129, 66, 65),
+                                   (300, 195, 190), (65541, 9, 6)])
+def test_projection_edges_against_oracle(gpu_lib, N, n, M):
+    """X and Y of the mode projection; the oracle's products round n <= 195 terms in
+    float64, at most 195 2^-53 = 2e-14 of the largest entry."""
+    from tdscha_gb300.preprocessing import project_modes
+    rng = np.random.default_rng(N + n)
+    u, f = rng.standard_normal((N, n)), 1e-3 * rng.standard_normal((N, n))
+    masses, mean = rng.uniform(1e3, 2e5, n), f.mean(0)
+    pols = np.linalg.qr(rng.standard_normal((n, max(M, 1))))[0][:, :M]
+    got = project_modes(u, f, masses, pols, mean, u_scale=0.5, f_scale=2.0)
+    ref = oracle.project_modes(u, f, masses, pols, mean, 0.5, 2.0)
+    for a, b in zip(got, ref):
+        assert _rel(a, b) <= 1e-13
+    u[0, 1] = np.nan
+    X, Y = project_modes(u, f, masses, pols, mean, u_scale=0.5, f_scale=2.0)
+    assert np.isnan(X[0]).all() and np.isfinite(X[1:]).all() and np.isfinite(Y).all()
