@@ -356,13 +356,13 @@ class QSpaceLanczos(Lanczos):
             raise ValueError("Must call build_q_pair_map (or prepare_mode_q) first")
         pkey = (self.iq_pert, self.q_pair_map.tobytes(), bool(self.ignore_harmonic),
                 bool(self.ignore_v3), bool(self.ignore_v4))
+        self._qctx.set_precision(self.precision)
         if self._qpert_key != pkey:
             P = self._qctx.set_pert(self.iq_pert, self.q_pair_map, self.ignore_harmonic,
                                     self.ignore_v3, self.ignore_v4)
             if P != self.get_psi_size():
                 raise AssertionError("psi layout mismatch")
             self._qpert_key = pkey
-        self._qctx.set_precision(self.precision)
         return self._qctx
 
     def _invalidate(self):

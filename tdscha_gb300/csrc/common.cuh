@@ -73,6 +73,7 @@ struct MixedStore {
 
 namespace tdscha {
 struct DigitStore;   // perturb_digits.cu
+struct QDigitStore;  // qspace_digits.cu
 }
 
 struct tdscha_ctx {
@@ -190,6 +191,7 @@ struct tdscha_qctx {
     double *dots = nullptr, *scal = nullptr, *hist_dev = nullptr, *stat_dev = nullptr;
     double *stat_host = nullptr, *pqn = nullptr, *rcoef = nullptr;
     int hist_cap = 0;
+    tdscha::QDigitStore *qd = nullptr;   // float64 averages by digit products (null: CUDA cores)
 };
 
 namespace tdscha {
@@ -244,6 +246,12 @@ int apply_full_L_dev(tdscha_ctx *c, const double *psi_in, double *psi_out, int t
                      int precision, cudaStream_t st);
 // qspace.cu
 int q_apply_full_L_dev(tdscha_qctx *c, const double *psi_in, double *psi_out, cudaStream_t st);
+// qspace_digits.cu
+void qdigits_release(tdscha_qctx *c);
+int qdigits_set_pert(tdscha_qctx *c);
+bool qdigits_ready(const tdscha_qctx *c);
+int qdigits_perturb(tdscha_qctx *c, int apply_d4, cudaStream_t st);
+int qdigits_check_error(tdscha_qctx *c);
 // preprocess.cu
 int apply_translation_projection(tdscha_ctx *c, cudaStream_t st);
 void free_translations(tdscha_ctx *c);

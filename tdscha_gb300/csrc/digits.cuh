@@ -5,6 +5,7 @@
 
 #include <algorithm>
 #include <climits>
+#include <cmath>
 
 #include "common.cuh"
 #include "tcgen05.cuh"
@@ -122,6 +123,98 @@ __device__ __forceinline__ double fixed_to_double(long long hi, long long lo, in
 // 2^e for the exponents of finite float64 rows
 __device__ __forceinline__ double pow2(int e) { return ldexp(1.0, e); }
 
+__device__ __forceinline__ void atomic_max_abs(unsigned long long *addr, double v) {
+    // absolute values order like their bit patterns (NaN above infinity)
+    atomicMax(addr, (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffULL);
+}
+
+
+// Sums of the squares of each digit over the 64 elements of a block's row, from
+// the eight lanes that hold it: nrm[digit * rows + row].
+__device__ __forceinline__ void digit_norms(const uint4 (&w)[kRes], int c, float *__restrict__ nrm,
+                                            int rows, int row) {
+#pragma unroll
+    for (int d = 0; d < kRes; ++d) {
+        const uint32_t v[4] = {w[d].x, w[d].y, w[d].z, w[d].w};
+        float s = 0.f;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&v[k]));
+            s = fmaf(f.x, f.x, fmaf(f.y, f.y, s));
+        }
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (c == 0) nrm[d * rows + row] = s;
+    }
+}
+
+// out[L - 3][digit]: largest norm (squared) over the accumulations of L = 3 +
+// blockIdx.y blocks of any row; nrm[tile][block][digit][rows], thread = row.
+static __global__ void k_dg_windows(const float *__restrict__ nrm, int nkb, float *__restrict__ out) {
+    const float *p = nrm + blockIdx.x * (long)nkb * kRes * blockDim.x + threadIdx.x;
+    const int L = kFlushMin + blockIdx.y;
+    float mx[kRes] = {};
+    for (int kb = 0; kb < nkb; kb += L) {
+        float s[kRes] = {};
+        for (int k = kb; k < min(nkb, kb + L); ++k)
+#pragma unroll
+            for (int d = 0; d < kRes; ++d) s[d] += p[((long)k * kRes + d) * blockDim.x];
+#pragma unroll
+        for (int d = 0; d < kRes; ++d) mx[d] = fmaxf(mx[d], s[d]);
+    }
+#pragma unroll
+    for (int d = 0; d < kRes; ++d) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) mx[d] = fmaxf(mx[d], __shfl_xor_sync(0xffffffffu, mx[d], o));
+        // non-negative floats order like their bit patterns
+        if ((threadIdx.x & 31) == 0)
+            atomicMax(reinterpret_cast<int *>(out + blockIdx.y * kRes + d), __float_as_int(mx[d]));
+    }
+}
+
+// The longest accumulation (K blocks) that keeps orders 0..4 below 2^24 for any
+// per-call operand: mx[L - 3][i] is the largest squared norm of digit i over L
+// blocks.  The other operand's digits are at most 64 (the first) and 128.
+inline int digits_flush(const float *mx) {
+    for (int L = kFlushMax; L > kFlushMin; --L) {
+        bool fits = true;
+        for (int o = 0; o <= 4 && fits; ++o) {
+            double sum = 0;
+            for (int i = 0; i <= o; ++i)
+                sum += std::sqrt((double)mx[(L - kFlushMin) * kRes + i] * kGK * L) *
+                       (i == o ? 64.0 : 128.0);
+            fits = sum <= 16777216.0;
+        }
+        if (fits) return L;
+    }
+    return kFlushMin;
+}
+
+// K blocks per split of a split-K contraction (of nkb blocks, accumulations of
+// `flush`) with `nat` A and `nbt` B tiles on `nsm` SMs: the fewest waves weighted
+// with what a wave costs: 4900 cycles a K block (35 products of 128 x 64 x 64 at
+// 4096 a cycle, and a tenth), 8000 to fill the ring and to write the tile; and the
+// partial tiles written and read again (both at about 3 KB a cycle).
+inline int dg_blocks_per_split(long nkb, int flush, int nat, int nbt, int nsm) {
+    const long tiles = (long)nat * nbt;
+    const double part = 16.0 * tiles * kGM * kGN / 3000.0;
+    double best = 1e300;
+    int kb_best = (int)nkb;
+    for (long n = 1; n <= std::min<long>(nkb, 96); ++n) {
+        long kb = (nkb + n - 1) / n;
+        // whole accumulations where a split has several
+        if (kb > flush) kb = (kb + flush - 1) / flush * flush;
+        const long ns = (nkb + kb - 1) / kb;
+        if (kb > 16384) continue;             // 64-bit sums of the orders
+        const double cost = (double)((tiles * ns + nsm - 1) / nsm) * (kb * 4900.0 + 8000.0) + part * ns;
+        if (cost < best * 0.999) {
+            best = cost;
+            kb_best = (int)kb;
+        }
+    }
+    return kb_best;
+}
+
 // -------------------------------------------------------- the contraction
 // Persistent, one CTA per SM, 512 threads, one 128 x 64 output tile at a time;
 // its accumulators, eight orders of 64 columns, fill the TMEM.
@@ -148,9 +241,9 @@ __device__ __forceinline__ double pow2(int e) { return ldexp(1.0, e); }
 // 12000 (stage A: two float64 products an element on the float64 pipe).  With 48
 // images stage A (976 us at M=189, N=10000) is bound by that pipe and the epilogue.
 // The copies (176 KB a K block) take 3700 cycles of a block's 4500 and do not show.
-// What becomes of a tile: row dots (stage A), split-K partials (stage B), or the
-// product itself
-enum { DG_DOTS = 0, DG_PARTS, DG_STORE };
+// What becomes of a tile: row dots (stage A), split-K partials (stage B), the
+// product itself, or the complex row dots of Bloch space (qspace_digits.cu)
+enum { DG_DOTS = 0, DG_PARTS, DG_STORE, DG_QDOTS };
 
 struct DgArgs {
     const __half *a, *b;
@@ -158,6 +251,14 @@ struct DgArgs {
     int kbps;              // K blocks per work item (stage A: nkb)
     int flush;             // K blocks per accumulation
     int nat, nbt;          // A and B tiles
+    // tiles that are partly empty:
+    int kk;                // 16-element steps of a K block
+    int hc;                // columns of an epilogue half: 32, or 16 with at most 32 in use
+    uint32_t abytes;       // bytes of one digit of an A block: kGA, or 1024 for every eight
+                           // rows of tiles with fewer (the others stay zero in shared memory)
+    // B tile of work item (at, bt): bt, or bmap[at] + bt.  The A tile is at (Bloch-space
+    // dots: bt nat + at)
+    const int *bmap;
     long nitems;
     int Mp;
     int *err;
@@ -168,12 +269,15 @@ struct DgArgs {
     double *qp;            // [image][column tile][4][R]
     long R;
     int nct;               // column tiles of one image
+    const int *cofs;       // Bloch-space dots: 4 o + kind of a tile column, whose x and g
+    int nr;                // begin at column (of 128 rows) o + nr x row tile of dt and gt
     // stage B
     const int *ec, *ew;
     double *gpart;         // [split][A rows][Mp]: H[b][a]
     int M;                 // columns in use (of an image)
-    long rows_b;           // rows (image, mode) in use
-    // product: out[R][M], row exponents er
+    int rmod, rlive;       // of the A rows, those with row % rmod < rlive ...
+    long rows_b;           // ... and row < rows_b are in use
+    // product: out[R][M], row exponents er (also of the Bloch-space dots, by A tile)
     const int *er;
     double *out;
 };
@@ -191,8 +295,8 @@ struct DgShape {
     static constexpr uint32_t bbytes = SB * kGB;
     static constexpr int bars = 2 * slots + 4 + 1 + kOrders + 1;
     static constexpr size_t ring = 2 * (size_t)bbytes + slots * (size_t)kGA;
-    static constexpr size_t smem = 1024 + ring + 2 * 2 * 128 * sizeof(double) +
-                                   2 * kGN * sizeof(int) + 8 * bars + 16;
+    static constexpr size_t smem = 1024 + ring + 2 * 4 * 128 * sizeof(double) +
+                                   4 * kGN * sizeof(int) + 8 * bars + 16;
 };
 static_assert(DgShape<DG_DOTS>::smem <= 232448 && DgShape<DG_PARTS>::smem <= 232448,
               "shared memory above the per-block limit");
@@ -211,17 +315,21 @@ __device__ __forceinline__ bool dg_sync_or(bool pred) {
     return out != 0;
 }
 
-template <int kMode>
+// kPart: tiles that are partly empty (kk, hc, abytes), the sizes of a full tile are
+// constants otherwise (read from the arguments they cost the M=573 call 3%)
+template <int kMode, bool kPart>
 __global__ void __launch_bounds__(kGThreads, 1) k_dg_gemm(const DgArgs args) {
+    const int hc = kPart ? args.hc : 32;
+    const uint32_t abytes = kPart ? args.abytes : kGA;
     using Sh = DgShape<kMode>;
     constexpr int SA = Sh::SA, SB = Sh::SB, slots = Sh::slots;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>(
         (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t *ring = smem + 2 * Sh::bbytes;
-    double *red = reinterpret_cast<double *>(smem + Sh::ring);        // [2][2][128]
-    int *cole = reinterpret_cast<int *>(red + 2 * 2 * 128);            // [2][64]
-    uint64_t *bars = reinterpret_cast<uint64_t *>(cole + 2 * kGN);
+    double *red = reinterpret_cast<double *>(smem + Sh::ring);        // [2][4][128]
+    int *cole = reinterpret_cast<int *>(red + 2 * 4 * 128);   // [2][64], offsets [2][64]
+    uint64_t *bars = reinterpret_cast<uint64_t *>(cole + 4 * kGN);
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + Sh::bars);
     volatile int *abort = reinterpret_cast<volatile int *>(tmem_slot + 1);
     const uint32_t afull = smem_u32(bars), aempty = afull + 8 * slots, bfull = aempty + 8 * slots,
@@ -244,6 +352,11 @@ __global__ void __launch_bounds__(kGThreads, 1) k_dg_gemm(const DgArgs args) {
         mbar_init(done, 1);
         *abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (kPart && abytes < kGA) {
+        for (uint32_t o = 16 * threadIdx.x; o < slots * kGA; o += 16 * kGThreads)
+            *reinterpret_cast<uint4 *>(ring + o) = make_uint4(0, 0, 0, 0);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     if (warp == 9) tmem_alloc<512>(smem_u32(tmem_slot));
@@ -288,6 +401,8 @@ __global__ void __launch_bounds__(kGThreads, 1) k_dg_gemm(const DgArgs args) {
             --left;
         }
     };
+    auto a_tile = [&](const Item &w) { return kMode == DG_QDOTS ? w.bt * args.nat + w.at : w.at; };
+    auto b_tile = [&](const Item &w) { return args.bmap ? args.bmap[w.at] + w.bt : w.bt; };
     // a ring's slot and the parity of its use
     struct Cursor {
         int s = 0;
@@ -309,9 +424,9 @@ __global__ void __launch_bounds__(kGThreads, 1) k_dg_gemm(const DgArgs args) {
             for (Item w(args); w.left > 0 && !fail_code; w.next()) {
                 const int kb0 = w.split * args.kbps, nkb = min(args.kbps, args.nkb - kb0);
                 const uint8_t *pa = reinterpret_cast<const uint8_t *>(args.a) +
-                                    ((long)w.at * args.nkb + kb0) * SA * (long)kGA;
+                                    ((long)a_tile(w) * args.nkb + kb0) * SA * (long)abytes;
                 const uint8_t *pb = reinterpret_cast<const uint8_t *>(args.b) +
-                                    ((long)w.bt * args.nkb + kb0) * SB * (long)kGB;
+                                    ((long)b_tile(w) * args.nkb + kb0) * SB * (long)kGB;
                 for (int kb = 0; kb < nkb && !fail_code; ++kb) {
                     if (gb >= 2 && !mbar_wait_ab(bempty + 8 * cb.s, cb.ph ^ 1, budget, abort)) {
                         fail_code = 1;
@@ -330,12 +445,12 @@ __global__ void __launch_bounds__(kGThreads, 1) k_dg_gemm(const DgArgs args) {
                             fail_code = 1;
                             break;
                         }
-                        mbar_expect_tx(afull + 8 * ca.s, kGA);
-                        bulk_load(smem_u32(ring + ca.s * kGA), pa + d * (long)kGA, kGA,
-                                  afull + 8 * ca.s);
+                        mbar_expect_tx(afull + 8 * ca.s, abytes);
+                        bulk_load(smem_u32(ring + ca.s * kGA), pa + d * (long)abytes,
+                                  abytes, afull + 8 * ca.s);
                         ca.next(slots);
                     }
-                    pa += SA * (long)kGA;
+                    pa += SA * (long)abytes;
                 }
             }
             if (fail_code) {
@@ -397,6 +512,7 @@ __global__ void __launch_bounds__(kGThreads, 1) k_dg_gemm(const DgArgs args) {
                         const int n1 = cnt > 4 ? (cnt + 1) / 2 : cnt;
 #pragma unroll
                         for (int kk = 0; kk < kGK / 16; ++kk) {
+                            if (kPart && kk >= args.kk) break;
                             // descriptor addresses count 16 bytes; the digits of B
                             // lie kGB apart
                             auto span = [&](int j0, int n, uint32_t acc) {
@@ -469,9 +585,11 @@ __global__ void __launch_bounds__(kGThreads, 1) k_dg_gemm(const DgArgs args) {
     }
     } else {
         regs_inc<kGRegsEpi>();
-        const int quad = warp & 3, half = warp >> 2;
+        const int quad = warp & 3, half = warp >> 2;   // half: columns c0 .. c0 + hc - 1
         const int row = quad * 32 + lane;
-        const uint32_t base = tmem + ((uint32_t)(quad * 32) << 16) + 32 * half;
+        const bool full = hc > 16;
+        const int c0 = half * hc;
+        const uint32_t base = tmem + ((uint32_t)(quad * 32) << 16) + c0;
         uint32_t nch = 0;
         bool bad = false;            // a wait of this warp gave up
         int i = 0;
@@ -480,8 +598,9 @@ __global__ void __launch_bounds__(kGThreads, 1) k_dg_gemm(const DgArgs args) {
             const int nkb = min(args.kbps, args.nkb - w.split * args.kbps);
             int *ce = cole + (i & 1) * kGN;
             if (threadIdx.x < kGN) {
-                const long c = (long)bt * kGN + threadIdx.x;
+                const long c = (long)b_tile(w) * kGN + threadIdx.x;
                 ce[threadIdx.x] = (kMode == DG_PARTS ? args.ec[c] : args.et[c]) + kUnit;
+                if (kMode == DG_QDOTS) ce[2 * kGN + threadIdx.x] = args.cofs[c] + 4 * at * args.nr;
             }
             const int nacc = (nkb + args.flush - 1) / args.flush;
             // An accumulator |a| <= 2^22 becomes a whole number by adding 1.5 2^23:
@@ -522,14 +641,14 @@ __global__ void __launch_bounds__(kGThreads, 1) k_dg_gemm(const DgArgs args) {
                 };
                 auto order = [&](int o, uint32_t w, long long(&acc)[32]) {
                     tmem_wait_ld();
-                    tmem_ld16(base + kGN * o + 16, v[1]);
+                    if (full) tmem_ld16(base + kGN * o + 16, v[1]);
                     add(v[0], w, acc);
-                    tmem_wait_ld();
+                    if (full) tmem_wait_ld();
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(tempty + 8 * o);
                     if (o > 0) tmem_ld16(base + kGN * (o - 1), v[0]);
-                    add(v[1], w, acc + 16);
+                    if (full) add(v[1], w, acc + 16);
                 };
 #pragma unroll 1
                 for (int k = 0; k < 4; ++k) order(7 - k, 1u << (8 * k), lo);
@@ -541,7 +660,6 @@ __global__ void __launch_bounds__(kGThreads, 1) k_dg_gemm(const DgArgs args) {
                 fail_code = 3;
                 break;
             }
-            const int c0 = half * 32;
             if (kMode == DG_DOTS) {
                 const long tile = ((long)at * args.Mp + (long)(bt % args.nct) * kGN + c0) * 128 + row;
                 const double *pd = args.dt + tile, *pg = args.gt + tile;
@@ -552,7 +670,8 @@ __global__ void __launch_bounds__(kGThreads, 1) k_dg_gemm(const DgArgs args) {
                     d[e] = pd[e * 128];
                     g[e] = pg[e * 128];
                 }
-                const int ncol = args.M - (bt % args.nct) * kGN - c0;    // the rest is padding
+                // the rest is padding
+                const int ncol = min(hc, args.M - (bt % args.nct) * kGN - c0);
 #pragma unroll
                 for (int e0 = 0; e0 < 32; e0 += 8) {
                     if (e0 >= ncol) break;
@@ -570,7 +689,7 @@ __global__ void __launch_bounds__(kGThreads, 1) k_dg_gemm(const DgArgs args) {
                         }
                     }
                 }
-                double *rb = red + (i & 1) * 2 * 128 + row;
+                double *rb = red + (i & 1) * 4 * 128 + row;
                 if (half) {
                     rb[0] = q;
                     rb[128] = p;
@@ -582,10 +701,73 @@ __global__ void __launch_bounds__(kGThreads, 1) k_dg_gemm(const DgArgs args) {
                     o[0] = q + rb[0];
                     o[args.R] = p + rb[128];
                 }
+            } else if (kMode == DG_QDOTS) {
+                // columns 2 n, 2 n + 1 are Re and Im of a band of u: sum conj(x) u and
+                // sum conj(u) g.  Of the former the second member of a pair (kind 2) has
+                // the conjugate of the first's (kind 1): twice that one's real part.
+                const int *co = ce + 2 * kGN + c0;
+                const double *px = args.dt + row, *pg = args.gt + row;
+                const int ncol = min(hc, args.M - c0);
+                double tr = 0, ti = 0, t2 = 0, br = 0, bi = 0, x[8], g[8];
+                auto load = [&](int e0) {
+#pragma unroll
+                    for (int e = 0; e < 8; e += 2) {
+                        const long o = (co[e0 + e] >> 2) * 128L;
+                        x[e] = px[o];
+                        x[e + 1] = px[o + 128];
+                        g[e] = pg[o];
+                        g[e + 1] = pg[o + 128];
+                    }
+                };
+                load(0);
+#pragma unroll
+                for (int e0 = 0; e0 < 32; e0 += 8) {
+                    if (e0 >= ncol) break;
+                    double v[8];
+#pragma unroll
+                    for (int e = 0; e < 8; ++e)
+                        v[e] = fixed_to_double(hi[e0 + e], lo[e0 + e], ce[c0 + e0 + e]);
+#pragma unroll
+                    for (int e = 0; e < 8; e += 2) {
+                        const int kind = co[e0 + e] & 3;
+                        if (kind == 0) {
+                            tr = fma(x[e], v[e], tr);
+                            tr = fma(x[e + 1], v[e + 1], tr);
+                            ti = fma(x[e], v[e + 1], ti);
+                            ti = fma(-x[e + 1], v[e], ti);
+                        } else if (kind == 1) {
+                            t2 = fma(x[e], v[e], t2);
+                            t2 = fma(x[e + 1], v[e + 1], t2);
+                        }
+                        br = fma(g[e], v[e], br);
+                        br = fma(g[e + 1], v[e + 1], br);
+                        bi = fma(g[e + 1], v[e], bi);
+                        bi = fma(-g[e], v[e + 1], bi);
+                    }
+                    if (e0 < 24) load(e0 + 8);
+                }
+                tr = fma(2.0, t2, tr);
+                double *rb = red + (i & 1) * 4 * 128 + row;
+                if (half) {
+                    rb[0] = tr;
+                    rb[128] = ti;
+                    rb[256] = br;
+                    rb[384] = bi;
+                }
+                asm volatile("bar.sync 1, 256;" ::: "memory");
+                const long r = (long)at * kGM + row;
+                if (!half && r < args.R) {
+                    const double f = pow2(args.er[(long)a_tile(w) * kGM + row]);
+                    double *o = args.qp + (long)bt * 4 * args.R + r;
+                    o[0] = (tr + rb[0]) * f;
+                    o[args.R] = (ti + rb[128]) * f;
+                    o[2 * args.R] = (br + rb[256]) * f;
+                    o[3 * args.R] = (bi + rb[384]) * f;
+                }
             } else if (kMode == DG_STORE) {
                 const long r = (long)at * kGM + row;
                 if (r < args.R) {
-                    const int er = args.er[r], ncol = args.M - bt * kGN - c0;
+                    const int er = args.er[r], ncol = min(hc, args.M - bt * kGN - c0);
                     double *o = args.out + r * args.M + (long)bt * kGN + c0;
 #pragma unroll
                     for (int e = 0; e < 32; ++e) {
@@ -595,13 +777,12 @@ __global__ void __launch_bounds__(kGThreads, 1) k_dg_gemm(const DgArgs args) {
                 }
             } else {
                 const long grow = (long)at * kGM + row;
-                const int b = (int)(grow % args.Mp);
-                const bool live = grow < args.rows_b && b < args.M;
+                const bool live = grow < args.rows_b && (int)(grow % args.rmod) < args.rlive;
                 if (live) {
                     const int eb = args.ew[grow];
                     double *o = args.gpart + ((long)w.split * args.nat * kGM + grow) * args.Mp +
                                 (long)bt * kGN + c0;
-                    const int ncol = args.M - bt * kGN - c0;
+                    const int ncol = min(hc, args.M - bt * kGN - c0);
 #pragma unroll
                     for (int e = 0; e < 32; e += 2) {
                         if (e >= ncol) break;
@@ -624,6 +805,19 @@ __global__ void __launch_bounds__(kGThreads, 1) k_dg_gemm(const DgArgs args) {
         tc_fence_after();
         tmem_dealloc<512>(tmem);
     }
+}
+
+template <int kMode, bool kPart>
+inline cudaError_t dg_setup() {
+    return cudaFuncSetAttribute(k_dg_gemm<kMode, kPart>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)DgShape<kMode>::smem);
+}
+
+// kk, hc and abytes of tiles that are partly empty, of full ones otherwise
+template <int kMode, bool kPart>
+inline cudaError_t dg_launch(const DgArgs &a, int nsm, cudaStream_t st) {
+    return launch_pdl(k_dg_gemm<kMode, kPart>, (int)std::min<long>(a.nitems, nsm), kGThreads,
+                      DgShape<kMode>::smem, st, a);
 }
 
 }  // namespace tdscha

@@ -1699,7 +1699,7 @@ extern "C" int tdscha_qlanczos_run(tdscha_qctx *ctx, double *basis_Q, double *ba
         set_error("qlanczos_run: %s", cudaGetErrorString(cudaGetLastError()));
         rc = TDSCHA_ERR_CUDA;
     }
-    return rc;
+    return rc == TDSCHA_OK ? qdigits_check_error(ctx) : rc;
 }
 
 // Many independent runs together (real-space and q-space contexts mixed): each
@@ -1789,7 +1789,9 @@ extern "C" int tdscha_lanczos_run_batch(tdscha_run *runs, int n_runs) {
             double *sh = r.kind == 0 ? ((tdscha_ctx *)r.ctx)->stat_host : ((tdscha_qctx *)r.ctx)->stat_host;
             int e = read_back_steps(hd, sd, sh, r.capacity, next[i], k, streams[i], r.hist,
                                     r.start_step, &r.steps_done, &r.converged, &stop);
-            if (e == TDSCHA_OK && r.kind == 0) e = mixed_check_error((tdscha_ctx *)r.ctx);
+            if (e == TDSCHA_OK)
+                e = r.kind == 0 ? mixed_check_error((tdscha_ctx *)r.ctx)
+                                : qdigits_check_error((tdscha_qctx *)r.ctx);
             if (e != TDSCHA_OK) { fail(i, e); continue; }
             next[i] = k + 1;
             if (stop || done[i] >= r.n_iter) active[i] = false;

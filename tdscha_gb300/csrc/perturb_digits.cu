@@ -66,11 +66,6 @@ struct __align__(32) RowScalars {
 };
 
 // ------------------------------------------------- once per ensemble
-__device__ __forceinline__ void atomic_max_abs(unsigned long long *addr, double v) {
-    // absolute values order like their bit patterns (NaN above infinity)
-    atomicMax(addr, (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffULL);
-}
-
 // Column maxima of |x| and |g|.
 __global__ void k_dg_colmax(const double *__restrict__ D, const double *__restrict__ F,
                             const double *__restrict__ fY, long R, int M, long rows_per_block,
@@ -143,49 +138,6 @@ __global__ void k_dg_rowexp(const double *__restrict__ dt, const int *__restrict
     if (g == 0) {
         for (int k = 1; k < 8; ++k) e = max(e, sh[k][row]);
         er[rt * 128 + row] = e == INT_MIN ? 0 : e;
-    }
-}
-
-// Sums of the squares of each digit over the 64 elements of a block's row, from
-// the eight lanes that hold it: nrm[digit * rows + row].
-__device__ __forceinline__ void digit_norms(const uint4 (&w)[kRes], int c, float *__restrict__ nrm,
-                                            int rows, int row) {
-#pragma unroll
-    for (int d = 0; d < kRes; ++d) {
-        const uint32_t v[4] = {w[d].x, w[d].y, w[d].z, w[d].w};
-        float s = 0.f;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&v[k]));
-            s = fmaf(f.x, f.x, fmaf(f.y, f.y, s));
-        }
-#pragma unroll
-        for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (c == 0) nrm[d * rows + row] = s;
-    }
-}
-
-// out[L - 3][digit]: largest norm (squared) over the accumulations of L = 3 +
-// blockIdx.y blocks of any row; nrm[tile][block][digit][rows], thread = row.
-__global__ void k_dg_windows(const float *__restrict__ nrm, int nkb, float *__restrict__ out) {
-    const float *p = nrm + blockIdx.x * (long)nkb * kRes * blockDim.x + threadIdx.x;
-    const int L = kFlushMin + blockIdx.y;
-    float mx[kRes] = {};
-    for (int kb = 0; kb < nkb; kb += L) {
-        float s[kRes] = {};
-        for (int k = kb; k < min(nkb, kb + L); ++k)
-#pragma unroll
-            for (int d = 0; d < kRes; ++d) s[d] += p[((long)k * kRes + d) * blockDim.x];
-#pragma unroll
-        for (int d = 0; d < kRes; ++d) mx[d] = fmaxf(mx[d], s[d]);
-    }
-#pragma unroll
-    for (int d = 0; d < kRes; ++d) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) mx[d] = fmaxf(mx[d], __shfl_xor_sync(0xffffffffu, mx[d], o));
-        // non-negative floats order like their bit patterns
-        if ((threadIdx.x & 31) == 0)
-            atomicMax(reinterpret_cast<int *>(out + blockIdx.y * kRes + d), __float_as_int(mx[d]));
     }
 }
 
@@ -535,49 +487,6 @@ struct DigitStore {
     long long budget = kDefaultBudget;
 };
 
-// K blocks per split of stage B for `nat` W tiles: the fewest waves of 152 SMs
-// weighted with what a wave costs: 4900 cycles a K block (35 products of 128 x 64
-// x 64 at 4096 a cycle, and a tenth), 8000 to fill the ring and to write the
-// tile; and the partial tiles written and read again (both at about 3 KB a cycle).
-static int dg_blocks_per_split(const DigitStore *x, int nat) {
-    const long tiles = (long)nat * x->nct, nkb = x->nkbR;
-    const double part = 16.0 * nat * kGM * x->Mp / 3000.0;
-    double best = 1e300;
-    int kb_best = (int)nkb;
-    for (long n = 1; n <= std::min<long>(nkb, 96); ++n) {
-        long kb = (nkb + n - 1) / n;
-        // whole accumulations where a split has several
-        if (kb > x->flushB) kb = (kb + x->flushB - 1) / x->flushB * x->flushB;
-        const long ns = (nkb + kb - 1) / kb;
-        if (kb > 16384) continue;             // 64-bit sums of the orders
-        const double cost = (double)((tiles * ns + x->nsm - 1) / x->nsm) * (kb * 4900.0 + 8000.0) +
-                            part * ns;
-        if (cost < best * 0.999) {
-            best = cost;
-            kb_best = (int)kb;
-        }
-    }
-    return kb_best;
-}
-
-// The longest accumulation (K blocks) that keeps orders 0..4 below 2^24 for any
-// per-call operand: mx[L - 3][i] is the largest squared norm of digit i over L
-// blocks.  The other operand's digits are at most 64 (the first) and 128.
-static int digits_flush(const float *mx) {
-    for (int L = kFlushMax; L > kFlushMin; --L) {
-        bool fits = true;
-        for (int o = 0; o <= 4 && fits; ++o) {
-            double sum = 0;
-            for (int i = 0; i <= o; ++i)
-                sum += std::sqrt((double)mx[(L - kFlushMin) * kRes + i] * kGK * L) *
-                       (i == o ? 64.0 : 128.0);
-            fits = sum <= 16777216.0;
-        }
-        if (fits) return L;
-    }
-    return kFlushMin;
-}
-
 void digits_release(tdscha_ctx *c) {
     if (!c->dg) return;
     cached_free(c->dg->slab);
@@ -624,7 +533,7 @@ int digits_prepare(tdscha_ctx *c) {
     size_t gbytes = 0;
     for (x->flushB = kFlushMax; ; --x->flushB) {      // ends at kFlushMin, its value until measured
         for (int n = 1; n <= cap; ++n) {
-            const int na = ceil_div((long)n * Mp, kGM), kb = dg_blocks_per_split(x, na);
+            const int na = ceil_div((long)n * Mp, kGM), kb = dg_blocks_per_split(x->nkbR, x->flushB, na, x->nct, x->nsm);
             gbytes = std::max(gbytes, (size_t)ceil_div(x->nkbR, kb) * na * kGM * Mp * sizeof(double));
         }
         if (x->flushB == kFlushMin) break;
@@ -717,10 +626,10 @@ int digits_prepare(tdscha_ctx *c) {
     x->flushA = digits_flush(h_fl);
     x->flushB = digits_flush(h_fl + kFlushes * kRes);
     TDS_CUDA(cudaFuncSetAttribute(k_dg_y1, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    TDS_CUDA(cudaFuncSetAttribute(k_dg_gemm<DG_DOTS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)DgShape<DG_DOTS>::smem));
-    TDS_CUDA(cudaFuncSetAttribute(k_dg_gemm<DG_PARTS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)DgShape<DG_PARTS>::smem));
+    TDS_CUDA((dg_setup<DG_DOTS, false>()));
+    TDS_CUDA((dg_setup<DG_DOTS, true>()));
+    TDS_CUDA((dg_setup<DG_PARTS, false>()));
+    TDS_CUDA((dg_setup<DG_PARTS, true>()));
     return TDSCHA_OK;
 }
 
@@ -750,6 +659,9 @@ static int digits_contract(tdscha_ctx *c, int nimg, const DgSources &src, int ap
     ga.b = x->yb;
     ga.nkb = ga.kbps = x->nkbM;
     ga.flush = x->flushA;
+    ga.kk = ceil_div(M, 16);             // (read where M <= 64)
+    ga.hc = M <= 32 ? 16 : 32;
+    ga.abytes = kGA;
     ga.nat = (int)(x->Rp / kGM);
     ga.nbt = nimg * x->nct;
     ga.nitems = (long)ga.nat * ga.nbt;
@@ -767,8 +679,8 @@ static int digits_contract(tdscha_ctx *c, int nimg, const DgSources &src, int ap
     ga.M = M;
     {
         ProfScope ps(c, 0, st);
-        TDS_CUDA(launch_pdl(k_dg_gemm<DG_DOTS>, (int)std::min<long>(ga.nitems, x->nsm), kGThreads,
-                            DgShape<DG_DOTS>::smem, st, ga));
+        TDS_CUDA((M <= kGK ? dg_launch<DG_DOTS, true>(ga, x->nsm, st)
+                           : dg_launch<DG_DOTS, false>(ga, x->nsm, st)));
     }
     {
         ProfScope ps(c, 1, st);
@@ -791,8 +703,11 @@ static int digits_contract(tdscha_ctx *c, int nimg, const DgSources &src, int ap
     gb.a = x->wa;
     gb.b = x->xb;
     gb.nkb = (int)x->nkbR;
-    gb.kbps = dg_blocks_per_split(x, nat);
+    gb.kbps = dg_blocks_per_split(x->nkbR, x->flushB, nat, x->nct, x->nsm);
     gb.flush = x->flushB;
+    gb.kk = kGK / 16;
+    gb.hc = M <= 32 ? 16 : 32;
+    gb.abytes = kGA;
     gb.nat = nat;
     gb.nbt = x->nct;
     *nsplit = ceil_div(x->nkbR, gb.kbps);
@@ -804,10 +719,12 @@ static int digits_contract(tdscha_ctx *c, int nimg, const DgSources &src, int ap
     gb.ew = x->ew;
     gb.gpart = x->gpart;
     gb.M = M;
+    gb.rmod = Mp;
+    gb.rlive = M;
     gb.rows_b = (long)nimg * Mp;
     ProfScope ps(c, 3, st);
-    TDS_CUDA(launch_pdl(k_dg_gemm<DG_PARTS>, (int)std::min<long>(gb.nitems, x->nsm), kGThreads,
-                        DgShape<DG_PARTS>::smem, st, gb));
+    TDS_CUDA((M <= 32 ? dg_launch<DG_PARTS, true>(gb, x->nsm, st)
+                      : dg_launch<DG_PARTS, false>(gb, x->nsm, st)));
     return TDSCHA_OK;
 }
 

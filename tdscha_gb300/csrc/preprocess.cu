@@ -250,8 +250,7 @@ struct DigitProduct {
 
     int set_b(const double *B) {
         TDS_CUDA(cudaMemsetAsync(err, 0, sizeof(int), 0));
-        TDS_CUDA(cudaFuncSetAttribute(k_dg_gemm<DG_STORE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)DgShape<DG_STORE>::smem));
+        TDS_CUDA((dg_setup<DG_STORE, false>()));
         k_dg_slice_cols<<<nbt * kGN, 128>>>(B, K, n, nkb, b, et);
         TDS_CHECK_LAUNCH();
         return TDSCHA_OK;
@@ -277,8 +276,7 @@ struct DigitProduct {
             g.R = nr;
             g.M = n;
             g.out = C + r0 * n;
-            TDS_CUDA(launch_pdl(k_dg_gemm<DG_STORE>, (int)std::min<long>(g.nitems, nsm), kGThreads,
-                                DgShape<DG_STORE>::smem, (cudaStream_t)0, g));
+            TDS_CUDA((dg_launch<DG_STORE, false>(g, nsm, (cudaStream_t)0)));
         }
         return TDSCHA_OK;
     }

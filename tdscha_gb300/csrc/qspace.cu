@@ -567,6 +567,7 @@ static int q_perturb_t(tdscha_qctx *c, int apply_d4, const T2 *Xr, const T2 *Yr,
 }
 
 static int q_perturb(tdscha_qctx *c, int apply_d4, cudaStream_t st) {
+    if (c->precision != TDSCHA_PREC_MIXED && qdigits_ready(c)) return qdigits_perturb(c, apply_d4, st);
     if (c->precision != TDSCHA_PREC_MIXED)
         return q_perturb_t<double2>(c, apply_d4, c->Xr, c->Yr, c->fY, c->fpsi, c->R1, c->alpha,
                                     c->rowc, st);
@@ -602,6 +603,7 @@ int q_apply_full_L_dev(tdscha_qctx *c, const double *psi_in, double *psi_out, cu
 
 static void q_free(tdscha_qctx *c) {
     if (!c) return;
+    qdigits_release(c);
     void *bufs[] = {c->Xr, c->Yr, c->fY, c->fpsi, c->rho, c->qpair, c->qrole, c->qpartner,
                     c->pair_q, c->elem, c->pcoef, c->mask, c->q_off, c->wpert, c->R1, c->alpha,
                     c->f, c->d2v, c->rowc, c->fpart, c->dpart, c->Lq, c->rk, c->sk, c->dots,
@@ -748,6 +750,7 @@ extern "C" int tdscha_qctx_set_pert(tdscha_qctx *ctx, int iq_pert, const int *q_
     ctx->ignore_v3 = ignore_v3 != 0;
     ctx->ignore_v4 = ignore_v4 != 0;
     TDS_TRY(q_build_layout(ctx, q_pair_map));
+    TDS_TRY(qdigits_set_pert(ctx));
     if (psi_size) *psi_size = ctx->P;
     if (n_pairs) *n_pairs = ctx->n_pairs;
     return TDSCHA_OK;
@@ -770,7 +773,10 @@ extern "C" int tdscha_qperturb_averages(tdscha_qctx *ctx, const double *R1, cons
     TDS_TRY(q_perturb(ctx, apply_d4, st));
     TDS_CUDA(cudaMemcpyAsync(f_out, ctx->f, sizeof(double2) * nb, outk, st));
     TDS_CUDA(cudaMemcpyAsync(d2v_out, ctx->d2v, sizeof(double2) * nbl, outk, st));
-    if (!device_ptrs) TDS_CUDA(cudaStreamSynchronize(st));
+    if (!device_ptrs) {
+        TDS_CUDA(cudaStreamSynchronize(st));
+        TDS_TRY(qdigits_check_error(ctx));
+    }
     return TDSCHA_OK;
 }
 
@@ -810,6 +816,8 @@ extern "C" int tdscha_qctx_set_precision(tdscha_qctx *ctx, int precision) {
     if (precision == TDSCHA_PREC_MIXED && ctx->n_pairs > 0 && !ctx->alpha32)
         TDS_CUDA(cudaMalloc(&ctx->alpha32, sizeof(float2) * (size_t)ctx->n_pairs * ctx->nb *
                                                ctx->nb));
+    const bool change = ctx->precision != precision;
     ctx->precision = precision;
+    if (change && ctx->n_pairs > 0) TDS_TRY(qdigits_set_pert(ctx));
     return TDSCHA_OK;
 }
