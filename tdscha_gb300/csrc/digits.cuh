@@ -253,7 +253,7 @@ struct DgArgs {
     int nat, nbt;          // A and B tiles
     // tiles that are partly empty:
     int kk;                // 16-element steps of a K block
-    int hc;                // columns of an epilogue half: 32, or 16 with at most 32 in use
+    int hc;                // columns of an epilogue warp: 16, or 8 with at most 32 in use
     uint32_t abytes;       // bytes of one digit of an A block: kGA, or 1024 for every eight
                            // rows of tiles with fewer (the others stay zero in shared memory)
     // B tile of work item (at, bt): bt, or bmap[at] + bt.  The A tile is at (Bloch-space
@@ -282,10 +282,7 @@ struct DgArgs {
     double *out;
 };
 
-// 512 threads of 128 registers; the epilogue's two warpgroups take 192 of each
-// thread, the other two 64: 256 * 192 + 256 * 64 = 512 * 128.
-constexpr int kGThreads = 512, kGRegsEpi = 192, kGRegsRest = 64;
-static_assert(256 * kGRegsEpi + 256 * kGRegsRest == kGThreads * 128, "register shares");
+constexpr int kEpi = 16;           // epilogue warps
 
 template <int kMode>
 struct DgShape {
@@ -295,19 +292,25 @@ struct DgShape {
     static constexpr uint32_t bbytes = SB * kGB;
     static constexpr int bars = 2 * slots + 4 + 1 + kOrders + 1;
     static constexpr size_t ring = 2 * (size_t)bbytes + slots * (size_t)kGA;
-    static constexpr size_t smem = 1024 + ring + 2 * 4 * 128 * sizeof(double) +
+    // registers: 61440 at launch, of which the epilogue takes the larger share
+    static constexpr int threads = 32 * (kEpi + (kMode == DG_DOTS ? 8 : 4));
+    static constexpr int regs = 61440 / threads, epi = kMode == DG_DOTS ? 96 : 104,
+                         rest = kMode == DG_DOTS ? 48 : 64;
+    static_assert(32 * kEpi * epi + (threads - 32 * kEpi) * rest == threads * regs, "register shares");
+    static constexpr int sums = kMode == DG_QDOTS ? 4 : 2;      // of a row
+    static constexpr size_t smem = 1024 + ring + 3 * sums * 128 * sizeof(double) +
                                    4 * kGN * sizeof(int) + 8 * bars + 16;
 };
-static_assert(DgShape<DG_DOTS>::smem <= 232448 && DgShape<DG_PARTS>::smem <= 232448,
+static_assert(DgShape<DG_QDOTS>::smem <= 232448 && DgShape<DG_PARTS>::smem <= 232448,
               "shared memory above the per-block limit");
 
-// Named barrier 1 over the 256 epilogue threads; true if `pred` was set in any.
+// Named barrier 1 over the 512 epilogue threads; true if `pred` was set in any.
 __device__ __forceinline__ bool dg_sync_or(bool pred) {
     uint32_t out;
     asm volatile(
         "{\n\t.reg .pred p, q;\n\t"
         "setp.ne.u32 p, %1, 0;\n\t"
-        "bar.red.or.pred q, 1, 256, p;\n\t"
+        "bar.red.or.pred q, 1, 512, p;\n\t"
         "selp.u32 %0, 1, 0, q;\n\t}"
         : "=r"(out)
         : "r"((uint32_t)pred)
@@ -318,8 +321,8 @@ __device__ __forceinline__ bool dg_sync_or(bool pred) {
 // kPart: tiles that are partly empty (kk, hc, abytes), the sizes of a full tile are
 // constants otherwise (read from the arguments they cost the M=573 call 3%)
 template <int kMode, bool kPart>
-__global__ void __launch_bounds__(kGThreads, 1) k_dg_gemm(const DgArgs args) {
-    const int hc = kPart ? args.hc : 32;
+__global__ void __launch_bounds__(DgShape<kMode>::threads, 1) k_dg_gemm(const DgArgs args) {
+    const int hc = kPart ? args.hc : 16;
     const uint32_t abytes = kPart ? args.abytes : kGA;
     using Sh = DgShape<kMode>;
     constexpr int SA = Sh::SA, SB = Sh::SB, slots = Sh::slots;
@@ -327,8 +330,8 @@ __global__ void __launch_bounds__(kGThreads, 1) k_dg_gemm(const DgArgs args) {
     uint8_t *smem = reinterpret_cast<uint8_t *>(
         (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t *ring = smem + 2 * Sh::bbytes;
-    double *red = reinterpret_cast<double *>(smem + Sh::ring);        // [2][4][128]
-    int *cole = reinterpret_cast<int *>(red + 2 * 4 * 128);   // [2][64], offsets [2][64]
+    double *red = reinterpret_cast<double *>(smem + Sh::ring);   // [sum][3][128]
+    int *cole = reinterpret_cast<int *>(red + 3 * Sh::sums * 128);   // [2][64], offsets [2][64]
     uint64_t *bars = reinterpret_cast<uint64_t *>(cole + 4 * kGN);
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + Sh::bars);
     volatile int *abort = reinterpret_cast<volatile int *>(tmem_slot + 1);
@@ -348,18 +351,18 @@ __global__ void __launch_bounds__(kGThreads, 1) k_dg_gemm(const DgArgs args) {
             mbar_init(bempty + 8 * s, 1);
         }
         mbar_init(tfull, 1);
-        for (int o = 0; o < kOrders; ++o) mbar_init(tempty + 8 * o, 8);
+        for (int o = 0; o < kOrders; ++o) mbar_init(tempty + 8 * o, kEpi);
         mbar_init(done, 1);
         *abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     if (kPart && abytes < kGA) {
-        for (uint32_t o = 16 * threadIdx.x; o < slots * kGA; o += 16 * kGThreads)
+        for (uint32_t o = 16 * threadIdx.x; o < slots * kGA; o += 16 * Sh::threads)
             *reinterpret_cast<uint4 *>(ring + o) = make_uint4(0, 0, 0, 0);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    if (warp == 9) tmem_alloc<512>(smem_u32(tmem_slot));
+    if (warp == kEpi + 1) tmem_alloc<512>(smem_u32(tmem_slot));
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -415,9 +418,9 @@ __global__ void __launch_bounds__(kGThreads, 1) k_dg_gemm(const DgArgs args) {
         }
     };
 
-    if (warp >= 8) {
-    regs_dec<kGRegsRest>();
-    if (warp == 8) {
+    if (warp >= kEpi) {
+    regs_dec<Sh::rest>();
+    if (warp == kEpi) {
         if (lane == 0) {
             Cursor ca, cb;
             long ga = 0, gb = 0;             // copies issued
@@ -462,7 +465,7 @@ __global__ void __launch_bounds__(kGThreads, 1) k_dg_gemm(const DgArgs args) {
                     mbar_wait(bfull + 8 * (int)(g & 1), (uint32_t)(g >> 1) & 1, kDefaultBudget);
             }
         }
-    } else if (warp == 9) {
+    } else if (warp == kEpi + 1) {
         {
             // the whole warp runs the loop, one lane issues
             const uint32_t one = elect_one();
@@ -548,12 +551,12 @@ __global__ void __launch_bounds__(kGThreads, 1) k_dg_gemm(const DgArgs args) {
             if (fail_code) *abort = 1;
             mma_commit_one(one, done);
         }
-    } else if (warp >= 12) {
+    } else if (warp >= kEpi + 4) {
         if (kMode == DG_DOTS) {
             // thread = row: its partial s and t over the tile's 64 modes, beside
             // the matrix work (in the epilogue these two products an element kept
             // the float64 pipe for longer than the tile's MMAs run)
-            const int row = (warp - 12) * 32 + lane;
+            const int row = (warp - kEpi - 4) * 32 + lane;
             for (Item w(args); w.left > 0; w.next()) {
                 const int at = w.at, bt = w.bt;
                 const long tile = ((long)at * args.Mp + (long)(bt % args.nct) * kGN) * 128 + row;
@@ -584,11 +587,11 @@ __global__ void __launch_bounds__(kGThreads, 1) k_dg_gemm(const DgArgs args) {
         }
     }
     } else {
-        regs_inc<kGRegsEpi>();
-        const int quad = warp & 3, half = warp >> 2;   // half: columns c0 .. c0 + hc - 1
+        regs_inc<Sh::epi>();
+        const int quad = warp & 3, part = warp >> 2;   // part: columns c0 .. c0 + hc - 1
         const int row = quad * 32 + lane;
-        const bool full = hc > 16;
-        const int c0 = half * hc;
+        const bool full = hc > 8;
+        const int c0 = part * hc;
         const uint32_t base = tmem + ((uint32_t)(quad * 32) << 16) + c0;
         uint32_t nch = 0;
         bool bad = false;            // a wait of this warp gave up
@@ -609,10 +612,10 @@ __global__ void __launch_bounds__(kGThreads, 1) k_dg_gemm(const DgArgs args) {
             // run at an eighth of this rate and took as long as an accumulation's
             // read may take.)
             constexpr uint32_t kMagic = 0x4B400000u;
-            long long hi[32], lo[32];
+            long long hi[16], lo[16];
             const long long start = -(long long)nacc * (long long)((uint64_t)kMagic * 0x01010101u);
 #pragma unroll
-            for (int e = 0; e < 32; ++e) hi[e] = lo[e] = start;
+            for (int e = 0; e < 16; ++e) hi[e] = lo[e] = start;
             for (int c = 0; c < nacc; ++c, ++nch) {
                 if (!bad && !mbar_all(tfull, nch & 1, budget, abort)) {
                     bad = true;
@@ -620,35 +623,32 @@ __global__ void __launch_bounds__(kGThreads, 1) k_dg_gemm(const DgArgs args) {
                 }
                 if (bad) continue;
                 tc_fence_after();
-                // Half an order (16 columns) at a time, the next half's read on its
-                // way while one is added.  Rolled: a small call runs this code once.
-                uint32_t v[2][16];
-                tmem_ld16(base + kGN * (kOrders - 1), v[0]);
-                auto add = [&](const uint32_t(&x)[16], uint32_t w, long long *acc) {
-                    uint32_t b[16], over = 0;
+                // Rolled: a small call runs this code once.
+                uint32_t v[16];
+                auto add = [&](uint32_t w, long long *acc, int e0) {
+                    uint32_t over = 0, b[8];
 #pragma unroll
-                    for (int e = 0; e < 16; ++e) {
-                        b[e] = __float_as_uint(__uint_as_float(x[e]) + 12582912.f);
+                    for (int e = 0; e < 8; ++e) {
+                        b[e] = __float_as_uint(__uint_as_float(v[e0 + e]) + 12582912.f);
                         over |= b[e] ^ 0x4B000000u;
                     }
                     if (__any_sync(0xffffffffu, over >> 23)) {
 #pragma unroll
-                        for (int e = 0; e < 16; ++e)
-                            b[e] = kMagic + (uint32_t)__float2int_rn(__uint_as_float(x[e]));
+                        for (int e = 0; e < 8; ++e)
+                            b[e] = kMagic + (uint32_t)__float2int_rn(__uint_as_float(v[e0 + e]));
                     }
 #pragma unroll
-                    for (int e = 0; e < 16; ++e) acc[e] += (long long)((uint64_t)b[e] * w);
+                    for (int e = 0; e < 8; ++e) acc[e0 + e] += (long long)((uint64_t)b[e] * w);
                 };
-                auto order = [&](int o, uint32_t w, long long(&acc)[32]) {
+                auto order = [&](int o, uint32_t w, long long(&acc)[16]) {
+                    if (full) tmem_ld16(base + kGN * o, v);
+                    else tmem_ld8(base + kGN * o, v);
                     tmem_wait_ld();
-                    if (full) tmem_ld16(base + kGN * o + 16, v[1]);
-                    add(v[0], w, acc);
-                    if (full) tmem_wait_ld();
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(tempty + 8 * o);
-                    if (o > 0) tmem_ld16(base + kGN * (o - 1), v[0]);
-                    if (full) add(v[1], w, acc + 16);
+                    add(w, acc, 0);
+                    if (full) add(w, acc, 8);
                 };
 #pragma unroll 1
                 for (int k = 0; k < 4; ++k) order(7 - k, 1u << (8 * k), lo);
@@ -663,43 +663,43 @@ __global__ void __launch_bounds__(kGThreads, 1) k_dg_gemm(const DgArgs args) {
             if (kMode == DG_DOTS) {
                 const long tile = ((long)at * args.Mp + (long)(bt % args.nct) * kGN + c0) * 128 + row;
                 const double *pd = args.dt + tile, *pg = args.gt + tile;
-                // eight modes' x and g on the way while the eight before are used
-                double q = 0, p = 0, d[8], g[8];
+                // four modes' x and g on the way while the four before are used
+                double q = 0, p = 0, d[4], g[4];
 #pragma unroll
-                for (int e = 0; e < 8; ++e) {
+                for (int e = 0; e < 4; ++e) {
                     d[e] = pd[e * 128];
                     g[e] = pg[e * 128];
                 }
                 // the rest is padding
                 const int ncol = min(hc, args.M - (bt % args.nct) * kGN - c0);
 #pragma unroll
-                for (int e0 = 0; e0 < 32; e0 += 8) {
+                for (int e0 = 0; e0 < 16; e0 += 4) {
                     if (e0 >= ncol) break;
-                    double v[8];
+                    double v[4];
 #pragma unroll
-                    for (int e = 0; e < 8; ++e)
+                    for (int e = 0; e < 4; ++e)
                         v[e] = fixed_to_double(hi[e0 + e], lo[e0 + e], ce[c0 + e0 + e]);
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) {
+                    for (int e = 0; e < 4; ++e) {
                         q = fma(d[e], v[e], q);
                         p = fma(g[e], v[e], p);
-                        if (e0 < 24) {
-                            d[e] = pd[(e0 + 8 + e) * 128];
-                            g[e] = pg[(e0 + 8 + e) * 128];
+                        if (e0 < 12) {
+                            d[e] = pd[(e0 + 4 + e) * 128];
+                            g[e] = pg[(e0 + 4 + e) * 128];
                         }
                     }
                 }
-                double *rb = red + (i & 1) * 4 * 128 + row;
-                if (half) {
-                    rb[0] = q;
-                    rb[128] = p;
+                double *rb = red + row;
+                if (part) {
+                    rb[(part - 1) * 128] = q;
+                    rb[(part + 2) * 128] = p;
                 }
-                asm volatile("bar.sync 1, 256;" ::: "memory");
+                asm volatile("bar.sync 1, 512;" ::: "memory");
                 const long r = (long)at * kGM + row;
-                if (!half && r < args.R) {
+                if (!part && r < args.R) {
                     double *o = args.qp + (long)bt * 4 * args.R + r;
-                    o[0] = q + rb[0];
-                    o[args.R] = p + rb[128];
+                    o[0] = (q + rb[0]) + (rb[128] + rb[256]);
+                    o[args.R] = (p + rb[384]) + (rb[512] + rb[640]);
                 }
             } else if (kMode == DG_QDOTS) {
                 // columns 2 n, 2 n + 1 are Re and Im of a band of u: sum conj(x) u and
@@ -708,10 +708,10 @@ __global__ void __launch_bounds__(kGThreads, 1) k_dg_gemm(const DgArgs args) {
                 const int *co = ce + 2 * kGN + c0;
                 const double *px = args.dt + row, *pg = args.gt + row;
                 const int ncol = min(hc, args.M - c0);
-                double tr = 0, ti = 0, t2 = 0, br = 0, bi = 0, x[8], g[8];
+                double tr = 0, ti = 0, t2 = 0, br = 0, bi = 0, x[4], g[4];
                 auto load = [&](int e0) {
 #pragma unroll
-                    for (int e = 0; e < 8; e += 2) {
+                    for (int e = 0; e < 4; e += 2) {
                         const long o = (co[e0 + e] >> 2) * 128L;
                         x[e] = px[o];
                         x[e + 1] = px[o + 128];
@@ -721,14 +721,14 @@ __global__ void __launch_bounds__(kGThreads, 1) k_dg_gemm(const DgArgs args) {
                 };
                 load(0);
 #pragma unroll
-                for (int e0 = 0; e0 < 32; e0 += 8) {
+                for (int e0 = 0; e0 < 16; e0 += 4) {
                     if (e0 >= ncol) break;
-                    double v[8];
+                    double v[4];
 #pragma unroll
-                    for (int e = 0; e < 8; ++e)
+                    for (int e = 0; e < 4; ++e)
                         v[e] = fixed_to_double(hi[e0 + e], lo[e0 + e], ce[c0 + e0 + e]);
 #pragma unroll
-                    for (int e = 0; e < 8; e += 2) {
+                    for (int e = 0; e < 4; e += 2) {
                         const int kind = co[e0 + e] & 3;
                         if (kind == 0) {
                             tr = fma(x[e], v[e], tr);
@@ -744,25 +744,29 @@ __global__ void __launch_bounds__(kGThreads, 1) k_dg_gemm(const DgArgs args) {
                         bi = fma(g[e + 1], v[e], bi);
                         bi = fma(-g[e], v[e + 1], bi);
                     }
-                    if (e0 < 24) load(e0 + 8);
+                    if (e0 < 12) load(e0 + 4);
                 }
                 tr = fma(2.0, t2, tr);
-                double *rb = red + (i & 1) * 4 * 128 + row;
-                if (half) {
-                    rb[0] = tr;
-                    rb[128] = ti;
-                    rb[256] = br;
-                    rb[384] = bi;
+                double *rb = red + row;
+                if (part) {
+                    double *o = rb + (part - 1) * 128;
+                    o[0] = tr;
+                    o[384] = ti;
+                    o[768] = br;
+                    o[1152] = bi;
                 }
-                asm volatile("bar.sync 1, 256;" ::: "memory");
+                asm volatile("bar.sync 1, 512;" ::: "memory");
                 const long r = (long)at * kGM + row;
-                if (!half && r < args.R) {
+                if (!part && r < args.R) {
                     const double f = pow2(args.er[(long)a_tile(w) * kGM + row]);
                     double *o = args.qp + (long)bt * 4 * args.R + r;
-                    o[0] = (tr + rb[0]) * f;
-                    o[args.R] = (ti + rb[128]) * f;
-                    o[2 * args.R] = (br + rb[256]) * f;
-                    o[3 * args.R] = (bi + rb[384]) * f;
+                    auto all = [&](double s, int k) {
+                        return ((s + rb[384 * k]) + (rb[384 * k + 128] + rb[384 * k + 256])) * f;
+                    };
+                    o[0] = all(tr, 0);
+                    o[args.R] = all(ti, 1);
+                    o[2 * args.R] = all(br, 2);
+                    o[3 * args.R] = all(bi, 3);
                 }
             } else if (kMode == DG_STORE) {
                 const long r = (long)at * kGM + row;
@@ -770,7 +774,7 @@ __global__ void __launch_bounds__(kGThreads, 1) k_dg_gemm(const DgArgs args) {
                     const int er = args.er[r], ncol = min(hc, args.M - bt * kGN - c0);
                     double *o = args.out + r * args.M + (long)bt * kGN + c0;
 #pragma unroll
-                    for (int e = 0; e < 32; ++e) {
+                    for (int e = 0; e < 16; ++e) {
                         if (e >= ncol) break;
                         o[e] = fixed_to_double(hi[e], lo[e], ce[c0 + e] + er);
                     }
@@ -784,7 +788,7 @@ __global__ void __launch_bounds__(kGThreads, 1) k_dg_gemm(const DgArgs args) {
                                 (long)bt * kGN + c0;
                     const int ncol = min(hc, args.M - bt * kGN - c0);
 #pragma unroll
-                    for (int e = 0; e < 32; e += 2) {
+                    for (int e = 0; e < 16; e += 2) {
                         if (e >= ncol) break;
                         double2 x;
                         x.x = fixed_to_double(hi[e], lo[e], ce[c0 + e] + eb);
@@ -799,7 +803,7 @@ __global__ void __launch_bounds__(kGThreads, 1) k_dg_gemm(const DgArgs args) {
     if (fail_code && lane == 0) *(volatile int *)args.err = 10 + fail_code;
     tc_fence_before();
     __syncthreads();
-    if (warp == 9) {
+    if (warp == kEpi + 1) {
         mbar_wait(done, 0, kDefaultBudget);
         __syncwarp();
         tc_fence_after();
@@ -816,8 +820,8 @@ inline cudaError_t dg_setup() {
 // kk, hc and abytes of tiles that are partly empty, of full ones otherwise
 template <int kMode, bool kPart>
 inline cudaError_t dg_launch(const DgArgs &a, int nsm, cudaStream_t st) {
-    return launch_pdl(k_dg_gemm<kMode, kPart>, (int)std::min<long>(a.nitems, nsm), kGThreads,
-                      DgShape<kMode>::smem, st, a);
+    return launch_pdl(k_dg_gemm<kMode, kPart>, (int)std::min<long>(a.nitems, nsm),
+                      DgShape<kMode>::threads, DgShape<kMode>::smem, st, a);
 }
 
 }  // namespace tdscha

@@ -660,7 +660,7 @@ static int digits_contract(tdscha_ctx *c, int nimg, const DgSources &src, int ap
     ga.nkb = ga.kbps = x->nkbM;
     ga.flush = x->flushA;
     ga.kk = ceil_div(M, 16);             // (read where M <= 64)
-    ga.hc = M <= 32 ? 16 : 32;
+    ga.hc = M <= 32 ? 8 : 16;
     ga.abytes = kGA;
     ga.nat = (int)(x->Rp / kGM);
     ga.nbt = nimg * x->nct;
@@ -706,7 +706,7 @@ static int digits_contract(tdscha_ctx *c, int nimg, const DgSources &src, int ap
     gb.kbps = dg_blocks_per_split(x->nkbR, x->flushB, nat, x->nct, x->nsm);
     gb.flush = x->flushB;
     gb.kk = kGK / 16;
-    gb.hc = M <= 32 ? 16 : 32;
+    gb.hc = M <= 32 ? 8 : 16;
     gb.abytes = kGA;
     gb.nat = nat;
     gb.nbt = x->nct;

@@ -658,7 +658,7 @@ int qdigits_perturb(tdscha_qctx *c, int apply_d4, cudaStream_t st) {
     a.b = x->yb;
     a.nkb = a.kbps = a.flush = 1;
     a.kk = ceil_div(live, 16);
-    a.hc = live <= 32 ? 16 : 32;
+    a.hc = live <= 32 ? 8 : 16;
     a.abytes = kGA;
     a.nat = (int)x->nrt;
     a.nbt = x->ngrp;
@@ -690,7 +690,7 @@ int qdigits_perturb(tdscha_qctx *c, int apply_d4, cudaStream_t st) {
     b.kbps = x->kbps;
     b.flush = x->flush;
     b.kk = kGK / 16;
-    b.hc = (x->nbq == 1 ? 2 * x->nr : x->nr) <= 32 ? 16 : 32;
+    b.hc = (x->nbq == 1 ? 2 * x->nr : x->nr) <= 32 ? 8 : 16;
     b.abytes = x->abytes;
     b.nat = x->n_pairs;
     b.nbt = x->nbq;
