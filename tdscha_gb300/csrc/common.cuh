@@ -245,12 +245,13 @@ int build_pair_coeffs(tdscha_ctx *c);
 int apply_full_L_dev(tdscha_ctx *c, const double *psi_in, double *psi_out, int transpose,
                      int precision, cudaStream_t st);
 // qspace.cu
+int q_averages_dev(tdscha_qctx *c, const double *psi_in, cudaStream_t st);
 int q_apply_full_L_dev(tdscha_qctx *c, const double *psi_in, double *psi_out, cudaStream_t st);
 // qspace_digits.cu
 void qdigits_release(tdscha_qctx *c);
 int qdigits_set_pert(tdscha_qctx *c);
 bool qdigits_ready(const tdscha_qctx *c);
-int qdigits_perturb(tdscha_qctx *c, int apply_d4, cudaStream_t st);
+int qdigits_perturb(tdscha_qctx *c, int apply_d4, const double *psi, cudaStream_t st);
 int qdigits_check_error(tdscha_qctx *c);
 // preprocess.cu
 int apply_translation_projection(tdscha_ctx *c, cudaStream_t st);

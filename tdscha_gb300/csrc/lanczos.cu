@@ -427,29 +427,38 @@ __device__ __forceinline__ double reduce_parts(const double *__restrict__ part, 
     return block_sum(v, sh);
 }
 
-// a = dot * p_norm and the axpy factors of the residuals (run_FT :6167-6232)
 // a = dot * p_norm and the axpy factors of the residuals (run_FT :6167-6232);
-// thread 0
+// one thread
+struct ScalA {
+    double a, pnorm, cq, cp;
+};
+__device__ __forceinline__ ScalA scal_a_value(double d, const double *hist, int k) {
+    ScalA v;
+    double c_old = k >= 1 ? hist[4 * (k - 1) + 2] : 1.0;
+    v.pnorm = hist[4 * k + 3] / c_old;
+    v.a = d * v.pnorm;
+    v.cq = v.cp = 0;
+    if (k >= 1) {
+        v.cq = hist[4 * (k - 1) + 2];
+        double old_p_norm = (k < 2) ? hist[4 * (k - 1) + 3] : hist[4 * (k - 1) + 3] / hist[4 * (k - 2) + 2];
+        v.cp = hist[4 * (k - 1) + 1] * (old_p_norm / v.pnorm);
+    }
+    return v;
+}
+__device__ __forceinline__ void scal_a_store(const ScalA &v, int k, double *scal, double *status) {
+    scal[SC_A] = v.a;
+    scal[SC_PNORM] = v.pnorm;
+    scal[SC_NAN] = isnan(v.a) ? 1.0 : 0.0;
+    status[k] = isnan(v.a) ? ST_NAN : ST_OK;
+    if (isnan(v.a)) scal[SC_HALT] = 1.0;
+    scal[SC_CQ] = v.cq;
+    scal[SC_CP] = v.cp;
+}
 __device__ __forceinline__ void scal_a_body(double d, const double *__restrict__ hist, int k,
                                             double *__restrict__ scal,
                                             double *__restrict__ status) {
     if (scal[SC_HALT] != 0.0) return;
-    double c_old = k >= 1 ? hist[4 * (k - 1) + 2] : 1.0;
-    double p_norm = hist[4 * k + 3] / c_old;
-    double a = d * p_norm;
-    scal[SC_A] = a;
-    scal[SC_PNORM] = p_norm;
-    scal[SC_NAN] = isnan(a) ? 1.0 : 0.0;
-    status[k] = isnan(a) ? ST_NAN : ST_OK;
-    if (isnan(a)) scal[SC_HALT] = 1.0;
-    double cq = 0, cp = 0;
-    if (k >= 1) {
-        cq = hist[4 * (k - 1) + 2];
-        double old_p_norm = (k < 2) ? hist[4 * (k - 1) + 3] : hist[4 * (k - 1) + 3] / hist[4 * (k - 2) + 2];
-        cp = hist[4 * (k - 1) + 1] * (old_p_norm / p_norm);
-    }
-    scal[SC_CQ] = cq;
-    scal[SC_CP] = cp;
+    scal_a_store(scal_a_value(d, hist, k), k, scal, status);
 }
 
 __global__ void k_scal_a(const double *__restrict__ part, int nblk, const double *__restrict__ hist,
@@ -545,34 +554,50 @@ __global__ void k_resid(const double *__restrict__ Lq, const double *__restrict_
     t = block_sum(sr, sh); if (threadIdx.x == 0) part[2 * nblk + blockIdx.x] = t;
 }
 
-// b, c, the new s_norm and the stop test (run_FT :6233-6306); thread 0
+// b, c, the new s_norm and the stop test (run_FT :6233-6306); one thread
+struct ScalBC {
+    double b, c, snorm, sraw, ib, is;
+    bool conv;
+};
+__device__ __forceinline__ ScalBC scal_bc_value(double ss, double rr, double sr, double pnorm,
+                                                double next) {
+    ScalBC v;
+    v.sraw = sqrt(ss);
+    v.snorm = v.sraw * pnorm;
+    v.b = sqrt(rr);
+    v.c = (sr / (v.sraw * v.b)) * v.snorm;
+    v.ib = 1.0 / v.b;
+    v.is = 1.0 / v.sraw;
+    v.conv = fabs(v.b) < kEps || fabs(v.c) < kEps || next != 0.0;
+    return v;
+}
+__device__ __forceinline__ void scal_bc_store(const ScalBC &v, double a, double *hist, int k,
+                                              double *scal, double *status) {
+    scal[SC_B] = v.b;
+    scal[SC_C] = v.c;
+    scal[SC_SNORM] = v.snorm;
+    scal[SC_SRAW] = v.sraw;
+    scal[SC_IB] = v.ib;
+    scal[SC_IS] = v.is;
+    scal[SC_CONV] = v.conv ? 1.0 : 0.0;
+    if (v.conv) {
+        status[k] = ST_CONV;
+        scal[SC_HALT] = 1.0;
+    }
+    hist[4 * k + 0] = a;
+    if (!v.conv) {
+        hist[4 * k + 1] = v.b;
+        hist[4 * k + 2] = v.c;
+        hist[4 * (k + 1) + 3] = v.snorm;
+    }
+}
 __device__ __forceinline__ void scal_bc_body(double ss, double rr, double sr,
                                              double *__restrict__ hist, int k,
                                              double *__restrict__ scal,
                                              double *__restrict__ status) {
     if (scal[SC_HALT] != 0.0) return;
-    double s_raw = sqrt(ss);
-    double s_norm = s_raw * scal[SC_PNORM];
-    double b = sqrt(rr);
-    double c = (sr / (s_raw * b)) * s_norm;
-    scal[SC_B] = b;
-    scal[SC_C] = c;
-    scal[SC_SNORM] = s_norm;
-    scal[SC_SRAW] = s_raw;
-    scal[SC_IB] = 1.0 / b;
-    scal[SC_IS] = 1.0 / s_raw;
-    bool conv = fabs(b) < kEps || fabs(c) < kEps || scal[SC_NEXT] != 0.0;
-    scal[SC_CONV] = conv ? 1.0 : 0.0;
-    if (conv) {
-        status[k] = ST_CONV;
-        scal[SC_HALT] = 1.0;
-    }
-    hist[4 * k + 0] = scal[SC_A];
-    if (!conv) {
-        hist[4 * k + 1] = b;
-        hist[4 * k + 2] = c;
-        hist[4 * (k + 1) + 3] = s_norm;
-    }
+    scal_bc_store(scal_bc_value(ss, rr, sr, scal[SC_PNORM], scal[SC_NEXT]), scal[SC_A], hist, k, scal,
+                  status);
 }
 
 __global__ void k_scal_bc(const double *__restrict__ part, int nblk, double *__restrict__ hist,
@@ -1125,6 +1150,234 @@ __global__ void k_qrenorm(const double *__restrict__ part, int nblk, double *__r
     }
 }
 
+// ---------------------------------------------------------------------------
+// Everything of a Hermitian (Bloch-space) step after the averages in one launch, for
+// short vectors: one cluster of blocks whose phases are separated by cluster barriers.
+// As thirteen launches of a few blocks each a step was bound by their starts and tails:
+// with the averages' kernels 142 -> 83 us
+// at 684 elements (12 steps of a 2x2x2 grid with 6 bands, N=2000).  Longer vectors, and more of them,
+// need more SMs than a cluster has.
+constexpr long kShortVector = 16384;          // elements: at most 64 blocks of partials
+constexpr int kShortBasis = 256;              // stored vectors
+constexpr long kShortSweep = 1L << 18;        // elements of all stored vectors
+
+struct RecurArgs {
+    // the operator on q (k_q_assemble)
+    const double *f, *d2v, *pcoef, *wpert;
+    const int *elem;
+    int nb, with_harm, with_anh;
+    double *Lq;
+    // the recurrence
+    const double *q, *p, *qprev, *pprev, *mask;
+    double *qn, *pn;
+    const double *Qb;
+    long n;                       // elements of a vector (and of a row of the basis)
+    int k, nblk, nvec, nch;       // nvec = 0: no re-orthogonalisation
+    double *rk, *sk, *scal, *part, *hist, *status, *pqn, *rpart;
+};
+
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::
+                     : "memory");
+}
+
+// block_sum of a group of 256 threads: its sum in the group's thread 0
+__device__ __forceinline__ double group_sum(double v, double *sh) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    const int bar = 1 + (threadIdx.x >> 8), tid = threadIdx.x & 255;
+    asm volatile("bar.sync %0, 256;" ::"r"(bar) : "memory");
+    if ((tid & 31) == 0) sh[tid >> 5] = v;
+    asm volatile("bar.sync %0, 256;" ::"r"(bar) : "memory");
+    double s = 0;
+    if (tid == 0)
+        for (int k = 0; k < 8; ++k) s += sh[k];
+    return s;
+}
+
+// Up to three sums of nblk <= 64 partials, part[s nblk ..], by the groups s; out[s] is
+// there after the next __syncthreads.
+__device__ __forceinline__ void sum_parts(const double *part, int nblk, int nsum, double (*sh)[8],
+                                          double *out) {
+    const int g = threadIdx.x >> 8, tid = threadIdx.x & 255, nw = (nblk + 31) / 32;
+    if (g < nsum && tid >> 5 < nw) {
+        double v = tid < nblk ? __ldcg(part + g * nblk + tid) : 0.0;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if ((tid & 31) == 0) sh[g][tid >> 5] = v;
+    }
+    __syncthreads();
+    if (g < nsum && tid == 0) {
+        double s = 0;
+        for (int k = 0; k < nw; ++k) s += sh[g][k];
+        out[g] = s;
+    }
+}
+
+// A group of 256 threads does what a block of k_dot1, k_resid, k_proj_dots ... does.
+// What another thread of the cluster wrote is read past the L1.
+__global__ void __launch_bounds__(1024, 1) k_qrecur(const RecurArgs r) {
+    __shared__ double sh[4][8], sums[4], cd[kShortBasis];
+    __shared__ ScalA sa;
+    __shared__ ScalBC sb;
+    pdl_enter();
+    int cta, ncta;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(cta));
+    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(ncta));
+    const int g = threadIdx.x >> 8, tid = threadIdx.x & 255, lane = threadIdx.x & 31,
+              warp = threadIdx.x >> 5;
+    const int v0 = g * ncta + cta, nv = 4 * ncta;
+    const long n = r.n, step = (long)r.nblk * 256;
+    const bool first = cta == 0 && threadIdx.x == 0;
+    if (__ldcg(r.scal + SC_HALT) != 0.0) return;          // (every thread of the cluster)
+    const double next = __ldcg(r.scal + SC_NEXT);
+
+    // An element of Lq, rk, sk, q_{k+1}, p_{k+1} is one thread's own throughout.
+    for (int vb = v0; vb < r.nblk; vb += nv) {
+        double acc = 0;
+        for (long e = vb * 256L + tid; e < n; e += step) {
+            const int code = r.elem[e >> 1], sector = code >> 28, i = (code >> 8) & 0xff;
+            double o = 0, v = r.q[e];
+            if (sector == 0) {
+                if (r.with_harm) o = v * r.wpert[i];
+                if (r.with_anh) o += r.f[2 * i + (e & 1)];
+            } else {
+                const long be = ((long)((code >> 16) & 0xfff) * r.nb + i) * r.nb + (code & 0xff);
+                const double *c = r.pcoef + be * 6;
+                if (r.with_harm) o = v * (sector == 1 ? c[0] : c[1]);
+                if (r.with_anh) o += r.d2v[2 * be + (e & 1)] * (sector == 1 ? c[4] : c[5]);
+            }
+            r.Lq[e] = o;
+            acc += r.p[e] * (o * r.mask[e]);
+        }
+        const double s = group_sum(acc, sh[g]);
+        if (tid == 0) r.part[vb] = s;
+    }
+    cluster_barrier();
+    sum_parts(r.part, r.nblk, 1, sh, sums);
+    if (threadIdx.x == 0) sa = scal_a_value(sums[0], r.hist, r.k);
+    __syncthreads();
+    if (first) scal_a_store(sa, r.k, r.scal, r.status);
+    if (isnan(sa.a)) return;
+    double *part2 = r.part + r.nblk;          // (the first sums may still be read)
+    for (int vb = v0; vb < r.nblk; vb += nv) {
+        double ss = 0, rr = 0, sr = 0;
+        for (long e = vb * 256L + tid; e < n; e += step) {
+            const double l = r.Lq[e], m = r.mask[e];
+            double a = l - sa.a * r.q[e], b = l - sa.a * r.p[e];
+            if (r.qprev) a -= sa.cq * r.qprev[e];
+            if (r.pprev) b -= sa.cp * r.pprev[e];
+            r.rk[e] = a;
+            r.sk[e] = b;
+            ss += b * (b * m);
+            rr += a * (a * m);
+            sr += b * (a * m);
+        }
+        double t;
+        t = group_sum(ss, sh[g]); if (tid == 0) part2[vb] = t;
+        t = group_sum(rr, sh[g]); if (tid == 0) part2[r.nblk + vb] = t;
+        t = group_sum(sr, sh[g]); if (tid == 0) part2[2 * r.nblk + vb] = t;
+    }
+    cluster_barrier();
+    sum_parts(part2, r.nblk, 3, sh, sums);
+    __syncthreads();
+    if (threadIdx.x == 0) sb = scal_bc_value(sums[0], sums[1], sums[2], sa.pnorm, next);
+    __syncthreads();
+    if (first) scal_bc_store(sb, sa.a, r.hist, r.k, r.scal, r.status);
+    if (sb.conv) return;
+    for (int vb = v0; vb < r.nblk; vb += nv)
+        for (long e = vb * 256L + tid; e < n; e += step) {
+            r.qn[e] = r.rk[e] * sb.ib;
+            r.pn[e] = r.sk[e] * sb.is;
+        }
+    if (r.nvec == 0) return;
+    cluster_barrier();
+    // one classical Gram-Schmidt pass of q_{k+1} (p_{k+1} becomes its copy)
+    for (int vb = v0; vb < r.nvec * r.nch; vb += nv) {
+        const int j = vb / r.nch, ch = vb % r.nch;
+        const double *qj = r.Qb + j * n;
+        const long e1 = n * (ch + 1) / r.nch;
+        double a = 0;
+        for (long e = n * ch / r.nch + tid; e < e1; e += 256)
+            a = fma(qj[e], __ldcg(r.qn + e) * r.mask[e], a);
+        const double t = group_sum(a, sh[g]);
+        if (tid == 0) r.rpart[vb] = t;
+    }
+    cluster_barrier();
+    // the coefficients, by every block for itself
+    for (int j = warp; j < r.nvec; j += 32) {
+        double s = 0;
+        for (int c = lane; c < r.nch; c += 32) s += __ldcg(r.rpart + j * r.nch + c);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) cd[j] = s / r.pqn[j];
+    }
+    __syncthreads();
+    for (int vb = v0; vb < r.nblk; vb += nv) {
+        double nn = 0;
+        for (long e = vb * 256L + tid; e < n; e += step) {
+            double q = r.qn[e];
+#pragma unroll 8
+            for (int j = 0; j < r.nvec; ++j) q = fma(-cd[j], r.Qb[j * n + e], q);
+            r.qn[e] = q;
+            nn += q * (q * r.mask[e]);
+        }
+        const double t = group_sum(nn, sh[g]);
+        if (tid == 0) r.part[vb] = t;
+    }
+    cluster_barrier();
+    // q_{k+1} / |q_{k+1}|, s_norm_{k+1} = c_k (QSpaceLanczos.py:1110-1125)
+    sum_parts(r.part, r.nblk, 1, sh, sums);
+    if (threadIdx.x == 0) {
+        const double nrm = sqrt(sums[0]);
+        sums[1] = 1.0 / nrm;
+        if (first) {
+            if (nrm < kEps) r.scal[SC_NEXT] = 1.0;
+            r.hist[4 * (r.k + 1) + 3] = sb.c;
+        }
+    }
+    __syncthreads();
+    const double iv = sums[1];
+    for (int vb = v0; vb < r.nblk; vb += nv) {
+        double nn = 0;
+        for (long e = vb * 256L + tid; e < n; e += step) {
+            const double v = r.qn[e] * iv;
+            r.qn[e] = v;
+            r.pn[e] = v;
+            nn = fma(v, v * r.mask[e], nn);
+        }
+        const double t = group_sum(nn, sh[g]);
+        if (tid == 0) part2[vb] = t;
+    }
+    cluster_barrier();
+    if (cta) return;
+    sum_parts(part2, r.nblk, 1, sh, sums);
+    if (first) r.pqn[r.k + 1] = sums[0];
+}
+
+inline bool short_vector(long n, int nvec) {
+    return n <= kShortVector && nvec <= kShortBasis && n * nvec <= kShortSweep;
+}
+
+static cudaError_t launch_qrecur(const RecurArgs &r, cudaStream_t st) {
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    // the portable limit: 1140 us a run of 12 steps with one block, 1063 with two, 1003
+    // with four, 1000 with eight
+    const unsigned c = 8;
+    attr[1].val.clusterDim.x = c;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = c;
+    cfg.blockDim = 1024;
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    return cudaLaunchKernelEx(&cfg, k_qrecur, r);
+}
+
 // Kernel polynomial method (QSpaceKPM.run_KPM, Modules/QSpaceKPM.py:260-454):
 // vp = 2 (L v - b v) / a - vm written over vm, and the moment finishers
 // moments[idx] = 2 <x, y>_M - moments[ref].
@@ -1623,6 +1876,18 @@ static int qz_step(tdscha_qctx *ctx, double *basis_Q, double *basis_P, int capac
     double *part = ctx->rcoef + 2 * (capacity + 1);
     double *q = basis_Q + (long)k * n, *p = basis_P + (long)k * n;
     // Hermitian operator: p_L = L q (QSpaceLanczos.py:1055-1057)
+    if (short_vector(n, reorthogonalize ? k + 1 : 0)) {
+        const int with_anh = !(ctx->ignore_v3 && ctx->ignore_v4);
+        if (with_anh) TDS_TRY(q_averages_dev(ctx, q, st));
+        RecurArgs r{(const double *)ctx->f, (const double *)ctx->d2v, ctx->pcoef, ctx->wpert, ctx->elem,
+                    ctx->nb, !ctx->ignore_harmonic, with_anh, ctx->Lq, q, p,
+                    k >= 1 ? q - n : nullptr, k >= 1 ? p - n : nullptr, mask, q + n, p + n, basis_Q, n,
+                    k, nb, reorthogonalize ? k + 1 : 0,
+                    reorthogonalize ? std::min(8, dot_chunks(n, k + 1)) : 0, ctx->rk, ctx->sk,
+                    ctx->scal, ctx->dots, ctx->hist_dev, ctx->stat_dev, ctx->pqn, part};
+        TDS_CUDA(launch_qrecur(r, st));
+        return TDSCHA_OK;
+    }
     TDS_TRY(q_apply_full_L_dev(ctx, q, ctx->Lq, st));
     k_dot1<<<nb, kDotThreads, 0, st>>>(p, ctx->Lq, mask, n, ctx->dots);
     k_scal_a<<<1, 256, 0, st>>>(ctx->dots, nb, ctx->hist_dev, k, ctx->scal, ctx->stat_dev);

@@ -17,9 +17,7 @@
 #include <cmath>
 #include <vector>
 
-#include "common.cuh"
-
-
+#include "qspace.cuh"
 
 namespace tdscha {
 
@@ -125,15 +123,6 @@ __global__ void k_q_expand(const double2 *__restrict__ X, const double2 *__restr
     }
 }
 
-// alpha1 blocks from psi (Wigner change of variables per pair element).
-// pcoef layout per pair element: [0] -(w1-w2)^2 vm, [1] -(w1+w2)^2 vm,
-// [2] w2X sqrt(-chi-/2), [3] w2X sqrt(chi+/2), [4] sqrt(-chi-/2), [5] -sqrt(chi+/2)
-__device__ __forceinline__ long q_store(int p, int i, int j, int nb, int full, const long *off) {
-    if (full) return off[p] + (long)i * nb + j;
-    // upper triangle rows from the diagonal, i <= j
-    return off[p] + (long)i * nb - (long)i * (i - 1) / 2 + (j - i);
-}
-
 __global__ void k_q_unpack(const double2 *__restrict__ psi, const int *__restrict__ pair_q,
                            const long *__restrict__ off_a, const long *__restrict__ off_b,
                            const double *__restrict__ pcoef, int n_pairs, int nb,
@@ -142,17 +131,7 @@ __global__ void k_q_unpack(const double2 *__restrict__ psi, const int *__restric
     for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < n; e += (long)gridDim.x * blockDim.x) {
         int p = (int)(e / (nb * nb));
         int i = (int)((e / nb) % nb), j = (int)(e % nb);
-        int full = pair_q[2 * p] < pair_q[2 * p + 1];
-        double2 a, b;
-        if (full || i <= j) {
-            a = psi[q_store(p, i, j, nb, full, off_a)];
-            b = psi[q_store(p, i, j, nb, full, off_b)];
-        } else {   // lower triangle of a Hermitian block
-            a = cconj(psi[q_store(p, j, i, nb, 0, off_a)]);
-            b = cconj(psi[q_store(p, j, i, nb, 0, off_b)]);
-        }
-        const double *c = pcoef + e * 6;
-        alpha[e] = make_double2(c[2] * a.x - c[3] * b.x, c[2] * a.y - c[3] * b.y);
+        alpha[e] = q_alpha1(psi, pair_q, off_a, off_b, pcoef, p, i, j, nb);
         if (e < nb) R1[e] = ignore_v3 ? make_double2(0, 0) : psi[e];
     }
 }
@@ -386,6 +365,7 @@ __global__ void k_q_assemble(const double2 *__restrict__ psi, const double2 *__r
                              const double *__restrict__ pcoef, const double *__restrict__ wpert,
                              long P, int nb, int with_harm, int with_anh,
                              double2 *__restrict__ out) {
+    pdl_enter();
     for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < P; e += (long)gridDim.x * blockDim.x) {
         int code = elem[e];
         int sector = code >> 28, p = (code >> 16) & 0xfff, i = (code >> 8) & 0xff, j = code & 0xff;
@@ -567,7 +547,8 @@ static int q_perturb_t(tdscha_qctx *c, int apply_d4, const T2 *Xr, const T2 *Yr,
 }
 
 static int q_perturb(tdscha_qctx *c, int apply_d4, cudaStream_t st) {
-    if (c->precision != TDSCHA_PREC_MIXED && qdigits_ready(c)) return qdigits_perturb(c, apply_d4, st);
+    if (c->precision != TDSCHA_PREC_MIXED && qdigits_ready(c))
+        return qdigits_perturb(c, apply_d4, nullptr, st);
     if (c->precision != TDSCHA_PREC_MIXED)
         return q_perturb_t<double2>(c, apply_d4, c->Xr, c->Yr, c->fY, c->fpsi, c->R1, c->alpha,
                                     c->rowc, st);
@@ -582,22 +563,26 @@ static int q_perturb(tdscha_qctx *c, int apply_d4, cudaStream_t st) {
                                c->alpha32, c->rowc32, st);
 }
 
-int q_apply_full_L_dev(tdscha_qctx *c, const double *psi_in, double *psi_out, cudaStream_t st) {
-    const int nb = c->nb;
-    const double2 *psi = reinterpret_cast<const double2 *>(psi_in);
-    int with_anh = !(c->ignore_v3 && c->ignore_v4);
-    if (with_anh) {
-        long n = (long)c->n_pairs * nb * nb;
-        k_q_unpack<<<std::max(1, std::min(ceil_div(n, 256), 1024)), 256, 0, st>>>(
-            psi, c->pair_q, c->q_off, c->q_off + c->n_pairs, c->pcoef, c->n_pairs, nb, c->ignore_v3,
-            c->R1, c->alpha);
-        TDS_CHECK_LAUNCH();
-        TDS_TRY(q_perturb(c, c->ignore_v4 ? 0 : 1, st));
-    }
-    k_q_assemble<<<std::max(1, std::min(ceil_div(c->P, 256), 4096)), 256, 0, st>>>(
-        psi, c->f, c->d2v, c->elem, c->pcoef, c->wpert, c->P, nb, !c->ignore_harmonic, with_anh,
-        reinterpret_cast<double2 *>(psi_out));
+// The averages of psi's perturbation into c->f, c->d2v
+int q_averages_dev(tdscha_qctx *c, const double *psi_in, cudaStream_t st) {
+    const int nb = c->nb, d4 = c->ignore_v4 ? 0 : 1;
+    if (c->precision != TDSCHA_PREC_MIXED && qdigits_ready(c)) return qdigits_perturb(c, d4, psi_in, st);
+    const long n = (long)c->n_pairs * nb * nb;
+    k_q_unpack<<<std::max(1, std::min(ceil_div(n, 256), 1024)), 256, 0, st>>>(
+        reinterpret_cast<const double2 *>(psi_in), c->pair_q, c->q_off, c->q_off + c->n_pairs, c->pcoef,
+        c->n_pairs, nb, c->ignore_v3, c->R1, c->alpha);
     TDS_CHECK_LAUNCH();
+    return q_perturb(c, d4, st);
+}
+
+int q_apply_full_L_dev(tdscha_qctx *c, const double *psi_in, double *psi_out, cudaStream_t st) {
+    int with_anh = !(c->ignore_v3 && c->ignore_v4);
+    if (with_anh) TDS_TRY(q_averages_dev(c, psi_in, st));
+    TDS_CUDA(launch_pdl(k_q_assemble, std::max(1, std::min(ceil_div(c->P, 256), 4096)), 256, 0, st,
+                        reinterpret_cast<const double2 *>(psi_in), (const double2 *)c->f,
+                        (const double2 *)c->d2v, (const int *)c->elem, (const double *)c->pcoef,
+                        (const double *)c->wpert, c->P, c->nb, (int)!c->ignore_harmonic, with_anh,
+                        reinterpret_cast<double2 *>(psi_out)));
     return TDSCHA_OK;
 }
 

@@ -16,13 +16,14 @@
 //           u2 and A2 with f2, are not needed and cost nothing: they fill a tile
 //           that would be empty.
 //
-// Measured (averages, one call): 4x4x4 grid, 12 bands, N=10000 2479 -> QAVG us.
+// Measured (averages, one call): 4x4x4 grid, 12 bands, N=10000 2479 -> 536 us.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <vector>
 
 #include "digits.cuh"
+#include "qspace.cuh"
 
 namespace tdscha {
 
@@ -207,8 +208,14 @@ __global__ void __launch_bounds__(256) k_qd_xb(const double *__restrict__ y,
 // (Re, -Im) and row 2 n + 1 (Im, Re) of complex row n.  The K axis carries the scales of
 // x's columns; outside x_k's the row is zero.  cofs: where x_q's column begins, and
 // whether q is its own partner, the first or the second of two.
-__global__ void __launch_bounds__(32) k_qd_alpha(const double2 *__restrict__ alpha,
-                                                 const int *__restrict__ qpair,
+struct QAlpha {                    // alpha1 itself, or the psi that it follows from
+    const double2 *alpha, *psi;
+    const int *pair_q;
+    const long *off;
+    const double *pcoef;
+    int n_pairs;
+};
+__global__ void __launch_bounds__(32) k_qd_alpha(const QAlpha src, const int *__restrict__ qpair,
                                                  const int *__restrict__ qrole,
                                                  const int *__restrict__ qpartner,
                                                  const int *__restrict__ ec, int nb, int G, int nrt,
@@ -218,19 +225,17 @@ __global__ void __launch_bounds__(32) k_qd_alpha(const double2 *__restrict__ alp
     __shared__ long long s[64];
     const int nr = 2 * nb, lane = threadIdx.x, grp = blockIdx.y / G, k0 = blockIdx.y % G * nr;
     const int q = qpartner[blockIdx.y], row = k0 + blockIdx.x, n = blockIdx.x >> 1;
-    const double2 *blk = alpha + (long)qpair[q] * nb * nb;
     const int *e2 = ec + grp * 64 + k0;
+    pdl_enter();
     s[lane] = s[lane + 32] = 0;
     __syncwarp();
     double v0 = 0, v1 = 0;                 // the two columns of band lane
     if (lane < nb) {
-        double2 a;
-        if (qrole[q] == 0) {
-            a = blk[n * nb + lane];
-        } else {
-            a = blk[lane * nb + n];
-            a.y = -a.y;
-        }
+        const int p = qpair[q], role = qrole[q], i = role ? lane : n, j = role ? n : lane;
+        double2 a = src.alpha ? src.alpha[((long)p * nb + i) * nb + j]
+                              : q_alpha1(src.psi, src.pair_q, src.off, src.off + src.n_pairs, src.pcoef,
+                                         p, i, j, nb);
+        if (role) a.y = -a.y;
         v0 = blockIdx.x & 1 ? a.y : a.x;
         v1 = blockIdx.x & 1 ? a.x : -a.y;
     }
@@ -278,6 +283,7 @@ __global__ void __launch_bounds__(256) k_qd_rows(const double *__restrict__ qp, 
     __shared__ double sum[8][4][64];
     const int part = threadIdx.x >> 6, i = threadIdx.x & 63;
     const long r = blockIdx.x * 64L + i;
+    pdl_enter();
     double s[8] = {};              // total, bfw, sum u conj(R1), sum y conj(R1)
     if (r < R) {
         const double *o = qp + 4 * part * R + r;
@@ -288,7 +294,7 @@ __global__ void __launch_bounds__(256) k_qd_rows(const double *__restrict__ qp, 
         const long base = (((long)iq_pert * nrt + (r >> 7)) * 2 * nb) * 128 + (r & 127);
 #pragma unroll 2
         for (int n = part; n < nb; n += 4) {
-            const double2 a = R1[n];
+            const double2 a = R1 ? R1[n] : make_double2(0, 0);
             const double ur = u[base + n * 256], ui = u[base + n * 256 + 128];
             const double yr = y[base + n * 256], yi = y[base + n * 256 + 128];
             s[4] = fma(ur, a.x, fma(ui, a.y, s[4]));
@@ -340,6 +346,7 @@ __global__ void __launch_bounds__(128) k_qd_wbuild(
     const int wide = max(1, 16 / nb);            // K blocks side by side
     const long kb0 = blockIdx.x * (long)per, kb1 = min(nkb, kb0 + per);
     const bool force = p == n_pairs;
+    pdl_enter();
     const int q1 = force ? iq_pert : pair_q[2 * p];
     if (force) {
         for (int n0 = 0; n0 < nb; n0 += 16) {
@@ -448,6 +455,7 @@ __global__ void __launch_bounds__(128) k_qd_final(const double *__restrict__ gpa
     const int nr = 2 * nb, ld = nbq * kGN, uc = nbq == 1 ? nr : kGN;
     const long n = (long)n_pairs * nb * nb, e = blockIdx.x * 16L + (threadIdx.x >> 3);
     const int k0 = threadIdx.x & 7;
+    pdl_enter();
     double re = 0, im = 0;
     double2 *out = nullptr;
     if (e < n) {
@@ -646,13 +654,17 @@ int qdigits_check_error(tdscha_qctx *c) {
     return TDSCHA_ERR_TIMEOUT;
 }
 
-// The averages of c->R1, c->alpha into c->f, c->d2v.
-int qdigits_perturb(tdscha_qctx *c, int apply_d4, cudaStream_t st) {
+// The averages of c->R1, c->alpha, or of psi's, into c->f, c->d2v.
+int qdigits_perturb(tdscha_qctx *c, int apply_d4, const double *psi, cudaStream_t st) {
     QDigitStore *x = c->qd;
     const int n_q = c->n_q, nb = c->nb, live = x->G * x->nr;
-    k_qd_alpha<<<dim3(x->nr, n_q), 32, 0, st>>>(c->alpha, c->qpair, c->qrole, c->qpartner, x->ec, nb,
-                                                x->G, (int)x->nrt, x->yb, x->et, x->cofs, x->absmax);
-    TDS_CHECK_LAUNCH();
+    const double2 *ps = reinterpret_cast<const double2 *>(psi);
+    const QAlpha src{ps ? nullptr : c->alpha, ps, c->pair_q, c->q_off, c->pcoef, c->n_pairs};
+    const double2 *R1 = !ps ? c->R1 : c->ignore_v3 ? nullptr : ps;
+    double2 *rowc = reinterpret_cast<double2 *>(x->rowc), *fpart = reinterpret_cast<double2 *>(x->fpart);
+    TDS_CUDA(launch_pdl(k_qd_alpha, dim3(x->nr, n_q), 32, 0, st, src, (const int *)c->qpair,
+                        (const int *)c->qrole, (const int *)c->qpartner, (const int *)x->ec, nb, x->G,
+                        (int)x->nrt, x->yb, x->et, x->cofs, x->absmax));
     DgArgs a{};
     a.a = x->xa;
     a.b = x->yb;
@@ -675,14 +687,14 @@ int qdigits_perturb(tdscha_qctx *c, int apply_d4, cudaStream_t st) {
     a.R = c->R;
     a.M = live;
     TDS_CUDA((dg_launch<DG_QDOTS, true>(a, x->nsm, st)));
-    k_qd_rows<<<(unsigned)x->nkb, 256, 0, st>>>(x->qp, x->ngrp, x->u, x->y, c->R1, c->rho, c->S, c->R,
-                                                x->nrt, nb, c->iq_pert, apply_d4, (double2 *)x->rowc,
-                                                x->absmax);
-    TDS_CHECK_LAUNCH();
-    k_qd_wbuild<<<dim3(x->nfc, x->n_pairs + 1), 128, 0, st>>>(
-        x->u, x->y, (const double2 *)x->rowc, x->absmax, x->umax, x->ymax, c->pair_q, x->n_pairs, nb,
-        c->iq_pert, x->nrt, x->nkb, x->per, x->abytes, x->wa, x->ew, (double2 *)x->fpart);
-    TDS_CHECK_LAUNCH();
+    TDS_CUDA(launch_pdl(k_qd_rows, (unsigned)x->nkb, 256, 0, st, (const double *)x->qp, x->ngrp,
+                        (const double *)x->u, (const double *)x->y, R1, (const double *)c->rho, c->S,
+                        c->R, x->nrt, nb, c->iq_pert, apply_d4, rowc, x->absmax));
+    TDS_CUDA(launch_pdl(k_qd_wbuild, dim3(x->nfc, x->n_pairs + 1), 128, 0, st, (const double *)x->u,
+                        (const double *)x->y, (const double2 *)rowc,
+                        (const unsigned long long *)x->absmax, (const unsigned long long *)x->umax,
+                        (const unsigned long long *)x->ymax, (const int *)c->pair_q, x->n_pairs, nb,
+                        c->iq_pert, x->nrt, x->nkb, x->per, x->abytes, x->wa, x->ew, fpart));
     DgArgs b{};
     b.a = x->wa;
     b.b = x->xb;
@@ -708,11 +720,9 @@ int qdigits_perturb(tdscha_qctx *c, int apply_d4, cudaStream_t st) {
     b.rows_b = (long)x->n_pairs * kGM;
     TDS_CUDA((dg_launch<DG_PARTS, true>(b, x->nsm, st)));
     const long n = (long)x->n_pairs * nb * nb + nb;
-    k_qd_final<<<ceil_div(n, 16), 128, 0, st>>>(x->gpart, x->ns, nb, x->n_pairs, x->nbq,
-                                                 (const double2 *)x->fpart, x->nfc,
-                                                 1.0 / (c->sum_rho * c->S), x->err, c->f,
-                                                 c->d2v);
-    TDS_CHECK_LAUNCH();
+    TDS_CUDA(launch_pdl(k_qd_final, ceil_div(n, 16), 128, 0, st, (const double *)x->gpart, x->ns, nb,
+                        x->n_pairs, x->nbq, (const double2 *)fpart, x->nfc,
+                        1.0 / (c->sum_rho * c->S), (const int *)x->err, c->f, c->d2v));
     return TDSCHA_OK;
 }
 

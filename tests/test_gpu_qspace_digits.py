@@ -132,3 +132,24 @@ def test_precision_and_perturbation_change(gpu_lib):
     again = lz.get_perturb_averages_q(R1, alpha, True)
     assert (first[0] == again[0]).all()
     assert all((x == y).all() for x, y in zip(first[1], again[1]))
+
+
+@pytest.mark.parametrize("dims,nb,N", [((1, 1, 1), 1, 40), ((2, 1, 1), 7, 60), ((2, 2, 1), 8, 60),
+                                       ((4, 2, 2), 22, 30), ((4, 2, 2), 23, 30)])
+@pytest.mark.parametrize("reorth", [False, True])
+def test_lanczos_vector_lengths(gpu_lib, dims, nb, N, reorth):
+    """The step in one launch (csrc/lanczos.cu, up to 16384 elements) and in several, on
+    both sides of its limit: the coefficients of the oracle up to a near-breakdown, to
+    1e-8: 1e-12 of an average, magnified by at most 1e4 = max|b| / b of the steps kept."""
+    _, lz, o, _, _ = _setup(dims, nb, N)
+    assert (2 * lz.get_psi_size() > 16384) == (nb == 23)
+    lz.prepare_mode_q(0, nb - 1)
+    o.psi[nb - 1] = 1.0
+    lz.run_FT(5, verbose=False, reorthogonalize=reorth)
+    o.run_FT(5, reorthogonalize=reorth)
+    b = np.abs(np.array(o.b_coeffs))
+    small = np.where(b < 1e-4 * b.max())[0] if len(b) else []
+    k = int(small[0]) + 1 if len(small) else len(b)
+    assert k >= min(5, len(o.b_coeffs)) - (nb == 1) * 4
+    for name in ("a_coeffs", "b_coeffs", "c_coeffs"):
+        np.testing.assert_allclose(getattr(lz, name)[:k], getattr(o, name)[:k], rtol=1e-8, atol=1e-14)
