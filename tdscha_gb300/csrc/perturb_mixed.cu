@@ -127,17 +127,17 @@ struct StageAArgs {
     long long budget;
 };
 
-// Named barrier 1 over the 128 epilogue threads; returns true if `pred` was
-// set in any of them.
-__device__ __forceinline__ bool epi_sync_or(bool pred) {
+// Named barrier `id` over 128 epilogue threads; returns true if `pred` was set in any
+// of them.
+__device__ __forceinline__ bool epi_sync_or(bool pred, int id = 1) {
     uint32_t out;
     asm volatile(
         "{\n\t.reg .pred p, q;\n\t"
         "setp.ne.u32 p, %1, 0;\n\t"
-        "bar.red.or.pred q, 1, 128, p;\n\t"
+        "bar.red.or.pred q, %2, 128, p;\n\t"
         "selp.u32 %0, 1, 0, q;\n\t}"
         : "=r"(out)
-        : "r"((uint32_t)pred)
+        : "r"((uint32_t)pred), "r"(id)
         : "memory");
     return out != 0;
 }
@@ -725,6 +725,313 @@ __global__ void __launch_bounds__(192, 1) k_stageA_tc1(const __grid_constant__ T
     tc_fence_before();
     __syncthreads();
     if (warp == 5) {
+        // every MMA has completed before the TMEM is freed
+        mbar_wait(done, 0, kDefaultBudget);
+        __syncwarp();
+        tc_fence_after();
+        tmem_dealloc<512>(tmem);
+    }
+}
+
+// ------------------------------ stage A with the ensemble's operands resident
+// With symmetry images every image multiplies the same rows of D and takes its row dots
+// with the same d and g.  k_stageA_tc read all of them again for each image: 192 KB of
+// operands and 128 KB of d and g for 4000 cycles of MMAs, at the 47 bytes a cycle that
+// reach an SM 10 400 cycles a tile (M=189, 48 images).  Here the rows' whole K range
+// (up to 192 modes, 96 KB) and d and g of 64 columns (64 KB) stay in shared memory while
+// the images go by, each with 16 KB of Y1 for a K block: 536 -> 212 us
+// a launch (both perturbations, N=10000).  Products, their order and the order of the
+// row dots are those of k_stageA_tc, so the results are the same bits: the second 64
+// columns of its tiles go on from the sums that the first left in qpst.
+//   warps 0-3, 4-7  epilogue, even and odd images (thread = tile row)
+//   warp 8   Y1 ring    warp 9   MMA issue (whole warp, one lane elected)
+//   warp 10  D, d and g
+// A CTA takes an even share of the (row tile, image) pairs, row tile major.
+constexpr int kIBN = 64;                                    // tile columns
+constexpr int kIMaxKb = 3;                                  // K blocks: Mp <= 192
+constexpr int kISlots = 4;                                  // of a K block of Y1, hi and lo
+constexpr int kIAcc = 4;                                    // tiles' accumulators: 4 x 2 x 64 columns
+constexpr uint32_t kILimbA = kBM * kBK * 2, kILimbB = kIBN * kBK * 2;
+constexpr uint32_t kISlotBytes = 2 * kILimbB;               // 16 KB
+constexpr uint32_t kIBox = kBM * kPEpiCols * 4;             // 16 columns of d or g
+constexpr uint32_t kIDgBytes = 2 * (kIBN / kPEpiCols) * kIBox;      // 64 KB
+constexpr int kIBars = 2 * kISlots + 2 * kIAcc + 4 + 1;     // ring, accumulators, A, dg, done
+constexpr size_t kISmem = 1024 + kIMaxKb * 2 * (size_t)kILimbA + kIDgBytes +
+                          kISlots * (size_t)kISlotBytes + 2 * 3 * kIBN * sizeof(float) +
+                          8 * kIBars + 16;
+static_assert(kISmem <= 232448, "stage A (images) shared memory above the per-block limit");
+
+__global__ void __launch_bounds__(352, 1) k_stageA_img(const __grid_constant__ TmaQuad tm,
+                                                        const __grid_constant__ TmaEpi te,
+                                                        const StageAArgs args) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t *smem = reinterpret_cast<uint8_t *>(
+        (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    uint8_t *dg = smem + kIMaxKb * 2 * kILimbA, *ring = dg + kIDgBytes;
+    float *colv = reinterpret_cast<float *>(ring + kISlots * kISlotBytes);   // [set][3][64]
+    uint64_t *bars = reinterpret_cast<uint64_t *>(colv + 2 * 3 * kIBN);
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + kIBars);
+    volatile int *abort = reinterpret_cast<volatile int *>(tmem_slot + 1);
+    const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8 * kISlots,
+                   tfull0 = empty0 + 8 * kISlots, tempty0 = tfull0 + 8 * kIAcc,
+                   afull = tempty0 + 8 * kIAcc, aempty = afull + 8, dgfull = aempty + 8,
+                   dgempty = dgfull + 8, done = dgempty + 8;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const long long budget = args.budget;
+    const int J = args.J, nkb = args.nkb, nct = args.Mp / kIBN;
+    // this CTA's pairs [p0, p1) of (row tile, image)
+    const int p0 = (int)(args.ntiles * blockIdx.x / gridDim.x),
+              p1 = (int)(args.ntiles * (blockIdx.x + 1) / gridDim.x);
+
+    if (threadIdx.x == 0) {
+        for (int b = 0; b < kISlots; ++b) {
+            mbar_init(full0 + 8 * b, 1);
+            mbar_init(empty0 + 8 * b, 1);
+        }
+        for (int b = 0; b < kIAcc; ++b) {
+            mbar_init(tfull0 + 8 * b, 1);
+            mbar_init(tempty0 + 8 * b, 128);
+        }
+        mbar_init(afull, 1);
+        mbar_init(aempty, 1);
+        mbar_init(dgfull, 1);
+        mbar_init(dgempty, 256);
+        mbar_init(done, 1);
+        *abort = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (warp == 9) tmem_alloc<512>(smem_u32(tmem_slot));
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    pdl_enter();
+    int fail_code = 0;
+
+    // Every role walks the segments (pairs of one row tile), in them the column tiles
+    // and in those the images.
+    if (warp == 8) {
+        if (lane == 0) {
+            int slot = 0;
+            uint32_t ph = 0;
+            long g = 0;
+            for (int p = p0; p < p1 && !fail_code;) {
+                const int rt = p / J, j0 = p - rt * J, j1 = min(J, j0 + p1 - p);
+                for (int ct = 0; ct < nct && !fail_code; ++ct)
+                    for (int j = j0; j < j1 && !fail_code; ++j)
+                        for (int kb = 0; kb < nkb; ++kb, ++g) {
+                            if (g >= kISlots &&
+                                !mbar_wait_ab(empty0 + 8 * slot, ph ^ 1, budget, abort)) {
+                                fail_code = 1;
+                                break;
+                            }
+                            const uint32_t base = smem_u32(ring + slot * kISlotBytes),
+                                           bar = full0 + 8 * slot;
+                            mbar_expect_tx(bar, kISlotBytes);
+                            tma_load_2d(base, &tm.b_hi, bar, kb * kBK, j * args.Mp + ct * kIBN);
+                            tma_load_2d(base + kILimbB, &tm.b_lo, bar, kb * kBK,
+                                        j * args.Mp + ct * kIBN);
+                            if (++slot == kISlots) {
+                                slot = 0;
+                                ph ^= 1;
+                            }
+                        }
+                p += j1 - j0;
+            }
+            if (fail_code) {
+                *abort = 1;
+                // every issued slot must land before the CTA exits
+                for (long gg = g > kISlots ? g - kISlots : 0; gg < g; ++gg)
+                    mbar_wait(full0 + 8 * (int)(gg % kISlots), (uint32_t)(gg / kISlots) & 1,
+                              kDefaultBudget);
+            }
+        }
+    } else if (warp == 9) {
+        const uint32_t one = elect_one();
+        constexpr uint32_t kIdesc = idesc_f16(kBM, kIBN);
+        int slot = 0, acc = 0;
+        uint32_t ph = 0, tph = 0, seg = 0;
+        long i = 0;
+        for (int p = p0; p < p1 && !fail_code; ++seg) {
+            const int rt = p / J, j0 = p - rt * J, j1 = min(J, j0 + p1 - p);
+            if (!mbar_all(afull, seg & 1, budget, abort)) {
+                fail_code = 2;
+                break;
+            }
+            const int ntile = nct * (j1 - j0);
+            for (int t = 0; t < ntile && !fail_code; ++t, ++i) {
+                if (i >= kIAcc && !mbar_all(tempty0 + 8 * acc, tph ^ 1, budget, abort)) {
+                    fail_code = 2;
+                    break;
+                }
+                const uint32_t d0 = tmem + 2 * kIBN * acc, d1 = d0 + kIBN;
+                for (int kb = 0; kb < nkb; ++kb) {
+                    if (!mbar_all(full0 + 8 * slot, ph, budget, abort)) {
+                        fail_code = 2;
+                        break;
+                    }
+                    tc_fence_after();
+                    const uint32_t a = smem_u32(smem + kb * 2 * kILimbA),
+                                   b = smem_u32(ring + slot * kISlotBytes);
+                    const uint64_t ah = sdesc_sw128(a), al = sdesc_sw128(a + kILimbA),
+                                   bh = sdesc_sw128(b), bl = sdesc_sw128(b + kILimbB);
+#pragma unroll
+                    for (int kk = 0; kk < kBK / 16; ++kk) {
+                        const uint32_t go = (kb | kk) != 0;
+                        mma_f16_one(one, d0, ah + 2 * kk, bh + 2 * kk, kIdesc, go);
+                        mma_f16_one(one, d1, ah + 2 * kk, bl + 2 * kk, kIdesc, go);
+                        mma_f16_one(one, d1, al + 2 * kk, bh + 2 * kk, kIdesc, 1);
+                    }
+                    mma_commit_one(one, empty0 + 8 * slot);
+                    if (++slot == kISlots) {
+                        slot = 0;
+                        ph ^= 1;
+                    }
+                }
+                if (fail_code) break;
+                mma_commit_one(one, tfull0 + 8 * acc);
+                if (++acc == kIAcc) {
+                    acc = 0;
+                    tph ^= 1;
+                }
+            }
+            if (fail_code) break;
+            mma_commit_one(one, aempty);
+            p += j1 - j0;
+        }
+        if (fail_code) *abort = 1;
+        mma_commit_one(one, done);   // tracks every MMA issued, also after a failure
+    } else if (warp == 10) {
+        if (lane == 0) {
+            uint32_t seg = 0, part = 0;         // loads issued
+            for (int p = p0; p < p1 && !fail_code; ++seg) {
+                const int rt = p / J, j0 = p - rt * J, j1 = min(J, j0 + p1 - p), row = rt * kBM;
+                if (seg > 0 && !mbar_wait_ab(aempty, (seg - 1) & 1, budget, abort)) {
+                    fail_code = 1;
+                    break;
+                }
+                mbar_expect_tx(afull, nkb * 2 * kILimbA);
+                for (int kb = 0; kb < nkb; ++kb) {
+                    const uint32_t a = smem_u32(smem + kb * 2 * kILimbA);
+                    tma_load_2d(a, &tm.a_hi, afull, kb * kBK, row);
+                    tma_load_2d(a + kILimbA, &tm.a_lo, afull, kb * kBK, row);
+                }
+                for (int ct = 0; ct < nct; ++ct, ++part) {
+                    if (part > 0 && !mbar_wait_ab(dgempty, (part - 1) & 1, budget, abort)) {
+                        fail_code = 1;
+                        ++seg;                  // (this segment's D is on its way)
+                        break;
+                    }
+                    mbar_expect_tx(dgfull, kIDgBytes);
+                    for (int b = 0; b < kIBN / kPEpiCols; ++b) {
+                        const uint32_t o = smem_u32(dg + 2 * b * kIBox);
+                        tma_load_2d(o, &te.d, dgfull, ct * kIBN + b * kPEpiCols, row);
+                        tma_load_2d(o + kIBox, &te.g, dgfull, ct * kIBN + b * kPEpiCols, row);
+                    }
+                }
+                if (fail_code) break;
+                p += j1 - j0;
+            }
+            if (fail_code) {
+                *abort = 1;
+                if (seg > 0) mbar_wait(afull, (seg - 1) & 1, kDefaultBudget);
+                if (part > 0) mbar_wait(dgfull, (part - 1) & 1, kDefaultBudget);
+            }
+        }
+    } else {
+        // ---- epilogue: set 0 takes the even images, set 1 the odd ones
+        const int set = warp >> 2, quad = warp & 3, row_in = quad * 32 + lane;
+        const uint32_t lane_base = tmem + ((uint32_t)(quad * 32) << 16);
+        const int sw = (row_in >> 1) & 3;
+        const long R = args.R;
+        long i = 0;
+        uint32_t part = 0;
+        for (int p = p0; p < p1 && !fail_code;) {
+            const int rt = p / J, j0 = p - rt * J, j1 = min(J, j0 + p1 - p);
+            const long row = (long)rt * kBM + row_in;
+            for (int ct = 0; ct < nct && !fail_code; ++ct, ++part) {
+                // Both sets wait for every part's d and g, also a set without an image in
+                // it: it would be ahead in dgempty's phases otherwise.
+                const bool here = mbar_wait_ab(dgfull, part & 1, budget, abort);
+                for (int j = j0; j < j1; ++j, ++i) {
+                    if ((j & 1) != set) continue;
+                    const int acc = (int)(i % kIAcc);
+                    float *cv = colv + set * 3 * kIBN;           // column factors
+                    for (int e = row_in; e < 3 * kIBN; e += 128) {
+                        const float *src = e < kIBN ? args.tcol : e < 2 * kIBN ? args.vec_s : args.vec_t;
+                        cv[e] = src[(long)j * args.Mp + ct * kIBN + (e & (kIBN - 1))];
+                    }
+                    float *o = args.qpst + ((long)j * ((nct + 1) / 2) + ct / 2) * 4 * R + row;
+                    float q = 0.f, pp = 0.f, sacc = 0.f, tacc = 0.f;
+                    if ((ct & 1) && row < R) {
+                        q = o[0];
+                        pp = o[R];
+                        sacc = o[2 * R];
+                        tacc = o[3 * R];
+                    }
+                    const bool ok = here && mbar_wait_ab(tfull0 + 8 * acc, (uint32_t)(i / kIAcc) & 1,
+                                                         budget, abort);
+                    __syncwarp();
+                    if (epi_sync_or(!ok, 1 + set)) {     // also publishes cv
+                        fail_code = 3;
+                        break;
+                    }
+                    tc_fence_after();
+#pragma unroll 1
+                    for (int chunk = 0; chunk < 2; ++chunk) {
+                        float v[32];
+                        tmem_combined(lane_base + 2 * kIBN * acc, chunk * 32, kIBN, v);
+                        if (chunk == 1) {
+                            tc_fence_before();
+                            mbar_arrive(tempty0 + 8 * acc);
+                        }
+#pragma unroll
+                        for (int half = 0; half < 2; ++half) {
+                            // 64-byte rows, 16-byte granule c stored at c ^ ((row >> 1) & 3)
+                            const uint8_t *bd = dg + 2 * (chunk * 2 + half) * kIBox + row_in * 64;
+                            const uint8_t *bg = bd + kIBox;
+                            const float *cp = cv + chunk * 32 + half * 16;
+#pragma unroll
+                            for (int ch = 0; ch < 4; ++ch) {
+                                float4 d4 = *reinterpret_cast<const float4 *>(bd + ((ch ^ sw) << 4));
+                                float4 g4 = *reinterpret_cast<const float4 *>(bg + ((ch ^ sw) << 4));
+                                float dd[4] = {d4.x, d4.y, d4.z, d4.w}, gg[4] = {g4.x, g4.y, g4.z, g4.w};
+#pragma unroll
+                                for (int k = 0; k < 4; ++k) {
+                                    int c = 4 * ch + k;
+                                    float vv = v[half * 16 + c] * cp[c];
+                                    q = fmaf(dd[k], vv, q);
+                                    pp = fmaf(gg[k], vv, pp);
+                                    sacc = fmaf(cp[kIBN + c], dd[k], sacc);
+                                    tacc = fmaf(cp[2 * kIBN + c], gg[k], tacc);
+                                }
+                            }
+                        }
+                    }
+                    // cv has been read
+                    asm volatile("bar.sync %0, 128;" ::"r"(1 + set) : "memory");
+                    if (row < R) {
+                        o[0] = q;
+                        o[R] = pp;
+                        o[2 * R] = sacc;
+                        o[3 * R] = tacc;
+                    }
+                }
+                if (!here) fail_code = 3;
+                if (fail_code) break;
+                // the reads of d and g are generic-proxy, their refill is a TMA write
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                mbar_arrive(dgempty);
+            }
+            p += j1 - j0;
+        }
+        if (fail_code) *abort = 1;
+    }
+    if (fail_code && lane == 0) *(volatile int *)args.err = fail_code;
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 9) {
         // every MMA has completed before the TMEM is freed
         mbar_wait(done, 0, kDefaultBudget);
         __syncwarp();
@@ -1640,6 +1947,7 @@ static int make_map_f32(CUtensorMap *m, const void *base, uint64_t inner, uint64
 
 struct MixedExtra {
     TmaQuad tmA, tmB;
+    TmaQuad tmA64;            // stage A operand maps for 64-row B boxes (images)
     TmaQuad tmA1;             // stage A operand maps for the 192-row B boxes (one accumulator)
     TmaEpi te;
     int bnA = 0;
@@ -1902,7 +2210,9 @@ int mixed_prepare(tdscha_ctx *c) {
     TDS_TRY(make_map(&x->tmA.a_lo, mx.d_lo, Mp, R, kBM));
     TDS_TRY(make_map(&x->tmA.b_hi, mx.y1_hi, Mp, (uint64_t)Jm * Mp, std::min(kPBN, Mp)));
     TDS_TRY(make_map(&x->tmA.b_lo, mx.y1_lo, Mp, (uint64_t)Jm * Mp, std::min(kPBN, Mp)));
-    x->tmA1 = x->tmA;
+    x->tmA1 = x->tmA64 = x->tmA;
+    TDS_TRY(make_map(&x->tmA64.b_hi, mx.y1_hi, Mp, (uint64_t)Jm * Mp, kIBN));
+    TDS_TRY(make_map(&x->tmA64.b_lo, mx.y1_lo, Mp, (uint64_t)Jm * Mp, kIBN));
     TDS_TRY(make_map(&x->tmA1.b_hi, mx.y1_hi, Mp, (uint64_t)Jm * Mp, std::min(kRBN, Mp)));
     TDS_TRY(make_map(&x->tmA1.b_lo, mx.y1_lo, Mp, (uint64_t)Jm * Mp, std::min(kRBN, Mp)));
     TDS_TRY(make_map(&x->tmB.a_hi, mx.ut_hi, Rp, Mp, kBM));
@@ -1915,6 +2225,8 @@ int mixed_prepare(tdscha_ctx *c) {
     if (!attr_done) {
         TDS_CUDA(cudaFuncSetAttribute(k_stageA_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)kPSmem));
+        TDS_CUDA(cudaFuncSetAttribute(k_stageA_img, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)kISmem));
         TDS_CUDA(cudaFuncSetAttribute(k_stageA_tc1, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)kRSmem));
         TDS_CUDA(cudaFuncSetAttribute(k_stageB_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2064,7 +2376,12 @@ static int perturb_mixed_src(tdscha_ctx *c, int apply_d4, const Y1FromPsi *psrc,
     {
         ProfScope ps(c, 0, st);
         int grid = (int)std::min<long>(ga.ntiles, x->nsm);
-        if (x->one_acc)
+        if (!x->one_acc && J > 1 && ga.nkb <= kIMaxKb) {
+            // images share the ensemble's operands, which fit
+            ga.ntiles = (long)ceil_div(R, kBM) * Jb;
+            grid = (int)std::min<long>(ga.ntiles, x->nsm);
+            TDS_CUDA(launch_pdl(k_stageA_img, grid, 352, kISmem, st, x->tmA64, x->te, ga));
+        } else if (x->one_acc)
             TDS_CUDA(launch_pdl(k_stageA_tc1, grid, 192, kRSmem, st, x->tmA1, x->te, ga));
         else
             TDS_CUDA(launch_pdl(k_stageA_tc, grid, 192, kPSmem, st, x->tmA, x->te, ga));
