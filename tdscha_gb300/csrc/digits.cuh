@@ -92,6 +92,10 @@ __device__ __forceinline__ uint32_t sw_place(int row, int c) {
     return (uint32_t)row * 128u + (uint32_t)((c ^ (row & 7)) << 4);
 }
 
+__device__ __forceinline__ double2 dg_two(const double *p) {
+    return *reinterpret_cast<const double2 *>(p);
+}
+
 // (hi 2^32 + lo) 2^e as float64, |hi| < 2^62, rounded to nearest to within 2^-60
 // of itself or one unit of lo.  About 25 whole-number operations: a conversion of
 // a 64-bit integer, like every float64 operation, runs at two per cycle per SM.
@@ -557,7 +561,8 @@ __global__ void __launch_bounds__(DgShape<kMode>::threads, 1) k_dg_gemm(const Dg
             // the matrix work (in the epilogue these two products an element kept
             // the float64 pipe for longer than the tile's MMAs run)
             const int row = (warp - kEpi - 4) * 32 + lane;
-            for (Item w(args); w.left > 0; w.next()) {
+            // (left out where s and t come from a product of their own)
+            for (Item w(args); args.vs && w.left > 0; w.next()) {
                 const int at = w.at, bt = w.bt;
                 const long tile = ((long)at * args.Mp + (long)(bt % args.nct) * kGN) * 128 + row;
                 const double *pd = args.dt + tile, *pg = args.gt + tile;

@@ -60,10 +60,8 @@
 
 namespace tdscha {
 
-// alpha, beta / 2 and the force weights of one (image, row)
-struct __align__(32) RowScalars {
-    double a, b, c1, c2;
-};
+// alpha, beta / 2 and the force weights (of g and of x) of the images' rows:
+// abcc[(4 image + k) Rp + row]
 
 // ------------------------------------------------- once per ensemble
 // Column maxima of |x| and |g|.
@@ -167,19 +165,45 @@ __global__ void __launch_bounds__(256) k_dg_xa(const double *__restrict__ D,
     }
 }
 
+// The same from the column layout (g): thread = (row, eight modes)
+__global__ void __launch_bounds__(256) k_dg_ga(const double *__restrict__ gt,
+                                               const int *__restrict__ ec,
+                                               const int *__restrict__ er, int M, int Mp, int nkb,
+                                               __half *__restrict__ ga) {
+    const long rt = blockIdx.x;
+    const int kb = blockIdx.y, row = threadIdx.x & 127;
+    uint8_t *out = reinterpret_cast<uint8_t *>(ga) + (rt * nkb + kb) * (long)kRes * kGA;
+    for (int c = threadIdx.x >> 7; c < 8; c += 2) {
+        long long q[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const int m = kb * kGK + c * 8 + k;
+            q[k] = m < M ? fixed_point(gt[(rt * Mp + m) * 128 + row], 55 - ec[m] - er[rt * kGM + row]) : 0;
+        }
+        uint4 w[kRes];
+        digits8<kRes>(q, w);
+#pragma unroll
+        for (int d = 0; d < kRes; ++d)
+            *reinterpret_cast<uint4 *>(out + d * kGA + sw_place(row, c)) = w[d];
+    }
+}
+
 __global__ void __launch_bounds__(256) k_dg_xb(const double *__restrict__ dt,
                                                const int *__restrict__ ec, int Mp, long nkb,
                                                __half *__restrict__ xb, float *__restrict__ nrm) {
     const long kb = blockIdx.x;
     const int at = blockIdx.y, c = threadIdx.x & 7;
     uint8_t *out = reinterpret_cast<uint8_t *>(xb) + (at * nkb + kb) * kRes * (long)kGB;
-    const long r0 = kb * kGK + c * 8;
     for (int row = threadIdx.x >> 3; row < kGN; row += 32) {
         const int a = at * kGN + row;
-        const double *src = dt + ((r0 >> 7) * Mp + a) * 128 + (r0 & 127);
+        const double *src = dt + ((kb >> 1) * Mp + a) * 128 + (kb & 1) * 64 + 8 * c;
         long long q[8];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) q[k] = fixed_point(src[k], 55 - ec[a]);
+        for (int j = 0; j < 4; ++j) {
+            const double2 v = dg_two(src + 2 * j);
+            q[2 * j] = fixed_point(v.x, 55 - ec[a]);
+            q[2 * j + 1] = fixed_point(v.y, 55 - ec[a]);
+        }
         uint4 w[kRes];
         digits8<kRes>(q, w);
 #pragma unroll
@@ -232,11 +256,13 @@ __device__ __forceinline__ double dg_y1(const DgSource &c, const double *__restr
 
 // Row n of image blockIdx.y of Y1 (symmetric): digits of y 2^(ec - et) with et
 // the exponent above the row's maximum, and the two vectors of the row scalars.
-// Also clears the image's maxima of alpha and beta.
+// Also clears the image's maxima of alpha, beta and the force weights.  With many
+// images rows M and M + 1 are those two vectors, digits of rows `image` of the tiles vb.
 __global__ void __launch_bounds__(128) k_dg_y1(const DgSources src, const double *__restrict__ fY,
-                                               const int *__restrict__ ec, int M, int Mp,
+                                               const int *__restrict__ ecol, int M, int Mp,
                                                __half *__restrict__ yb, int *__restrict__ et,
                                                double *__restrict__ vs, double *__restrict__ vt,
+                                               __half *__restrict__ vb, int *__restrict__ etv,
                                                unsigned long long *__restrict__ absmax) {
     pdl_enter();
     extern __shared__ double yrow[];     // M
@@ -245,9 +271,15 @@ __global__ void __launch_bounds__(128) k_dg_y1(const DgSources src, const double
     const long img = blockIdx.y, rel = img - is;
     const DgSource &c = src.s[is];
     const double *Y = c.Y + rel * c.ystride;
+    auto vec = [&](int m, bool of_s) {
+        const double r = c.no_r ? 0.0 : c.R[rel * c.rstride + m];
+        return of_s && c.S ? c.S[rel * c.rstride + m] : fY[m] * r;
+    };
+    const int v2 = n - M;             // 0, 1: s and t
+    const int *ec = ecol + (v2 == 1 ? Mp : 0);
     int e = INT_MIN;
     for (int m = threadIdx.x; m < M; m += blockDim.x) {
-        const double v = dg_y1(c, Y, M, n, m);
+        const double v = v2 >= 0 ? vec(m, v2 == 0) : dg_y1(c, Y, M, n, m);
         yrow[m] = v;
         if (v != 0) e = max(e, isfinite(v) ? exp_above(v) + ec[m] : kBadExp);
     }
@@ -258,8 +290,10 @@ __global__ void __launch_bounds__(128) k_dg_y1(const DgSources src, const double
     e = max(max(sh[0], sh[1]), max(sh[2], sh[3]));
     if (e == INT_MIN) e = 0;
     const bool bad = e >= kBadExp / 2;
-    const int nkb = Mp / kGK, row = n % kGN;
-    uint8_t *out = reinterpret_cast<uint8_t *>(yb) + (img * (Mp / kGN) + n / kGN) * nkb * (long)kCall * kGB;
+    const int nkb = Mp / kGK, row = v2 >= 0 ? (int)img : n % kGN;
+    uint8_t *out = v2 >= 0 ? reinterpret_cast<uint8_t *>(vb) + v2 * (long)nkb * kCall * kGB
+                           : reinterpret_cast<uint8_t *>(yb) +
+                                 (img * (Mp / kGN) + n / kGN) * nkb * (long)kCall * kGB;
     for (int ch = threadIdx.x; ch < Mp / 8; ch += blockDim.x) {
         const int kb = ch >> 3, c8 = ch & 7;
         long long q[8];
@@ -274,76 +308,108 @@ __global__ void __launch_bounds__(128) k_dg_y1(const DgSources src, const double
         for (int d = 0; d < kCall; ++d)
             *reinterpret_cast<uint4 *>(out + (kb * (long)kCall + d) * kGB + sw_place(row, c8)) = w[d];
     }
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == 0 && v2 >= 0) {
+        etv[v2 * kGN + img] = e;
+    } else if (threadIdx.x == 0) {
         et[img * Mp + n] = e;
-        const double r = c.no_r ? 0.0 : c.R[rel * c.rstride + n];
-        vs[img * Mp + n] = c.S ? c.S[rel * c.rstride + n] : fY[n] * r;
-        vt[img * Mp + n] = fY[n] * r;
-        if (n == 0) absmax[2 * img] = absmax[2 * img + 1] = 0ULL;
+        vs[img * Mp + n] = vec(n, true);
+        vt[img * Mp + n] = vec(n, false);
+        if (n == 0)
+            for (int k = 0; k < 4; ++k) absmax[4 * img + k] = 0ULL;
     }
 }
 
-// Row scalars of the image blockIdx.y from the stage A partials; max |alpha|
-// and max |beta / 2| of the image.  Rows past the end get zeros.
-__global__ void __launch_bounds__(128) k_dg_rows(const double *__restrict__ qp, int nct, long R,
+// Row scalars of the image blockIdx.y from the stage A partials (s and t of many images
+// from st, [2 Rp][images]); max |alpha|, max |beta / 2| and the maxima of the force
+// weights of the image.  Rows past the end get zeros.
+template <bool kMany>
+__global__ void __launch_bounds__(128) k_dg_rows(const double *__restrict__ qp,
+                                                 const double *__restrict__ st, int nct, long R,
                                                  long Rp, int rho_div,
                                                  const double *__restrict__ rho,
                                                  const int *__restrict__ er, int apply_d4,
-                                                 RowScalars *__restrict__ abcc,
+                                                 double *__restrict__ abcc,
                                                  unsigned long long *__restrict__ absmax) {
     pdl_enter();
-    __shared__ unsigned long long red[2][4];
+    constexpr int kMax = kMany ? 4 : 2;
+    __shared__ unsigned long long red[kMax][4];
     const long img = blockIdx.y, r = blockIdx.x * 128L + threadIdx.x;
-    RowScalars v = {0, 0, 0, 0};
+    double w[4] = {0, 0, 0, 0};
     if (r < R) {
         double q = 0, p = 0, s = 0, t = 0;
         const double *o = qp + img * nct * 4 * R + r;
         for (int ct = 0; ct < nct; ++ct, o += 4 * R) {
             q += o[0];
             p += o[R];
-            s += o[2 * R];
-            t += o[3 * R];
+            if (!kMany) {
+                s += o[2 * R];
+                t += o[3 * R];
+            }
         }
-        const double f = pow2(er[r]), rw = rho[r / rho_div], d4 = apply_d4 ? 1.0 : 0.0;
+        if (kMany) {
+            s = st[r * gridDim.y + img];
+            t = st[(Rp + r) * gridDim.y + img];
+        }
+        const double f = pow2(er[r]), rw = rho[r / rho_div];
         q *= f;
         p *= f;
-        v.a = rw * (s / 3 - d4 * q / 8);
-        v.b = 0.5 * (rw * (t / 3 - d4 * p / 4));
-        v.c1 = -rw * q / 6;
-        v.c2 = -rw * p / 3;
+        // rho / 3 by the reciprocal and one residual step: a warp's float64 operation
+        // takes 64 cycles, a division ten of them
+        constexpr double third = 1.0 / 3.0;
+        const double y = rw * third, t3 = fma(fma(-y, 3.0, rw), third, y), h3 = 0.5 * t3,
+                     t8 = apply_d4 ? 0.125 * rw : 0.0;
+        w[0] = fma(s, t3, -q * t8);           // rho (s / 3 - q / 8)
+        w[1] = fma(t, h3, -p * t8);           // rho (t / 3 - p / 4) / 2
+        w[2] = -q * h3;
+        w[3] = -p * t3;
     }
-    if (r < Rp) abcc[img * Rp + r] = v;
-    unsigned long long a = (unsigned long long)__double_as_longlong(v.a) & 0x7fffffffffffffffULL;
-    unsigned long long b = (unsigned long long)__double_as_longlong(v.b) & 0x7fffffffffffffffULL;
+    if (r < Rp) {
+        double *o = abcc + 4 * img * Rp + r;
+        o[0] = w[0];
+        o[Rp] = w[1];
+        o[2 * Rp] = w[2];
+        o[3 * Rp] = w[3];
+    }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        a = max(a, __shfl_xor_sync(0xffffffffu, a, o));
-        b = max(b, __shfl_xor_sync(0xffffffffu, b, o));
-    }
-    if ((threadIdx.x & 31) == 0) {
-        red[0][threadIdx.x >> 5] = a;
-        red[1][threadIdx.x >> 5] = b;
+    for (int k = 0; k < kMax; ++k) {
+        unsigned long long a = (unsigned long long)__double_as_longlong(w[k]) & 0x7fffffffffffffffULL;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) a = max(a, __shfl_xor_sync(0xffffffffu, a, o));
+        if ((threadIdx.x & 31) == 0) red[k][threadIdx.x >> 5] = a;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int k = 1; k < 4; ++k) {
-            a = max(a, red[0][k]);
-            b = max(b, red[1][k]);
-        }
-        atomicMax(absmax + 2 * img, a);
-        atomicMax(absmax + 2 * img + 1, b);
+    if (threadIdx.x < kMax) {
+        unsigned long long a = red[threadIdx.x][0];
+        for (int k = 1; k < 4; ++k) a = max(a, red[threadIdx.x][k]);
+        atomicMax(absmax + 4 * img + threadIdx.x, a);
     }
+}
+
+// Exponent above max|alpha| max|g| + max|beta/2| max|x| of a mode of an image, kBadExp
+// where that is not finite; am: the image's four maxima.
+__device__ __forceinline__ int dg_wexp(const unsigned long long *__restrict__ am, double dm, double gm) {
+    // a little above the bound: w itself is rounded
+    const double bound = (__longlong_as_double((long long)am[0]) * gm +
+                          __longlong_as_double((long long)am[1]) * dm) * (1.0 + 0x1p-40);
+    return !isfinite(bound) ? kBadExp : bound > 0 ? exp_above(bound) : 0;
+}
+
+// Digits of eight numbers as row `row` of the A block blk, chunk c
+__device__ __forceinline__ void dg_put(const long long (&q)[8], uint8_t *blk, int row, int c) {
+    uint4 w[kCall];
+    digits8<kCall>(q, w);
+    blk += sw_place(row, c);
+#pragma unroll
+    for (int d = 0; d < kCall; ++d) *reinterpret_cast<uint4 *>(blk + d * kGA) = w[d];
 }
 
 // W digits: block = (group of K blocks, tile of 128 rows (image, mode)); thread
 // = (mode, eight rows of the ensemble) for 32 modes at a time, so that a warp
-// reads 512 contiguous bytes of x and g a mode and writes whole 128-byte rows of
-// every digit.  The scale of a mode is the exponent above
-// max|alpha| max|g| + max|beta/2| max|x|.  The force partials
+// writes whole 128-byte rows of every digit.  The force partials
 // fpart[(img nfc + group) M + b] ride along.
 __global__ void __launch_bounds__(256) k_dg_wbuild(
     const double *__restrict__ dt, const double *__restrict__ gt,
-    const RowScalars *__restrict__ abcc, const unsigned long long *__restrict__ absmax,
+    const double *__restrict__ abcc, const unsigned long long *__restrict__ absmax,
     const unsigned long long *__restrict__ dmax, const unsigned long long *__restrict__ gmax,
     const double *__restrict__ fY, int M, int Mp, long Rp, int nimg, long nkb, int per,
     __half *__restrict__ wa, int *__restrict__ ew, double *__restrict__ fpart) {
@@ -357,48 +423,128 @@ __global__ void __launch_bounds__(256) k_dg_wbuild(
         // (the eight lanes of a mode take the same branch; padding rows of wa
         // are zero from the start)
         const bool live = img < nimg && b < M;
-        double facc = 0;
+        double f1 = 0, f2 = 0;
         if (live) {
-            const double am = __longlong_as_double((long long)absmax[2 * img]),
-                         bm = __longlong_as_double((long long)absmax[2 * img + 1]),
-                         dm = __longlong_as_double((long long)dmax[b]),
-                         gm = __longlong_as_double((long long)gmax[b]);
-            // a little above the bound: w itself is rounded
-            const double bound = (am * gm + bm * dm) * (1.0 + 0x1p-40);
-            const bool bad = !isfinite(bound);
-            const int e = bad ? kBadExp : bound > 0 ? exp_above(bound) : 0;
+            const int e = dg_wexp(absmax + 4 * img, __longlong_as_double((long long)dmax[b]),
+                                  __longlong_as_double((long long)gmax[b]));
+            const bool bad = e == kBadExp;
             const int K = 62 - e;
             if (blockIdx.x == 0 && c == 0) ew[grow] = e;
             for (long kb = kb0; kb < kb1; ++kb) {
-                const long r0 = kb * kGK + c * 8;
-                const long o = ((r0 >> 7) * Mp + b) * 128 + (r0 & 127);
-                const double2 *d2 = reinterpret_cast<const double2 *>(dt + o);
-                const double2 *g2 = reinterpret_cast<const double2 *>(gt + o);
-                const RowScalars *ab = abcc + img * Rp + r0;
+                const long o = ((kb >> 1) * Mp + b) * 128 + (kb & 1) * 64 + 8 * c;
+                const double *pa = abcc + 4L * img * Rp + kb * kGK + 8 * c;
                 long long q[8];
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const double2 d = d2[k], g = g2[k];
-                    const RowScalars s0 = ab[2 * k], s1 = ab[2 * k + 1];
-                    const double w0 = fma(s0.a, g.x, s0.b * d.x), w1 = fma(s1.a, g.y, s1.b * d.y);
-                    q[2 * k] = bad ? 0 : fixed_point(w0, K);
-                    q[2 * k + 1] = bad ? 0 : fixed_point(w1, K);
-                    facc = fma(s0.c1, g.x, facc);
-                    facc = fma(s0.c2, d.x, facc);
-                    facc = fma(s1.c1, g.y, facc);
-                    facc = fma(s1.c2, d.y, facc);
+                for (int j = 0; j < 4; ++j) {
+                    const double2 d = dg_two(dt + o + 2 * j), g = dg_two(gt + o + 2 * j);
+                    const double *pr = pa + 2 * j;
+                    const double2 sa = dg_two(pr), sb = dg_two(pr + Rp), c1 = dg_two(pr + 2 * Rp),
+                                  c2 = dg_two(pr + 3 * Rp);
+                    const double w0 = fma(sa.x, g.x, sb.x * d.x),
+                                 w1 = fma(sa.y, g.y, sb.y * d.y);
+                    q[2 * j] = bad ? 0 : fixed_point(w0, K);
+                    q[2 * j + 1] = bad ? 0 : fixed_point(w1, K);
+                    f1 = fma(c1.x, g.x, f1);
+                    f2 = fma(c2.x, d.x, f2);
+                    f1 = fma(c1.y, g.y, f1);
+                    f2 = fma(c2.y, d.y, f2);
                 }
-                uint4 w[kCall];
-                digits8<kCall>(q, w);
-                uint8_t *blk = out + kb * kCall * (long)kGA + sw_place(row, c);
-#pragma unroll
-                for (int d = 0; d < kCall; ++d) *reinterpret_cast<uint4 *>(blk + d * kGA) = w[d];
+                dg_put(q, out + kb * kCall * (long)kGA, row, c);
             }
         }
+        double facc = f1 + f2;
 #pragma unroll
         for (int o = 4; o > 0; o >>= 1) facc += __shfl_xor_sync(0xffffffffu, facc, o);
         if (live && c == 0) fpart[((long)img * gridDim.x + blockIdx.x) * M + b] = facc * fY[b];
     }
+}
+
+// The same for many images: block = (K block, 32 modes, kWImages images); x and g of a
+// thread's rows stay in registers while the images go by.  The forces are products of
+// their own with the rows that the blocks blockIdx.y == modes / 32 build in wf: digits
+// of the weights of x (rows 0 .. 63: images) and of g (rows 64 .. 127); as two float64
+// products an element they were half of this kernel's work.  M=189, N=10000, 48 images:
+// 781 us with the forces and every image its own pass over x and g, 376 so.
+constexpr int kWImages = 8;
+__global__ void __launch_bounds__(256) k_dg_wimages(
+    const double *__restrict__ dt, const double *__restrict__ gt,
+    const double *__restrict__ abcc, const unsigned long long *__restrict__ absmax,
+    const unsigned long long *__restrict__ dmax, const unsigned long long *__restrict__ gmax, int M,
+    int Mp, long Rp, int nimg, long nkb, __half *__restrict__ wa, int *__restrict__ ew,
+    __half *__restrict__ wf, int *__restrict__ ewf) {
+    pdl_enter();
+    const int c = threadIdx.x & 7, slot = threadIdx.x >> 3, i0 = blockIdx.z * kWImages,
+              i1 = min(nimg, i0 + kWImages);
+    const long kb = blockIdx.x;
+    if (blockIdx.y == gridDim.y - 1) {
+        // (an image in both halves of the tile)
+        const int img = i0 + slot / 2, row = img + (slot & 1 ? 64 : 0), k = slot & 1 ? 2 : 3;
+        if (img >= i1) return;
+        const double top = __longlong_as_double((long long)absmax[4 * img + k]);
+        const int e = !isfinite(top) ? kBadExp : top > 0 ? exp_above(top) : 0;
+        if (kb == 0 && c == 0) ewf[row] = e;
+        const double *src = abcc + (4L * img + k) * Rp + kb * kGK + 8 * c;
+        long long q[8];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const double2 v = dg_two(src + 2 * j);
+            q[2 * j] = e == kBadExp ? 0 : fixed_point(v.x, 62 - e);
+            q[2 * j + 1] = e == kBadExp ? 0 : fixed_point(v.y, 62 - e);
+        }
+        dg_put(q, reinterpret_cast<uint8_t *>(wf) + kb * kCall * (long)kGA, row, c);
+        return;
+    }
+    __shared__ int sexp[kWImages][32];
+    const int b0 = blockIdx.y * 32, b = b0 + slot;
+    for (int t = threadIdx.x; t < (i1 - i0) * 32; t += blockDim.x) {
+        const int img = i0 + (t >> 5), m = b0 + (t & 31);
+        int e = 0;
+        if (m < M)
+            e = dg_wexp(absmax + 4 * img, __longlong_as_double((long long)dmax[m]),
+                        __longlong_as_double((long long)gmax[m]));
+        sexp[t >> 5][t & 31] = e;
+        if (kb == 0 && m < M) ew[(long)img * Mp + m] = e;
+    }
+    __syncthreads();
+    if (b >= M) return;
+    const long o = ((kb >> 1) * Mp + b) * 128 + (kb & 1) * 64 + 8 * c;
+    double2 d[4], g[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        d[j] = dg_two(dt + o + 2 * j);
+        g[j] = dg_two(gt + o + 2 * j);
+    }
+#pragma unroll 1
+    for (int img = i0; img < i1; ++img) {
+        const int e = sexp[img - i0][slot];
+        const double *pa = abcc + 4L * img * Rp + kb * kGK + 8 * c;
+        long long q[8];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const double2 sa = dg_two(pa + 2 * j), sb = dg_two(pa + Rp + 2 * j);
+            const double w0 = fma(sa.x, g[j].x, sb.x * d[j].x), w1 = fma(sa.y, g[j].y, sb.y * d[j].y);
+            q[2 * j] = e == kBadExp ? 0 : fixed_point(w0, 62 - e);
+            q[2 * j + 1] = e == kBadExp ? 0 : fixed_point(w1, 62 - e);
+        }
+        const long grow = (long)img * Mp + b;
+        dg_put(q, reinterpret_cast<uint8_t *>(wa) + ((grow >> 7) * nkb + kb) * kCall * (long)kGA,
+               (int)(grow & 127), c);
+    }
+}
+
+// fpart[img][m] from the products gf[split][128][2 Mp] of the force weights' rows with
+// [x | g]
+__global__ void __launch_bounds__(128) k_dg_force(const double *__restrict__ gf, int ns, int M, int Mp,
+                                                  const double *__restrict__ fY,
+                                                  double *__restrict__ fpart) {
+    pdl_enter();
+    const int m = blockIdx.x * 128 + threadIdx.x, img = blockIdx.y;
+    if (m >= M) return;
+    const double *p = gf + (long)img * 2 * Mp + m, *q = p + (long)64 * 2 * Mp + Mp;
+    double a = 0;
+#pragma unroll 4
+    for (int s = 0; s < ns; ++s, p += (long)kGM * 2 * Mp, q += (long)kGM * 2 * Mp) a += *p + *q;
+    fpart[(long)img * M + m] = a * fY[m];
 }
 
 // sum_s p[s * stride] in split order, eight loads in flight
@@ -475,11 +621,18 @@ struct DigitStore {
     long Rp = 0, nkbR = 0;
     int cap = 1;                 // images that the per-call buffers hold
     int per = 1, nfc = 1;        // K blocks of one W block, force partials an image
+    // s, t and the forces as digit products of their own (many symmetry images): g's
+    // digits behind x's in xa and xb, its exponents behind x's in er and ec
+    bool many = false;
+    int kbF = 1, nsF = 1;
+    double *st = nullptr, *gf = nullptr;
+    __half *vb = nullptr, *wf = nullptr;
+    int *etv = nullptr, *ewf = nullptr, *bmap = nullptr;
     int flushA = kFlushMin, flushB = kFlushMin;   // K blocks per accumulation of the stages
     void *slab = nullptr;
     double *dt = nullptr, *gt = nullptr, *vs = nullptr, *vt = nullptr, *qp = nullptr,
            *gpart = nullptr, *fpart = nullptr, *fo = nullptr, *d2vo = nullptr;
-    RowScalars *abcc = nullptr;
+    double *abcc = nullptr;
     unsigned long long *dmax = nullptr, *gmax = nullptr, *absmax = nullptr;
     __half *xa = nullptr, *xb = nullptr, *yb = nullptr, *wa = nullptr;
     int *ec = nullptr, *er = nullptr, *et = nullptr, *ew = nullptr;
@@ -522,11 +675,19 @@ int digits_prepare(tdscha_ctx *c) {
     const size_t per_img = elems * 2 * kCall;
     const size_t most = std::max<size_t>(1, (size_t(6) << 30) / per_img);
     if (c->J > 1)
-        x->cap = (int)std::min<size_t>(c->J, most);
+        x->cap = (int)std::min<size_t>(std::min(c->J, 64), most);
     else
         x->cap = (int)std::max(std::min<size_t>(2, most),
                                std::min<size_t>(32, (size_t(256) << 20) / per_img));
     const int cap = x->cap, nat = ceil_div((long)cap * Mp, kGM);
+    // From 8 images on (one tile of 64 takes them, 128 rows the forces' weights), where
+    // the four float64 products an element that it saves, 6.2 us a million, are worth
+    // three more launches: M=60, N=300, 48 images (0.9 million) 153 us with it and 119
+    // without; M=189, N=10000, 48 images (92 million) 2106 and 2632.
+    x->many = cap >= 8 && c->J > 1 && (double)cap * M * R >= 4e6;
+    x->kbF = dg_blocks_per_split(x->nkbR, kFlushMin, 1, 2 * x->nct, x->nsm);
+    x->nsF = ceil_div(x->nkbR, x->kbF);
+    const size_t two = x->many ? 2 : 1, one = x->many ? 1 : 0;
     // about eight W blocks per SM, at most 16 K blocks each
     x->per = (int)std::max<long>(1, std::min<long>(16, x->nkbR * nat / (152L * 8)));
     x->nfc = ceil_div(x->nkbR, x->per);
@@ -548,20 +709,27 @@ int digits_prepare(tdscha_ctx *c) {
     std::vector<Part> parts = {
         {(void **)&x->dt, d * elems, false},
         {(void **)&x->gt, d * elems, false},
-        {(void **)&x->xa, 2 * kRes * elems, false},
-        {(void **)&x->xb, 2 * kRes * elems, false},
-        {(void **)&x->er, i4 * x->Rp, false},
+        {(void **)&x->xa, two * 2 * kRes * elems, false},
+        {(void **)&x->xb, two * 2 * kRes * elems, false},
+        {(void **)&x->er, two * i4 * x->Rp, false},
+        {(void **)&x->st, one * d * 2 * cap * x->Rp, false},
+        {(void **)&x->gf, one * d * x->nsF * kGM * 2 * Mp, false},
+        {(void **)&x->bmap, one * i4 * 2 * nrt, false},
         {(void **)&x->qp, d * 4 * x->nct * (size_t)cap * R, false},
-        {(void **)&x->abcc, sizeof(RowScalars) * (size_t)cap * x->Rp, false},
+        {(void **)&x->abcc, d * 4 * (size_t)cap * x->Rp, false},
         {(void **)&x->gpart, gbytes, false},
         {(void **)&x->fpart, d * (size_t)cap * x->nfc * M, false},
         {(void **)&x->fo, c->J == 1 ? d * cap * M : 0, false},
         {(void **)&x->d2vo, c->J == 1 ? d * (size_t)cap * M * M : 0, false},
-        {(void **)&x->ec, i4 * Mp, false},
+        {(void **)&x->ec, two * i4 * Mp, false},
         // zero from the start: maxima, and the rows of padding modes
         {(void **)&x->dmax, u8 * Mp, true},
         {(void **)&x->gmax, u8 * Mp, true},
-        {(void **)&x->absmax, u8 * 2 * cap, true},
+        {(void **)&x->absmax, u8 * 4 * cap, true},
+        {(void **)&x->etv, one * i4 * 2 * kGN, true},
+        {(void **)&x->ewf, one * i4 * kGM, true},
+        {(void **)&x->vb, one * 2 * (size_t)x->nkbM * kCall * kGB, true},
+        {(void **)&x->wf, one * (size_t)x->nkbR * kCall * kGA, true},
         {(void **)&x->vs, d * cap * Mp, true},
         {(void **)&x->vt, d * cap * Mp, true},
         {(void **)&x->et, i4 * cap * Mp, true},
@@ -620,6 +788,22 @@ int digits_prepare(tdscha_ctx *c) {
     TDS_CHECK_LAUNCH();
     k_dg_windows<<<dim3(x->nct, kFlushes), kGN>>>(nrm, (int)x->nkbR, fl + kFlushes * kRes);
     TDS_CHECK_LAUNCH();
+    if (x->many) {
+        __half *ga = x->xa + kRes * elems, *gb = x->xb + kRes * elems;
+        int *ecg = x->ec + Mp, *erg = x->er + x->Rp;
+        k_dg_colexp<<<ceil_div(Mp, 128), 128>>>(x->gmax, M, Mp, ecg);
+        TDS_CHECK_LAUNCH();
+        k_dg_rowexp<<<(unsigned)nrt, dim3(128, 8)>>>(x->gt, ecg, M, Mp, erg);
+        TDS_CHECK_LAUNCH();
+        k_dg_ga<<<dim3((unsigned)nrt, x->nkbM), 256>>>(x->gt, ecg, erg, M, Mp, x->nkbM, ga);
+        TDS_CHECK_LAUNCH();
+        k_dg_xb<<<dim3((unsigned)x->nkbR, x->nct), 256>>>(x->gt, ecg, Mp, x->nkbR, gb, nrm);
+        TDS_CHECK_LAUNCH();
+        std::vector<int> bm(2 * nrt, 0);
+        std::fill(bm.begin() + nrt, bm.end(), 1);
+        TDS_CUDA(cudaMemcpy(x->bmap, bm.data(), i4 * 2 * nrt, cudaMemcpyHostToDevice));
+        TDS_CUDA((dg_setup<DG_STORE, false>()));
+    }
     TDS_CUDA(cudaMemsetAsync(nrm, 0, sizeof(float) * kRes * (elems / kGK), 0));
     float h_fl[2 * kFlushes * kRes];
     TDS_CUDA(cudaMemcpy(h_fl, fl, sizeof(h_fl), cudaMemcpyDeviceToHost));
@@ -650,9 +834,29 @@ static int digits_contract(tdscha_ctx *c, int nimg, const DgSources &src, int ap
     const long R = c->Nrows;
     {
         ProfScope ps(c, 5, st);
-        TDS_CUDA(launch_pdl(k_dg_y1, dim3(M, nimg), 128, sizeof(double) * M, st, src,
-                            (const double *)c->fY, (const int *)x->ec, M, Mp, x->yb, x->et, x->vs,
-                            x->vt, x->absmax));
+        TDS_CUDA(launch_pdl(k_dg_y1, dim3(x->many ? M + 2 : M, nimg), 128, sizeof(double) * M, st,
+                            src, (const double *)c->fY, (const int *)x->ec, M, Mp, x->yb, x->et,
+                            x->vs, x->vt, x->vb, x->etv, x->absmax));
+        if (x->many) {
+            // s and t of all images: [x; g] times their vectors
+            DgArgs g{};
+            g.a = x->xa;
+            g.b = x->vb;
+            g.nkb = g.kbps = x->nkbM;
+            g.flush = kFlushMin;
+            g.nat = (int)(2 * x->Rp / kGM);
+            g.nbt = 1;
+            g.nitems = g.nat;
+            g.bmap = x->bmap;
+            g.err = x->err;
+            g.budget = x->budget;
+            g.et = x->etv;
+            g.er = x->er;
+            g.R = 2 * x->Rp;
+            g.M = nimg;
+            g.out = x->st;
+            TDS_CUDA((dg_launch<DG_STORE, false>(g, x->nsm, st)));
+        }
     }
     DgArgs ga{};
     ga.a = x->xa;
@@ -670,7 +874,7 @@ static int digits_contract(tdscha_ctx *c, int nimg, const DgSources &src, int ap
     ga.budget = x->budget;
     ga.dt = x->dt;
     ga.gt = x->gt;
-    ga.vs = x->vs;
+    ga.vs = x->many ? nullptr : x->vs;
     ga.vt = x->vt;
     ga.et = x->et;
     ga.qp = x->qp;
@@ -684,20 +888,29 @@ static int digits_contract(tdscha_ctx *c, int nimg, const DgSources &src, int ap
     }
     {
         ProfScope ps(c, 1, st);
-        TDS_CUDA(launch_pdl(k_dg_rows, dim3((unsigned)(x->Rp / 128), nimg), 128, 0, st,
-                            (const double *)x->qp, x->nct, R, x->Rp, c->rho_div,
+        TDS_CUDA(launch_pdl(x->many ? k_dg_rows<true> : k_dg_rows<false>, dim3((unsigned)(x->Rp / 128), nimg), 128, 0, st,
+                            (const double *)x->qp, (const double *)x->st,
+                            x->nct, R, x->Rp, c->rho_div,
                             (const double *)c->rho, (const int *)x->er, apply_d4, x->abcc,
                             x->absmax));
     }
     const int nat = ceil_div((long)nimg * Mp, kGM);
     {
         ProfScope ps(c, 2, st);
-        TDS_CUDA(launch_pdl(k_dg_wbuild, dim3(x->nfc, nat), 256, 0, st, (const double *)x->dt,
-                            (const double *)x->gt, (const RowScalars *)x->abcc,
-                            (const unsigned long long *)x->absmax,
-                            (const unsigned long long *)x->dmax,
-                            (const unsigned long long *)x->gmax, (const double *)c->fY, M, Mp,
-                            x->Rp, nimg, x->nkbR, x->per, x->wa, x->ew, x->fpart));
+        if (x->many)
+            TDS_CUDA(launch_pdl(k_dg_wimages, dim3(x->nkbR, Mp / 32 + 1, ceil_div(nimg, kWImages)), 256,
+                                0, st, (const double *)x->dt, (const double *)x->gt,
+                                (const double *)x->abcc, (const unsigned long long *)x->absmax,
+                                (const unsigned long long *)x->dmax,
+                                (const unsigned long long *)x->gmax, M, Mp, x->Rp, nimg, x->nkbR,
+                                x->wa, x->ew, x->wf, x->ewf));
+        else
+            TDS_CUDA(launch_pdl(k_dg_wbuild, dim3(x->nfc, nat), 256, 0, st, (const double *)x->dt,
+                                (const double *)x->gt, (const double *)x->abcc,
+                                (const unsigned long long *)x->absmax,
+                                (const unsigned long long *)x->dmax,
+                                (const unsigned long long *)x->gmax, (const double *)c->fY, M, Mp,
+                                x->Rp, nimg, x->nkbR, x->per, x->wa, x->ew, x->fpart));
     }
     DgArgs gb{};
     gb.a = x->wa;
@@ -725,6 +938,25 @@ static int digits_contract(tdscha_ctx *c, int nimg, const DgSources &src, int ap
     ProfScope ps(c, 3, st);
     TDS_CUDA((M <= 32 ? dg_launch<DG_PARTS, true>(gb, x->nsm, st)
                       : dg_launch<DG_PARTS, false>(gb, x->nsm, st)));
+    if (x->many) {
+        // the forces: the weights' rows times [x | g]
+        DgArgs g = gb;
+        g.a = x->wf;
+        g.kbps = x->kbF;
+        g.flush = kFlushMin;
+        g.nat = 1;
+        g.nbt = 2 * x->nct;
+        g.nitems = (long)g.nbt * x->nsF;
+        g.Mp = g.M = 2 * Mp;
+        g.ew = x->ewf;
+        g.gpart = x->gf;
+        g.rmod = kGM;
+        g.rlive = kGM;
+        g.rows_b = kGM;
+        TDS_CUDA((dg_launch<DG_PARTS, false>(g, x->nsm, st)));
+        TDS_CUDA(launch_pdl(k_dg_force, dim3(ceil_div(M, 128), nimg), 128, 0, st,
+                            (const double *)x->gf, x->nsF, M, Mp, (const double *)c->fY, x->fpart));
+    }
     return TDSCHA_OK;
 }
 
@@ -770,7 +1002,7 @@ int perturb_digits(tdscha_ctx *c, int apply_d4, cudaStream_t st) {
         TDS_TRY(digits_contract(c, nj, {{s}, 1}, apply_d4, &ns, st));
         const int nat = ceil_div((long)nj * Mp, kGM);
         TDS_TRY(psi_hsum64(c, x->gpart, ns, (long)nat * kGM * Mp, (long)Mp * Mp, Mp, x->fpart,
-                           x->nfc, c->fY, j0, nj, st));
+                           x->many ? 1 : x->nfc, c->fY, j0, nj, st));
     }
     return psi_reduce64(c, st);
 }

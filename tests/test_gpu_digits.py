@@ -176,3 +176,39 @@ def test_projection_edges_against_oracle(gpu_lib, N, n, M):
     u[0, 1] = np.nan
     X, Y = project_modes(u, f, masses, pols, mean, u_scale=0.5, f_scale=2.0)
     assert np.isnan(X[0]).all() and np.isfinite(X[1:]).all() and np.isfinite(Y).all()
+
+
+@pytest.mark.parametrize("M,N,S", [(189, 460, 48), (192, 900, 24), (252, 2100, 8), (129, 1300, 24)])
+@pytest.mark.parametrize("d4", [0, 1])
+def test_many_images(gpu_lib, M, N, S, d4):
+    """From 8 images and 4 million elements on: the row scalars and the forces as
+    products of their own.  N S <= 3.2e4 here: 7e-13 by the estimate above."""
+    ens = make_ensemble(M, N, seed=M, n_syms=S, rho_sigma=0.1)
+    assert min(S, 64) * M * N >= 4e6
+    R1, Y1 = random_R1(M, 1), random_sym(M, 2, scale=1e-3)
+    ref = oracle.perturb_averages(ens["X"], ens["Y"], ens["w"], ens["rho"], R1, Y1, ens["T"], d4,
+                                  *_tables(ens, M), n_threads=8)
+    ctx = _context(ens)
+    got = _call(ctx, R1, Y1, d4)
+    ctx.close()
+    assert _rel(got[1], ref[1]) < TOL
+    assert np.abs(got[0] - ref[0]).max() < TOL * max(np.abs(ref[0]).max(), 1e-300)
+
+
+def test_many_images_matches_core_kernels(gpu_lib, monkeypatch):
+    """Zero and non-finite perturbations, a scaled ensemble, a repeated call."""
+    ens = make_ensemble(63, 1400, seed=3, n_syms=48, rho_sigma=0.1)
+    R1, Y1 = random_R1(63, 1), random_sym(63, 2, scale=1e-3)
+    ctx, cores = _context(ens), _context(ens, monkeypatch, cores=True)
+    for r, y in ((R1, Y1), (R1 * 0, Y1), (R1, Y1 * 0), (R1 * 1e100, Y1), (R1, Y1 * 1e-200), (R1, Y1)):
+        a, b = _call(ctx, r, y), _call(cores, r, y)
+        for u, v in zip(a, b):
+            assert np.abs(u - v).max() <= 3e-12 * np.abs(v).max()     # N S = 6.7e4 on both sides
+    for bad in (np.nan, np.inf):
+        y = Y1.copy()
+        y[3, 5] = y[5, 3] = bad
+        a, b = _call(ctx, R1, y), _call(cores, R1, y)
+        for u, v in zip(a, b):
+            assert (np.isfinite(u) == np.isfinite(v)).all()
+    ctx.close()
+    cores.close()
