@@ -377,17 +377,59 @@ enum { ST_OK = 0, ST_NAN = 1, ST_CONV = 2 };
 
 constexpr int kDotThreads = 256;
 
-__device__ __forceinline__ double block_sum(double v, double *sh) {
+// Float64 runs at one operation a warp per 64 cycles and subcore here, however few of
+// its lanes take part (measured), so the sums below are short of operations rather than
+// of lanes: K sums share one shuffle tree, warps that hold zeros only are left out, and
+// the serial ends run side by side in lanes.  Every sum keeps the order of its own tree
+// (lane l + lane l ^ o, o = 16 .. 1, then the warps in order) and with it its bits.
+// k_resid_bc at 2400 elements: 11.8 us with one tree after the other, 8.6 so.
+
+// K <= 4 sums over the warp's lanes, in lanes 0, 16, 8, 24
+template <int K>
+__device__ __forceinline__ double warp_sums(const double (&v)[K]) {
+    const int lane = threadIdx.x & 31;
+    // two sums through one step: half the lanes add up one, half the other
+    auto fold = [&](double a, double b, int o) {
+        const bool up = lane & o;
+        const double got = __shfl_xor_sync(0xffffffffu, up ? a : b, o);
+        return (up ? b : a) + got;
+    };
+    double x = K > 1 ? fold(v[0], v[K > 1 ? 1 : 0], 16) : v[0] + __shfl_xor_sync(0xffffffffu, v[0], 16);
+    if (K > 2) {
+        const double c = v[K > 2 ? 2 : 0];
+        const double y = K > 3 ? fold(c, v[K > 3 ? 3 : 0], 16) : c + __shfl_xor_sync(0xffffffffu, c, 16);
+        x = fold(x, y, 8);
+    } else {
+        x += __shfl_xor_sync(0xffffffffu, x, 8);
+    }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    for (int o = 4; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    return x;
+}
+
+// K sums over the block, of which only the first nw warps hold anything; sum k in
+// thread k.  sh: K x 32
+template <int K>
+__device__ __forceinline__ double block_sums(const double (&v)[K], double *sh, int nw) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     __syncthreads();
-    if (lane == 0) sh[wid] = v;
+    if (wid < nw) {
+        const double x = warp_sums(v);
+        constexpr int at[4] = {0, 16, 8, 24};
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+            if (lane == at[k]) sh[32 * k + wid] = x;
+    }
     __syncthreads();
     double s = 0;
-    if (threadIdx.x == 0)
-        for (int k = 0; k < (int)(blockDim.x >> 5); ++k) s += sh[k];
-    return s;   // valid in thread 0
+    if (threadIdx.x < K)
+        for (int k = 0; k < nw; ++k) s += sh[32 * threadIdx.x + k];
+    return s;
+}
+
+__device__ __forceinline__ double block_sum(double v, double *sh) {
+    const double a[1] = {v};
+    return block_sums<1>(a, sh, blockDim.x >> 5);   // valid in thread 0
 }
 
 // y * mask[e], or y where there is no mask.  The kernels below take the mask
@@ -413,35 +455,42 @@ __device__ __forceinline__ double dot1_range(const double *__restrict__ x,
 __global__ void k_dot1(const double *__restrict__ x, const double *__restrict__ y,
                        const double *__restrict__ mask, long n, double *__restrict__ part) {
     pdl_enter();
-    __shared__ double sh[32];
+    __shared__ double sh[96];
     double acc = mask ? dot1_range<true>(x, y, mask, n) : dot1_range<false>(x, y, mask, n);
     double s = block_sum(acc, sh);
     if (threadIdx.x == 0) part[blockIdx.x] = s;
 }
 
-// Sum of nblk block partials by one block (fixed order: thread stride, then tree).
-__device__ __forceinline__ double reduce_parts(const double *__restrict__ part, int nblk,
-                                               double *sh) {
-    double v = 0;
-    for (int b = threadIdx.x; b < nblk; b += blockDim.x) v += part[b];
-    return block_sum(v, sh);
+// K sums of nblk block partials each, part[k nblk ..], by one block (fixed order: thread
+// stride, then tree); sum k in thread k
+template <int K>
+__device__ __forceinline__ double reduce_parts(const double *part, int nblk, double *sh) {
+    double v[K] = {};
+    for (int b = threadIdx.x; b < nblk; b += blockDim.x)
+#pragma unroll
+        // written by other blocks, perhaps of this kernel: past the L1
+        for (int k = 0; k < K; ++k) v[k] += __ldcg(part + k * nblk + b);
+    return block_sums<K>(v, sh, min((int)(blockDim.x >> 5), (nblk + 31) / 32));
 }
 
-// a = dot * p_norm and the axpy factors of the residuals (run_FT :6167-6232);
-// one thread
+// a = dot * p_norm and the axpy factors of the residuals (run_FT :6167-6232).  By a whole
+// warp: the two norms divide side by side in lanes 0 and 1.  pnorm, cq and cp do not
+// depend on the dot.
 struct ScalA {
     double a, pnorm, cq, cp;
 };
-__device__ __forceinline__ ScalA scal_a_value(double d, const double *hist, int k) {
-    ScalA v;
-    double c_old = k >= 1 ? hist[4 * (k - 1) + 2] : 1.0;
-    v.pnorm = hist[4 * k + 3] / c_old;
-    v.a = d * v.pnorm;
-    v.cq = v.cp = 0;
+__device__ __forceinline__ ScalA scal_a_norms(const double *hist, int k) {
+    const int one = threadIdx.x & 1, j = k - one;      // norms of steps k and k - 1
+    ScalA v = {0, 0, 0, 0};
+    double x = 0, c = 1.0;
+    if (j >= 0) x = hist[4 * j + 3];
+    if (j >= 1) c = hist[4 * (j - 1) + 2];
+    const double norm = x / c;
+    v.pnorm = __shfl_sync(0xffffffffu, norm, 0);
+    const double old = __shfl_sync(0xffffffffu, norm, 1);
     if (k >= 1) {
         v.cq = hist[4 * (k - 1) + 2];
-        double old_p_norm = (k < 2) ? hist[4 * (k - 1) + 3] : hist[4 * (k - 1) + 3] / hist[4 * (k - 2) + 2];
-        v.cp = hist[4 * (k - 1) + 1] * (old_p_norm / v.pnorm);
+        v.cp = hist[4 * (k - 1) + 1] * (old / v.pnorm);
     }
     return v;
 }
@@ -454,28 +503,27 @@ __device__ __forceinline__ void scal_a_store(const ScalA &v, int k, double *scal
     scal[SC_CQ] = v.cq;
     scal[SC_CP] = v.cp;
 }
-__device__ __forceinline__ void scal_a_body(double d, const double *__restrict__ hist, int k,
-                                            double *__restrict__ scal,
-                                            double *__restrict__ status) {
-    if (scal[SC_HALT] != 0.0) return;
-    scal_a_store(scal_a_value(d, hist, k), k, scal, status);
+// From the dot in thread 0 of a block; warp 1 has divided meanwhile
+__device__ __forceinline__ void scal_a_finish(double d, const double *hist, int k, double *scal,
+                                              double *status) {
+    __shared__ ScalA v;
+    if (threadIdx.x >> 5 == 1) {
+        const ScalA n = scal_a_norms(hist, k);
+        if ((threadIdx.x & 31) == 0) v = n;
+    }
+    __syncthreads();
+    if (threadIdx.x || scal[SC_HALT] != 0.0) return;
+    ScalA w = v;
+    w.a = d * w.pnorm;
+    scal_a_store(w, k, scal, status);
 }
 
 __global__ void k_scal_a(const double *__restrict__ part, int nblk, const double *__restrict__ hist,
                          int k, double *__restrict__ scal, double *__restrict__ status) {
     pdl_enter();
-    __shared__ double sh[32];
-    double d = reduce_parts(part, nblk, sh);
-    if (threadIdx.x == 0) scal_a_body(d, hist, k, scal, status);
-}
-
-// Sum of nblk block partials written by other blocks of the same kernel:
-// loads from L2 (this SM's L1 may hold the buffer from an earlier step)
-__device__ __forceinline__ double reduce_parts_cg(const double *__restrict__ part, int nblk,
-                                                  double *sh) {
-    double v = 0;
-    for (int b = threadIdx.x; b < nblk; b += blockDim.x) v += __ldcg(part + b);
-    return block_sum(v, sh);
+    __shared__ double sh[96];
+    const double d = reduce_parts<1>(part, nblk, sh);
+    scal_a_finish(d, hist, k, scal, status);
 }
 
 // Whether this block is the last of the grid to have written its partials
@@ -483,6 +531,7 @@ __device__ __forceinline__ double reduce_parts_cg(const double *__restrict__ par
 // of the separate reduction kernel and resets the counter for the next launch.
 // No block waits for another.
 __device__ __forceinline__ bool last_block(unsigned *__restrict__ ctr, bool *flag) {
+    __syncwarp();                 // (threads of warp 0 wrote them)
     if (threadIdx.x == 0) {
         __threadfence();
         *flag = atomicAdd(ctr, 1u) == gridDim.x - 1;
@@ -498,17 +547,15 @@ __global__ void k_dot1_a(const double *__restrict__ x, const double *__restrict_
                          const double *__restrict__ hist, int k, double *__restrict__ scal,
                          double *__restrict__ status, unsigned *__restrict__ ctr) {
     pdl_enter();
-    __shared__ double sh[32];
+    __shared__ double sh[96];
     __shared__ bool flag;
     double acc = mask ? dot1_range<true>(x, y, mask, n) : dot1_range<false>(x, y, mask, n);
     double s = block_sum(acc, sh);
     if (threadIdx.x == 0) part[blockIdx.x] = s;
     if (!last_block(ctr, &flag)) return;
-    const double d = reduce_parts_cg(part, gridDim.x, sh);
-    if (threadIdx.x == 0) {
-        *ctr = 0u;
-        scal_a_body(d, hist, k, scal, status);
-    }
+    const double d = reduce_parts<1>(part, gridDim.x, sh);
+    if (threadIdx.x == 0) *ctr = 0u;
+    scal_a_finish(d, hist, k, scal, status);
 }
 
 template <bool kMasked>
@@ -542,32 +589,35 @@ __global__ void k_resid(const double *__restrict__ Lq, const double *__restrict_
                         double *__restrict__ rk, double *__restrict__ sk, double *__restrict__ part,
                         int nblk) {
     pdl_enter();
-    __shared__ double sh[32];
+    __shared__ double sh[96];
     double ss = 0, rr = 0, sr = 0;
     if (mask)
         resid_range<true>(Lq, pL, q, p, qprev, pprev, mask, scal, n, rk, sk, ss, rr, sr);
     else
         resid_range<false>(Lq, pL, q, p, qprev, pprev, mask, scal, n, rk, sk, ss, rr, sr);
-    double t;
-    t = block_sum(ss, sh); if (threadIdx.x == 0) part[blockIdx.x] = t;
-    t = block_sum(rr, sh); if (threadIdx.x == 0) part[nblk + blockIdx.x] = t;
-    t = block_sum(sr, sh); if (threadIdx.x == 0) part[2 * nblk + blockIdx.x] = t;
+    const double v[3] = {ss, rr, sr};
+    const double t = block_sums<3>(v, sh, blockDim.x >> 5);
+    if (threadIdx.x < 3) part[threadIdx.x * nblk + blockIdx.x] = t;
 }
 
-// b, c, the new s_norm and the stop test (run_FT :6233-6306); one thread
+// b, c, the new s_norm and the stop test (run_FT :6233-6306)
 struct ScalBC {
     double b, c, snorm, sraw, ib, is;
     bool conv;
 };
-__device__ __forceinline__ ScalBC scal_bc_value(double ss, double rr, double sr, double pnorm,
-                                                double next) {
+// by a whole warp, lanes 0, 1, 2 with ss, rr, sr: the roots and the quotients side by side
+__device__ __forceinline__ ScalBC scal_bc_value(double sum, double pnorm, double next) {
+    const int lane = threadIdx.x & 31;
     ScalBC v;
-    v.sraw = sqrt(ss);
+    const double root = sqrt(sum);
+    v.sraw = __shfl_sync(0xffffffffu, root, 0);
+    v.b = __shfl_sync(0xffffffffu, root, 1);
+    const double quot = (lane == 2 ? sum : 1.0) /
+                        (lane == 0 ? v.sraw : lane == 1 ? v.b : v.sraw * v.b);
+    v.is = __shfl_sync(0xffffffffu, quot, 0);
+    v.ib = __shfl_sync(0xffffffffu, quot, 1);
     v.snorm = v.sraw * pnorm;
-    v.b = sqrt(rr);
-    v.c = (sr / (v.sraw * v.b)) * v.snorm;
-    v.ib = 1.0 / v.b;
-    v.is = 1.0 / v.sraw;
+    v.c = __shfl_sync(0xffffffffu, quot, 2) * v.snorm;
     v.conv = fabs(v.b) < kEps || fabs(v.c) < kEps || next != 0.0;
     return v;
 }
@@ -591,23 +641,19 @@ __device__ __forceinline__ void scal_bc_store(const ScalBC &v, double a, double 
         hist[4 * (k + 1) + 3] = v.snorm;
     }
 }
-__device__ __forceinline__ void scal_bc_body(double ss, double rr, double sr,
-                                             double *__restrict__ hist, int k,
-                                             double *__restrict__ scal,
-                                             double *__restrict__ status) {
-    if (scal[SC_HALT] != 0.0) return;
-    scal_bc_store(scal_bc_value(ss, rr, sr, scal[SC_PNORM], scal[SC_NEXT]), scal[SC_A], hist, k, scal,
-                  status);
+__device__ __forceinline__ void scal_bc_finish(double sum, double *hist, int k, double *scal,
+                                               double *status) {
+    if (threadIdx.x >= 32 || scal[SC_HALT] != 0.0) return;
+    const ScalBC v = scal_bc_value(sum, scal[SC_PNORM], scal[SC_NEXT]);
+    if (threadIdx.x == 0) scal_bc_store(v, scal[SC_A], hist, k, scal, status);
 }
 
 __global__ void k_scal_bc(const double *__restrict__ part, int nblk, double *__restrict__ hist,
                           int k, double *__restrict__ scal, double *__restrict__ status) {
     pdl_enter();
-    __shared__ double sh[32];
-    double ss = reduce_parts(part, nblk, sh);
-    double rr = reduce_parts(part + nblk, nblk, sh);
-    double sr = reduce_parts(part + 2 * nblk, nblk, sh);
-    if (threadIdx.x == 0) scal_bc_body(ss, rr, sr, hist, k, scal, status);
+    __shared__ double sh[96];
+    const double sum = reduce_parts<3>(part, nblk, sh);
+    scal_bc_finish(sum, hist, k, scal, status);
 }
 
 // k_resid and k_scal_bc in one launch (the real-space recurrence)
@@ -619,7 +665,7 @@ __global__ void k_resid_bc(const double *__restrict__ Lq, const double *__restri
                            double *__restrict__ part, double *__restrict__ hist, int k,
                            double *__restrict__ status, unsigned *__restrict__ ctr) {
     pdl_enter();
-    __shared__ double sh[32];
+    __shared__ double sh[96];
     __shared__ bool flag;
     const int nblk = gridDim.x;
     double ss = 0, rr = 0, sr = 0;
@@ -627,18 +673,13 @@ __global__ void k_resid_bc(const double *__restrict__ Lq, const double *__restri
         resid_range<true>(Lq, pL, q, p, qprev, pprev, mask, scal, n, rk, sk, ss, rr, sr);
     else
         resid_range<false>(Lq, pL, q, p, qprev, pprev, mask, scal, n, rk, sk, ss, rr, sr);
-    double t;
-    t = block_sum(ss, sh); if (threadIdx.x == 0) part[blockIdx.x] = t;
-    t = block_sum(rr, sh); if (threadIdx.x == 0) part[nblk + blockIdx.x] = t;
-    t = block_sum(sr, sh); if (threadIdx.x == 0) part[2 * nblk + blockIdx.x] = t;
+    const double v[3] = {ss, rr, sr};
+    const double t = block_sums<3>(v, sh, blockDim.x >> 5);
+    if (threadIdx.x < 3) part[threadIdx.x * nblk + blockIdx.x] = t;
     if (!last_block(ctr, &flag)) return;
-    const double a = reduce_parts_cg(part, nblk, sh);
-    const double b = reduce_parts_cg(part + nblk, nblk, sh);
-    const double c = reduce_parts_cg(part + 2 * nblk, nblk, sh);
-    if (threadIdx.x == 0) {
-        *ctr = 0u;
-        scal_bc_body(a, b, c, hist, k, scal, status);
-    }
+    const double sum = reduce_parts<3>(part, nblk, sh);
+    if (threadIdx.x == 0) *ctr = 0u;
+    scal_bc_finish(sum, hist, k, scal, status);
 }
 
 // ---------------------------------------------------------------------------
@@ -733,7 +774,7 @@ __global__ void k_proj_dots(const double *__restrict__ Qb, const double *__restr
                             const double *__restrict__ mask, long n, long ld,
                             double *__restrict__ part) {
     pdl_enter();
-    __shared__ double sh[32];
+    __shared__ double sh[96];
     int j = blockIdx.x;
     const long nch = gridDim.y;
     long e0 = n * blockIdx.y / nch, e1 = n * (blockIdx.y + 1) / nch;
@@ -743,22 +784,21 @@ __global__ void k_proj_dots(const double *__restrict__ Qb, const double *__restr
         proj_dots_range<true>(pj, qj, qn, pn, mask, e0, e1, a, b);
     else
         proj_dots_range<false>(pj, qj, qn, pn, mask, e0, e1, a, b);
-    double t = block_sum(a, sh);
-    if (threadIdx.x == 0) part[((long)j * nch + blockIdx.y) * 2] = t;
-    t = block_sum(b, sh);
-    if (threadIdx.x == 0) part[((long)j * nch + blockIdx.y) * 2 + 1] = t;
+    const double v[2] = {a, b};
+    const double t = block_sums<2>(v, sh, blockDim.x >> 5);
+    if (threadIdx.x < 2) part[((long)j * nch + blockIdx.y) * 2 + threadIdx.x] = t;
 }
 
-// Sum of the nch chunk partials part[(j * nch + c) * stride + off] by one warp
-// (lane-strided, then a fixed shuffle tree): the same order on every run.
-__device__ __forceinline__ double warp_chunk_sum(const double *__restrict__ part, long j, int nch,
-                                                 int stride, int off) {
+// Sums of the nch chunk partials part[(j * nch + c) * K + k], k < K, by one warp
+// (lane-strided, then a fixed shuffle tree: the same order on every run), in lanes 0, 16
+template <int K>
+__device__ __forceinline__ double warp_chunk_sums(const double *__restrict__ part, long j, int nch) {
     const int lane = threadIdx.x & 31;
-    double a = 0;
-    for (int c = lane; c < nch; c += 32) a += part[(j * nch + c) * stride + off];
+    double a[K] = {};
+    for (int c = lane; c < nch; c += 32)
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-    return a;
+        for (int k = 0; k < K; ++k) a[k] += part[(j * nch + c) * K + k];
+    return warp_sums(a);
 }
 
 // coef[2j], coef[2j+1] = chunk sums / (p_j . q_j); one warp per j
@@ -767,13 +807,8 @@ __global__ void k_proj_scale(const double *__restrict__ part, const double *__re
     pdl_enter();
     const int j = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (j >= nvec) return;   // whole warps
-    double a = warp_chunk_sum(part, j, nch, 2, 0);
-    double b = warp_chunk_sum(part, j, nch, 2, 1);
-    if ((threadIdx.x & 31) == 0) {
-        double inv = 1.0 / pqn[j];
-        coef[2 * j] = a * inv;
-        coef[2 * j + 1] = b * inv;
-    }
+    const double c = warp_chunk_sums<2>(part, j, nch) * (1.0 / pqn[j]);
+    if ((threadIdx.x & 15) == 0) coef[2 * j + ((threadIdx.x & 31) >> 4)] = c;
 }
 
 constexpr int kProjMax = 2048;   // coefficients cached in shared memory per pass
@@ -785,7 +820,7 @@ __global__ void k_proj_apply(const double *__restrict__ Qb, const double *__rest
                              const double *__restrict__ mask, double *__restrict__ pq_part) {
     pdl_enter();
     __shared__ double cs[2 * kProjMax];
-    __shared__ double sh[32];
+    __shared__ double sh[96];
     for (int t = threadIdx.x; t < 2 * nvec; t += blockDim.x) cs[t] = coef[2 * j0 + t];
     __syncthreads();
     double pq = 0;
@@ -833,7 +868,7 @@ __global__ void k_rdots(const double *__restrict__ Qb, const double *__restrict_
                         const float2 *__restrict__ vs, long n, long ldv, long ld,
                         double *__restrict__ part) {
     pdl_enter();
-    __shared__ double sh[32];
+    __shared__ double sh[96];
     const int j = blockIdx.x;
     const long nch = gridDim.y;
     const long e0 = n * blockIdx.y / nch, e1 = n * (blockIdx.y + 1) / nch;
@@ -863,10 +898,9 @@ __global__ void k_rdots(const double *__restrict__ Qb, const double *__restrict_
         df_fma_acc(as, ac, split_f64(pj[e]), qm[e]);
         df_fma_acc(bs, bc, split_f64(qj[e]), pm[e]);
     }
-    double t = block_sum((double)as + (double)ac, sh);
-    if (threadIdx.x == 0) part[((long)j * nch + blockIdx.y) * 2] = t;
-    t = block_sum((double)bs + (double)bc, sh);
-    if (threadIdx.x == 0) part[((long)j * nch + blockIdx.y) * 2 + 1] = t;
+    const double v[2] = {(double)as + (double)ac, (double)bs + (double)bc};
+    const double t = block_sums<2>(v, sh, blockDim.x >> 5);
+    if (threadIdx.x < 2) part[((long)j * nch + blockIdx.y) * 2 + threadIdx.x] = t;
 }
 
 // coef[j] = split(c_j), split(d_j) with c_j, d_j = chunk sums / (p_j . q_j)
@@ -876,13 +910,8 @@ __global__ void k_rscale(const double *__restrict__ part, const double *__restri
     pdl_enter();
     const int j = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (j >= nvec) return;   // whole warps
-    double a = warp_chunk_sum(part, j, nch, 2, 0);
-    double b = warp_chunk_sum(part, j, nch, 2, 1);
-    if ((threadIdx.x & 31) == 0) {
-        const double inv = 1.0 / pqn[j];
-        const float2 c = split_f64(a * inv), d = split_f64(b * inv);
-        coef[j] = make_float4(c.x, c.y, d.x, d.y);
-    }
+    const float2 c = split_f64(warp_chunk_sums<2>(part, j, nch) * (1.0 / pqn[j]));
+    if ((threadIdx.x & 15) == 0) reinterpret_cast<float2 *>(coef + j)[(threadIdx.x & 31) >> 4] = c;
 }
 
 constexpr int kRProjMax = 1024;   // coefficients per apply pass (16 KB of shared memory)
@@ -899,7 +928,7 @@ __global__ void __launch_bounds__(256) k_rapply(const double *__restrict__ Qb,
                                                 double *__restrict__ pq_part) {
     pdl_enter();
     __shared__ float4 cs[kRProjMax];
-    __shared__ double sh[32];
+    __shared__ double sh[96];
     for (int t = threadIdx.x; t < nvec; t += blockDim.x) cs[t] = coef[j0 + t];
     __syncthreads();
     const double *Q0 = Qb + (long)j0 * ld, *P0 = Pb + (long)j0 * ld;
@@ -955,7 +984,7 @@ __global__ void k_rdots2(const double *__restrict__ Qb, const double *__restrict
                          const float2 *__restrict__ vs, long n, long ldv, long ld,
                          double *__restrict__ part) {
     pdl_enter();
-    __shared__ double sh[32];
+    __shared__ double sh[96];
     const int j = blockIdx.x;
     const long nch = gridDim.y, npair = n >> 1;
     const long i0 = npair * blockIdx.y / nch, i1 = npair * (blockIdx.y + 1) / nch;
@@ -999,10 +1028,9 @@ __global__ void k_rdots2(const double *__restrict__ Qb, const double *__restrict
         df_fma_acc(as, ac, split_f64(pj[e]), vs[e]);
         df_fma_acc(bs, bc, split_f64(qj[e]), vs[ldv + e]);
     }
-    double t = block_sum((double)as + (double)ac, sh);
-    if (threadIdx.x == 0) part[((long)j * nch + blockIdx.y) * 2] = t;
-    t = block_sum((double)bs + (double)bc, sh);
-    if (threadIdx.x == 0) part[((long)j * nch + blockIdx.y) * 2 + 1] = t;
+    const double v[2] = {(double)as + (double)ac, (double)bs + (double)bc};
+    const double t = block_sums<2>(v, sh, blockDim.x >> 5);
+    if (threadIdx.x < 2) part[((long)j * nch + blockIdx.y) * 2 + threadIdx.x] = t;
 }
 
 // k_rapply over tiles of 64 elements, one tile per block: lane l of warp w
@@ -1019,7 +1047,7 @@ __global__ void __launch_bounds__(32 * kTileWarps) k_rapply2(
     pdl_enter();
     __shared__ float4 cs[kRProjMax];
     __shared__ float4 red[kTileWarps][64];
-    __shared__ double sh[32];
+    __shared__ double sh[96];
     for (int t = threadIdx.x; t < nvec; t += blockDim.x) cs[t] = coef[j0 + t];
     __syncthreads();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -1084,7 +1112,8 @@ __global__ void __launch_bounds__(32 * kTileWarps) k_rapply2(
         }
     }
     if (pq_part) {
-        const double t = block_sum(pq, sh);
+        const double v[1] = {pq};
+        const double t = block_sums<1>(v, sh, 2);
         if (threadIdx.x == 0) pq_part[blockIdx.x] = t;
     }
 }
@@ -1093,8 +1122,8 @@ __global__ void __launch_bounds__(32 * kTileWarps) k_rapply2(
 __global__ void k_pq_reduce(const double *__restrict__ part, int nblk, double *__restrict__ pqn,
                             int k) {
     pdl_enter();
-    __shared__ double sh[32];
-    double s = reduce_parts(part, nblk, sh);
+    __shared__ double sh[96];
+    double s = reduce_parts<1>(part, nblk, sh);
     if (threadIdx.x == 0) pqn[k] = s;
 }
 
@@ -1102,7 +1131,7 @@ __global__ void k_pq_reduce(const double *__restrict__ part, int nblk, double *_
 __global__ void k_pq_part(const double *__restrict__ Qb, const double *__restrict__ Pb,
                           const double *__restrict__ mask, long n, long ld, int j0,
                           double *__restrict__ part) {
-    __shared__ double sh[32];
+    __shared__ double sh[96];
     int j = j0 + blockIdx.x;
     const long nch = gridDim.y;
     long e0 = n * blockIdx.y / nch, e1 = n * (blockIdx.y + 1) / nch;
@@ -1119,7 +1148,7 @@ __global__ void k_pq_finish(const double *__restrict__ part, int cnt, int j0, in
                             double *__restrict__ out) {
     const int j = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (j >= cnt) return;   // whole warps
-    double a = warp_chunk_sum(part, j, nch, 1, 0);
+    double a = warp_chunk_sums<1>(part, j, nch);
     if ((threadIdx.x & 31) == 0) out[j0 + j] = a;
 }
 
@@ -1129,10 +1158,10 @@ __global__ void k_pq_finish(const double *__restrict__ part, int cnt, int j0, in
 __global__ void k_qrenorm(const double *__restrict__ part, int nblk, double *__restrict__ scal,
                           double *__restrict__ hist, int k, long n, double *__restrict__ qn,
                           double *__restrict__ pn) {
-    __shared__ double sh[32];
+    __shared__ double sh[96];
     __shared__ double inv_s;
     if (scal[SC_HALT] != 0.0) return;
-    double s = reduce_parts(part, nblk, sh);
+    double s = reduce_parts<1>(part, nblk, sh);
     if (threadIdx.x == 0) {
         double nrm = sqrt(s);
         inv_s = 1.0 / nrm;
@@ -1181,43 +1210,53 @@ __device__ __forceinline__ void cluster_barrier() {
                      : "memory");
 }
 
-// block_sum of a group of 256 threads: its sum in the group's thread 0
-__device__ __forceinline__ double group_sum(double v, double *sh) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    const int bar = 1 + (threadIdx.x >> 8), tid = threadIdx.x & 255;
+// block_sums of a group of 256 threads: sum k in the group's thread k.  sh: K x 8
+template <int K>
+__device__ __forceinline__ double group_sums(const double (&v)[K], double *sh) {
+    const int bar = 1 + (threadIdx.x >> 8), tid = threadIdx.x & 255, lane = tid & 31;
+    const double x = warp_sums(v);
     asm volatile("bar.sync %0, 256;" ::"r"(bar) : "memory");
-    if ((tid & 31) == 0) sh[tid >> 5] = v;
+    constexpr int at[4] = {0, 16, 8, 24};
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+        if (lane == at[k]) sh[8 * k + (tid >> 5)] = x;
     asm volatile("bar.sync %0, 256;" ::"r"(bar) : "memory");
     double s = 0;
-    if (tid == 0)
-        for (int k = 0; k < 8; ++k) s += sh[k];
+    if (tid < K)
+        for (int k = 0; k < 8; ++k) s += sh[8 * tid + k];
     return s;
 }
+__device__ __forceinline__ double group_sum(double v, double *sh) {
+    const double a[1] = {v};
+    return group_sums<1>(a, sh);
+}
 
-// Up to three sums of nblk <= 64 partials, part[s nblk ..], by the groups s; out[s] is
-// there after the next __syncthreads.
-__device__ __forceinline__ void sum_parts(const double *part, int nblk, int nsum, double (*sh)[8],
-                                          double *out) {
-    const int g = threadIdx.x >> 8, tid = threadIdx.x & 255, nw = (nblk + 31) / 32;
-    if (g < nsum && tid >> 5 < nw) {
-        double v = tid < nblk ? __ldcg(part + g * nblk + tid) : 0.0;
+// K sums of nblk <= 64 partials, part[k nblk ..], in threads k of the block.  sh: K x 2
+template <int K>
+__device__ __forceinline__ double sum_parts(const double *part, int nblk, double *sh) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = (nblk + 31) / 32;
+    if (warp < nw) {
+        double v[K];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if ((tid & 31) == 0) sh[g][tid >> 5] = v;
+        for (int k = 0; k < K; ++k)
+            v[k] = (int)threadIdx.x < nblk ? __ldcg(part + k * nblk + threadIdx.x) : 0.0;
+        const double x = warp_sums(v);
+        constexpr int at[4] = {0, 16, 8, 24};
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+            if (lane == at[k]) sh[2 * k + warp] = x;
     }
     __syncthreads();
-    if (g < nsum && tid == 0) {
-        double s = 0;
-        for (int k = 0; k < nw; ++k) s += sh[g][k];
-        out[g] = s;
-    }
+    double s = 0;
+    if (threadIdx.x < K)
+        for (int k = 0; k < nw; ++k) s += sh[2 * threadIdx.x + k];
+    return s;
 }
 
 // A group of 256 threads does what a block of k_dot1, k_resid, k_proj_dots ... does.
 // What another thread of the cluster wrote is read past the L1.
 __global__ void __launch_bounds__(1024, 1) k_qrecur(const RecurArgs r) {
-    __shared__ double sh[4][8], sums[4], cd[kShortBasis];
+    __shared__ double sh[4][24], inv_s, cd[kShortBasis];
     __shared__ ScalA sa;
     __shared__ ScalBC sb;
     pdl_enter();
@@ -1254,8 +1293,14 @@ __global__ void __launch_bounds__(1024, 1) k_qrecur(const RecurArgs r) {
         if (tid == 0) r.part[vb] = s;
     }
     cluster_barrier();
-    sum_parts(r.part, r.nblk, 1, sh, sums);
-    if (threadIdx.x == 0) sa = scal_a_value(sums[0], r.hist, r.k);
+    // (warp 4 divides while warp 0 adds up)
+    const double dot = sum_parts<1>(r.part, r.nblk, sh[0]);
+    if (warp == 4) {
+        const ScalA v = scal_a_norms(r.hist, r.k);
+        if (lane == 0) sa = v;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) sa.a = dot * sa.pnorm;
     __syncthreads();
     if (first) scal_a_store(sa, r.k, r.scal, r.status);
     if (isnan(sa.a)) return;
@@ -1273,15 +1318,15 @@ __global__ void __launch_bounds__(1024, 1) k_qrecur(const RecurArgs r) {
             rr += a * (a * m);
             sr += b * (a * m);
         }
-        double t;
-        t = group_sum(ss, sh[g]); if (tid == 0) part2[vb] = t;
-        t = group_sum(rr, sh[g]); if (tid == 0) part2[r.nblk + vb] = t;
-        t = group_sum(sr, sh[g]); if (tid == 0) part2[2 * r.nblk + vb] = t;
+        const double v[3] = {ss, rr, sr}, t = group_sums<3>(v, sh[g]);
+        if (tid < 3) part2[tid * r.nblk + vb] = t;
     }
     cluster_barrier();
-    sum_parts(part2, r.nblk, 3, sh, sums);
-    __syncthreads();
-    if (threadIdx.x == 0) sb = scal_bc_value(sums[0], sums[1], sums[2], sa.pnorm, next);
+    const double sum = sum_parts<3>(part2, r.nblk, sh[0]);
+    if (warp == 0) {
+        const ScalBC v = scal_bc_value(sum, sa.pnorm, next);
+        if (lane == 0) sb = v;
+    }
     __syncthreads();
     if (first) scal_bc_store(sb, sa.a, r.hist, r.k, r.scal, r.status);
     if (sb.conv) return;
@@ -1327,17 +1372,17 @@ __global__ void __launch_bounds__(1024, 1) k_qrecur(const RecurArgs r) {
     }
     cluster_barrier();
     // q_{k+1} / |q_{k+1}|, s_norm_{k+1} = c_k (QSpaceLanczos.py:1110-1125)
-    sum_parts(r.part, r.nblk, 1, sh, sums);
+    const double nsq = sum_parts<1>(r.part, r.nblk, sh[0]);
     if (threadIdx.x == 0) {
-        const double nrm = sqrt(sums[0]);
-        sums[1] = 1.0 / nrm;
+        const double nrm = sqrt(nsq);
+        inv_s = 1.0 / nrm;
         if (first) {
             if (nrm < kEps) r.scal[SC_NEXT] = 1.0;
             r.hist[4 * (r.k + 1) + 3] = sb.c;
         }
     }
     __syncthreads();
-    const double iv = sums[1];
+    const double iv = inv_s;
     for (int vb = v0; vb < r.nblk; vb += nv) {
         double nn = 0;
         for (long e = vb * 256L + tid; e < n; e += step) {
@@ -1351,8 +1396,8 @@ __global__ void __launch_bounds__(1024, 1) k_qrecur(const RecurArgs r) {
     }
     cluster_barrier();
     if (cta) return;
-    sum_parts(part2, r.nblk, 1, sh, sums);
-    if (first) r.pqn[r.k + 1] = sums[0];
+    const double pq = sum_parts<1>(part2, r.nblk, sh[0]);
+    if (first) r.pqn[r.k + 1] = pq;
 }
 
 inline bool short_vector(long n, int nvec) {
@@ -1389,8 +1434,8 @@ __global__ void k_kpm_combine(const double *__restrict__ Lv, const double *__res
 
 __global__ void k_kpm_moment(const double *__restrict__ part, int nblk, double *__restrict__ moments,
                              int idx, int ref) {
-    __shared__ double sh[32];
-    double s = reduce_parts(part, nblk, sh);
+    __shared__ double sh[96];
+    double s = reduce_parts<1>(part, nblk, sh);
     if (threadIdx.x == 0) moments[idx] = 2 * s - moments[ref];
 }
 
