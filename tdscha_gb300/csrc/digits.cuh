@@ -6,6 +6,7 @@
 #include <algorithm>
 #include <climits>
 #include <cmath>
+#include <type_traits>
 
 #include "common.cuh"
 #include "tcgen05.cuh"
@@ -257,7 +258,8 @@ struct DgArgs {
     int nat, nbt;          // A and B tiles
     // tiles that are partly empty:
     int kk;                // 16-element steps of a K block
-    int hc;                // columns of an epilogue warp: 16, or 8 with at most 32 in use
+    int hc;                // columns of an epilogue warp: 16, or 8 or 4 of narrower tiles
+    int win;               // work items that share a tile: each ends its own 4 hc columns
     uint32_t abytes;       // bytes of one digit of an A block: kGA, or 1024 for every eight
                            // rows of tiles with fewer (the others stay zero in shared memory)
     // B tile of work item (at, bt): bt, or bmap[at] + bt.  The A tile is at (Bloch-space
@@ -326,7 +328,7 @@ __device__ __forceinline__ bool dg_sync_or(bool pred) {
 // constants otherwise (read from the arguments they cost the M=573 call 3%)
 template <int kMode, bool kPart>
 __global__ void __launch_bounds__(DgShape<kMode>::threads, 1) k_dg_gemm(const DgArgs args) {
-    const int hc = kPart ? args.hc : 16;
+    const int hc = kPart ? args.hc : 16, win = kPart ? args.win : 1;
     const uint32_t abytes = kPart ? args.abytes : kGA;
     using Sh = DgShape<kMode>;
     constexpr int SA = Sh::SA, SB = Sh::SB, slots = Sh::slots;
@@ -409,7 +411,7 @@ __global__ void __launch_bounds__(DgShape<kMode>::threads, 1) k_dg_gemm(const Dg
         }
     };
     auto a_tile = [&](const Item &w) { return kMode == DG_QDOTS ? w.bt * args.nat + w.at : w.at; };
-    auto b_tile = [&](const Item &w) { return args.bmap ? args.bmap[w.at] + w.bt : w.bt; };
+    auto b_tile = [&](const Item &w) { return args.bmap ? args.bmap[w.at] + w.bt : kPart ? w.bt / win : w.bt; };
     // a ring's slot and the parity of its use
     struct Cursor {
         int s = 0;
@@ -563,13 +565,14 @@ __global__ void __launch_bounds__(DgShape<kMode>::threads, 1) k_dg_gemm(const Dg
             const int row = (warp - kEpi - 4) * 32 + lane;
             // (left out where s and t come from a product of their own)
             for (Item w(args); args.vs && w.left > 0; w.next()) {
-                const int at = w.at, bt = w.bt;
-                const long tile = ((long)at * args.Mp + (long)(bt % args.nct) * kGN) * 128 + row;
+                const int at = w.at, bt = w.bt, tb = kPart ? bt / win : bt;
+                const int cw = 4 * hc, w0 = kPart ? bt % win * cw : 0;
+                const long tile = ((long)at * args.Mp + (long)(tb % args.nct) * kGN + w0) * 128 + row;
                 const double *pd = args.dt + tile, *pg = args.gt + tile;
-                const double *vs = args.vs + (long)bt * kGN, *vt = args.vt + (long)bt * kGN;
+                const double *vs = args.vs + (long)tb * kGN + w0, *vt = args.vt + (long)tb * kGN + w0;
                 double s = 0, t = 0;
 #pragma unroll 1
-                for (int c = 0; c < kGN; c += 8) {
+                for (int c = 0; c < cw; c += 8) {
                     double d[8], g[8];
 #pragma unroll
                     for (int e = 0; e < 8; ++e) {
@@ -596,13 +599,13 @@ __global__ void __launch_bounds__(DgShape<kMode>::threads, 1) k_dg_gemm(const Dg
         const int quad = warp & 3, part = warp >> 2;   // part: columns c0 .. c0 + hc - 1
         const int row = quad * 32 + lane;
         const bool full = hc > 8;
-        const int c0 = part * hc;
-        const uint32_t base = tmem + ((uint32_t)(quad * 32) << 16) + c0;
+        const uint32_t base = tmem + ((uint32_t)(quad * 32) << 16);
         uint32_t nch = 0;
         bool bad = false;            // a wait of this warp gave up
         int i = 0;
         for (Item w(args); w.left > 0; w.next(), ++i) {
-            const int at = w.at, bt = w.bt;
+            const int at = w.at, bt = w.bt, tb = kPart ? bt / win : bt;
+            const int c0 = (kPart ? bt % win * 4 * hc : 0) + part * hc;
             const int nkb = min(args.kbps, args.nkb - w.split * args.kbps);
             int *ce = cole + (i & 1) * kGN;
             if (threadIdx.x < kGN) {
@@ -630,30 +633,39 @@ __global__ void __launch_bounds__(DgShape<kMode>::threads, 1) k_dg_gemm(const Dg
                 tc_fence_after();
                 // Rolled: a small call runs this code once.
                 uint32_t v[16];
-                auto add = [&](uint32_t w, long long *acc, int e0) {
-                    uint32_t over = 0, b[8];
+                auto add = [&](uint32_t w, long long *acc, int e0, auto count) {
+                    constexpr int n = decltype(count)::value;
+                    uint32_t over = 0, b[n];
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) {
+                    for (int e = 0; e < n; ++e) {
                         b[e] = __float_as_uint(__uint_as_float(v[e0 + e]) + 12582912.f);
                         over |= b[e] ^ 0x4B000000u;
                     }
                     if (__any_sync(0xffffffffu, over >> 23)) {
 #pragma unroll
-                        for (int e = 0; e < 8; ++e)
+                        for (int e = 0; e < n; ++e)
                             b[e] = kMagic + (uint32_t)__float2int_rn(__uint_as_float(v[e0 + e]));
                     }
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) acc[e0 + e] += (long long)((uint64_t)b[e] * w);
+                    for (int e = 0; e < n; ++e) acc[e0 + e] += (long long)((uint64_t)b[e] * w);
                 };
+                using Eight = std::integral_constant<int, 8>;
+                using Four = std::integral_constant<int, 4>;
                 auto order = [&](int o, uint32_t w, long long(&acc)[16]) {
-                    if (full) tmem_ld16(base + kGN * o, v);
-                    else tmem_ld8(base + kGN * o, v);
+                    const uint32_t from = base + c0 + kGN * o;
+                    if (full) tmem_ld16(from, v);
+                    else if (hc > 4) tmem_ld8(from, v);
+                    else tmem_ld4(from, v);
                     tmem_wait_ld();
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(tempty + 8 * o);
-                    add(w, acc, 0);
-                    if (full) add(w, acc, 8);
+                    if (kPart && hc == 4) {
+                        add(w, acc, 0, Four());
+                    } else {
+                        add(w, acc, 0, Eight());
+                        if (full) add(w, acc, 8, Eight());
+                    }
                 };
 #pragma unroll 1
                 for (int k = 0; k < 4; ++k) order(7 - k, 1u << (8 * k), lo);
@@ -666,7 +678,7 @@ __global__ void __launch_bounds__(DgShape<kMode>::threads, 1) k_dg_gemm(const Dg
                 break;
             }
             if (kMode == DG_DOTS) {
-                const long tile = ((long)at * args.Mp + (long)(bt % args.nct) * kGN + c0) * 128 + row;
+                const long tile = ((long)at * args.Mp + (long)(tb % args.nct) * kGN + c0) * 128 + row;
                 const double *pd = args.dt + tile, *pg = args.gt + tile;
                 // four modes' x and g on the way while the four before are used
                 double q = 0, p = 0, d[4], g[4];
@@ -676,7 +688,7 @@ __global__ void __launch_bounds__(DgShape<kMode>::threads, 1) k_dg_gemm(const Dg
                     g[e] = pg[e * 128];
                 }
                 // the rest is padding
-                const int ncol = min(hc, args.M - (bt % args.nct) * kGN - c0);
+                const int ncol = min(hc, args.M - (tb % args.nct) * kGN - c0);
 #pragma unroll
                 for (int e0 = 0; e0 < 16; e0 += 4) {
                     if (e0 >= ncol) break;

@@ -417,7 +417,7 @@ __global__ void __launch_bounds__(256) k_dg_wbuild(
     const int c = threadIdx.x & 7;
     const long wt = blockIdx.y, kb0 = blockIdx.x * (long)per, kb1 = min(nkb, kb0 + per);
     uint8_t *out = reinterpret_cast<uint8_t *>(wa) + wt * nkb * kCall * (long)kGA;
-    for (int row = threadIdx.x >> 3; row < kGM; row += 32) {
+    for (int row = blockIdx.z * 32 + (threadIdx.x >> 3); row < kGM; row += 32 * gridDim.z) {
         const long grow = wt * kGM + row;
         const int img = (int)(grow / Mp), b = (int)(grow % Mp);
         // (the eight lanes of a mode take the same branch; padding rows of wa
@@ -564,52 +564,63 @@ __device__ __forceinline__ double dg_split_sum(const double *__restrict__ p, int
 
 // d2v = -f_Y,a f_Y,b (H + H^T) / norm and f = sum fpart / norm of the image blockIdx.y (no
 // symmetry images): one block per 8-row slab of a pair (A, B), A <= B, of
-// 32 x 32 tiles, each element summed over the splits once.
-__global__ void __launch_bounds__(256) k_dg_final(const double *__restrict__ gpart, int nsplit,
-                                                  long stride, int M, int Mp,
-                                                  const double *__restrict__ fpart, int nfc,
-                                                  const double *__restrict__ fY, double norm,
-                                                  double *__restrict__ f,
-                                                  double *__restrict__ d2v) {
+// 32 x 32 tiles, each element summed over the splits once.  kRows = 2 and four groups
+// of threads, each with every fourth split, where slabs of 8 rows would leave SMs idle:
+// an addition takes a warp 64 cycles and the loads wait for one another (32 splits of
+// M=48: 11.4 us with the slabs of 8, 6.9 so).
+template <int kRows, int kGroups>
+__global__ void __launch_bounds__(32 * kRows * kGroups) k_dg_final(
+    const double *__restrict__ gpart, int nsplit, long stride, int M, int Mp,
+    const double *__restrict__ fpart, int nfc, const double *__restrict__ fY, double inv,
+    double *__restrict__ f, double *__restrict__ d2v) {
     pdl_enter();
     gpart += blockIdx.y * (long)Mp * Mp;
     fpart += blockIdx.y * (long)nfc * M;
     f += blockIdx.y * (long)M;
     d2v += blockIdx.y * (long)M * M;
-    __shared__ double tr[32][9], red[8][33];
-    const int nt = (M + 31) / 32, slab = blockIdx.x & 3;
-    int A = 0, rem = blockIdx.x >> 2;
+    constexpr int kSlabs = 32 / kRows;
+    constexpr int kThreads = 32 * kRows;
+    __shared__ double tr[kGroups][32][kRows + 1], red[kGroups][kRows][33];
+    const int nt = (M + 31) / 32, slab = blockIdx.x % kSlabs;
+    const int group = threadIdx.x / kThreads, t = threadIdx.x % kThreads;
+    int A = 0, rem = blockIdx.x / kSlabs;
     while (rem >= nt - A) {
         rem -= nt - A;
         ++A;
     }
-    const int B = A + rem, a0 = A * 32 + slab * 8, b0 = B * 32;
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const double inv = 1.0 / norm;
+    const int B = A + rem, a0 = A * 32 + slab * kRows, b0 = B * 32;
+    const int tx = t & 31, ty = t >> 5;
+    const int mine = (nsplit - group + kGroups - 1) / kGroups;
+    gpart += group * stride;
     {
-        const int ao = threadIdx.x & 7, bo = threadIdx.x >> 3;
+        const int ao = t % kRows, bo = t / kRows;
         const int b = b0 + bo, a = a0 + ao;
-        tr[bo][ao] = (a < M && b < M) ? dg_split_sum(gpart + (long)b * Mp + a, nsplit, stride) : 0.0;
+        tr[group][bo][ao] =
+            (a < M && b < M) ? dg_split_sum(gpart + (long)b * Mp + a, mine, kGroups * stride) : 0.0;
     }
+    const int a = a0 + ty, b = b0 + tx;
+    const bool in = a < M && b < M;
+    double h = in ? dg_split_sum(gpart + (long)a * Mp + b, mine, kGroups * stride) : 0.0;
+    if (kGroups > 1) red[group][ty][tx] = h;
     __syncthreads();
-    {
-        const int a = a0 + ty, b = b0 + tx;
-        if (a < M && b < M) {
-            const double h = dg_split_sum(gpart + (long)a * Mp + b, nsplit, stride) + tr[tx][ty];
-            const double v = -(h * fY[a]) * fY[b] * inv;
-            d2v[(long)a * M + b] = v;
-            if (A != B) d2v[(long)b * M + a] = v;
-        }
+    if (group == 0 && in) {
+        for (int k = 1; k < kGroups; ++k) h += red[k][ty][tx];
+        for (int k = 0; k < kGroups; ++k) h += tr[k][tx][ty];
+        const double v = -(h * fY[a]) * fY[b] * inv;
+        d2v[(long)a * M + b] = v;
+        if (A != B) d2v[(long)b * M + a] = v;
     }
     if (A == 0 && slab == 0) {
         const int e = b0 + tx;
         double acc = 0;
         if (e < M)
-            for (int ch = ty; ch < nfc; ch += 8) acc += fpart[(long)ch * M + e];
-        red[ty][tx] = acc;
+            for (int ch = group * kRows + ty; ch < nfc; ch += kGroups * kRows) acc += fpart[(long)ch * M + e];
         __syncthreads();
-        if (ty == 0 && e < M) {
-            for (int k = 1; k < 8; ++k) acc += red[k][tx];
+        red[group][ty][tx] = acc;
+        __syncthreads();
+        if (threadIdx.x < 32 && e < M) {
+            acc = 0;
+            for (int k = 0; k < kGroups * kRows; ++k) acc += red[k / kRows][k % kRows][tx];
             f[e] = acc * inv;
         }
     }
@@ -715,7 +726,8 @@ int digits_prepare(tdscha_ctx *c) {
         {(void **)&x->st, one * d * 2 * cap * x->Rp, false},
         {(void **)&x->gf, one * d * x->nsF * kGM * 2 * Mp, false},
         {(void **)&x->bmap, one * i4 * 2 * nrt, false},
-        {(void **)&x->qp, d * 4 * x->nct * (size_t)cap * R, false},
+        // (the column parts of small tiles are at most as many as there are SMs)
+        {(void **)&x->qp, d * 4 * std::max((size_t)x->nct * cap, (size_t)(x->nsm / nrt)) * R, false},
         {(void **)&x->abcc, d * 4 * (size_t)cap * x->Rp, false},
         {(void **)&x->gpart, gbytes, false},
         {(void **)&x->fpart, d * (size_t)cap * x->nfc * M, false},
@@ -864,10 +876,20 @@ static int digits_contract(tdscha_ctx *c, int nimg, const DgSources &src, int ap
     ga.nkb = ga.kbps = x->nkbM;
     ga.flush = x->flushA;
     ga.kk = ceil_div(M, 16);             // (read where M <= 64)
+    // At most 64 modes: where that leaves SMs, two or four work items end a tile, each a
+    // part of its columns (and do all of its products): with one, 16 row tiles at M=48
+    // spend 16 000 cycles on the float64 operations of the row dots: 23.3 us at M=48,
+    // N=2000, 13.0 so.
+    int win = 1;
     ga.hc = M <= 32 ? 8 : 16;
+    while (M <= kGN && ga.hc > 4 && 2 * ga.hc < M && 2 * win * nimg * (x->Rp / kGM) <= x->nsm) {
+        win *= 2;
+        ga.hc /= 2;
+    }
+    ga.win = win;
     ga.abytes = kGA;
     ga.nat = (int)(x->Rp / kGM);
-    ga.nbt = nimg * x->nct;
+    ga.nbt = nimg * x->nct * win;
     ga.nitems = (long)ga.nat * ga.nbt;
     ga.Mp = Mp;
     ga.err = x->err;
@@ -890,7 +912,7 @@ static int digits_contract(tdscha_ctx *c, int nimg, const DgSources &src, int ap
         ProfScope ps(c, 1, st);
         TDS_CUDA(launch_pdl(x->many ? k_dg_rows<true> : k_dg_rows<false>, dim3((unsigned)(x->Rp / 128), nimg), 128, 0, st,
                             (const double *)x->qp, (const double *)x->st,
-                            x->nct, R, x->Rp, c->rho_div,
+                            x->nct * win, R, x->Rp, c->rho_div,
                             (const double *)c->rho, (const int *)x->er, apply_d4, x->abcc,
                             x->absmax));
     }
@@ -905,7 +927,9 @@ static int digits_contract(tdscha_ctx *c, int nimg, const DgSources &src, int ap
                                 (const unsigned long long *)x->gmax, M, Mp, x->Rp, nimg, x->nkbR,
                                 x->wa, x->ew, x->wf, x->ewf));
         else
-            TDS_CUDA(launch_pdl(k_dg_wbuild, dim3(x->nfc, nat), 256, 0, st, (const double *)x->dt,
+            // (few blocks: a group of 32 modes each)
+            TDS_CUDA(launch_pdl(k_dg_wbuild, dim3(x->nfc, nat, x->nfc * nat <= 2 * x->nsm ? 4 : 1),
+                                256, 0, st, (const double *)x->dt,
                                 (const double *)x->gt, (const double *)x->abcc,
                                 (const unsigned long long *)x->absmax,
                                 (const unsigned long long *)x->dmax,
@@ -920,6 +944,7 @@ static int digits_contract(tdscha_ctx *c, int nimg, const DgSources &src, int ap
     gb.flush = x->flushB;
     gb.kk = kGK / 16;
     gb.hc = M <= 32 ? 8 : 16;
+    gb.win = 1;
     gb.abytes = kGA;
     gb.nat = nat;
     gb.nbt = x->nct;
@@ -974,10 +999,12 @@ static int digits_averages(tdscha_ctx *c, int nimg, const DgSources &src, int ap
     TDS_TRY(digits_contract(c, nimg, src, apply_d4, &ns, st));
     ProfScope ps(c, 4, st);
     const int nt = ceil_div(M, 32), nat = ceil_div((long)nimg * Mp, kGM);
-    TDS_CUDA(launch_pdl(k_dg_final, dim3(4 * (nt * (nt + 1) / 2), nimg), 256, 0, st,
-                        (const double *)x->gpart, ns, (long)nat * kGM * Mp, M, Mp,
-                        (const double *)x->fpart, x->nfc, (const double *)c->fY,
-                        c->sum_rho * c->S, f, d2v));
+    const int pairs = nt * (nt + 1) / 2;
+    const bool small = 4 * pairs * nimg < x->nsm;
+    TDS_CUDA(launch_pdl(small ? k_dg_final<2, 4> : k_dg_final<8, 1>,
+                        dim3((small ? 16 : 4) * pairs, nimg), 256, 0, st, (const double *)x->gpart, ns,
+                        (long)nat * kGM * Mp, M, Mp, (const double *)x->fpart, x->nfc,
+                        (const double *)c->fY, 1.0 / (c->sum_rho * c->S), f, d2v));
     return TDSCHA_OK;
 }
 

@@ -212,3 +212,18 @@ def test_many_images_matches_core_kernels(gpu_lib, monkeypatch):
             assert (np.isfinite(u) == np.isfinite(v)).all()
     ctx.close()
     cores.close()
+
+
+@pytest.mark.parametrize("M,N", [(16, 100), (17, 300), (32, 129), (33, 700), (48, 2500), (64, 4800),
+                                 (64, 9800)])
+def test_column_parts(gpu_lib, M, N):
+    """Up to 64 modes and few rows: several work items share a tile (stage A), blocks of
+    32 modes (W), slabs of two rows (the end)."""
+    ens = make_ensemble(M, N, seed=M + N, rho_sigma=0.1)
+    R1, Y1 = random_R1(M, 3), random_sym(M, 4, scale=1e-5)
+    ctx = _context(ens)
+    got = _call(ctx, R1, Y1)
+    ctx.close()
+    ref = oracle.perturb_averages(ens["X"], ens["Y"], ens["w"], ens["rho"], R1, Y1, ens["T"], 1,
+                                  *_tables(ens, M), n_threads=8)
+    assert _rel(got[0], ref[0]) <= TOL and _rel(got[1], ref[1]) <= TOL
