@@ -1830,7 +1830,7 @@ __device__ __forceinline__ double gsum_one(const float *__restrict__ g, int nspl
 __global__ void __launch_bounds__(256) k_gfinal(const float *__restrict__ gpart, int nsplit,
                                                 long lda, long stride, int M, int Mp,
                                                 const float *__restrict__ fpart, int nfchunk,
-                                                double norm, double *__restrict__ f,
+                                                double inv, double *__restrict__ f,
                                                 double *__restrict__ d2v, double *__restrict__ f2,
                                                 double *__restrict__ d2v2) {
     pdl_enter();
@@ -1854,7 +1854,6 @@ __global__ void __launch_bounds__(256) k_gfinal(const float *__restrict__ gpart,
         ++A;
     }
     const int B = A + rem;
-    const double inv = 1.0 / norm;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;   // 8 x 32
     const int a0 = A * 32 + slab * 8, b0 = B * 32;
     {
@@ -2439,7 +2438,7 @@ static int perturb_mixed_src(tdscha_ctx *c, int apply_d4, const Y1FromPsi *psrc,
         const int nt = ceil_div(M, 32);
         TDS_CUDA(launch_pdl(k_gfinal, dim3(4 * (nt * (nt + 1) / 2), nsrc), 256, 0, st, mx.gpart,
                             mx.nsplit, (long)ldGb, sstride, M, Mp, x->fpart, x->nfchunk,
-                            c->sum_rho * c->S, f, d2v, c->f2, c->d2v2));
+                            1.0 / (c->sum_rho * c->S), f, d2v, c->f2, c->d2v2));
     }
     return TDSCHA_OK;
 }
