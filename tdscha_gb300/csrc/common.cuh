@@ -142,6 +142,7 @@ struct tdscha_ctx {
     double *pqn = nullptr;      // p_j . q_j of the stored basis (full reorthogonalisation)
     double *rcoef = nullptr;    // projection coefficients (2 per basis vector)
     int pqn_cap = 0;
+    int pq_pending = 0;      // partials of the last pair's weight, not yet added up (lz_step)
     float2 *vsplit = nullptr;   // 2 x ldv: double-float splits of the masked new pair
     long basis_ld = 0;          // row stride of the Lanczos basis buffers (0: P)
     double *host_pinned = nullptr;

@@ -970,14 +970,28 @@ __global__ void k_rdots(const double *__restrict__ Qb, const double *__restrict_
 }
 
 // coef[j] = split(c_j), split(d_j) with c_j, d_j = chunk sums / (p_j . q_j)
-// (float64 sums and division); one warp per j
-__global__ void k_rscale(const double *__restrict__ part, const double *__restrict__ pqn,
-                         int nvec, int nch, float4 *__restrict__ coef) {
+// (float64 sums and division); one warp per j.  The weight p_j . q_j of the last vector
+// comes from the npq block partials of its own step's update (npq > 0; added up as
+// k_pq_reduce does, without a launch for it).
+__global__ void k_rscale(const double *__restrict__ part, double *pqn, int nvec, int nch,
+                         float4 *__restrict__ coef, const double *__restrict__ pq, int npq) {
     pdl_enter();
-    const int j = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const int j = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (j >= nvec) return;   // whole warps
-    const float2 c = split_f64(warp_chunk_sums<2>(part, j, nch) * (1.0 / pqn[j]));
-    if ((threadIdx.x & 15) == 0) reinterpret_cast<float2 *>(coef + j)[(threadIdx.x & 31) >> 4] = c;
+    double weight;
+    if (npq > 0 && j == nvec - 1) {
+        weight = 0;
+        for (int b = 0; b < npq; b += 32) {
+            const double v[1] = {b + lane < npq ? 0.0 + pq[b + lane] : 0.0};
+            weight += warp_sums(v);
+        }
+        if (lane == 0) pqn[j] = weight;
+        weight = __shfl_sync(0xffffffffu, weight, 0);
+    } else {
+        weight = pqn[j];
+    }
+    const float2 c = split_f64(warp_chunk_sums<2>(part, j, nch) * (1.0 / weight));
+    if ((lane & 15) == 0) reinterpret_cast<float2 *>(coef + j)[lane >> 4] = c;
 }
 
 constexpr int kRProjMax = 1024;   // coefficients per apply pass (16 KB of shared memory)
@@ -1645,6 +1659,7 @@ namespace tdscha {
 static int lz_begin(tdscha_ctx *ctx, double *basis_Q, double *basis_P, long ld, int capacity,
                     int start_step, int run_simm, int full_reorth, const double *hist,
                     cudaStream_t st) {
+    ctx->pq_pending = 0;
     const long P = ctx->P;
     const double *mask = run_simm ? ctx->mask : nullptr;
     if (ctx->hist_cap < capacity + 1) {
@@ -1731,6 +1746,8 @@ static int lz_step(tdscha_ctx *ctx, double *basis_Q, double *basis_P, long ld, i
         int nvec = k + 1;
         double *part = ctx->rcoef + 2 * (capacity + 1);
         const int nch = dot_chunks(P, nvec);
+        // partials of the weight, past those of the sums that come before the next k_rscale
+        double *pq = ctx->dots + (nb <= kFewParts ? 4 * kFewParts : 0);
         float4 *coef = reinterpret_cast<float4 *>(ctx->rcoef);
         const float2 *vs = ctx->vsplit;
         // two elements per load where every row starts on 16 bytes
@@ -1744,24 +1761,30 @@ static int lz_step(tdscha_ctx *ctx, double *basis_Q, double *basis_P, long ld, i
             else
                 launch_pdl(k_rdots, dim3(nvec, nch), 256, 0, st, basis_Q, basis_P, vs, P, ldv, ld,
                            part);
-            launch_pdl(k_rscale, ceil_div(nvec, 8), 256, 0, st, part, ctx->pqn, nvec, nch, coef);
+            // (the weight of the step before, where it is still in partials)
+            launch_pdl(k_rscale, ceil_div(nvec, 8), 256, 0, st, part, ctx->pqn, nvec, nch, coef,
+                       (const double *)pq, ctx->pq_pending);
         }
         ProfScope ps(ctx, 7, st);
         const int ntile = (int)ceil_div(P, 64L);
         const int npq = vec ? ntile : nbw;
+        const bool keep = nb <= kFewParts;      // npq <= 128: the next step's k_rscale adds up
         for (int j0 = 0; j0 < nvec; j0 += kRProjMax) {
             bool last = j0 + kRProjMax >= nvec;
             if (vec)
                 launch_pdl(k_rapply2, ntile, 32 * kTileWarps, 0, st, basis_Q, basis_P,
                            (const float4 *)coef, P, j0, std::min(kRProjMax, nvec - j0), ld, qn,
-                           pn, mask, last ? ctx->dots : nullptr);
+                           pn, mask, last ? pq : nullptr);
             else
                 launch_pdl(k_rapply, nbw, 256, 0, st, basis_Q, basis_P, (const float4 *)coef, P,
                            j0, std::min(kRProjMax, nvec - j0), ld, qn, pn, mask,
-                           last ? ctx->dots : nullptr);
+                           last ? pq : nullptr);
         }
         // weight p_{k+1} . q_{k+1} of the new pair from the apply pass's partials
-        launch_pdl(k_pq_reduce, 1, 512, 0, st, ctx->dots, npq, ctx->pqn, k + 1);
+        if (keep)
+            ctx->pq_pending = npq;
+        else
+            launch_pdl(k_pq_reduce, 1, 512, 0, st, pq, npq, ctx->pqn, k + 1);
     }
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) { set_error("lanczos_run launch: %s", cudaGetErrorString(e)); return TDSCHA_ERR_CUDA; }
