@@ -221,31 +221,33 @@ inline int dg_blocks_per_split(long nkb, int flush, int nat, int nbt, int nsm) {
 }
 
 // -------------------------------------------------------- the contraction
-// Persistent, one CTA per SM, 512 threads, one 128 x 64 output tile at a time;
-// its accumulators, eight orders of 64 columns, fill the TMEM.
-//   warp 8  copies: B blocks (all digits of 64 rows) into two buffers, A digits
+// Persistent, one CTA per SM, one 128 x 64 output tile at a time; its accumulators,
+// eight orders of 64 columns, fill the TMEM.
+//   warps 0-15  every `flush` K blocks the accumulators are read, order 7 first, and
+//           added to two 64-bit integers an element (warp w: lanes 32 (w % 4), columns
+//           16 (w / 4) of every order).  Each order has its own release, so the MMAs of
+//           the next blocks start on order 7 while the lower ones are still read.  At
+//           the end of a tile the sums become float64: row dots, a partial tile or a
+//           product.
+//   warp 16  copies: B blocks (all digits of 64 rows) into two buffers, A digits
 //           (128 rows each) into a ring
-//   warp 9  MMA issue: A digit i against the B digits 0 .. 7 - i at once, which
+//   warp 17  MMA issue: A digit i against the B digits 0 .. 7 - i at once, which
 //           lie behind one another in shared memory as their accumulators do in
 //           TMEM, so one instruction covers up to four orders (N = 256).  i
 //           runs downwards: the light high orders come first.
-//   warps 12-15  (stage A) s and t
-//   warps 0-7  every three K blocks the accumulators are read, order 7 first,
-//           and added to two 64-bit integers an element (warp w: lanes 32 (w % 4),
-//           columns 32 (w / 4) of every order).  Each order has its own
-//           release, so the MMAs of the next blocks start on order 7 while the
-//           lower ones are still read.  At the end of a tile the sums become
-//           float64: row dots (stage A) or a partial tile (stage B).
+//   warps 20-23  (row dots of the real-space stage A) s and t
 // Bounded waits and the abort flag as in perturb_mixed.cu.
 //
-// What it takes at M=573, N=50000 (1.95 GHz): stage A 700 us, stage B 774 us; the
+// What it takes at M=573, N=50000 (1.95 GHz): stage A 673 us, stage B 759 us; the
 // 35 products alone are 0.93 and 1.04 million cycles an SM, 480 and 530 us.  The
 // same loop on one thread (`if (lane == 0)`) took 794 and 928 us, with 64-bit
 // divisions for the ring slots 1165 and 1098.  Reading an accumulation back takes
-// the epilogue 8000 cycles, of which 1200 stand before the next MMAs; a tile's end
-// 12000 (stage A: two float64 products an element on the float64 pipe).  With 48
-// images stage A (976 us at M=189, N=10000) is bound by that pipe and the epilogue.
-// The copies (176 KB a K block) take 3700 cycles of a block's 4500 and do not show.
+// the sixteen epilogue warps 6300 cycles, of which the next products wait for about
+// 2900 (eight warps of 32 columns: 8000); the end of a tile with row dots 12 000 to
+// 15 000: two float64 products an element, and as many for s and t beside them.  With
+// 48 images at M=189, N=10000 stage A (783 us) is bound by that and the reading back,
+// 20 000 cycles a tile against 13 400 of products.  The copies (176 KB a K block) take
+// 3700 cycles of a block's 4500 and do not show.
 // What becomes of a tile: row dots (stage A), split-K partials (stage B), the
 // product itself, or the complex row dots of Bloch space (qspace_digits.cu)
 enum { DG_DOTS = 0, DG_PARTS, DG_STORE, DG_QDOTS };

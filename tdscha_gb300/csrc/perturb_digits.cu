@@ -33,8 +33,8 @@
 // of perturb_fp64.cu: M=573 N=2000 6.9e-16 7.0e-16 | 1.3e-15 1.2e-15; with Y1 over
 // six decades 7.9e-16 7.7e-16 | 1.4e-15 1.2e-15; M=192 N=3000 1.5e-15 1.5e-15 |
 // 1.7e-15 1.6e-15; M=24 N=400 48 images 1.3e-15 5.3e-16 | 3.1e-15 5.6e-16.
-// One call: M=573 N=50000 57.1 -> 1.77 ms; M=189 N=10000 48 images 62.8 -> 2.68 ms;
-// M=97 N=4999 554 -> 86 us; M=21 N=1000 245 -> 61 us.
+// One call: M=573 N=50000 57.1 -> 1.71 ms; M=189 N=10000 48 images 62.8 -> 2.10 ms;
+// M=97 N=4999 554 -> 66 us; M=21 N=1000 245 -> 34 us.
 //
 // Form of the contractions, with g = y / f_Y (= f_psi y) so that both operands
 // of the second stage come from x and g alone (u = f_Y x, y = f_Y g):

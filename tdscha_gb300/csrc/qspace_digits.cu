@@ -16,7 +16,8 @@
 //           u2 and A2 with f2, are not needed and cost nothing: they fill a tile
 //           that would be empty.
 //
-// Measured (averages, one call): 4x4x4 grid, 12 bands, N=10000 2479 -> 536 us.
+// Measured (averages, one call): 4x4x4 grid, 12 bands, N=10000 2479 -> 530 us
+// (row dots 216, W 132, d2v 146 of them).
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
