@@ -260,7 +260,7 @@ struct DgArgs {
     int nat, nbt;          // A and B tiles
     // tiles that are partly empty:
     int kk;                // 16-element steps of a K block
-    int hc;                // columns of an epilogue warp: 16, or 8 or 4 of narrower tiles
+    int hc;                // columns of an epilogue warp: 16, or 12, 8, 4 of narrower tiles
     int win;               // work items that share a tile: each ends its own 4 hc columns
     uint32_t abytes;       // bytes of one digit of an A block: kGA, or 1024 for every eight
                            // rows of tiles with fewer (the others stay zero in shared memory)
@@ -289,6 +289,10 @@ struct DgArgs {
     const int *er;
     double *out;
 };
+
+// hc where `cols` of a tile's columns are in use: a quarter of them, in fours (Bloch-space
+// averages with 12 bands, 48 columns of a tile: 538 us with three warps of 16, 530 so)
+inline int dg_part_cols(int cols) { return std::min(16, (cols + 15) / 16 * 4); }
 
 constexpr int kEpi = 16;           // epilogue warps
 

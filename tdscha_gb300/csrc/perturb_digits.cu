@@ -886,6 +886,7 @@ static int digits_contract(tdscha_ctx *c, int nimg, const DgSources &src, int ap
         win *= 2;
         ga.hc /= 2;
     }
+    if (win == 1) ga.hc = dg_part_cols(M);
     ga.win = win;
     ga.abytes = kGA;
     ga.nat = (int)(x->Rp / kGM);
@@ -943,7 +944,7 @@ static int digits_contract(tdscha_ctx *c, int nimg, const DgSources &src, int ap
     gb.kbps = dg_blocks_per_split(x->nkbR, x->flushB, nat, x->nct, x->nsm);
     gb.flush = x->flushB;
     gb.kk = kGK / 16;
-    gb.hc = M <= 32 ? 8 : 16;
+    gb.hc = dg_part_cols(M);
     gb.win = 1;
     gb.abytes = kGA;
     gb.nat = nat;

@@ -671,7 +671,7 @@ int qdigits_perturb(tdscha_qctx *c, int apply_d4, const double *psi, cudaStream_
     a.b = x->yb;
     a.nkb = a.kbps = a.flush = 1;
     a.kk = ceil_div(live, 16);
-    a.hc = live <= 32 ? 8 : 16;
+    a.hc = dg_part_cols(live);
     a.win = 1;
     a.abytes = kGA;
     a.nat = (int)x->nrt;
@@ -704,7 +704,7 @@ int qdigits_perturb(tdscha_qctx *c, int apply_d4, const double *psi, cudaStream_
     b.kbps = x->kbps;
     b.flush = x->flush;
     b.kk = kGK / 16;
-    b.hc = (x->nbq == 1 ? 2 * x->nr : x->nr) <= 32 ? 8 : 16;
+    b.hc = dg_part_cols(x->nbq == 1 ? 2 * x->nr : x->nr);
     b.win = 1;
     b.abytes = x->abytes;
     b.nat = x->n_pairs;
