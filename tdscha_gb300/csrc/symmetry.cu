@@ -34,6 +34,7 @@ namespace tdscha {
 __global__ void k_psi_vec(const int *__restrict__ sc_idx, const double *__restrict__ sc_val,
                           const double *__restrict__ fY, const double *__restrict__ R1, int J,
                           int M, int md, double *__restrict__ vs, double *__restrict__ vt) {
+    pdl_enter();
     long n = (long)J * M;
     for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < n; e += (long)gridDim.x * blockDim.x) {
         const int *ix = sc_idx + e * md;
@@ -54,6 +55,7 @@ __global__ void k_psi_vec(const int *__restrict__ sc_idx, const double *__restri
 __global__ void k_psi_y1(const int *__restrict__ sc_idx, const double *__restrict__ sc_val,
                          const double *__restrict__ Y1, int J, int M, int md,
                          double *__restrict__ Y1all) {
+    pdl_enter();
     long MM = (long)M * M, n = (long)J * MM;
     for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < n; e += (long)gridDim.x * blockDim.x) {
         long j = e / MM;
@@ -100,6 +102,7 @@ __global__ void __launch_bounds__(256) k_psi_hsum(const double *__restrict__ g, 
                                                   const double *__restrict__ fpart, int nfc,
                                                   const double *__restrict__ fY, int M,
                                                   double *__restrict__ hs, double *__restrict__ fs) {
+    pdl_enter();
     __shared__ double t1[32][33], t2[32][33];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;    // 32 x 8
     const int nt = (M + 31) / 32;
@@ -149,6 +152,7 @@ __global__ void k_psi_sandwich(const int *__restrict__ sr_idx, const double *__r
                                const double *__restrict__ hs, const double *__restrict__ fs,
                                int J, int M, int md, double *__restrict__ tj,
                                double *__restrict__ tf) {
+    pdl_enter();
     const long MM = (long)M * M, n = (long)J * MM;
     for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < n; e += (long)gridDim.x * blockDim.x) {
         const long j = e / MM;
@@ -172,6 +176,7 @@ __global__ void k_psi_sandwich(const int *__restrict__ sr_idx, const double *__r
 // d2v[a][b] = -inv sum_j tj[j][a][b], f[a] = inv sum_j tf[j][a], in image order.
 __global__ void k_psi_jsum(const double *__restrict__ tj, const double *__restrict__ tf, int J,
                            int M, double inv, double *__restrict__ f, double *__restrict__ d2v) {
+    pdl_enter();
     const long MM = (long)M * M;
     for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < MM; e += (long)gridDim.x * blockDim.x) {
         d2v[e] = -split_sum(tj + e, J, MM) * inv;
@@ -209,6 +214,7 @@ __global__ void __launch_bounds__(256) k_psi_hsum_df(const float *__restrict__ g
                                                      const float *__restrict__ fpart, int nfc,
                                                      int M, float2 *__restrict__ hs,
                                                      float2 *__restrict__ fs) {
+    pdl_enter();
     __shared__ float2 t1[32][33], t2[32][33];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;    // 32 x 8
     const int nt = (M + 31) / 32;
@@ -254,6 +260,7 @@ __global__ void k_psi_sandwich_df(const int *__restrict__ sr_idx, const float2 *
                                   const float2 *__restrict__ hs, const float2 *__restrict__ fs,
                                   int J, int M, int md, float2 *__restrict__ tj,
                                   float2 *__restrict__ tf) {
+    pdl_enter();
     const long MM = (long)M * M, n = (long)J * MM;
     for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < n; e += (long)gridDim.x * blockDim.x) {
         const long j = e / MM;
@@ -281,6 +288,7 @@ __global__ void __launch_bounds__(256) k_psi_jsum_df(const float2 *__restrict__ 
                                                      const float2 *__restrict__ tf, int J, int M,
                                                      double inv, double *__restrict__ f,
                                                      double *__restrict__ d2v) {
+    pdl_enter();
     __shared__ float2 red[2][4][64];
     const long MM = (long)M * M;
     const int x = threadIdx.x, y = threadIdx.y;
@@ -408,13 +416,11 @@ void psi_free(tdscha_ctx *c) {
 
 int psi_perturbation64(tdscha_ctx *c, cudaStream_t st) {
     const int M = c->M, J = c->J, md = c->maxdeg;
-    k_psi_vec<<<grid_for((long)J * M), 256, 0, st>>>(c->sc_idx, c->sc_val, c->fY, c->R1, J, M, md,
-                                                     c->vsv, c->vsv + (long)J * M);
-    TDS_CHECK_LAUNCH();
+    TDS_CUDA(launch_pdl(k_psi_vec, grid_for((long)J * M), 256, 0, st, c->sc_idx, c->sc_val, c->fY,
+                        c->R1, J, M, md, c->vsv, c->vsv + (long)J * M));
     if (!c->Y1all) TDS_CUDA(cached_malloc(&c->Y1all, sizeof(double) * (size_t)J * M * M));
-    k_psi_y1<<<grid_for((long)J * M * M), 256, 0, st>>>(c->sc_idx, c->sc_val, c->Y1, J, M, md,
-                                                        c->Y1all);
-    TDS_CHECK_LAUNCH();
+    TDS_CUDA(launch_pdl(k_psi_y1, grid_for((long)J * M * M), 256, 0, st, c->sc_idx, c->sc_val, c->Y1,
+                        J, M, md, c->Y1all));
     return TDSCHA_OK;
 }
 
@@ -427,9 +433,8 @@ int psi_hsum64(tdscha_ctx *c, const double *gpart, int nsplit, long sstride, lon
     ProfScope ps(c, 4, st);
     const int nt = ceil_div(M, 32);
     dim3 gt(nt * (nt + 1) / 2, nj);
-    k_psi_hsum<<<gt, 256, 0, st>>>(gpart, nsplit, sstride, jstride, lda, fpart, nfchunk, fY, M,
-                                   hs + j0 * MM, fs + (size_t)j0 * M);
-    TDS_CHECK_LAUNCH();
+    TDS_CUDA(launch_pdl(k_psi_hsum, gt, 256, 0, st, gpart, nsplit, sstride, jstride, lda, fpart, nfchunk,
+                        fY, M, hs + j0 * MM, fs + (size_t)j0 * M));
     return TDSCHA_OK;
 }
 
@@ -438,12 +443,10 @@ int psi_reduce64(tdscha_ctx *c, cudaStream_t st) {
     const size_t JMM = (size_t)J * M * M, JM = (size_t)J * M;
     double *hs = c->hs, *tj = hs + JMM, *fs = tj + JMM, *tf = fs + JM;
     ProfScope ps(c, 4, st);
-    k_psi_sandwich<<<grid_for((long)JMM), 256, 0, st>>>(c->sr_idx, c->sr_val, hs, fs, J, M,
-                                                        c->maxdeg, tj, tf);
-    TDS_CHECK_LAUNCH();
-    k_psi_jsum<<<std::max(1, ceil_div((long)M * M, 64)), 64, 0, st>>>(
-        tj, tf, J, M, 1.0 / (c->sum_rho * c->S), c->f, c->d2v);
-    TDS_CHECK_LAUNCH();
+    TDS_CUDA(launch_pdl(k_psi_sandwich, grid_for((long)JMM), 256, 0, st, c->sr_idx, c->sr_val, hs, fs, J,
+                        M, c->maxdeg, tj, tf));
+    TDS_CUDA(launch_pdl(k_psi_jsum, std::max(1, ceil_div((long)M * M, 64)), 64, 0, st, tj, tf, J, M,
+                        1.0 / (c->sum_rho * c->S), c->f, c->d2v));
     return TDSCHA_OK;
 }
 
@@ -464,15 +467,12 @@ int psi_finalize32(tdscha_ctx *c, const float *gpart, int nsplit, long sstride, 
     ProfScope ps(c, 4, st);
     const int nt = ceil_div(M, 32);
     dim3 gt(nt * (nt + 1) / 2, J);
-    k_psi_hsum_df<<<gt, 256, 0, st>>>(gpart, nsplit, sstride, jstride, lda, fpart, nfchunk, M, hs,
-                                      fs);
-    TDS_CHECK_LAUNCH();
-    k_psi_sandwich_df<<<grid_for((long)JMM), 256, 0, st>>>(c->sr_idx, c->sr_val2, hs, fs, J, M,
-                                                           c->maxdeg, tj, tf);
-    TDS_CHECK_LAUNCH();
-    k_psi_jsum_df<<<std::max(1, ceil_div((long)M * M, 64)), dim3(64, 4), 0, st>>>(
-        tj, tf, J, M, 1.0 / (c->sum_rho * c->S), f_out, d2v_out);
-    TDS_CHECK_LAUNCH();
+    TDS_CUDA(launch_pdl(k_psi_hsum_df, gt, 256, 0, st, gpart, nsplit, sstride, jstride, lda, fpart,
+                        nfchunk, M, hs, fs));
+    TDS_CUDA(launch_pdl(k_psi_sandwich_df, grid_for((long)JMM), 256, 0, st, c->sr_idx, c->sr_val2, hs, fs,
+                        J, M, c->maxdeg, tj, tf));
+    TDS_CUDA(launch_pdl(k_psi_jsum_df, std::max(1, ceil_div((long)M * M, 64)), dim3(64, 4), 0, st, tj, tf,
+                        J, M, 1.0 / (c->sum_rho * c->S), f_out, d2v_out));
     return TDSCHA_OK;
 }
 
