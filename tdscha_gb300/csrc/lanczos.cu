@@ -1211,6 +1211,7 @@ __global__ void k_pq_reduce(const double *__restrict__ part, int nblk, double *_
 __global__ void k_pq_part(const double *__restrict__ Qb, const double *__restrict__ Pb,
                           const double *__restrict__ mask, long n, long ld, int j0,
                           double *__restrict__ part) {
+    pdl_enter();
     __shared__ double sh[96];
     int j = j0 + blockIdx.x;
     const long nch = gridDim.y;
@@ -1226,6 +1227,7 @@ __global__ void k_pq_part(const double *__restrict__ Qb, const double *__restric
 
 __global__ void k_pq_finish(const double *__restrict__ part, int cnt, int j0, int nch,
                             double *__restrict__ out) {
+    pdl_enter();
     const int j = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (j >= cnt) return;   // whole warps
     double a = warp_chunk_sums<1>(part, j, nch);
@@ -1238,6 +1240,7 @@ __global__ void k_pq_finish(const double *__restrict__ part, int cnt, int j0, in
 __global__ void k_qrenorm(const double *__restrict__ part, int nblk, double *__restrict__ scal,
                           double *__restrict__ hist, int k, long n, double *__restrict__ qn,
                           double *__restrict__ pn) {
+    pdl_enter();
     __shared__ double sh[96];
     __shared__ double inv_s;
     if (scal[SC_HALT] != 0.0) return;
@@ -1508,12 +1511,14 @@ static cudaError_t launch_qrecur(const RecurArgs &r, cudaStream_t st) {
 // moments[idx] = 2 <x, y>_M - moments[ref].
 __global__ void k_kpm_combine(const double *__restrict__ Lv, const double *__restrict__ v,
                               double *__restrict__ vm, double a, double b, long n) {
+    pdl_enter();
     for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < n; e += (long)gridDim.x * blockDim.x)
         vm[e] = 2 * ((Lv[e] - b * v[e]) / a) - vm[e];
 }
 
 __global__ void k_kpm_moment(const double *__restrict__ part, int nblk, double *__restrict__ moments,
                              int idx, int ref) {
+    pdl_enter();
     __shared__ double sh[96];
     double s = reduce_parts<1>(part, nblk, sh);
     if (threadIdx.x == 0) moments[idx] = 2 * s - moments[ref];
@@ -2057,32 +2062,38 @@ static int qz_step(tdscha_qctx *ctx, double *basis_Q, double *basis_P, int capac
         return TDSCHA_OK;
     }
     TDS_TRY(q_apply_full_L_dev(ctx, q, ctx->Lq, st));
-    k_dot1<<<nb, kDotThreads, 0, st>>>(p, ctx->Lq, mask, n, ctx->dots);
-    k_scal_a<<<1, 256, 0, st>>>(ctx->dots, nb, ctx->hist_dev, k, ctx->scal, ctx->stat_dev);
+    TDS_CUDA(launch_pdl(k_dot1, nb, kDotThreads, 0, st, p, ctx->Lq, mask, n, ctx->dots));
+    TDS_CUDA(launch_pdl(k_scal_a, 1, 256, 0, st, ctx->dots, nb, ctx->hist_dev, k, ctx->scal,
+                        ctx->stat_dev));
     const double *qprev = k >= 1 ? basis_Q + (long)(k - 1) * n : nullptr;
     const double *pprev = k >= 1 ? basis_P + (long)(k - 1) * n : nullptr;
-    k_resid<<<nb, kDotThreads, 0, st>>>(ctx->Lq, ctx->Lq, q, p, qprev, pprev, mask, ctx->scal, n,
-                                         ctx->rk, ctx->sk, ctx->dots, nb);
-    k_scal_bc<<<1, 256, 0, st>>>(ctx->dots, nb, ctx->hist_dev, k, ctx->scal, ctx->stat_dev);
+    TDS_CUDA(launch_pdl(k_resid, nb, kDotThreads, 0, st, ctx->Lq, ctx->Lq, q, p, qprev, pprev, mask,
+                        ctx->scal, n, ctx->rk, ctx->sk, ctx->dots, nb));
+    TDS_CUDA(launch_pdl(k_scal_bc, 1, 256, 0, st, ctx->dots, nb, ctx->hist_dev, k, ctx->scal,
+                        ctx->stat_dev));
     double *qn = basis_Q + (long)(k + 1) * n, *pn = basis_P + (long)(k + 1) * n;
-    k_normalize<<<nb, kDotThreads, 0, st>>>(ctx->rk, ctx->sk, ctx->scal, n, qn, pn, nullptr, nullptr,
-                                            0L);
+    TDS_CUDA(launch_pdl(k_normalize, nb, kDotThreads, 0, st, ctx->rk, ctx->sk, ctx->scal, n, qn, pn,
+                        nullptr, nullptr, 0L));
     if (reorthogonalize) {
         // one classical Gram-Schmidt pass of q_{k+1} against q_0..q_k with the
         // real mask product (the p side of the shared kernels runs on the
         // p_{k+1} slot, which the renormalisation then overwrites)
         int nvec = k + 1;
         const int nch = dot_chunks(n, nvec);
-        k_proj_dots<<<dim3(nvec, nch), 256, 0, st>>>(basis_Q, basis_Q, qn, pn, mask, n, n, part);
-        k_proj_scale<<<ceil_div(nvec, 8), 256, 0, st>>>(part, ctx->pqn, nvec, nch, ctx->rcoef);
+        TDS_CUDA(launch_pdl(k_proj_dots, dim3(nvec, nch), 256, 0, st, basis_Q, basis_Q, qn, pn,
+                            mask, n, n, part));
+        TDS_CUDA(launch_pdl(k_proj_scale, ceil_div(nvec, 8), 256, 0, st, part, ctx->pqn, nvec, nch,
+                            ctx->rcoef));
         for (int j0 = 0; j0 < nvec; j0 += kProjMax)
-            k_proj_apply<<<nb, 256, 0, st>>>(basis_Q, basis_Q, ctx->rcoef, n, j0,
-                                             std::min(kProjMax, nvec - j0), n, qn, pn, nullptr,
-                                             nullptr);
-        k_dot1<<<nb, kDotThreads, 0, st>>>(qn, qn, mask, n, ctx->dots);
-        k_qrenorm<<<nb, kDotThreads, 0, st>>>(ctx->dots, nb, ctx->scal, ctx->hist_dev, k, n, qn, pn);
-        k_pq_part<<<dim3(1, nch), 256, 0, st>>>(basis_Q, basis_Q, mask, n, n, k + 1, part);
-        k_pq_finish<<<1, 32, 0, st>>>(part, 1, k + 1, nch, ctx->pqn);
+            TDS_CUDA(launch_pdl(k_proj_apply, nb, 256, 0, st, basis_Q, basis_Q, ctx->rcoef, n, j0,
+                                std::min(kProjMax, nvec - j0), n, qn, pn, nullptr,
+                                nullptr));
+        TDS_CUDA(launch_pdl(k_dot1, nb, kDotThreads, 0, st, qn, qn, mask, n, ctx->dots));
+        TDS_CUDA(launch_pdl(k_qrenorm, nb, kDotThreads, 0, st, ctx->dots, nb, ctx->scal,
+                            ctx->hist_dev, k, n, qn, pn));
+        TDS_CUDA(launch_pdl(k_pq_part, dim3(1, nch), 256, 0, st, basis_Q, basis_Q, mask, n, n,
+                            k + 1, part));
+        TDS_CUDA(launch_pdl(k_pq_finish, 1, 32, 0, st, part, 1, k + 1, nch, ctx->pqn));
     }
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) { set_error("qlanczos_run launch: %s", cudaGetErrorString(e)); return TDSCHA_ERR_CUDA; }
@@ -2254,13 +2265,14 @@ extern "C" int tdscha_qkpm_run(tdscha_qctx *ctx, double *vm, double *v, double *
     double *a = vm, *b = v;
     *swapped = 0;
     for (int k = n_start; 2 * k < n_moments; ++k) {
-        k_dot1<<<nb, kDotThreads, 0, st>>>(b, b, ctx->mask, n, ctx->dots);
-        k_kpm_moment<<<1, 256, 0, st>>>(ctx->dots, nb, moments, 2 * k, 0);
+        TDS_CUDA(launch_pdl(k_dot1, nb, kDotThreads, 0, st, b, b, ctx->mask, n, ctx->dots));
+        TDS_CUDA(launch_pdl(k_kpm_moment, 1, 256, 0, st, ctx->dots, nb, moments, 2 * k, 0));
         if (2 * k + 1 >= n_moments) break;
         TDS_TRY(q_apply_full_L_dev(ctx, b, work, st));
-        k_kpm_combine<<<nb, kDotThreads, 0, st>>>(work, b, a, rescale_a, rescale_b, n);
-        k_dot1<<<nb, kDotThreads, 0, st>>>(a, b, ctx->mask, n, ctx->dots);
-        k_kpm_moment<<<1, 256, 0, st>>>(ctx->dots, nb, moments, 2 * k + 1, 1);
+        TDS_CUDA(launch_pdl(k_kpm_combine, nb, kDotThreads, 0, st, work, b, a, rescale_a, rescale_b,
+                            n));
+        TDS_CUDA(launch_pdl(k_dot1, nb, kDotThreads, 0, st, a, b, ctx->mask, n, ctx->dots));
+        TDS_CUDA(launch_pdl(k_kpm_moment, 1, 256, 0, st, ctx->dots, nb, moments, 2 * k + 1, 1));
         TDS_CHECK_LAUNCH();
         double *t = a;   // (vm, v) <- (v, vp)
         a = b;

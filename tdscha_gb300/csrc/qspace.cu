@@ -84,6 +84,16 @@ __global__ void k_q_to32(const double *__restrict__ a, long n, float *__restrict
         b[e] = (float)a[e];
 }
 
+// the same for a call's two arrays
+__global__ void k_q_call32(const double *__restrict__ a, long n, float *__restrict__ b,
+                           const double *__restrict__ a2, long n2, float *__restrict__ b2) {
+    pdl_enter();
+    for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < n + n2; e += (long)gridDim.x * blockDim.x) {
+        if (e < n) b[e] = (float)a[e];
+        else b2[e - n] = (float)a2[e - n];
+    }
+}
+
 // x_rot = S_j x_i for every image row, S_j in CSR (identity when n_syms == 0).
 // bad = 1 if any of the n entries of a or b is not finite
 __global__ void k_q_finite(const double *__restrict__ a, const double *__restrict__ b, long n,
@@ -127,6 +137,7 @@ __global__ void k_q_unpack(const double2 *__restrict__ psi, const int *__restric
                            const long *__restrict__ off_a, const long *__restrict__ off_b,
                            const double *__restrict__ pcoef, int n_pairs, int nb,
                            int ignore_v3, double2 *__restrict__ R1, double2 *__restrict__ alpha) {
+    pdl_enter();
     long n = (long)n_pairs * nb * nb;
     for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < n; e += (long)gridDim.x * blockDim.x) {
         int p = (int)(e / (nb * nb));
@@ -157,6 +168,7 @@ __global__ void __launch_bounds__(256, 4) k_q_rows(
         const int *__restrict__ qrole, const int *__restrict__ qpartner,
         int n_q, int nb, int S, long R, int iq_pert, int apply_d4, int rpb,
         T2 *__restrict__ rowc) {
+    pdl_enter();
     using T = typename CReal<T2>::type;
     __shared__ double red[8][8];   // per warp: tot, bfw, wR, wRf (re, im)
     const int lw = blockDim.x / rpb;
@@ -242,6 +254,7 @@ __global__ void k_q_favg(const T2 *__restrict__ Xr, const T2 *__restrict__ Yr,
                          const typename CReal<T2>::type *__restrict__ fY,
                          const T2 *__restrict__ rowc, int L, int nb, int iq_pert, long R,
                          long chunk, double2 *__restrict__ fpart) {
+    pdl_enter();
     using T = typename CReal<T2>::type;
     __shared__ double sh[2][32];
     int nu = blockIdx.x;
@@ -284,6 +297,7 @@ __global__ void k_q_d2v(const T2 *__restrict__ Xr, const T2 *__restrict__ Yr,
                         const typename CReal<T2>::type *__restrict__ fY,
                         const T2 *__restrict__ rowc, const int *__restrict__ pair_q, int L, int nb,
                         long R, long chunk, int n_pairs, double2 *__restrict__ dpart) {
+    pdl_enter();
     extern __shared__ __align__(16) unsigned char sm_raw[];
     T2 *sm = reinterpret_cast<T2 *>(sm_raw);   // kQRows x 4 nb, reused for the phase sum
     const int p = blockIdx.x;
@@ -345,6 +359,7 @@ __global__ void k_q_d2v(const T2 *__restrict__ Xr, const T2 *__restrict__ Yr,
 __global__ void k_q_finalize(const double2 *__restrict__ fpart, int nfchunk,
                              const double2 *__restrict__ dpart, int nbchunk, int nb, int n_pairs,
                              double inv_norm, double2 *__restrict__ f, double2 *__restrict__ d2v) {
+    pdl_enter();
     long n = (long)n_pairs * nb * nb;
     for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < n; e += (long)gridDim.x * blockDim.x) {
         double2 s = make_double2(0, 0);
@@ -524,25 +539,21 @@ static int q_perturb_t(tdscha_qctx *c, int apply_d4, const T2 *Xr, const T2 *Yr,
     const int nb = c->nb, L = c->L;
     const long R = c->R;
     const int rpb = q_rows_per_block(L);
-    k_q_rows<T2><<<ceil_div(R, rpb), 256, 0, st>>>(Xr, Yr, fY, fpsi, c->rho, R1, alpha, c->qpair,
-                                                    c->qrole, c->qpartner, c->n_q, nb, c->S, R,
-                                                    c->iq_pert, apply_d4, rpb, rowc);
-    TDS_CHECK_LAUNCH();
+    TDS_CUDA(launch_pdl(k_q_rows<T2>, ceil_div(R, rpb), 256, 0, st, Xr, Yr, fY, fpsi, c->rho, R1,
+                        alpha, c->qpair, c->qrole, c->qpartner, c->n_q, nb, c->S, R, c->iq_pert,
+                        apply_d4, rpb, rowc));
     long fchunk = (R + c->nfchunk - 1) / c->nfchunk;
-    k_q_favg<T2><<<dim3(nb, c->nfchunk), 256, 0, st>>>(Xr, Yr, fY, rowc, L, nb, c->iq_pert, R,
-                                                       fchunk, c->fpart);
-    TDS_CHECK_LAUNCH();
+    TDS_CUDA(launch_pdl(k_q_favg<T2>, dim3(nb, c->nfchunk), 256, 0, st, Xr, Yr, fY, rowc, L, nb,
+                        c->iq_pert, R, fchunk, c->fpart));
     long bchunk = (R + c->nbchunk - 1) / c->nbchunk;
     const int dthreads = q_d2v_threads(nb);
     size_t smem = sizeof(double2) * std::max(kQRows * 4 * nb, dthreads);
-    k_q_d2v<T2><<<dim3(c->n_pairs, c->nbchunk), dthreads, smem, st>>>(
-        Xr, Yr, fY, rowc, c->pair_q, L, nb, R, bchunk, c->n_pairs, c->dpart);
-    TDS_CHECK_LAUNCH();
+    TDS_CUDA(launch_pdl(k_q_d2v<T2>, dim3(c->n_pairs, c->nbchunk), dthreads, smem, st, Xr, Yr, fY,
+                        rowc, c->pair_q, L, nb, R, bchunk, c->n_pairs, c->dpart));
     long n = (long)c->n_pairs * nb * nb;
-    k_q_finalize<<<std::max(1, std::min(ceil_div(n, 256), 1024)), 256, 0, st>>>(
-        c->fpart, c->nfchunk, c->dpart, c->nbchunk, nb, c->n_pairs, 1.0 / (c->sum_rho * c->S),
-        c->f, c->d2v);
-    TDS_CHECK_LAUNCH();
+    TDS_CUDA(launch_pdl(k_q_finalize, std::max(1, std::min(ceil_div(n, 256), 1024)), 256, 0, st,
+                        c->fpart, c->nfchunk, c->dpart, c->nbchunk, nb, c->n_pairs,
+                        1.0 / (c->sum_rho * c->S), c->f, c->d2v));
     return TDSCHA_OK;
 }
 
@@ -553,12 +564,10 @@ static int q_perturb(tdscha_qctx *c, int apply_d4, cudaStream_t st) {
         return q_perturb_t<double2>(c, apply_d4, c->Xr, c->Yr, c->fY, c->fpsi, c->R1, c->alpha,
                                     c->rowc, st);
     const long na = 2L * c->n_pairs * c->nb * c->nb, nr = 2L * c->nb;
-    k_q_to32<<<std::max(1, std::min(ceil_div(na, 256), 256)), 256, 0, st>>>(
-        reinterpret_cast<const double *>(c->alpha), na, reinterpret_cast<float *>(c->alpha32));
-    TDS_CHECK_LAUNCH();
-    k_q_to32<<<1, 64, 0, st>>>(reinterpret_cast<const double *>(c->R1), nr,
-                               reinterpret_cast<float *>(c->R1_32));
-    TDS_CHECK_LAUNCH();
+    TDS_CUDA(launch_pdl(k_q_call32, std::max(1, std::min(ceil_div(na + nr, 256), 256)), 256, 0, st,
+                        reinterpret_cast<const double *>(c->alpha), na,
+                        reinterpret_cast<float *>(c->alpha32),
+                        reinterpret_cast<const double *>(c->R1), nr, reinterpret_cast<float *>(c->R1_32)));
     return q_perturb_t<float2>(c, apply_d4, c->Xr32, c->Yr32, c->fY32, c->fpsi32, c->R1_32,
                                c->alpha32, c->rowc32, st);
 }
@@ -568,10 +577,9 @@ int q_averages_dev(tdscha_qctx *c, const double *psi_in, cudaStream_t st) {
     const int nb = c->nb, d4 = c->ignore_v4 ? 0 : 1;
     if (c->precision != TDSCHA_PREC_MIXED && qdigits_ready(c)) return qdigits_perturb(c, d4, psi_in, st);
     const long n = (long)c->n_pairs * nb * nb;
-    k_q_unpack<<<std::max(1, std::min(ceil_div(n, 256), 1024)), 256, 0, st>>>(
-        reinterpret_cast<const double2 *>(psi_in), c->pair_q, c->q_off, c->q_off + c->n_pairs, c->pcoef,
-        c->n_pairs, nb, c->ignore_v3, c->R1, c->alpha);
-    TDS_CHECK_LAUNCH();
+    TDS_CUDA(launch_pdl(k_q_unpack, std::max(1, std::min(ceil_div(n, 256), 1024)), 256, 0, st,
+                        reinterpret_cast<const double2 *>(psi_in), c->pair_q, c->q_off,
+                        c->q_off + c->n_pairs, c->pcoef, c->n_pairs, nb, c->ignore_v3, c->R1, c->alpha));
     return q_perturb(c, d4, st);
 }
 

@@ -58,6 +58,7 @@ __device__ __forceinline__ long tri_index_s(int i, int j, int M) {
 // R1 = psi_R; Y1_ab = -2 (psi_W(ab) Upsilon_a) Upsilon_b
 __global__ void k_unpack_static(const double *__restrict__ psi, const double *__restrict__ Yw,
                                 int M, double *__restrict__ R1, double *__restrict__ Y1) {
+    pdl_enter();
     long n = (long)M * M;
     for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < n; e += (long)gridDim.x * blockDim.x) {
         int a = (int)(e / M), b = (int)(e % M);
@@ -83,6 +84,7 @@ __global__ void k_assemble_static(const double *__restrict__ psi, const double *
                                   const double *__restrict__ lam, const int *__restrict__ tri,
                                   int M, long H, int harm, int anh, double power,
                                   double *__restrict__ out) {
+    pdl_enter();
     // vector blockIdx.y of a batch
     psi += blockIdx.y * (M + H);
     out += blockIdx.y * (M + H);
@@ -203,23 +205,21 @@ extern "C" int tdscha_static_L(tdscha_ctx *ctx, int nvec, const double *psi_in, 
         double *f, *d2v;
         TDS_TRY(digits_from_static(ctx, ctx->ignore_v4 ? 0 : 1, n, psi_in + (long)v * Ps, &f, &d2v,
                                    st));
-        k_assemble_static<<<dim3(nba, n), 256, 0, st>>>(psi_in + (long)v * Ps, f, d2v, ctx->w,
-                                                        ctx->lam_static, ctx->tri, M, H, harm, anh,
-                                                        power, psi_out + (long)v * Ps);
-        TDS_CHECK_LAUNCH();
+        TDS_CUDA(launch_pdl(k_assemble_static, dim3(nba, n), 256, 0, st, psi_in + (long)v * Ps, f,
+                            d2v, ctx->w, ctx->lam_static, ctx->tri, M, H, harm, anh, power,
+                            psi_out + (long)v * Ps));
     }
     if (batch > 0) return TDSCHA_OK;
     for (int v = 0; v < nvec; ++v) {
         const double *in = psi_in + (long)v * Ps;
         double *out = psi_out + (long)v * Ps;
         if (anh) {
-            k_unpack_static<<<nbu, 256, 0, st>>>(in, ctx->Yw, M, ctx->R1, ctx->Y1);
-            TDS_CHECK_LAUNCH();
+            TDS_CUDA(launch_pdl(k_unpack_static, nbu, 256, 0, st, in, ctx->Yw, M, ctx->R1,
+                                ctx->Y1));
             TDS_TRY(run_perturb(ctx, ctx->ignore_v4 ? 0 : 1, precision, st));
         }
-        k_assemble_static<<<nba, 256, 0, st>>>(in, ctx->f, ctx->d2v, ctx->w, ctx->lam_static,
-                                               ctx->tri, M, H, harm, anh, power, out);
-        TDS_CHECK_LAUNCH();
+        TDS_CUDA(launch_pdl(k_assemble_static, nba, 256, 0, st, in, ctx->f, ctx->d2v, ctx->w,
+                            ctx->lam_static, ctx->tri, M, H, harm, anh, power, out));
     }
     return TDSCHA_OK;
 }
