@@ -468,14 +468,13 @@ __global__ void __launch_bounds__(DgShape<kMode>::threads, 1) k_dg_gemm(const Dg
                     pa += SA * (long)abytes;
                 }
             }
-            if (fail_code) {
-                *abort = 1;
-                // every issued copy must land before the CTA exits
-                for (long g = ga > slots ? ga - slots : 0; g < ga; ++g)
-                    mbar_wait(afull + 8 * (int)(g % slots), (uint32_t)(g / slots) & 1, kDefaultBudget);
-                for (long g = gb > 2 ? gb - 2 : 0; g < gb; ++g)
-                    mbar_wait(bfull + 8 * (int)(g & 1), (uint32_t)(g >> 1) & 1, kDefaultBudget);
-            }
+            if (fail_code) *abort = 1;
+            // every issued copy must land before the CTA exits, also where it is another
+            // role that has given up
+            for (long g = ga > slots ? ga - slots : 0; g < ga; ++g)
+                mbar_wait(afull + 8 * (int)(g % slots), (uint32_t)(g / slots) & 1, kDefaultBudget);
+            for (long g = gb > 2 ? gb - 2 : 0; g < gb; ++g)
+                mbar_wait(bfull + 8 * (int)(g & 1), (uint32_t)(g >> 1) & 1, kDefaultBudget);
         }
     } else if (warp == kEpi + 1) {
         {

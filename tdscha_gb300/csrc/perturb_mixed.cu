@@ -217,13 +217,12 @@ __global__ void __launch_bounds__(192, 1) k_stageA_tc(const __grid_constant__ Tm
                     tma_load_2d(base + 2 * kPLimbA + kPLimbB, &tm.b_lo, bar, kx, brow);
                 }
             }
-            if (fail_code) {
-                *abort = 1;
-                // every issued stage must land before the CTA exits
-                for (long gg = g > kPStages ? g - kPStages : 0; gg < g; ++gg)
-                    mbar_wait(full0 + 8 * (int)(gg % kPStages), (uint32_t)(gg / kPStages) & 1,
-                              kDefaultBudget);
-            }
+            if (fail_code) *abort = 1;
+            // every issued stage must land before the CTA exits, also where it is another
+            // role that has given up
+            for (long gg = g > kPStages ? g - kPStages : 0; gg < g; ++gg)
+                mbar_wait(full0 + 8 * (int)(gg % kPStages), (uint32_t)(gg / kPStages) & 1,
+                          kDefaultBudget);
         }
     } else if (warp == 5) {
         if (lane == 0) {
@@ -523,13 +522,12 @@ __global__ void __launch_bounds__(192, 1) k_stageA_tc1(const __grid_constant__ T
                                 brow);
                 }
             }
-            if (fail_code) {
-                *abort = 1;
-                // every issued slot must land before the CTA exits
-                for (long gg = g > kRSlots ? g - kRSlots : 0; gg < g; ++gg)
-                    mbar_wait(full0 + 8 * (int)(gg % kRSlots), (uint32_t)(gg / kRSlots) & 1,
-                              kDefaultBudget);
-            }
+            if (fail_code) *abort = 1;
+            // every issued slot must land before the CTA exits, also where it is another
+            // role that has given up
+            for (long gg = g > kRSlots ? g - kRSlots : 0; gg < g; ++gg)
+                mbar_wait(full0 + 8 * (int)(gg % kRSlots), (uint32_t)(gg / kRSlots) & 1,
+                          kDefaultBudget);
         }
     } else if (warp == 5) {
         if (lane == 0) {
@@ -839,13 +837,12 @@ __global__ void __launch_bounds__(352, 1) k_stageA_img(const __grid_constant__ T
                         }
                 p += j1 - j0;
             }
-            if (fail_code) {
-                *abort = 1;
-                // every issued slot must land before the CTA exits
-                for (long gg = g > kISlots ? g - kISlots : 0; gg < g; ++gg)
-                    mbar_wait(full0 + 8 * (int)(gg % kISlots), (uint32_t)(gg / kISlots) & 1,
-                              kDefaultBudget);
-            }
+            if (fail_code) *abort = 1;
+            // every issued slot must land before the CTA exits, also where it is another
+            // role that has given up
+            for (long gg = g > kISlots ? g - kISlots : 0; gg < g; ++gg)
+                mbar_wait(full0 + 8 * (int)(gg % kISlots), (uint32_t)(gg / kISlots) & 1,
+                          kDefaultBudget);
         }
     } else if (warp == 9) {
         const uint32_t one = elect_one();
@@ -933,11 +930,9 @@ __global__ void __launch_bounds__(352, 1) k_stageA_img(const __grid_constant__ T
                 if (fail_code) break;
                 p += j1 - j0;
             }
-            if (fail_code) {
-                *abort = 1;
-                if (seg > 0) mbar_wait(afull, (seg - 1) & 1, kDefaultBudget);
-                if (part > 0) mbar_wait(dgfull, (part - 1) & 1, kDefaultBudget);
-            }
+            if (fail_code) *abort = 1;
+            if (seg > 0) mbar_wait(afull, (seg - 1) & 1, kDefaultBudget);
+            if (part > 0) mbar_wait(dgfull, (part - 1) & 1, kDefaultBudget);
         }
     } else {
         // ---- epilogue: set 0 takes the even images, set 1 the odd ones
@@ -1140,12 +1135,12 @@ __global__ void __launch_bounds__(192, 1) k_stageB_tc(const __grid_constant__ Tm
                     tma_load_2d(base + 2 * kABytes + kBNB * kBK * 2, &tm.b_lo, bar, kx, brow);
                 }
             }
-            if (fail_code) {
-                *abort = 1;
-                for (long gg = g > kQStages ? g - kQStages : 0; gg < g; ++gg)
-                    mbar_wait(full0 + 8 * (int)(gg % kQStages), (uint32_t)(gg / kQStages) & 1,
-                              kDefaultBudget);
-            }
+            if (fail_code) *abort = 1;
+            // every issued stage must land before the CTA exits, also where it is another
+            // role that has given up
+            for (long gg = g > kQStages ? g - kQStages : 0; gg < g; ++gg)
+                mbar_wait(full0 + 8 * (int)(gg % kQStages), (uint32_t)(gg / kQStages) & 1,
+                          kDefaultBudget);
         }
     } else if (warp == 5) {
         if (lane == 0) {
