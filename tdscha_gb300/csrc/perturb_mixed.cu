@@ -1013,7 +1013,13 @@ __global__ void __launch_bounds__(352, 1) k_stageA_img(const __grid_constant__ T
                         o[3 * R] = tacc;
                     }
                 }
-                if (!here) fail_code = 3;
+                // (without an image of its own the set has not compared notes yet: threads
+                // that parted here would miss each other at the next named barrier)
+                const bool mine = j1 - j0 > 1 || (j0 & 1) == set;
+                if (!mine) {
+                    __syncwarp();
+                    if (epi_sync_or(!here, 1 + set)) fail_code = 3;
+                }
                 if (fail_code) break;
                 // the reads of d and g are generic-proxy, their refill is a TMA write
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");

@@ -28,7 +28,9 @@ def _call(ctx, R1, Y1, precision):
 @pytest.mark.parametrize("M,N,S,precision", [
     (20, 100, 1, nat.PREC_FP64), (66, 700, 1, nat.PREC_FP64), (129, 9000, 1, nat.PREC_FP64),
     (24, 400, 48, nat.PREC_FP64), (63, 1400, 48, nat.PREC_FP64), (189, 2000, 8, nat.PREC_FP64),
-    (20, 100, 1, nat.PREC_MIXED), (66, 700, 1, nat.PREC_MIXED), (129, 9000, 1, nat.PREC_MIXED)])
+    (20, 100, 1, nat.PREC_MIXED), (66, 700, 1, nat.PREC_MIXED), (129, 9000, 1, nat.PREC_MIXED),
+    # blocks with a single image of a row tile, so that one epilogue set has none
+    (24, 130, 24, nat.PREC_MIXED), (63, 1400, 48, nat.PREC_MIXED), (189, 2000, 8, nat.PREC_MIXED)])
 def test_averages(gpu_lib, monkeypatch, M, N, S, precision):
     ens = make_ensemble(M, N, seed=M + S, n_syms=S)
     tables = ((ens["symmetries"], ens["degenerate_space"], ens["sym_block_id"]) if S > 1
