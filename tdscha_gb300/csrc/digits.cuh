@@ -705,7 +705,9 @@ __global__ void __launch_bounds__(DgShape<kMode>::threads, 1) k_dg_gemm(const Dg
                     for (int e = 0; e < 4; ++e) {
                         q = fma(d[e], v[e], q);
                         p = fma(g[e], v[e], p);
-                        if (e0 < 12) {
+                        // (never past this warp's columns: the last part of a shared
+                        // tile ends with the tile, and the last tile with the array)
+                        if (e0 + 4 < ncol) {
                             d[e] = pd[(e0 + 4 + e) * 128];
                             g[e] = pg[(e0 + 4 + e) * 128];
                         }
