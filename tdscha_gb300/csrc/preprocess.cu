@@ -124,12 +124,13 @@ __global__ void k_prologue(const double *__restrict__ a, long n, int K, int widt
     }
 }
 
-// Digits of the rows a' of k_prologue (real data), one warp per row, and the
-// exponent above each row's maximum.  Rows past n (of the last tile) are zero.
+// Digits of the rows a' of k_prologue (real data), one warp per row, and the exponent
+// above each row's largest |a'| 2^-ec.  Rows past n (of the last tile) are zero.
 __global__ void __launch_bounds__(256) k_dg_slice_rows(const double *__restrict__ a, long n, int K,
                                                        int nkb, double s,
                                                        const double *__restrict__ sub,
                                                        const double *__restrict__ mul,
+                                                       const int *__restrict__ ec,
                                                        __half *__restrict__ out,
                                                        int *__restrict__ er) {
     const long r = blockIdx.x * 8L + (threadIdx.x >> 5);
@@ -144,7 +145,7 @@ __global__ void __launch_bounds__(256) k_dg_slice_rows(const double *__restrict_
     if (r < n)
         for (int k = lane; k < K; k += 32) {
             const double v = value(k);
-            if (v != 0) e = max(e, isfinite(v) ? exp_above(v) : kBadExp);
+            if (v != 0) e = max(e, isfinite(v) ? exp_above(v) - ec[k] : kBadExp);
         }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, o));
@@ -158,7 +159,7 @@ __global__ void __launch_bounds__(256) k_dg_slice_rows(const double *__restrict_
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             const int m = ch * 8 + k;
-            q[k] = m < K && !bad ? fixed_point(value(m), 55 - e) : 0;
+            q[k] = m < K && !bad ? fixed_point(value(m), 55 - ec[m] - e) : 0;
         }
         uint4 w[kRes];
         digits8<kRes>(q, w);
@@ -169,9 +170,10 @@ __global__ void __launch_bounds__(256) k_dg_slice_rows(const double *__restrict_
     }
 }
 
-// Digits of the columns of b (K x n): block = column (up to a multiple of 64, the
+// Digits of the columns of b 2^ec (K x n): block = column (up to a multiple of 64, the
 // padding zero)
-__global__ void __launch_bounds__(128) k_dg_slice_cols(const double *__restrict__ b, int K, int n,
+__global__ void __launch_bounds__(128) k_dg_slice_cols(const double *__restrict__ b,
+                                                       const int *__restrict__ ec, int K, int n,
                                                        int nkb, __half *__restrict__ out,
                                                        int *__restrict__ et) {
     __shared__ int sh[4];
@@ -180,7 +182,7 @@ __global__ void __launch_bounds__(128) k_dg_slice_cols(const double *__restrict_
     if (c < n)
         for (int k = threadIdx.x; k < K; k += blockDim.x) {
             const double v = b[(long)k * n + c];
-            if (v != 0) e = max(e, isfinite(v) ? exp_above(v) : kBadExp);
+            if (v != 0) e = max(e, isfinite(v) ? exp_above(v) + ec[k] : kBadExp);
         }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, o));
@@ -196,7 +198,7 @@ __global__ void __launch_bounds__(128) k_dg_slice_cols(const double *__restrict_
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             const int m = ch * 8 + k;
-            q[k] = m < K && !bad ? fixed_point(b[(long)m * n + c], 62 - e) : 0;
+            q[k] = m < K && !bad ? fixed_point(b[(long)m * n + c], 62 + ec[m] - e) : 0;
         }
         uint4 w[kCall];
         digits8<kCall>(q, w);
@@ -208,11 +210,14 @@ __global__ void __launch_bounds__(128) k_dg_slice_cols(const double *__restrict_
 }
 
 // C (rows x n) = A' B by digit products: A' the rows of k_prologue, B K x n.  The
-// digits of 2^16 rows at a time (14 bytes an element) beside those of B.
+// digits of 2^16 rows at a time (14 bytes an element) beside those of B.  The columns of A'
+// (coordinates) have scales of their own, which B's rows carry: atoms of unequal mass have
+// displacements and forces of unequal size, and a mode of the smaller ones keeps its bits.
 struct DigitProduct {
     void *slab = nullptr;
     __half *a = nullptr, *b = nullptr;
-    int *er = nullptr, *et = nullptr, *err = nullptr;
+    int *er = nullptr, *et = nullptr, *ec = nullptr, *err = nullptr;
+    unsigned long long *stat = nullptr;
     int K = 0, n = 0, nkb = 0, nbt = 0, nsm = 1;
     long chunk = 0;
     long long budget = kDefaultBudget;
@@ -233,8 +238,9 @@ struct DigitProduct {
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
         auto pad = [](size_t x) { return (x + 1023) & ~size_t(1023); };
         const size_t ba = (size_t)chunk * nkb * kGK * 2 * kRes, bb = (size_t)nbt * nkb * kCall * kGB,
-                     be = pad(sizeof(int) * chunk), bt = pad(sizeof(int) * nbt * kGN);
-        if (cached_malloc(&slab, ba + bb + be + bt + 1024) != cudaSuccess) {
+                     be = pad(sizeof(int) * chunk), bt = pad(sizeof(int) * nbt * kGN),
+                     bs = pad(sizeof(*stat) * 2 * K), bc = pad(sizeof(int) * K);
+        if (cached_malloc(&slab, ba + bb + be + bt + bs + bc + 1024) != cudaSuccess) {
             cudaGetLastError();
             slab = nullptr;
             return false;
@@ -244,22 +250,35 @@ struct DigitProduct {
         b = reinterpret_cast<__half *>(p + ba);
         er = reinterpret_cast<int *>(p + ba + bb);
         et = reinterpret_cast<int *>(p + ba + bb + be);
-        err = reinterpret_cast<int *>(p + ba + bb + be + bt);
+        stat = reinterpret_cast<unsigned long long *>(p + ba + bb + be + bt);
+        ec = reinterpret_cast<int *>(p + ba + bb + be + bt + bs);
+        err = reinterpret_cast<int *>(p + ba + bb + be + bt + bs + bc);
         return true;
     }
 
-    int set_b(const double *B) {
+    int begin() {
         TDS_CUDA(cudaMemsetAsync(err, 0, sizeof(int), 0));
         TDS_CUDA((dg_setup<DG_STORE, false>()));
-        k_dg_slice_cols<<<nbt * kGN, 128>>>(B, K, n, nkb, b, et);
-        TDS_CHECK_LAUNCH();
         return TDSCHA_OK;
     }
 
-    int product(const double *A, long rows, double s, const double *sub, const double *mul, double *C) {
+    int product(const double *A, long rows, double s, const double *sub, const double *mul,
+                const double *B, double *C) {
+        // rows a block walks one after the other: 64, more where the grid would not hold them
+        const long per = std::max<long>(64, (rows + 65534) / 65535);
+        TDS_CUDA(cudaMemsetAsync(stat, 0, sizeof(*stat) * 2 * K, 0));
+        k_dg_colstat<<<dim3(ceil_div(K, 128), ceil_div(rows, per)), 128>>>(A, rows, K, per, s, sub, nullptr,
+                                                                           1, stat);
+        TDS_CHECK_LAUNCH();
+        // (with a mean taken off, s is in what was counted)
+        k_dg_colscale<<<ceil_div(K, 128), 128>>>(stat, K, K, sub ? 1.0 : s, mul, 0, ec);
+        TDS_CHECK_LAUNCH();
+        k_dg_slice_cols<<<nbt * kGN, 128>>>(B, ec, K, n, nkb, b, et);
+        TDS_CHECK_LAUNCH();
         for (long r0 = 0; r0 < rows; r0 += chunk) {
             const long nr = std::min(chunk, rows - r0), nrp = (nr + kGM - 1) / kGM * kGM;
-            k_dg_slice_rows<<<(unsigned)(nrp / 8), 256>>>(A + r0 * K, nr, K, nkb, s, sub, mul, a, er);
+            k_dg_slice_rows<<<(unsigned)(nrp / 8), 256>>>(A + r0 * K, nr, K, nkb, s, sub, mul, ec, a,
+                                                                er);
             TDS_CHECK_LAUNCH();
             DgArgs g{};
             g.a = a;
@@ -413,14 +432,14 @@ extern "C" int tdscha_project_modes(int N, int n_cart, int M, const double *u, c
     PCU(cudaMemcpy(d_vec + n_cart, isq.data(), sizeof(double) * n_cart, cudaMemcpyHostToDevice));
     if (f_mean) PCU(cudaMemcpy(d_vec + 2 * n_cart, sub.data(), sizeof(double) * n_cart, cudaMemcpyHostToDevice));
     int nb = std::max(1, std::min(ceil_div((long)nu, 256), 152 * 8)), rc = TDSCHA_OK;
-    if (digits && (rc = dg.set_b(d_pols)) != TDSCHA_OK) return done(rc);
+    if (digits && (rc = dg.begin()) != TDSCHA_OK) return done(rc);
     for (int pass = 0; pass < 2; ++pass) {
         PCU(cudaMemcpy(d_in, pass == 0 ? u : f, sizeof(double) * nu, cudaMemcpyHostToDevice));
         const double scale = pass == 0 ? u_scale : f_scale;
         const double *sub = pass == 1 && f_mean ? d_vec + 2 * n_cart : nullptr;
         const double *mul = pass == 0 ? d_vec : d_vec + n_cart;
         if (digits) {
-            rc = dg.product(d_in, N, scale, sub, mul, d_out);
+            rc = dg.product(d_in, N, scale, sub, mul, d_pols, d_out);
         } else {
             k_prologue<<<nb, 256>>>(d_in, N, n_cart, 1, scale, sub, mul, d_tmp);
             PCU(cudaGetLastError());
