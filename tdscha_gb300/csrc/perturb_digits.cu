@@ -778,8 +778,10 @@ int digits_prepare(tdscha_ctx *c) {
     x->err = reinterpret_cast<int *>(c->host_pinned);
     *x->err = 0;
     TDS_CUDA(cudaMemsetAsync((uint8_t *)x->slab + zero0, 0, total - zero0, 0));
-    // rows a block walks one after the other: 8 in a small ensemble, at most 128
-    const long walk = std::min<long>(128, std::max<long>(8, R / 400));
+    // rows a block walks one after the other: 8 in a small ensemble, 128 in a large one, more
+    // where the grid's second dimension (65535) would not hold the blocks
+    const long walk = std::max<long>(std::min<long>(128, std::max<long>(8, R / 400)),
+                                     (R + 65534) / 65535);
     k_dg_colmax<<<dim3(ceil_div(M, 128), ceil_div(R, walk)), 128>>>(c->D, c->F, c->fY, R, M, walk,
                                                                     x->dmax, x->gmax);
     TDS_CHECK_LAUNCH();
