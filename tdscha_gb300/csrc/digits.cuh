@@ -24,6 +24,7 @@ constexpr int kFlushMax = 9;
 constexpr int kFlushes = kFlushMax - kFlushMin + 1;
 constexpr int kUnit = -69;      // one unit of the order-7 accumulator: 2^(-7-6-56)
 constexpr int kBadExp = 1 << 20;   // exponent of a row with a non-finite element
+constexpr int kZeroExp = -8192;    // of a row of zeros: 2^kZeroExp counts as 0
 constexpr uint32_t kGA = kGM * kGK * 2;   // bytes of one digit of an A block
 constexpr uint32_t kGB = kGN * kGK * 2;   // and of a B block
 
@@ -125,14 +126,10 @@ __device__ __forceinline__ double fixed_to_double(long long hi, long long lo, in
     return __longlong_as_double((long long)(bits | ((uint64_t)(sgn & 0x80000000u) << 32)));
 }
 
-// 2^e for the exponents of finite float64 rows
-__device__ __forceinline__ double pow2(int e) { return ldexp(1.0, e); }
-
-__device__ __forceinline__ void atomic_max_abs(unsigned long long *addr, double v) {
-    // absolute values order like their bit patterns (NaN above infinity)
-    atomicMax(addr, (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffULL);
+// 2^e for the exponents of finite float64 rows (0 below the normal numbers)
+__device__ __forceinline__ double pow2(int e) {
+    return __longlong_as_double((long long)(e < -1022 ? 0 : min(e + 1023, 2047)) << 52);
 }
-
 
 // Scales of the columns of an operand whose rows get a scale each as well.  A row's scale
 // is the exponent above its largest |a| 2^-ec, so any ec keeps the digits in range; what
@@ -179,8 +176,8 @@ static __global__ void k_dg_colscale(const unsigned long long *__restrict__ stat
     if (k < K && stat[K + k]) {
         const long long sum = (long long)stat[k], n = (long long)stat[K + k], t = 2 * sum + n;
         e = (int)((t - (t < 0 ? 2 * n - 1 : 0)) / (2 * n));        // rounded, ties upwards
-        if (mul) e += inverse ? -exp_above(mul[k]) : exp_above(mul[k]);
-        e += exp_above(s);
+        if (mul) e += inverse ? -exp_above(mul[k]) : exp_above(mul[k]) - 1;
+        e += exp_above(s) - 1;
     }
     ec[k] = e;
 }

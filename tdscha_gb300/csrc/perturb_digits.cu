@@ -36,6 +36,14 @@
 // One call: M=573 N=50000 57.1 -> 1.71 ms; M=189 N=10000 48 images 62.8 -> 2.10 ms;
 // M=97 N=4999 554 -> 66 us; M=21 N=1000 245 -> 34 us.
 //
+// Scales: a mode's is the mean exponent of its elements (k_dg_colscale), a configuration's
+// the exponent above its largest element in those units.  Both are powers of two and both
+// operands of stage B are without the configuration's: W's rows carry it instead.  So a
+// configuration that the weights take out, or nearly so, costs the others nothing, however
+// far out it lies.  With the columns' maxima over all configurations as their only scales
+// one outlier of weight 0, 1e6 times the others, took 20 bits from all of them: errors of
+// d2v of 2e-11 (and 2e-9 at 1e8).
+//
 // Form of the contractions, with g = y / f_Y (= f_psi y) so that both operands
 // of the second stage come from x and g alone (u = f_Y x, y = f_Y g):
 //
@@ -64,23 +72,6 @@ namespace tdscha {
 // abcc[(4 image + k) Rp + row]
 
 // ------------------------------------------------- once per ensemble
-// Column maxima of |x| and |g|.
-__global__ void k_dg_colmax(const double *__restrict__ D, const double *__restrict__ F,
-                            const double *__restrict__ fY, long R, int M, long rows_per_block,
-                            unsigned long long *__restrict__ dmax,
-                            unsigned long long *__restrict__ gmax) {
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= M) return;
-    const long rb = blockIdx.y * rows_per_block, re = min(R, rb + rows_per_block);
-    double a = 0, b = 0;
-    for (long r = rb; r < re; ++r) {
-        a = fmax(a, fabs(D[r * M + m]));
-        b = fmax(b, fabs(F[r * M + m]));
-    }
-    atomic_max_abs(dmax + m, a);
-    atomic_max_abs(gmax + m, b / fY[m]);
-}
-
 // dt, gt: 128 rows x 32 modes per block through shared memory.  Rows and modes
 // past the end are zero.  g = y / f_Y by the reciprocal and one residual step
 // (a division costs about ten float64 operations), so that f_Y g is y to one
@@ -111,16 +102,7 @@ __global__ void k_dg_cols(const double *__restrict__ D, const double *__restrict
     }
 }
 
-// ec[m]: exponent above the column's maximum; 0 for a zero or padding column
-__global__ void k_dg_colexp(const unsigned long long *__restrict__ dmax, int M, int Mp,
-                            int *__restrict__ ec) {
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= Mp) return;
-    const double d = m < M ? __longlong_as_double((long long)dmax[m]) : 0.0;
-    ec[m] = d > 0 ? exp_above(d) : 0;
-}
-
-// er[r]: exponent above the maximum over the modes of |x| 2^-ec (0 for a zero row)
+// er[r]: exponent above the maximum over the modes of |x| 2^-ec (kZeroExp for a zero row)
 __global__ void k_dg_rowexp(const double *__restrict__ dt, const int *__restrict__ ec, int M,
                             int Mp, int *__restrict__ er) {
     __shared__ int sh[8][128];
@@ -135,7 +117,7 @@ __global__ void k_dg_rowexp(const double *__restrict__ dt, const int *__restrict
     __syncthreads();
     if (g == 0) {
         for (int k = 1; k < 8; ++k) e = max(e, sh[k][row]);
-        er[rt * 128 + row] = e == INT_MIN ? 0 : e;
+        er[rt * 128 + row] = e == INT_MIN ? kZeroExp : e;
     }
 }
 
@@ -189,7 +171,8 @@ __global__ void __launch_bounds__(256) k_dg_ga(const double *__restrict__ gt,
 }
 
 __global__ void __launch_bounds__(256) k_dg_xb(const double *__restrict__ dt,
-                                               const int *__restrict__ ec, int Mp, long nkb,
+                                               const int *__restrict__ ec,
+                                               const int *__restrict__ er, int Mp, long nkb,
                                                __half *__restrict__ xb, float *__restrict__ nrm) {
     const long kb = blockIdx.x;
     const int at = blockIdx.y, c = threadIdx.x & 7;
@@ -201,8 +184,9 @@ __global__ void __launch_bounds__(256) k_dg_xb(const double *__restrict__ dt,
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const double2 v = dg_two(src + 2 * j);
-            q[2 * j] = fixed_point(v.x, 55 - ec[a]);
-            q[2 * j + 1] = fixed_point(v.y, 55 - ec[a]);
+            const int2 e = *reinterpret_cast<const int2 *>(er + kb * kGK + 8 * c + 2 * j);
+            q[2 * j] = fixed_point(v.x, 55 - ec[a] - e.x);
+            q[2 * j + 1] = fixed_point(v.y, 55 - ec[a] - e.y);
         }
         uint4 w[kRes];
         digits8<kRes>(q, w);
@@ -320,21 +304,23 @@ __global__ void __launch_bounds__(128) k_dg_y1(const DgSources src, const double
 }
 
 // Row scalars of the image blockIdx.y from the stage A partials (s and t of many images
-// from st, [2 Rp][images]); max |alpha|, max |beta / 2| and the maxima of the force
-// weights of the image.  Rows past the end get zeros.
+// from st, [2 Rp][images]), those of W times the row's scale of x, which the row of xb
+// does without; max |alpha| and max |beta / 2| with the scales of g's and x's row, and with
+// many images the same of the force weights.  Rows past the end get zeros.
 template <bool kMany>
 __global__ void __launch_bounds__(128) k_dg_rows(const double *__restrict__ qp,
                                                  const double *__restrict__ st, int nct, long R,
                                                  long Rp, int rho_div,
                                                  const double *__restrict__ rho,
-                                                 const int *__restrict__ er, int apply_d4,
+                                                 const int *__restrict__ er,
+                                                 const int *__restrict__ erg, int apply_d4,
                                                  double *__restrict__ abcc,
                                                  unsigned long long *__restrict__ absmax) {
     pdl_enter();
     constexpr int kMax = kMany ? 4 : 2;
     __shared__ unsigned long long red[kMax][4];
     const long img = blockIdx.y, r = blockIdx.x * 128L + threadIdx.x;
-    double w[4] = {0, 0, 0, 0};
+    double w[4] = {0, 0, 0, 0}, top[4] = {0, 0, 0, 0};
     if (r < R) {
         double q = 0, p = 0, s = 0, t = 0;
         const double *o = qp + img * nct * 4 * R + r;
@@ -350,7 +336,7 @@ __global__ void __launch_bounds__(128) k_dg_rows(const double *__restrict__ qp,
             s = st[r * gridDim.y + img];
             t = st[(Rp + r) * gridDim.y + img];
         }
-        const double f = pow2(er[r]), rw = rho[r / rho_div];
+        const double f = pow2(er[r]), fg = pow2(erg[r]), rw = rho[r / rho_div];
         q *= f;
         p *= f;
         // rho / 3 by the reciprocal and one residual step: a warp's float64 operation
@@ -358,10 +344,16 @@ __global__ void __launch_bounds__(128) k_dg_rows(const double *__restrict__ qp,
         constexpr double third = 1.0 / 3.0;
         const double y = rw * third, t3 = fma(fma(-y, 3.0, rw), third, y), h3 = 0.5 * t3,
                      t8 = apply_d4 ? 0.125 * rw : 0.0;
-        w[0] = fma(s, t3, -q * t8);           // rho (s / 3 - q / 8)
-        w[1] = fma(t, h3, -p * t8);           // rho (t / 3 - p / 4) / 2
+        w[0] = fma(s, t3, -q * t8) * f;       // rho (s / 3 - q / 8)
+        w[1] = fma(t, h3, -p * t8) * f;       // rho (t / 3 - p / 4) / 2
         w[2] = -q * h3;
         w[3] = -p * t3;
+        top[0] = w[0] * fg;
+        top[1] = w[1] * f;
+        if (kMany) {
+            w[2] = top[2] = w[2] * fg;
+            w[3] = top[3] = w[3] * f;
+        }
     }
     if (r < Rp) {
         double *o = abcc + 4 * img * Rp + r;
@@ -372,7 +364,7 @@ __global__ void __launch_bounds__(128) k_dg_rows(const double *__restrict__ qp,
     }
 #pragma unroll
     for (int k = 0; k < kMax; ++k) {
-        unsigned long long a = (unsigned long long)__double_as_longlong(w[k]) & 0x7fffffffffffffffULL;
+        unsigned long long a = (unsigned long long)__double_as_longlong(top[k]) & 0x7fffffffffffffffULL;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) a = max(a, __shfl_xor_sync(0xffffffffu, a, o));
         if ((threadIdx.x & 31) == 0) red[k][threadIdx.x >> 5] = a;
@@ -385,13 +377,19 @@ __global__ void __launch_bounds__(128) k_dg_rows(const double *__restrict__ qp,
     }
 }
 
-// Exponent above max|alpha| max|g| + max|beta/2| max|x| of a mode of an image, kBadExp
-// where that is not finite; am: the image's four maxima.
-__device__ __forceinline__ int dg_wexp(const unsigned long long *__restrict__ am, double dm, double gm) {
-    // a little above the bound: w itself is rounded
-    const double bound = (__longlong_as_double((long long)am[0]) * gm +
-                          __longlong_as_double((long long)am[1]) * dm) * (1.0 + 0x1p-40);
-    return !isfinite(bound) ? kBadExp : bound > 0 ? exp_above(bound) : 0;
+// Exponent above |w| of a mode of an image, kBadExp where that is not finite: am, the
+// image's maxima of the rows' weights with their scales, times the scales of the mode in
+// g and x (an element is below its row's and its column's scale).  Whole numbers only: every
+// row of a W block asks for it, and four float64 operations each were 6 of the 250 us of
+// 24 vectors at M=60, N=5000.
+__device__ __forceinline__ int dg_wexp(const unsigned long long *__restrict__ am, int ex, int eg) {
+    constexpr unsigned long long kInf = 0x7ff0000000000000ULL;
+    const unsigned long long a = am[0], b = am[1];
+    if (a >= kInf || b >= kInf) return kBadExp;
+    if (!(a | b)) return 0;
+    const int ea = a ? exp_above(__longlong_as_double((long long)a)) + eg : INT_MIN,
+              eb = b ? exp_above(__longlong_as_double((long long)b)) + ex : INT_MIN;
+    return max(ea, eb) + 1;             // of the sum of both
 }
 
 // Digits of eight numbers as row `row` of the A block blk, chunk c
@@ -410,8 +408,8 @@ __device__ __forceinline__ void dg_put(const long long (&q)[8], uint8_t *blk, in
 __global__ void __launch_bounds__(256) k_dg_wbuild(
     const double *__restrict__ dt, const double *__restrict__ gt,
     const double *__restrict__ abcc, const unsigned long long *__restrict__ absmax,
-    const unsigned long long *__restrict__ dmax, const unsigned long long *__restrict__ gmax,
-    const double *__restrict__ fY, int M, int Mp, long Rp, int nimg, long nkb, int per,
+    const int *__restrict__ ec, const double *__restrict__ fY, int M, int Mp, long Rp, int nimg,
+    long nkb, int per,
     __half *__restrict__ wa, int *__restrict__ ew, double *__restrict__ fpart) {
     pdl_enter();
     const int c = threadIdx.x & 7;
@@ -425,8 +423,7 @@ __global__ void __launch_bounds__(256) k_dg_wbuild(
         const bool live = img < nimg && b < M;
         double f1 = 0, f2 = 0;
         if (live) {
-            const int e = dg_wexp(absmax + 4 * img, __longlong_as_double((long long)dmax[b]),
-                                  __longlong_as_double((long long)gmax[b]));
+            const int e = dg_wexp(absmax + 4 * img, ec[b], ec[Mp + b]);
             const bool bad = e == kBadExp;
             const int K = 62 - e;
             if (blockIdx.x == 0 && c == 0) ew[grow] = e;
@@ -469,8 +466,8 @@ constexpr int kWImages = 8;
 __global__ void __launch_bounds__(256) k_dg_wimages(
     const double *__restrict__ dt, const double *__restrict__ gt,
     const double *__restrict__ abcc, const unsigned long long *__restrict__ absmax,
-    const unsigned long long *__restrict__ dmax, const unsigned long long *__restrict__ gmax, int M,
-    int Mp, long Rp, int nimg, long nkb, __half *__restrict__ wa, int *__restrict__ ew,
+    const int *__restrict__ ec, int M, int Mp, long Rp, int nimg, long nkb,
+    __half *__restrict__ wa, int *__restrict__ ew,
     __half *__restrict__ wf, int *__restrict__ ewf) {
     pdl_enter();
     const int c = threadIdx.x & 7, slot = threadIdx.x >> 3, i0 = blockIdx.z * kWImages,
@@ -500,8 +497,7 @@ __global__ void __launch_bounds__(256) k_dg_wimages(
         const int img = i0 + (t >> 5), m = b0 + (t & 31);
         int e = 0;
         if (m < M)
-            e = dg_wexp(absmax + 4 * img, __longlong_as_double((long long)dmax[m]),
-                        __longlong_as_double((long long)gmax[m]));
+            e = dg_wexp(absmax + 4 * img, ec[m], ec[Mp + m]);
         sexp[t >> 5][t & 31] = e;
         if (kb == 0 && m < M) ew[(long)img * Mp + m] = e;
     }
@@ -633,7 +629,7 @@ struct DigitStore {
     int cap = 1;                 // images that the per-call buffers hold
     int per = 1, nfc = 1;        // K blocks of one W block, force partials an image
     // s, t and the forces as digit products of their own (many symmetry images): g's
-    // digits behind x's in xa and xb, its exponents behind x's in er and ec
+    // digits behind x's in xa and xb.  (Its exponents are always behind x's in er and ec.)
     bool many = false;
     int kbF = 1, nsF = 1;
     double *st = nullptr, *gf = nullptr;
@@ -644,7 +640,7 @@ struct DigitStore {
     double *dt = nullptr, *gt = nullptr, *vs = nullptr, *vt = nullptr, *qp = nullptr,
            *gpart = nullptr, *fpart = nullptr, *fo = nullptr, *d2vo = nullptr;
     double *abcc = nullptr;
-    unsigned long long *dmax = nullptr, *gmax = nullptr, *absmax = nullptr;
+    unsigned long long *absmax = nullptr;
     __half *xa = nullptr, *xb = nullptr, *yb = nullptr, *wa = nullptr;
     int *ec = nullptr, *er = nullptr, *et = nullptr, *ew = nullptr;
     int *err = nullptr;          // bounded-wait failure code (pinned host memory)
@@ -711,6 +707,7 @@ int digits_prepare(tdscha_ctx *c) {
         if (x->flushB == kFlushMin) break;
     }
     float *fl = nullptr;         // largest digit norms of xa and of xb
+    unsigned long long *stat = nullptr;
     struct Part {
         void **p;
         size_t bytes;
@@ -722,7 +719,7 @@ int digits_prepare(tdscha_ctx *c) {
         {(void **)&x->gt, d * elems, false},
         {(void **)&x->xa, two * 2 * kRes * elems, false},
         {(void **)&x->xb, two * 2 * kRes * elems, false},
-        {(void **)&x->er, two * i4 * x->Rp, false},
+        {(void **)&x->er, 2 * i4 * x->Rp, false},
         {(void **)&x->st, one * d * 2 * cap * x->Rp, false},
         {(void **)&x->gf, one * d * x->nsF * kGM * 2 * Mp, false},
         {(void **)&x->bmap, one * i4 * 2 * nrt, false},
@@ -733,10 +730,9 @@ int digits_prepare(tdscha_ctx *c) {
         {(void **)&x->fpart, d * (size_t)cap * x->nfc * M, false},
         {(void **)&x->fo, c->J == 1 ? d * cap * M : 0, false},
         {(void **)&x->d2vo, c->J == 1 ? d * (size_t)cap * M * M : 0, false},
-        {(void **)&x->ec, two * i4 * Mp, false},
-        // zero from the start: maxima, and the rows of padding modes
-        {(void **)&x->dmax, u8 * Mp, true},
-        {(void **)&x->gmax, u8 * Mp, true},
+        {(void **)&x->ec, 2 * i4 * Mp, false},
+        // zero from the start: sums, maxima, and the rows of padding modes
+        {(void **)&stat, u8 * 4 * M, true},
         {(void **)&x->absmax, u8 * 4 * cap, true},
         {(void **)&x->etv, one * i4 * 2 * kGN, true},
         {(void **)&x->ewf, one * i4 * kGM, true},
@@ -782,15 +778,22 @@ int digits_prepare(tdscha_ctx *c) {
     // where the grid's second dimension (65535) would not hold the blocks
     const long walk = std::max<long>(std::min<long>(128, std::max<long>(8, R / 400)),
                                      (R + 65534) / 65535);
-    k_dg_colmax<<<dim3(ceil_div(M, 128), ceil_div(R, walk)), 128>>>(c->D, c->F, c->fY, R, M, walk,
-                                                                    x->dmax, x->gmax);
+    int *ecg = x->ec + Mp, *erg = x->er + x->Rp;
+    const dim3 cols(ceil_div(M, 128), ceil_div(R, walk));
+    k_dg_colstat<<<cols, 128>>>(c->D, R, M, walk, 1.0, nullptr, c->rho, c->rho_div, stat);
     TDS_CHECK_LAUNCH();
-    k_dg_colexp<<<ceil_div(Mp, 128), 128>>>(x->dmax, M, Mp, x->ec);
+    k_dg_colstat<<<cols, 128>>>(c->F, R, M, walk, 1.0, nullptr, c->rho, c->rho_div, stat + 2 * M);
+    TDS_CHECK_LAUNCH();
+    k_dg_colscale<<<ceil_div(Mp, 128), 128>>>(stat, M, Mp, 1.0, nullptr, 0, x->ec);
+    TDS_CHECK_LAUNCH();
+    k_dg_colscale<<<ceil_div(Mp, 128), 128>>>(stat + 2 * M, M, Mp, 1.0, c->fY, 1, ecg);
     TDS_CHECK_LAUNCH();
     k_dg_cols<<<dim3((unsigned)nrt, Mp / 32), dim3(32, 8)>>>(c->D, c->F, c->fY, R, M, Mp, x->dt,
                                                               x->gt);
     TDS_CHECK_LAUNCH();
     k_dg_rowexp<<<(unsigned)nrt, dim3(128, 8)>>>(x->dt, x->ec, M, Mp, x->er);
+    TDS_CHECK_LAUNCH();
+    k_dg_rowexp<<<(unsigned)nrt, dim3(128, 8)>>>(x->gt, ecg, M, Mp, erg);
     TDS_CHECK_LAUNCH();
     // the digit norms pass through the W digits' space, which is zeroed again
     float *nrm = reinterpret_cast<float *>(x->wa);
@@ -798,20 +801,15 @@ int digits_prepare(tdscha_ctx *c) {
     TDS_CHECK_LAUNCH();
     k_dg_windows<<<dim3((unsigned)nrt, kFlushes), kGM>>>(nrm, x->nkbM, fl);
     TDS_CHECK_LAUNCH();
-    k_dg_xb<<<dim3((unsigned)x->nkbR, x->nct), 256>>>(x->dt, x->ec, Mp, x->nkbR, x->xb, nrm);
+    k_dg_xb<<<dim3((unsigned)x->nkbR, x->nct), 256>>>(x->dt, x->ec, x->er, Mp, x->nkbR, x->xb, nrm);
     TDS_CHECK_LAUNCH();
     k_dg_windows<<<dim3(x->nct, kFlushes), kGN>>>(nrm, (int)x->nkbR, fl + kFlushes * kRes);
     TDS_CHECK_LAUNCH();
     if (x->many) {
         __half *ga = x->xa + kRes * elems, *gb = x->xb + kRes * elems;
-        int *ecg = x->ec + Mp, *erg = x->er + x->Rp;
-        k_dg_colexp<<<ceil_div(Mp, 128), 128>>>(x->gmax, M, Mp, ecg);
-        TDS_CHECK_LAUNCH();
-        k_dg_rowexp<<<(unsigned)nrt, dim3(128, 8)>>>(x->gt, ecg, M, Mp, erg);
-        TDS_CHECK_LAUNCH();
         k_dg_ga<<<dim3((unsigned)nrt, x->nkbM), 256>>>(x->gt, ecg, erg, M, Mp, x->nkbM, ga);
         TDS_CHECK_LAUNCH();
-        k_dg_xb<<<dim3((unsigned)x->nkbR, x->nct), 256>>>(x->gt, ecg, Mp, x->nkbR, gb, nrm);
+        k_dg_xb<<<dim3((unsigned)x->nkbR, x->nct), 256>>>(x->gt, ecg, erg, Mp, x->nkbR, gb, nrm);
         TDS_CHECK_LAUNCH();
         std::vector<int> bm(2 * nrt, 0);
         std::fill(bm.begin() + nrt, bm.end(), 1);
@@ -916,8 +914,8 @@ static int digits_contract(tdscha_ctx *c, int nimg, const DgSources &src, int ap
         TDS_CUDA(launch_pdl(x->many ? k_dg_rows<true> : k_dg_rows<false>, dim3((unsigned)(x->Rp / 128), nimg), 128, 0, st,
                             (const double *)x->qp, (const double *)x->st,
                             x->nct * win, R, x->Rp, c->rho_div,
-                            (const double *)c->rho, (const int *)x->er, apply_d4, x->abcc,
-                            x->absmax));
+                            (const double *)c->rho, (const int *)x->er,
+                            (const int *)x->er + x->Rp, apply_d4, x->abcc, x->absmax));
     }
     const int nat = ceil_div((long)nimg * Mp, kGM);
     {
@@ -926,8 +924,7 @@ static int digits_contract(tdscha_ctx *c, int nimg, const DgSources &src, int ap
             TDS_CUDA(launch_pdl(k_dg_wimages, dim3(x->nkbR, Mp / 32 + 1, ceil_div(nimg, kWImages)), 256,
                                 0, st, (const double *)x->dt, (const double *)x->gt,
                                 (const double *)x->abcc, (const unsigned long long *)x->absmax,
-                                (const unsigned long long *)x->dmax,
-                                (const unsigned long long *)x->gmax, M, Mp, x->Rp, nimg, x->nkbR,
+                                (const int *)x->ec, M, Mp, x->Rp, nimg, x->nkbR,
                                 x->wa, x->ew, x->wf, x->ewf));
         else
             // (few blocks: a group of 32 modes each)
@@ -935,9 +932,8 @@ static int digits_contract(tdscha_ctx *c, int nimg, const DgSources &src, int ap
                                 256, 0, st, (const double *)x->dt,
                                 (const double *)x->gt, (const double *)x->abcc,
                                 (const unsigned long long *)x->absmax,
-                                (const unsigned long long *)x->dmax,
-                                (const unsigned long long *)x->gmax, (const double *)c->fY, M, Mp,
-                                x->Rp, nimg, x->nkbR, x->per, x->wa, x->ew, x->fpart));
+                                (const int *)x->ec, (const double *)c->fY, M, Mp, x->Rp, nimg,
+                                x->nkbR, x->per, x->wa, x->ew, x->fpart));
     }
     DgArgs gb{};
     gb.a = x->wa;

@@ -6,7 +6,9 @@ measured against the part in question, not against the largest part."""
 import numpy as np
 import pytest
 
+import oracle
 from tdscha_gb300 import _native as nat
+from tdscha_gb300.synthetic import make_ensemble, random_R1, random_sym
 
 pytestmark = pytest.mark.gpu
 
@@ -38,3 +40,39 @@ def test_projection_of_two_sublattices(gpu_lib, ratio):
         ref = a @ p
         for part in (slice(0, n), slice(n, 2 * n)):
             assert np.abs(got[:, part] - ref[:, part]).max() <= 2e-15 * np.abs(ref[:, part]).max()
+
+
+def _outlier(a, what, size):
+    a = a.copy()
+    if what == "row":
+        a[37] *= size
+    elif what == "element":
+        a[37, 5] *= size
+    return a
+
+
+@pytest.mark.parametrize("S", [1, 48])
+@pytest.mark.parametrize("x,y", [("row", "row"), ("row", ""), ("", "row"), ("element", "element"),
+                                 ("element", ""), ("", "element")])
+@pytest.mark.parametrize("weight,size", [(0.0, 1e3), (0.0, 1e6), (0.0, 1e8), (1e-40, 1e6),
+                                         (1e-24, 1e6), (1e-12, 1e3)])
+def test_outlier_of_little_weight(gpu_lib, x, y, weight, size, S):
+    """One configuration far out in displacements, forces or one of their elements, with a
+    weight of zero, one that makes it vanish, or one that leaves it a part in the sums.  The
+    oracle adds up N S <= 2e4 float64 terms: 5e-13 of the largest entry (as for ordinary
+    ensembles, tests/test_gpu_digits.py)."""
+    M, N = (63, 2000) if S == 1 else (24, 400)
+    ens = make_ensemble(M, N, seed=12, n_syms=S, rho_sigma=0.1)
+    tables = ((ens["symmetries"], ens["degenerate_space"], ens["sym_block_id"]) if S > 1
+              else oracle.identity_symmetries(M))
+    X, Y, rho = _outlier(ens["X"], x, size), _outlier(ens["Y"], y, size), ens["rho"].copy()
+    rho[37] = weight
+    R1, Y1 = random_R1(M, 3), random_sym(M, 4, scale=1e-5)
+    ref = oracle.perturb_averages(X, Y, ens["w"], rho, R1, Y1, ens["T"], 1, *tables, n_threads=8)
+    ctx = nat.Context(X, Y, ens["w"], rho, ens["T"], *tables)
+    f, d2v = np.zeros(M), np.zeros((M, M))
+    nat.check(nat.load().tdscha_perturb_averages(ctx.handle, nat.dp(R1), nat.dp(Y1), 1, nat.PREC_FP64,
+                                                 nat.dp(f), nat.dp(d2v), 0, None))
+    ctx.close()
+    for a, b in zip((f, d2v), ref):
+        assert np.abs(a - b).max() <= 1e-12 * np.abs(b).max()
