@@ -83,6 +83,7 @@ struct tdscha_ctx {
     long P = 0;                 // psi length M + M(M+1)
     long H = 0;                 // M(M+1)/2
     double T = 0, sum_rho = 0;  // sum_rho accumulated in config order
+    int rho_top = 0;            // exponent of the largest weight (frexp)
     int with_mixed = 0;     // 0 float64 only, 1 float64 + mixed, 2 mixed with 4-byte storage only
     // operator options
     int use_wigner = 1, ignore_harmonic = 0, ignore_v3 = 0, ignore_v4 = 0, reverse_L = 0;

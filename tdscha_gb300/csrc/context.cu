@@ -305,10 +305,11 @@ extern "C" int tdscha_ctx_create(tdscha_ctx **out, int M, int N, const double *X
     // X and Y are checked for non-finite entries on the device (k_expand_images)
     for (int mu = 0; mu < M; ++mu)
         if (!(w[mu] > 0) || !std::isfinite(w[mu])) { set_error("ctx_create: frequency w[%d]=%g must be positive", mu, w[mu]); return TDSCHA_ERR_ARG; }
-    double sum_rho = 0;
+    double sum_rho = 0, max_rho = 0;
     for (int i = 0; i < N; ++i) {
         if (!std::isfinite(rho[i])) { set_error("ctx_create: non-finite rho[%d]", i); return TDSCHA_ERR_NAN; }
         sum_rho += rho[i];
+        max_rho = std::max(max_rho, std::fabs(rho[i]));
     }
     if (sum_rho == 0) { set_error("ctx_create: sum of weights is zero"); return TDSCHA_ERR_ARG; }
 
@@ -318,6 +319,7 @@ extern "C" int tdscha_ctx_create(tdscha_ctx **out, int M, int N, const double *X
     c->H = (long)M * (M + 1) / 2;
     c->P = M + 2 * c->H;
     c->T = T; c->sum_rho = sum_rho;
+    std::frexp(max_rho, &c->rho_top);
     c->with_mixed = with_mixed;
 
     int rc = TDSCHA_OK;

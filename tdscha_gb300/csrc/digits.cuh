@@ -166,6 +166,12 @@ static __global__ void __launch_bounds__(128) k_dg_colstat(const double *__restr
     atomicAdd(stat + K + k, (unsigned long long)cnt);
 }
 
+// sum / n rounded, ties upwards
+__device__ __forceinline__ int dg_mean_exp(long long sum, long long n) {
+    const long long t = 2 * sum + n;
+    return (int)((t - (t < 0 ? 2 * n - 1 : 0)) / (2 * n));
+}
+
 // ec[k] = mean exponent of column k, and of mul[k] (or of 1 / mul[k]) and s beside it
 // where they multiply the elements that were counted; 0 of a column without any
 static __global__ void k_dg_colscale(const unsigned long long *__restrict__ stat, int K, int Kp, double s,
@@ -174,12 +180,17 @@ static __global__ void k_dg_colscale(const unsigned long long *__restrict__ stat
     if (k >= Kp) return;
     int e = 0;
     if (k < K && stat[K + k]) {
-        const long long sum = (long long)stat[k], n = (long long)stat[K + k], t = 2 * sum + n;
-        e = (int)((t - (t < 0 ? 2 * n - 1 : 0)) / (2 * n));        // rounded, ties upwards
+        e = dg_mean_exp((long long)stat[k], (long long)stat[K + k]);
         if (mul) e += inverse ? -exp_above(mul[k]) : exp_above(mul[k]) - 1;
         e += exp_above(s) - 1;
     }
     ec[k] = e;
+}
+
+// What a configuration's element counts for in the scale of its column: its exponent, less
+// what its weight is below the largest one (exponent rtop); INT_MIN of nothing.
+__device__ __forceinline__ int dg_weighted_exp(double x, double rho, int rtop) {
+    return x != 0 && rho != 0 ? exp_above(x) + min(0, exp_above(rho) - rtop) : INT_MIN;
 }
 
 // Sums of the squares of each digit over the 64 elements of a block's row, from

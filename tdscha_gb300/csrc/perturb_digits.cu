@@ -36,13 +36,17 @@
 // One call: M=573 N=50000 57.1 -> 1.71 ms; M=189 N=10000 48 images 62.8 -> 2.10 ms;
 // M=97 N=4999 554 -> 66 us; M=21 N=1000 245 -> 34 us.
 //
-// Scales: a mode's is the mean exponent of its elements (k_dg_colscale), a configuration's
-// the exponent above its largest element in those units.  Both are powers of two and both
-// operands of stage B are without the configuration's: W's rows carry it instead.  So a
-// configuration that the weights take out, or nearly so, costs the others nothing, however
-// far out it lies.  With the columns' maxima over all configurations as their only scales
-// one outlier of weight 0, 1e6 times the others, took 20 bits from all of them: errors of
-// d2v of 2e-11 (and 2e-9 at 1e8).
+// Scales: a mode's is the largest exponent of its elements, each less what its
+// configuration's weight is below the largest weight; a configuration's is the exponent
+// above its largest element in those units.  Both are powers of two and both operands of
+// stage B are without the configuration's: W's rows carry it instead.  So a configuration
+// that the weights take out, or nearly so, costs the others nothing, however far out it
+// lies, and loses itself at most as many bits as its weight is smaller (a scale of a
+// configuration is never further above 1 than that).  With the columns' maxima over all
+// configurations as the only scales one outlier of weight 0, 1e6 times the others, took 20
+// bits from all of them: errors of d2v of 2e-11 (and 2e-9 at 1e8).  The mean exponent of a
+// mode's elements as its scale leaves a mode of rounding noise over many decades, as
+// symmetry makes them, to set the scales of the configurations.
 //
 // Form of the contractions, with g = y / f_Y (= f_psi y) so that both operands
 // of the second stage come from x and g alone (u = f_Y x, y = f_Y g):
@@ -72,6 +76,32 @@ namespace tdscha {
 // abcc[(4 image + k) Rp + row]
 
 // ------------------------------------------------- once per ensemble
+// ec[m], ec[Mp + m]: largest weighted exponents of column m of D and of F (before: kNone)
+constexpr int kNone = (int)0x80808080u;
+__global__ void __launch_bounds__(128) k_dg_colexp(const double *__restrict__ D,
+                                                   const double *__restrict__ F,
+                                                   const double *__restrict__ rho, int rho_div, int rtop,
+                                                   long R, int M, int Mp, long per,
+                                                   int *__restrict__ ec) {
+    const int m = blockIdx.x * 128 + threadIdx.x;
+    if (m >= M) return;
+    const double *a = blockIdx.z ? F : D;
+    const long r0 = blockIdx.y * per, r1 = min(R, r0 + per);
+    int e = INT_MIN;
+#pragma unroll 4
+    for (long r = r0; r < r1; ++r)
+        e = max(e, dg_weighted_exp(a[r * M + m], rho[rho_div == 1 ? r : r / rho_div], rtop));
+    atomicMax(ec + blockIdx.z * Mp + m, e);
+}
+
+// From there: 0 of a column without an element, and g's scales from y's
+__global__ void k_dg_colend(const double *__restrict__ fY, int M, int Mp, int *__restrict__ ec) {
+    const int m = blockIdx.x * blockDim.x + threadIdx.x;
+    if (m >= 2 * Mp) return;
+    const int e = ec[m], k = m % Mp;
+    ec[m] = e == kNone ? 0 : m >= Mp ? e - exp_above(fY[k]) : e;
+}
+
 // dt, gt: 128 rows x 32 modes per block through shared memory.  Rows and modes
 // past the end are zero.  g = y / f_Y by the reciprocal and one residual step
 // (a division costs about ten float64 operations), so that f_Y g is y to one
@@ -707,7 +737,6 @@ int digits_prepare(tdscha_ctx *c) {
         if (x->flushB == kFlushMin) break;
     }
     float *fl = nullptr;         // largest digit norms of xa and of xb
-    unsigned long long *stat = nullptr;
     struct Part {
         void **p;
         size_t bytes;
@@ -731,8 +760,7 @@ int digits_prepare(tdscha_ctx *c) {
         {(void **)&x->fo, c->J == 1 ? d * cap * M : 0, false},
         {(void **)&x->d2vo, c->J == 1 ? d * (size_t)cap * M * M : 0, false},
         {(void **)&x->ec, 2 * i4 * Mp, false},
-        // zero from the start: sums, maxima, and the rows of padding modes
-        {(void **)&stat, u8 * 4 * M, true},
+        // zero from the start: maxima, and the rows of padding modes
         {(void **)&x->absmax, u8 * 4 * cap, true},
         {(void **)&x->etv, one * i4 * 2 * kGN, true},
         {(void **)&x->ewf, one * i4 * kGM, true},
@@ -779,14 +807,11 @@ int digits_prepare(tdscha_ctx *c) {
     const long walk = std::max<long>(std::min<long>(128, std::max<long>(8, R / 400)),
                                      (R + 65534) / 65535);
     int *ecg = x->ec + Mp, *erg = x->er + x->Rp;
-    const dim3 cols(ceil_div(M, 128), ceil_div(R, walk));
-    k_dg_colstat<<<cols, 128>>>(c->D, R, M, walk, 1.0, nullptr, c->rho, c->rho_div, stat);
+    TDS_CUDA(cudaMemsetAsync(x->ec, kNone & 0xff, i4 * 2 * Mp, 0));
+    k_dg_colexp<<<dim3(ceil_div(M, 128), ceil_div(R, walk), 2), 128>>>(
+        c->D, c->F, c->rho, c->rho_div, c->rho_top, R, M, Mp, walk, x->ec);
     TDS_CHECK_LAUNCH();
-    k_dg_colstat<<<cols, 128>>>(c->F, R, M, walk, 1.0, nullptr, c->rho, c->rho_div, stat + 2 * M);
-    TDS_CHECK_LAUNCH();
-    k_dg_colscale<<<ceil_div(Mp, 128), 128>>>(stat, M, Mp, 1.0, nullptr, 0, x->ec);
-    TDS_CHECK_LAUNCH();
-    k_dg_colscale<<<ceil_div(Mp, 128), 128>>>(stat + 2 * M, M, Mp, 1.0, c->fY, 1, ecg);
+    k_dg_colend<<<ceil_div(2 * Mp, 128), 128>>>(c->fY, M, Mp, x->ec);
     TDS_CHECK_LAUNCH();
     k_dg_cols<<<dim3((unsigned)nrt, Mp / 32), dim3(32, 8)>>>(c->D, c->F, c->fY, R, M, Mp, x->dt,
                                                               x->gt);

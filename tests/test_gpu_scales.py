@@ -76,3 +76,28 @@ def test_outlier_of_little_weight(gpu_lib, x, y, weight, size, S):
     ctx.close()
     for a, b in zip((f, d2v), ref):
         assert np.abs(a - b).max() <= 1e-12 * np.abs(b).max()
+
+
+@pytest.mark.parametrize("S", [1, 48])
+@pytest.mark.parametrize("x,y", [(True, False), (False, True), (True, True)])
+def test_mode_of_noise(gpu_lib, x, y, S):
+    """Modes that symmetry holds at zero, up to rounding noise over 40 decades: the others
+    keep their accuracy.  Tolerance as above."""
+    M, N = (63, 2000) if S == 1 else (24, 400)
+    ens = make_ensemble(M, N, seed=13, n_syms=S, rho_sigma=0.1)
+    tables = ((ens["symmetries"], ens["degenerate_space"], ens["sym_block_id"]) if S > 1
+              else oracle.identity_symmetries(M))
+    rng = np.random.default_rng(2)
+    X, Y = ens["X"].copy(), ens["Y"].copy()
+    for a, on in ((X, x), (Y, y)):
+        if on:
+            a[:, 3:6] = rng.standard_normal((N, 3)) * 10.0 ** rng.uniform(-57, -17, (N, 3))
+    R1, Y1 = random_R1(M, 3), random_sym(M, 4, scale=1e-5)
+    ref = oracle.perturb_averages(X, Y, ens["w"], ens["rho"], R1, Y1, ens["T"], 1, *tables, n_threads=8)
+    ctx = nat.Context(X, Y, ens["w"], ens["rho"], ens["T"], *tables)
+    f, d2v = np.zeros(M), np.zeros((M, M))
+    nat.check(nat.load().tdscha_perturb_averages(ctx.handle, nat.dp(R1), nat.dp(Y1), 1, nat.PREC_FP64,
+                                                 nat.dp(f), nat.dp(d2v), 0, None))
+    ctx.close()
+    for a, b in zip((f, d2v), ref):
+        assert np.abs(a - b).max() <= 1e-12 * np.abs(b).max()
