@@ -131,62 +131,6 @@ __device__ __forceinline__ double pow2(int e) {
     return __longlong_as_double((long long)(e < -1022 ? 0 : min(e + 1023, 2047)) << 52);
 }
 
-// Scales of the columns of an operand whose rows get a scale each as well.  A row's scale
-// is the exponent above its largest |a| 2^-ec, so any ec keeps the digits in range; what
-// counts is that it makes the columns alike.  The mean exponent of a column's non-zero
-// elements does, and a few rows with outliers do not move it as they move the maximum (one
-// element a million times larger took 20 of 55 bits from its column in every other row).
-//
-// stat[k], stat[K + k]: sum of the exponents of a s - sub (sub may be null) over the
-// non-zero finite elements of column k, and their number; rows of weight 0 do not count
-// (rho may be null; row r has rho[r / rho_div]).  Whole numbers: the same in any order.
-static __global__ void __launch_bounds__(128) k_dg_colstat(const double *__restrict__ a, long rows, int K,
-                                                           long per, double s,
-                                                           const double *__restrict__ sub,
-                                                           const double *__restrict__ rho, int rho_div,
-                                                           unsigned long long *__restrict__ stat) {
-    const int k = blockIdx.x * 128 + threadIdx.x;
-    if (k >= K) return;
-    const long r0 = blockIdx.y * per, r1 = min(rows, r0 + per);
-    const double m = sub ? -sub[k] : 0.0;
-    long long sum = 0;
-    int cnt = 0;
-#pragma unroll 8
-    for (long r = r0; r < r1; ++r) {
-        double v = a[r * K + k];
-        if (sub) v = fma(v, s, m);
-        const int e = (int)((__double_as_longlong(v) >> 52) & 0x7ff);
-        if (e != 0 && e != 0x7ff && !(rho && rho[r / rho_div] == 0.0)) {
-            sum += e - 1022;
-            ++cnt;
-        }
-    }
-    if (!cnt) return;
-    atomicAdd(stat + k, (unsigned long long)sum);
-    atomicAdd(stat + K + k, (unsigned long long)cnt);
-}
-
-// sum / n rounded, ties upwards
-__device__ __forceinline__ int dg_mean_exp(long long sum, long long n) {
-    const long long t = 2 * sum + n;
-    return (int)((t - (t < 0 ? 2 * n - 1 : 0)) / (2 * n));
-}
-
-// ec[k] = mean exponent of column k, and of mul[k] (or of 1 / mul[k]) and s beside it
-// where they multiply the elements that were counted; 0 of a column without any
-static __global__ void k_dg_colscale(const unsigned long long *__restrict__ stat, int K, int Kp, double s,
-                                     const double *__restrict__ mul, int inverse, int *__restrict__ ec) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= Kp) return;
-    int e = 0;
-    if (k < K && stat[K + k]) {
-        e = dg_mean_exp((long long)stat[k], (long long)stat[K + k]);
-        if (mul) e += inverse ? -exp_above(mul[k]) : exp_above(mul[k]) - 1;
-        e += exp_above(s) - 1;
-    }
-    ec[k] = e;
-}
-
 // What a configuration's element counts for in the scale of its column: its exponent, less
 // what its weight is below the largest one (exponent rtop); INT_MIN of nothing.
 __device__ __forceinline__ int dg_weighted_exp(double x, double rho, int rtop) {

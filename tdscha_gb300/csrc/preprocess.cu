@@ -124,6 +124,44 @@ __global__ void k_prologue(const double *__restrict__ a, long n, int K, int widt
     }
 }
 
+// Scales of the columns of a'.  A row's scale is the exponent above its largest
+// |a'| 2^-ec, so any ec keeps the digits in range; what counts is that it makes the columns
+// alike.  Every row is a result of its own here, so ec is the mean over blocks of rows of the
+// largest exponent of a block: an outlier moves it by its block's share only, and a column
+// of rounding noise over many decades counts by its largest elements.
+//
+// stat[k], stat[K + k]: sum over the blocks of `per` rows of the largest exponent of
+// a s - sub (or of a, without sub) in column k, and the number of blocks that have one
+__global__ void __launch_bounds__(128) k_dg_colstat(const double *__restrict__ a, long rows, int K, long per,
+                                                    double s, const double *__restrict__ sub,
+                                                    unsigned long long *__restrict__ stat) {
+    const int k = blockIdx.x * 128 + threadIdx.x;
+    if (k >= K) return;
+    const long r0 = blockIdx.y * per, r1 = min(rows, r0 + per);
+    const double m = sub ? -sub[k] : 0.0;
+    int e = INT_MIN;
+#pragma unroll 8
+    for (long r = r0; r < r1; ++r) {
+        double v = a[r * K + k];
+        if (sub) v = fma(v, s, m);
+        if (v != 0 && isfinite(v)) e = max(e, exp_above(v));
+    }
+    if (e == INT_MIN) return;
+    atomicAdd(stat + k, (unsigned long long)(long long)e);
+    atomicAdd(stat + K + k, 1ULL);
+}
+
+// ec[k]: the mean, and the exponents of mul[k] and of s where they multiply what was
+// counted; 0 of a column without an element
+__global__ void k_dg_colscale(const unsigned long long *__restrict__ stat, int K, double s,
+                              const double *__restrict__ mul, int *__restrict__ ec) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= K) return;
+    const long long n = (long long)stat[K + k], t = 2 * (long long)stat[k] + n;
+    // rounded, ties upwards
+    ec[k] = n == 0 ? 0 : (int)((t - (t < 0 ? 2 * n - 1 : 0)) / (2 * n)) + exp_above(mul[k]) + exp_above(s) - 2;
+}
+
 // Digits of the rows a' of k_prologue (real data), one warp per row, and the exponent
 // above each row's largest |a'| 2^-ec.  Rows past n (of the last tile) are zero.
 __global__ void __launch_bounds__(256) k_dg_slice_rows(const double *__restrict__ a, long n, int K,
@@ -264,14 +302,14 @@ struct DigitProduct {
 
     int product(const double *A, long rows, double s, const double *sub, const double *mul,
                 const double *B, double *C) {
-        // rows a block walks one after the other: 64, more where the grid would not hold them
-        const long per = std::max<long>(64, (rows + 65534) / 65535);
+        // rows a block walks one after the other: 64, fewer where there would be less than
+        // 64 blocks, more where the grid would not hold them
+        const long per = std::max(std::min<long>(64, std::max<long>(4, rows / 64)), (rows + 65534) / 65535);
         TDS_CUDA(cudaMemsetAsync(stat, 0, sizeof(*stat) * 2 * K, 0));
-        k_dg_colstat<<<dim3(ceil_div(K, 128), ceil_div(rows, per)), 128>>>(A, rows, K, per, s, sub, nullptr,
-                                                                           1, stat);
+        k_dg_colstat<<<dim3(ceil_div(K, 128), ceil_div(rows, per)), 128>>>(A, rows, K, per, s, sub, stat);
         TDS_CHECK_LAUNCH();
         // (with a mean taken off, s is in what was counted)
-        k_dg_colscale<<<ceil_div(K, 128), 128>>>(stat, K, K, sub ? 1.0 : s, mul, 0, ec);
+        k_dg_colscale<<<ceil_div(K, 128), 128>>>(stat, K, sub ? 1.0 : s, mul, ec);
         TDS_CHECK_LAUNCH();
         k_dg_slice_cols<<<nbt * kGN, 128>>>(B, ec, K, n, nkb, b, et);
         TDS_CHECK_LAUNCH();

@@ -42,6 +42,32 @@ def test_projection_of_two_sublattices(gpu_lib, ratio):
             assert np.abs(got[:, part] - ref[:, part]).max() <= 2e-15 * np.abs(ref[:, part]).max()
 
 
+@pytest.mark.parametrize("what", ["row", "element", "noise"])
+def test_projection_of_outliers_and_noise(gpu_lib, what):
+    """One configuration, or one element of it, 1e6 times the others: each of the others
+    keeps its accuracy; and coordinates of rounding noise over 40 decades: all do.  2e-15 of
+    the largest entry of X, Y in ordinary configurations, as above."""
+    from tdscha_gb300.preprocessing import project_modes
+    rng = np.random.default_rng(9)
+    N, n, M = 2000, 60, 57
+    u, f = rng.standard_normal((N, n)), rng.standard_normal((N, n))
+    masses = rng.uniform(1.0, 10.0, n)
+    pols = np.linalg.qr(rng.standard_normal((n, n)))[0][:, :M]
+    ordinary = np.ones(N, dtype=bool)
+    for a in (u, f):
+        if what == "noise":
+            a[:, 6:9] *= 10.0 ** rng.uniform(-57, -17, (N, 3))
+        else:
+            a[37, slice(None) if what == "row" else 5] *= 1e6
+            ordinary[37] = False
+    X, Y = project_modes(u, f, masses, pols, None, u_scale=0.5, f_scale=2.0)
+    root, p = np.sqrt(masses).astype(LD), pols.astype(LD)
+    for got, a in ((X, u.astype(LD) * LD(0.5) * root), (Y, f.astype(LD) * 2 / root)):
+        ref = a @ p
+        assert np.abs(got - ref)[ordinary].max() <= 2e-15 * np.abs(ref[ordinary]).max()
+        assert np.abs(got - ref)[37].max() <= 2e-15 * np.abs(ref[37]).max()
+
+
 def _outlier(a, what, size):
     a = a.copy()
     if what == "row":
