@@ -94,12 +94,15 @@ __global__ void __launch_bounds__(128) k_dg_colexp(const double *__restrict__ D,
     atomicMax(ec + blockIdx.z * Mp + m, e);
 }
 
-// From there: 0 of a column without an element, and g's scales from y's
-__global__ void k_dg_colend(const double *__restrict__ fY, int M, int Mp, int *__restrict__ ec) {
+// From there: g's scales from y's, and 0 of a column without an element; eb has kZeroExp
+// there, for what is scaled with it: Y1's rows and the bounds of W
+__global__ void k_dg_colend(const double *__restrict__ fY, int M, int Mp, int *__restrict__ ec,
+                            int *__restrict__ eb) {
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= 2 * Mp) return;
-    const int e = ec[m], k = m % Mp;
-    ec[m] = e == kNone ? 0 : m >= Mp ? e - exp_above(fY[k]) : e;
+    const int e = ec[m], k = m % Mp, s = m >= Mp && k < M ? e - exp_above(fY[k]) : e;
+    ec[m] = e == kNone ? 0 : s;
+    eb[m] = e == kNone ? kZeroExp : s;
 }
 
 // dt, gt: 128 rows x 32 modes per block through shared memory.  Rows and modes
@@ -268,7 +271,7 @@ __device__ __forceinline__ double dg_y1(const DgSource &c, const double *__restr
     return n == m ? a : 0.5 * (a + b);
 }
 
-// Row n of image blockIdx.y of Y1 (symmetric): digits of y 2^(ec - et) with et
+// Row n of image blockIdx.y of Y1 (symmetric): digits of y 2^(eb - et) with et
 // the exponent above the row's maximum, and the two vectors of the row scalars.
 // Also clears the image's maxima of alpha, beta and the force weights.  With many
 // images rows M and M + 1 are those two vectors, digits of rows `image` of the tiles vb.
@@ -438,7 +441,7 @@ __device__ __forceinline__ void dg_put(const long long (&q)[8], uint8_t *blk, in
 __global__ void __launch_bounds__(256) k_dg_wbuild(
     const double *__restrict__ dt, const double *__restrict__ gt,
     const double *__restrict__ abcc, const unsigned long long *__restrict__ absmax,
-    const int *__restrict__ ec, const double *__restrict__ fY, int M, int Mp, long Rp, int nimg,
+    const int *__restrict__ eb, const double *__restrict__ fY, int M, int Mp, long Rp, int nimg,
     long nkb, int per,
     __half *__restrict__ wa, int *__restrict__ ew, double *__restrict__ fpart) {
     pdl_enter();
@@ -453,7 +456,7 @@ __global__ void __launch_bounds__(256) k_dg_wbuild(
         const bool live = img < nimg && b < M;
         double f1 = 0, f2 = 0;
         if (live) {
-            const int e = dg_wexp(absmax + 4 * img, ec[b], ec[Mp + b]);
+            const int e = dg_wexp(absmax + 4 * img, eb[b], eb[Mp + b]);
             const bool bad = e == kBadExp;
             const int K = 62 - e;
             if (blockIdx.x == 0 && c == 0) ew[grow] = e;
@@ -496,7 +499,7 @@ constexpr int kWImages = 8;
 __global__ void __launch_bounds__(256) k_dg_wimages(
     const double *__restrict__ dt, const double *__restrict__ gt,
     const double *__restrict__ abcc, const unsigned long long *__restrict__ absmax,
-    const int *__restrict__ ec, int M, int Mp, long Rp, int nimg, long nkb,
+    const int *__restrict__ eb, int M, int Mp, long Rp, int nimg, long nkb,
     __half *__restrict__ wa, int *__restrict__ ew,
     __half *__restrict__ wf, int *__restrict__ ewf) {
     pdl_enter();
@@ -527,7 +530,7 @@ __global__ void __launch_bounds__(256) k_dg_wimages(
         const int img = i0 + (t >> 5), m = b0 + (t & 31);
         int e = 0;
         if (m < M)
-            e = dg_wexp(absmax + 4 * img, ec[m], ec[Mp + m]);
+            e = dg_wexp(absmax + 4 * img, eb[m], eb[Mp + m]);
         sexp[t >> 5][t & 31] = e;
         if (kb == 0 && m < M) ew[(long)img * Mp + m] = e;
     }
@@ -672,7 +675,7 @@ struct DigitStore {
     double *abcc = nullptr;
     unsigned long long *absmax = nullptr;
     __half *xa = nullptr, *xb = nullptr, *yb = nullptr, *wa = nullptr;
-    int *ec = nullptr, *er = nullptr, *et = nullptr, *ew = nullptr;
+    int *ec = nullptr, *eb = nullptr, *er = nullptr, *et = nullptr, *ew = nullptr;
     int *err = nullptr;          // bounded-wait failure code (pinned host memory)
     long long budget = kDefaultBudget;
 };
@@ -760,6 +763,7 @@ int digits_prepare(tdscha_ctx *c) {
         {(void **)&x->fo, c->J == 1 ? d * cap * M : 0, false},
         {(void **)&x->d2vo, c->J == 1 ? d * (size_t)cap * M * M : 0, false},
         {(void **)&x->ec, 2 * i4 * Mp, false},
+        {(void **)&x->eb, 2 * i4 * Mp, false},
         // zero from the start: maxima, and the rows of padding modes
         {(void **)&x->absmax, u8 * 4 * cap, true},
         {(void **)&x->etv, one * i4 * 2 * kGN, true},
@@ -811,7 +815,7 @@ int digits_prepare(tdscha_ctx *c) {
     k_dg_colexp<<<dim3(ceil_div(M, 128), ceil_div(R, walk), 2), 128>>>(
         c->D, c->F, c->rho, c->rho_div, c->rho_top, R, M, Mp, walk, x->ec);
     TDS_CHECK_LAUNCH();
-    k_dg_colend<<<ceil_div(2 * Mp, 128), 128>>>(c->fY, M, Mp, x->ec);
+    k_dg_colend<<<ceil_div(2 * Mp, 128), 128>>>(c->fY, M, Mp, x->ec, x->eb);
     TDS_CHECK_LAUNCH();
     k_dg_cols<<<dim3((unsigned)nrt, Mp / 32), dim3(32, 8)>>>(c->D, c->F, c->fY, R, M, Mp, x->dt,
                                                               x->gt);
@@ -872,7 +876,7 @@ static int digits_contract(tdscha_ctx *c, int nimg, const DgSources &src, int ap
     {
         ProfScope ps(c, 5, st);
         TDS_CUDA(launch_pdl(k_dg_y1, dim3(x->many ? M + 2 : M, nimg), 128, sizeof(double) * M, st,
-                            src, (const double *)c->fY, (const int *)x->ec, M, Mp, x->yb, x->et,
+                            src, (const double *)c->fY, (const int *)x->eb, M, Mp, x->yb, x->et,
                             x->vs, x->vt, x->vb, x->etv, x->absmax));
         if (x->many) {
             // s and t of all images: [x; g] times their vectors
@@ -949,7 +953,7 @@ static int digits_contract(tdscha_ctx *c, int nimg, const DgSources &src, int ap
             TDS_CUDA(launch_pdl(k_dg_wimages, dim3(x->nkbR, Mp / 32 + 1, ceil_div(nimg, kWImages)), 256,
                                 0, st, (const double *)x->dt, (const double *)x->gt,
                                 (const double *)x->abcc, (const unsigned long long *)x->absmax,
-                                (const int *)x->ec, M, Mp, x->Rp, nimg, x->nkbR,
+                                (const int *)x->eb, M, Mp, x->Rp, nimg, x->nkbR,
                                 x->wa, x->ew, x->wf, x->ewf));
         else
             // (few blocks: a group of 32 modes each)
@@ -957,7 +961,7 @@ static int digits_contract(tdscha_ctx *c, int nimg, const DgSources &src, int ap
                                 256, 0, st, (const double *)x->dt,
                                 (const double *)x->gt, (const double *)x->abcc,
                                 (const unsigned long long *)x->absmax,
-                                (const int *)x->ec, (const double *)c->fY, M, Mp, x->Rp, nimg,
+                                (const int *)x->eb, (const double *)c->fY, M, Mp, x->Rp, nimg,
                                 x->nkbR, x->per, x->wa, x->ew, x->fpart));
     }
     DgArgs gb{};

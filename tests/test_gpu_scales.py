@@ -127,3 +127,29 @@ def test_mode_of_noise(gpu_lib, x, y, S):
     ctx.close()
     for a, b in zip((f, d2v), ref):
         assert np.abs(a - b).max() <= 1e-12 * np.abs(b).max()
+
+
+@pytest.mark.parametrize("S", [1, 48])
+@pytest.mark.parametrize("x,y", [(True, False), (False, True)])
+@pytest.mark.parametrize("scale", [2.0 ** -40, 2.0 ** 40])
+def test_mode_of_zeros(gpu_lib, x, y, scale, S):
+    """Modes without displacements, or without forces, in ensembles of small and of large
+    numbers (multiplied by a power of two).  Tolerance as above."""
+    M, N = (63, 2000) if S == 1 else (24, 400)
+    ens = make_ensemble(M, N, seed=14, n_syms=S, rho_sigma=0.1)
+    tables = ((ens["symmetries"], ens["degenerate_space"], ens["sym_block_id"]) if S > 1
+              else oracle.identity_symmetries(M))
+    X, Y = scale * ens["X"], scale * ens["Y"]
+    if x:
+        X[:, 3:6] = 0
+    if y:
+        Y[:, 3:6] = 0
+    R1, Y1 = random_R1(M, 3), random_sym(M, 4, scale=1e-5)
+    ref = oracle.perturb_averages(X, Y, ens["w"], ens["rho"], R1, Y1, ens["T"], 1, *tables, n_threads=8)
+    ctx = nat.Context(X, Y, ens["w"], ens["rho"], ens["T"], *tables)
+    f, d2v = np.zeros(M), np.zeros((M, M))
+    nat.check(nat.load().tdscha_perturb_averages(ctx.handle, nat.dp(R1), nat.dp(Y1), 1, nat.PREC_FP64,
+                                                 nat.dp(f), nat.dp(d2v), 0, None))
+    ctx.close()
+    for a, b in ((f, ref[0]), (d2v, ref[1]), (d2v[3:6], ref[1][3:6])):
+        assert np.abs(a - b).max() <= 1e-12 * np.abs(b).max()
