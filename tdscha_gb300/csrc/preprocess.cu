@@ -152,14 +152,14 @@ __global__ void __launch_bounds__(128) k_dg_colstat(const double *__restrict__ a
 }
 
 // ec[k]: the mean, and the exponents of mul[k] and of s where they multiply what was
-// counted; 0 of a column without an element
+// counted; kZeroExp of a column without an element, which leaves it out of B's scales
 __global__ void k_dg_colscale(const unsigned long long *__restrict__ stat, int K, double s,
                               const double *__restrict__ mul, int *__restrict__ ec) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= K) return;
     const long long n = (long long)stat[K + k], t = 2 * (long long)stat[k] + n;
     // rounded, ties upwards
-    ec[k] = n == 0 ? 0 : (int)((t - (t < 0 ? 2 * n - 1 : 0)) / (2 * n)) + exp_above(mul[k]) + exp_above(s) - 2;
+    ec[k] = n == 0 ? kZeroExp : (int)((t - (t < 0 ? 2 * n - 1 : 0)) / (2 * n)) + exp_above(mul[k]) + exp_above(s) - 2;
 }
 
 // Digits of the rows a' of k_prologue (real data), one warp per row, and the exponent

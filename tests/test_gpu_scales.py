@@ -42,11 +42,12 @@ def test_projection_of_two_sublattices(gpu_lib, ratio):
             assert np.abs(got[:, part] - ref[:, part]).max() <= 2e-15 * np.abs(ref[:, part]).max()
 
 
-@pytest.mark.parametrize("what", ["row", "element", "noise"])
+@pytest.mark.parametrize("what", ["row", "element", "noise", "zeros"])
 def test_projection_of_outliers_and_noise(gpu_lib, what):
     """One configuration, or one element of it, 1e6 times the others: each of the others
-    keeps its accuracy; and coordinates of rounding noise over 40 decades: all do.  2e-15 of
-    the largest entry of X, Y in ordinary configurations, as above."""
+    keeps its accuracy; coordinates of rounding noise over 40 decades, and of zeros beside
+    small numbers: all do.  2e-15 of the largest entry of X, Y in ordinary configurations,
+    as above."""
     from tdscha_gb300.preprocessing import project_modes
     rng = np.random.default_rng(9)
     N, n, M = 2000, 60, 57
@@ -57,6 +58,9 @@ def test_projection_of_outliers_and_noise(gpu_lib, what):
     for a in (u, f):
         if what == "noise":
             a[:, 6:9] *= 10.0 ** rng.uniform(-57, -17, (N, 3))
+        elif what == "zeros":
+            a *= 2.0 ** -40
+            a[:, 6:9] = 0
         else:
             a[37, slice(None) if what == "row" else 5] *= 1e6
             ordinary[37] = False
