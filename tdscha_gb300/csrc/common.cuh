@@ -161,6 +161,7 @@ struct tdscha_qctx {
     long R = 0;          // image rows N * S
     int L = 0;           // n_q * nb (length of one image row)
     double T = 0, sum_rho = 0;
+    int rho_top = 0;     // exponent of the largest weight (frexp)
     double2 *Xr = nullptr, *Yr = nullptr;      // R x L image rows
     double *fY = nullptr, *fpsi = nullptr;     // [q][nu] (0 for masked modes)
     double *rho = nullptr;

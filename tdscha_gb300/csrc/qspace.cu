@@ -642,12 +642,16 @@ extern "C" int tdscha_qctx_create(tdscha_qctx **out, int n_q, int nb, int N, con
             if (sym_col[t] < 0 || sym_col[t] >= L) { set_error("qctx_create: symmetry column %ld out of range", t); return TDSCHA_ERR_ARG; }
     }
     // X_q and Y_q are checked for non-finite entries on the device after the upload
-    double sum_rho = 0;
-    for (int i = 0; i < N; ++i) sum_rho += rho[i];
+    double sum_rho = 0, max_rho = 0;
+    for (int i = 0; i < N; ++i) {
+        sum_rho += rho[i];
+        max_rho = std::max(max_rho, std::fabs(rho[i]));
+    }
     if (!(sum_rho != 0) || !std::isfinite(sum_rho)) { set_error("qctx_create: bad weights"); return TDSCHA_ERR_ARG; }
     tdscha_qctx *c = new tdscha_qctx();
     c->n_q = n_q; c->nb = nb; c->N = N; c->S = n_syms > 0 ? n_syms : 1;
     c->R = (long)N * c->S; c->L = L; c->T = T; c->sum_rho = sum_rho;
+    std::frexp(max_rho, &c->rho_top);
     c->w_q.assign(w_q, w_q + (size_t)nb * n_q);
     c->valid.assign((size_t)nb * n_q, 1);
     if (valid)

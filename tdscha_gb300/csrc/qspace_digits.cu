@@ -16,6 +16,10 @@
 //           u2 and A2 with f2, are not needed and cost nothing: they fill a tile
 //           that would be empty.
 //
+// Scales as in perturb_digits.cu: a column's is the largest weighted exponent of its
+// elements; a configuration has one for y and one for u of each q-point, the exponent above its largest
+// element there.  The rows of [f2 | u2] are without it and those of A1 and A2 carry it.
+//
 // Measured (averages, one call): 4x4x4 grid, 12 bands, N=10000 2479 -> 530 us
 // (row dots 216, W 132, d2v 146 of them).
 #include <algorithm>
@@ -37,9 +41,9 @@ struct QDigitStore {
     void *slab = nullptr, *pslab = nullptr;
     double *x = nullptr, *g = nullptr, *u = nullptr, *y = nullptr, *qp = nullptr;
     __half *xa = nullptr, *xb = nullptr, *yb = nullptr;
-    unsigned long long *xmax = nullptr, *ymax = nullptr, *umax = nullptr, *absmax = nullptr;
     int *ec = nullptr, *er = nullptr, *ecb = nullptr, *et = nullptr, *cofs = nullptr,
-        *err = nullptr;
+        *wtop = nullptr, *err = nullptr;
+    int2 *erb = nullptr;          // a row's scales in y and in u, [q][Rp]
     double *rowc = nullptr;       // 8 doubles a row
     // per perturbation
     uint32_t abytes = 0;          // of a digit of a W block: rows up to a multiple of eight
@@ -85,49 +89,56 @@ __global__ void __launch_bounds__(256) k_qd_cols(const double *__restrict__ Xr,
     }
 }
 
-// Maxima of |x|, |y|, |u| of each column, and the exponents of the columns of xa
-// (ec) and of the tiles [y | u] (ecb)
-__global__ void __launch_bounds__(128) k_qd_colmax(const double *__restrict__ x,
-                                                   const double *__restrict__ y,
-                                                   const double *__restrict__ u, long nrt, int nr,
-                                                   int nbq, int G, unsigned long long *__restrict__ ymax,
-                                                   unsigned long long *__restrict__ umax,
-                                                   int *__restrict__ ec, int *__restrict__ ecb) {
-    __shared__ double sh[3][4];
+// Scales of the columns, their largest weighted exponents (dg_weighted_exp): of x in ec, of y
+// and u as the tiles [y | u] have them in ecb.  A column without an element (the imaginary
+// parts at Gamma, masked modes) has kZeroExp, which leaves it out of the rows' scales of A_q
+// and of W's bounds.
+__global__ void __launch_bounds__(128) k_qd_colscale(const double *__restrict__ x,
+                                                     const double *__restrict__ y,
+                                                     const double *__restrict__ u,
+                                                     const double *__restrict__ rho, int S, int rtop,
+                                                     long R, long nrt, int nr, int nbq, int G,
+                                                     int *__restrict__ ec, int *__restrict__ ecb) {
+    __shared__ int sh[4][3];
     const int c = blockIdx.x, q = blockIdx.y;
-    double a = 0, b = 0, d = 0;
+    int e[3] = {INT_MIN, INT_MIN, INT_MIN};
     for (long rt = 0; rt < nrt; ++rt) {
-        const long o = (((long)q * nrt + rt) * nr + c) * 128 + threadIdx.x;
-        a = fmax(a, fabs(x[o]));
-        b = fmax(b, fabs(y[o]));
-        d = fmax(d, fabs(u[o]));
+        const long o = (((long)q * nrt + rt) * nr + c) * 128 + threadIdx.x, r = rt * 128 + threadIdx.x;
+        if (r >= R) break;
+        const double w = rho[(unsigned)r / (unsigned)S];
+        e[0] = max(e[0], dg_weighted_exp(x[o], w, rtop));
+        e[1] = max(e[1], dg_weighted_exp(y[o], w, rtop));
+        e[2] = max(e[2], dg_weighted_exp(u[o], w, rtop));
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        a = fmax(a, __shfl_xor_sync(0xffffffffu, a, o));
-        b = fmax(b, __shfl_xor_sync(0xffffffffu, b, o));
-        d = fmax(d, __shfl_xor_sync(0xffffffffu, d, o));
-    }
-    if ((threadIdx.x & 31) == 0) {
-        sh[0][threadIdx.x >> 5] = a;
-        sh[1][threadIdx.x >> 5] = b;
-        sh[2][threadIdx.x >> 5] = d;
+    for (int k = 0; k < 3; ++k) {
+        e[k] = __reduce_max_sync(0xffffffffu, e[k]);
+        if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5][k] = e[k];
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int k = 1; k < 4; ++k) {
-            a = fmax(a, sh[0][k]);
-            b = fmax(b, sh[1][k]);
-            d = fmax(d, sh[2][k]);
-        }
-        ymax[q * nr + c] = (unsigned long long)__double_as_longlong(b);
-        umax[q * nr + c] = (unsigned long long)__double_as_longlong(d);
-        ec[q / G * 64 + q % G * nr + c] = a > 0 ? exp_above(a) : 0;
-        int *e = ecb + (long)q * nbq * kGN;
-        const int uc = nbq == 1 ? nr + c : kGN + c;
-        e[c] = b > 0 ? exp_above(b) : 0;
-        e[uc] = d > 0 ? exp_above(d) : 0;
+    if (threadIdx.x >= 3) return;
+    const int k = threadIdx.x;
+    int top = max(max(sh[0][k], sh[1][k]), max(sh[2][k], sh[3][k]));
+    if (top == INT_MIN) top = kZeroExp;
+    if (k == 0) ec[q / G * 64 + q % G * nr + c] = top;
+    else ecb[(long)q * nbq * kGN + (k == 1 ? c : nbq == 1 ? nr + c : kGN + c)] = top;
+}
+
+// erb[q][r]: exponents above the largest |y| 2^-ecb and |u| 2^-ecb of a row
+__global__ void __launch_bounds__(128) k_qd_rowscale(const double *__restrict__ y,
+                                                     const double *__restrict__ u,
+                                                     const int *__restrict__ ecb, int nr, int nbq,
+                                                     int2 *__restrict__ erb) {
+    const int q = blockIdx.y, *e = ecb + (long)q * nbq * kGN;
+    const long t = (long)q * gridDim.x + blockIdx.x;
+    int ey = INT_MIN, eu = INT_MIN;
+#pragma unroll 4
+    for (int c = 0; c < nr; ++c) {
+        const double a = y[(t * nr + c) * 128 + threadIdx.x], b = u[(t * nr + c) * 128 + threadIdx.x];
+        if (a != 0) ey = max(ey, exp_above(a) - e[c]);
+        if (b != 0) eu = max(eu, exp_above(b) - e[nbq == 1 ? nr + c : kGN + c]);
     }
+    erb[t * 128 + threadIdx.x] = make_int2(ey == INT_MIN ? kZeroExp : ey, eu == INT_MIN ? kZeroExp : eu);
 }
 
 // er[group][r]: exponent above the largest |x| 2^-ec of a row
@@ -139,9 +150,11 @@ __global__ void __launch_bounds__(128) k_qd_rowexp(const double *__restrict__ x,
     for (int m = 0; m < nc; ++m) {
         const int q = blockIdx.y * G + m / nr;
         const double v = x[(((long)q * gridDim.x + blockIdx.x) * nr + m % nr) * 128 + threadIdx.x];
-        if (v != 0) e = max(e, exp_above(v) - ec[blockIdx.y * 64 + m]);
+        // (what a column of kZeroExp has is in rows of weight 0)
+        if (v != 0 && ec[blockIdx.y * 64 + m] != kZeroExp)
+            e = max(e, exp_above(v) - ec[blockIdx.y * 64 + m]);
     }
-    er[(blockIdx.x + (long)blockIdx.y * gridDim.x) * 128 + threadIdx.x] = e == INT_MIN ? 0 : e;
+    er[(blockIdx.x + (long)blockIdx.y * gridDim.x) * 128 + threadIdx.x] = e == INT_MIN ? kZeroExp : e;
 }
 
 // xa: [group][row tile][digit 7][128 x 64], thread = (row, eight columns)
@@ -157,9 +170,11 @@ __global__ void __launch_bounds__(256) k_qd_xa(const double *__restrict__ x,
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             const int m = c * 8 + k, q = blockIdx.y * G + m / nr;
-            v[k] = m >= nc ? 0
-                           : fixed_point(x[(((long)q * gridDim.x + blockIdx.x) * nr + m % nr) * 128 + row],
-                                         55 - ec[blockIdx.y * 64 + m] - er[t * 128 + row]);
+            const int e = m < nc ? ec[blockIdx.y * 64 + m] : kZeroExp;
+            v[k] = e == kZeroExp
+                       ? 0
+                       : fixed_point(x[(((long)q * gridDim.x + blockIdx.x) * nr + m % nr) * 128 + row],
+                                     55 - e - er[t * 128 + row]);
         }
         uint4 w[kRes];
         digits8<kRes>(v, w);
@@ -173,7 +188,8 @@ __global__ void __launch_bounds__(256) k_qd_xa(const double *__restrict__ x,
 // eight rows), and the digits' norms
 __global__ void __launch_bounds__(256) k_qd_xb(const double *__restrict__ y,
                                                const double *__restrict__ u,
-                                               const int *__restrict__ ecb, int nr, int nbq,
+                                               const int *__restrict__ ecb,
+                                               const int2 *__restrict__ erb, int nr, int nbq,
                                                long nrt, long nkb, __half *__restrict__ xb,
                                                float *__restrict__ nrm) {
     const long kb = blockIdx.x, t = blockIdx.y;                   // t = q nbq + tile
@@ -189,11 +205,14 @@ __global__ void __launch_bounds__(256) k_qd_xb(const double *__restrict__ y,
             src = j == 0 ? y : u;
         }
         const int cc = nbq == 1 && col >= nr ? col - nr : col;
+        const bool of_y = src == y;
         const int e = ecb[t * kGN + col];
+        const int2 *es = erb + q * nrt * 128 + r0;
         if (src) src += (((long)q * nrt + (r0 >> 7)) * nr + cc) * 128 + (r0 & 127);
         long long v[8];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) v[k] = src ? fixed_point(src[k], 55 - e) : 0;
+        for (int k = 0; k < 8; ++k)
+            v[k] = src ? fixed_point(src[k], 55 - e - (of_y ? es[k].x : es[k].y)) : 0;
         uint4 w[kRes];
         digits8<kRes>(v, w);
 #pragma unroll
@@ -222,7 +241,7 @@ __global__ void __launch_bounds__(32) k_qd_alpha(const QAlpha src, const int *__
                                                  const int *__restrict__ ec, int nb, int G, int nrt,
                                                  __half *__restrict__ yb, int *__restrict__ et,
                                                  int *__restrict__ cofs,
-                                                 unsigned long long *__restrict__ absmax) {
+                                                 int *__restrict__ wtop) {
     __shared__ long long s[64];
     const int nr = 2 * nb, lane = threadIdx.x, grp = blockIdx.y / G, k0 = blockIdx.y % G * nr;
     const int q = qpartner[blockIdx.y], row = k0 + blockIdx.x, n = blockIdx.x >> 1;
@@ -262,26 +281,32 @@ __global__ void __launch_bounds__(32) k_qd_alpha(const QAlpha src, const int *__
         for (int d = 0; d < kCall; ++d)
             *reinterpret_cast<uint4 *>(out + d * kGB + sw_place(row, lane)) = w[d];
     }
+    // (there are no more pairs than q-points)
+    if (blockIdx.x == 0 && (int)blockIdx.y < src.n_pairs && lane < 3) wtop[4 * blockIdx.y + lane] = INT_MIN;
     if (lane == 0) {
         et[grp * 64 + row] = e;
         cofs[grp * 64 + row] =
             4 * (q * nrt * nr + (int)blockIdx.x) + (qpartner[q] == q ? 0 : 1 + qrole[q]);
-        if (blockIdx.x == 0 && blockIdx.y == 0) absmax[0] = absmax[1] = 0ULL;
     }
 }
 
 // Row weights (k_q_rows of qspace.cu): 64 rows a block, four threads a row, each a
 // quarter of the sums (with one thread a row its loads took 13 us at 2000 rows).
-// Rows past the end get zeros.
+// Rows past the end get zeros.  wtop, of each pair (q1, q2): the largest exponents of
+// w_cross with its row's scales in u of q1 and y of q2, of w_cross with those in y of q1
+// and u of q2, and of w_diag with those in u of both; kBadExp of one that is not finite.
 __global__ void __launch_bounds__(256) k_qd_rows(const double *__restrict__ qp, int ngrp,
                                                  const double *__restrict__ u,
                                                  const double *__restrict__ y,
                                                  const double2 *__restrict__ R1,
                                                  const double *__restrict__ rho, int S, long R,
                                                  long nrt, int nb, int iq_pert, int apply_d4,
+                                                 const int2 *__restrict__ erb,
+                                                 const int *__restrict__ pair_q, int n_pairs,
                                                  double2 *__restrict__ rowc,
-                                                 unsigned long long *__restrict__ absmax) {
+                                                 int *__restrict__ wtop) {
     __shared__ double sum[8][4][64];
+    __shared__ int we[2][64];      // exponents of w_cross, w_diag
     const int part = threadIdx.x >> 6, i = threadIdx.x & 63;
     const long r = blockIdx.x * 64L + i;
     pdl_enter();
@@ -307,40 +332,62 @@ __global__ void __launch_bounds__(256) k_qd_rows(const double *__restrict__ qp, 
 #pragma unroll
     for (int k = 0; k < 8; ++k) sum[k][part][i] = s[k];
     __syncthreads();
-    if (threadIdx.x >= 64) return;
-    double2 w[4] = {};
-    if (r < R) {
+    if (threadIdx.x < 64) {
+        double2 w[4] = {};
+        if (r < R) {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) s[k] = (sum[k][0][i] + sum[k][1][i]) + (sum[k][2][i] + sum[k][3][i]);
-        const double rw = rho[(unsigned)r / (unsigned)S], d4 = apply_d4 ? 1.0 : 0.0;
-        const double t3 = rw / 3.0, t8 = -d4 * rw / 8.0, t4 = -d4 * rw / 4.0;
-        w[0] = make_double2(s[0] * (-0.5 * t3), s[1] * (-0.5 * t3));
-        w[1] = make_double2(s[2] * -t3, s[3] * -t3);
-        w[2] = make_double2(fma(s[4], t3, s[0] * t8), fma(s[5], t3, s[1] * t8));
-        w[3] = make_double2(fma(s[6], t3, s[2] * t4), fma(s[7], t3, s[3] * t4));
+            for (int k = 0; k < 8; ++k)
+                s[k] = (sum[k][0][i] + sum[k][1][i]) + (sum[k][2][i] + sum[k][3][i]);
+            const double rw = rho[(unsigned)r / (unsigned)S], d4 = apply_d4 ? 1.0 : 0.0;
+            const double t3 = rw / 3.0, t8 = -d4 * rw / 8.0, t4 = -d4 * rw / 4.0;
+            w[0] = make_double2(s[0] * (-0.5 * t3), s[1] * (-0.5 * t3));
+            w[1] = make_double2(s[2] * -t3, s[3] * -t3);
+            w[2] = make_double2(fma(s[4], t3, s[0] * t8), fma(s[5], t3, s[1] * t8));
+            w[3] = make_double2(fma(s[6], t3, s[2] * t4), fma(s[7], t3, s[3] * t4));
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) rowc[4 * r + k] = w[k];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const unsigned long long a =
+                max((unsigned long long)__double_as_longlong(w[2 + k].x) & 0x7fffffffffffffffULL,
+                    (unsigned long long)__double_as_longlong(w[2 + k].y) & 0x7fffffffffffffffULL);
+            we[k][i] = a >= 0x7ff0000000000000ULL ? kBadExp
+                       : a ? exp_above(__longlong_as_double((long long)a)) : INT_MIN;
+        }
     }
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    for (int p = threadIdx.x >> 5; p < n_pairs; p += 8) {
+        const int2 *s1 = erb + pair_q[2 * p] * nrt * 128 + blockIdx.x * 64L,
+                   *s2 = erb + pair_q[2 * p + 1] * nrt * 128 + blockIdx.x * 64L;
+        int top[3] = {INT_MIN, INT_MIN, INT_MIN};
 #pragma unroll
-    for (int k = 0; k < 4; ++k) rowc[4 * r + k] = w[k];
+        for (int h = 0; h < 64; h += 32) {
+            const int c = we[0][h + lane], d = we[1][h + lane];
+            const int2 a = s1[h + lane], b = s2[h + lane];
+            auto with = [](int e, int x) { return e == INT_MIN || e == kBadExp ? e : e + x; };
+            top[0] = max(top[0], with(c, a.y + b.x));
+            top[1] = max(top[1], with(c, a.x + b.y));
+            top[2] = max(top[2], with(d, a.y + b.y));
+        }
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-        unsigned long long a =
-            max((unsigned long long)__double_as_longlong(w[2 + k].x) & 0x7fffffffffffffffULL,
-                (unsigned long long)__double_as_longlong(w[2 + k].y) & 0x7fffffffffffffffULL);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) a = max(a, __shfl_xor_sync(0xffffffffu, a, o));
-        if ((threadIdx.x & 31) == 0) atomicMax(absmax + k, a);
+        for (int k = 0; k < 3; ++k) {
+            const int e = __reduce_max_sync(0xffffffffu, top[k]);
+            if (lane == k) atomicMax(wtop + 4 * p + k, e);
+        }
     }
 }
 
 // Digits of the rows [A1 | A2] of pair blockIdx.y over a group of K blocks: thread =
 // (band, eight rows), which makes four rows of digits; with few bands several K blocks
-// side by side.  The scales are bounds from the maxima of the weights and of the
-// columns.  blockIdx.y == n_pairs: the partial f of the group's rows.
+// side by side.  The scales are bounds from those of the weights and of the columns; a
+// row's own scale goes into the shift that cuts the digits.  blockIdx.y == n_pairs: the partial f of the group's rows.
 __global__ void __launch_bounds__(128) k_qd_wbuild(
     const double *__restrict__ u, const double *__restrict__ y, const double2 *__restrict__ rowc,
-    const unsigned long long *__restrict__ absmax, const unsigned long long *__restrict__ umax,
-    const unsigned long long *__restrict__ ymax, const int *__restrict__ pair_q, int n_pairs, int nb,
-    int iq_pert, long nrt, long nkb, int per, uint32_t abytes, __half *__restrict__ wa,
+    const int *__restrict__ wtop, const int *__restrict__ ecb, const int2 *__restrict__ erb,
+    const int *__restrict__ pair_q, int n_pairs, int nb, int nbq, int iq_pert, long nrt, long nkb,
+    int per, uint32_t abytes, __half *__restrict__ wa,
     int *__restrict__ ew, double2 *__restrict__ fpart) {
     __shared__ double2 fs[16];
     const int c = threadIdx.x & 7, m = threadIdx.x >> 3, nr = 2 * nb, p = blockIdx.y;
@@ -385,21 +432,20 @@ __global__ void __launch_bounds__(128) k_qd_wbuild(
         }
         return;
     }
-    const double ac = __longlong_as_double((long long)absmax[0]),
-                 ad = __longlong_as_double((long long)absmax[1]);
+    const int *wt = wtop + 4 * p;
+    const int2 *es2 = erb + pair_q[2 * p + 1] * nrt * 128;
     uint8_t *out = reinterpret_cast<uint8_t *>(wa) + p * nkb * kCall * (long)abytes;
     for (int n0 = 0; n0 < nb; n0 += 16) {
         const int n = n0 + (nb < 16 ? m % nb : m);
         if (n >= nb || m >= nb * wide) break;
-        auto top = [&](const unsigned long long *mx) {
-            return fmax(__longlong_as_double((long long)mx[q1 * nr + 2 * n]),
-                        __longlong_as_double((long long)mx[q1 * nr + 2 * n + 1]));
-        };
-        const double um = top(umax), ym = top(ymax);
-        const double b1 = 2 * ac * um * (1.0 + 0x1p-40), b2 = 2 * (ac * ym + ad * um) * (1.0 + 0x1p-40);
-        const bool bad1 = !isfinite(b1), bad2 = !isfinite(b2);
-        const int e1 = bad1 ? kBadExp : b1 > 0 ? exp_above(b1) : 0;
-        const int e2 = bad2 ? kBadExp : b2 > 0 ? exp_above(b2) : 0;
+        const int *ey = ecb + (long)q1 * nbq * kGN + 2 * n, *eu = ey + (nbq == 1 ? nr : kGN);
+        const int ym = max(ey[0], ey[1]), um = max(eu[0], eu[1]);
+        // real and imaginary part: two products each, and two of them in A2
+        auto bound = [](int a, int e) { return a == INT_MIN ? INT_MIN : a + e; };
+        const int b1 = bound(wt[0], um), b2 = max(bound(wt[1], ym), bound(wt[2], um));
+        const bool bad1 = wt[0] == kBadExp, bad2 = wt[1] == kBadExp || wt[2] == kBadExp;
+        const int e1 = bad1 ? kBadExp : b1 == INT_MIN ? 0 : b1 + 1;
+        const int e2 = bad2 ? kBadExp : b2 == INT_MIN ? 0 : b2 + 2;
         if (blockIdx.x == 0 && c == 0) {
             ew[p * kGM + 2 * n] = ew[p * kGM + 2 * n + 1] = e1;
             ew[p * kGM + nr + 2 * n] = ew[p * kGM + nr + 2 * n + 1] = e2;
@@ -419,13 +465,14 @@ __global__ void __launch_bounds__(128) k_qd_wbuild(
                     const double pu = h ? vur.y : vur.x, pv = h ? vui.y : vui.x;
                     const double py = h ? vyr.y : vyr.x, pz = h ? vyi.y : vyi.x;
                     const double2 wc = rowc[4 * (r0 + k + h) + 2], wd = rowc[4 * (r0 + k + h) + 3];
+                    const int2 es = es2[r0 + k + h];
                     const double xr = fma(wc.y, pv, -wc.x * pu), xi = fma(-wc.x, pv, -wc.y * pu);
                     const double zr = fma(wd.y, pv, fma(-wd.x, pu, fma(wc.y, pz, -wc.x * py)));
                     const double zi = fma(-wd.x, pv, fma(-wd.y, pu, fma(-wc.x, pz, -wc.y * py)));
-                    a1r[k + h] = bad1 ? 0 : fixed_point(xr, 62 - e1);
-                    a1i[k + h] = bad1 ? 0 : fixed_point(xi, 62 - e1);
-                    a2r[k + h] = bad2 ? 0 : fixed_point(zr, 62 - e2);
-                    a2i[k + h] = bad2 ? 0 : fixed_point(zi, 62 - e2);
+                    a1r[k + h] = bad1 ? 0 : fixed_point(xr, 62 - e1 + es.x);
+                    a1i[k + h] = bad1 ? 0 : fixed_point(xi, 62 - e1 + es.x);
+                    a2r[k + h] = bad2 ? 0 : fixed_point(zr, 62 - e2 + es.y);
+                    a2i[k + h] = bad2 ? 0 : fixed_point(zi, 62 - e2 + es.y);
                 }
             }
             uint8_t *blk = out + kb * kCall * (long)abytes;
@@ -554,9 +601,8 @@ static int qdigits_prepare(tdscha_qctx *c) {
         {(void **)&x->rowc, sizeof(double) * 8 * x->Rp},
         {(void **)&x->er, sizeof(int) * x->ngrp * x->Rp},
         {(void **)&nrm, sizeof(float) * kRes * (size_t)n_q * x->nbq * kGN * x->nkb},
-        {(void **)&x->ymax, sizeof(unsigned long long) * n_q * nr},
-        {(void **)&x->umax, sizeof(unsigned long long) * n_q * nr},
-        {(void **)&x->absmax, sizeof(unsigned long long) * 2},
+        {(void **)&x->erb, sizeof(int2) * rows},
+        {(void **)&x->wtop, sizeof(int) * 4 * n_q},
         // zero from the start: exponents of padding columns, rows of padding bands
         {(void **)&x->ec, sizeof(int) * x->ngrp * 64},
         {(void **)&x->ecb, sizeof(int) * (size_t)n_q * x->nbq * kGN},
@@ -580,16 +626,18 @@ static int qdigits_prepare(tdscha_qctx *c) {
     k_qd_cols<<<gt, 256>>>((const double *)c->Xr, (const double *)c->Yr, c->fY, c->fpsi, c->L, nb,
                            c->R, x->x, x->g, x->u, x->y);
     TDS_CHECK_LAUNCH();
-    k_qd_colmax<<<dim3(nr, n_q), 128>>>(x->x, x->y, x->u, x->nrt, nr, x->nbq, x->G, x->ymax,
-                                        x->umax, x->ec, x->ecb);
+    k_qd_colscale<<<dim3(nr, n_q), 128>>>(x->x, x->y, x->u, c->rho, c->S, c->rho_top, c->R, x->nrt, nr,
+                                          x->nbq, x->G, x->ec, x->ecb);
+    TDS_CHECK_LAUNCH();
+    k_qd_rowscale<<<gt, 128>>>(x->y, x->u, x->ecb, nr, x->nbq, x->erb);
     TDS_CHECK_LAUNCH();
     const dim3 gg((unsigned)x->nrt, x->ngrp);
     k_qd_rowexp<<<gg, 128>>>(x->x, x->ec, nr, x->G, n_q, x->er);
     TDS_CHECK_LAUNCH();
     k_qd_xa<<<gg, 256>>>(x->x, x->ec, x->er, nr, x->G, n_q, x->xa);
     TDS_CHECK_LAUNCH();
-    k_qd_xb<<<dim3((unsigned)x->nkb, n_q * x->nbq), 256>>>(x->y, x->u, x->ecb, nr, x->nbq, x->nrt,
-                                                           x->nkb, x->xb, nrm);
+    k_qd_xb<<<dim3((unsigned)x->nkb, n_q * x->nbq), 256>>>(x->y, x->u, x->ecb, x->erb, nr, x->nbq,
+                                                           x->nrt, x->nkb, x->xb, nrm);
     TDS_CHECK_LAUNCH();
     k_dg_windows<<<dim3(n_q * x->nbq, kFlushes), kGN>>>(nrm, (int)x->nkb, fl);
     TDS_CHECK_LAUNCH();
@@ -665,7 +713,7 @@ int qdigits_perturb(tdscha_qctx *c, int apply_d4, const double *psi, cudaStream_
     double2 *rowc = reinterpret_cast<double2 *>(x->rowc), *fpart = reinterpret_cast<double2 *>(x->fpart);
     TDS_CUDA(launch_pdl(k_qd_alpha, dim3(x->nr, n_q), 32, 0, st, src, (const int *)c->qpair,
                         (const int *)c->qrole, (const int *)c->qpartner, (const int *)x->ec, nb, x->G,
-                        (int)x->nrt, x->yb, x->et, x->cofs, x->absmax));
+                        (int)x->nrt, x->yb, x->et, x->cofs, x->wtop));
     DgArgs a{};
     a.a = x->xa;
     a.b = x->yb;
@@ -691,12 +739,12 @@ int qdigits_perturb(tdscha_qctx *c, int apply_d4, const double *psi, cudaStream_
     TDS_CUDA((dg_launch<DG_QDOTS, true>(a, x->nsm, st)));
     TDS_CUDA(launch_pdl(k_qd_rows, (unsigned)x->nkb, 256, 0, st, (const double *)x->qp, x->ngrp,
                         (const double *)x->u, (const double *)x->y, R1, (const double *)c->rho, c->S,
-                        c->R, x->nrt, nb, c->iq_pert, apply_d4, rowc, x->absmax));
+                        c->R, x->nrt, nb, c->iq_pert, apply_d4, (const int2 *)x->erb,
+                        (const int *)c->pair_q, x->n_pairs, rowc, x->wtop));
     TDS_CUDA(launch_pdl(k_qd_wbuild, dim3(x->nfc, x->n_pairs + 1), 128, 0, st, (const double *)x->u,
                         (const double *)x->y, (const double2 *)rowc,
-                        (const unsigned long long *)x->absmax, (const unsigned long long *)x->umax,
-                        (const unsigned long long *)x->ymax, (const int *)c->pair_q, x->n_pairs, nb,
-                        c->iq_pert, x->nrt, x->nkb, x->per, x->abytes, x->wa, x->ew, fpart));
+                        (const int *)x->wtop, (const int *)x->ecb, (const int2 *)x->erb,
+                        (const int *)c->pair_q, x->n_pairs, nb, x->nbq, c->iq_pert, x->nrt, x->nkb, x->per, x->abytes, x->wa, x->ew, fpart));
     DgArgs b{};
     b.a = x->wa;
     b.b = x->xb;

@@ -157,3 +157,62 @@ def test_mode_of_zeros(gpu_lib, x, y, scale, S):
     ctx.close()
     for a, b in ((f, ref[0]), (d2v, ref[1]), (d2v[3:6], ref[1][3:6])):
         assert np.abs(a - b).max() <= 1e-12 * np.abs(b).max()
+
+
+def _bloch_averages(e, rho, iq):
+    """f and the blocks of d2v, from the GPU and from the oracle."""
+    import oracle.qspace as oq
+    from tdscha_gb300.QSpaceLanczos import QSpaceLanczos
+    nb = e["X_q"].shape[2]
+    lz = QSpaceLanczos.from_arrays(e["X_q"], e["Y_q"], e["w_q"], rho, e["T"], q_points=e["q"])
+    valid = np.ones((nb, 3), dtype=bool)
+    valid[0, 0] = False
+    lz.valid_modes_q = valid
+    lz.prepare_symmetrization(symmetries=None)
+    lz.build_q_pair_map(iq)
+    o = oq.OracleQSpaceLanczos(e["X_q"], e["Y_q"], e["w_q"], rho, e["T"], lz.q_pair_map, iq, valid=valid)
+    rng = np.random.default_rng(3)
+    R1 = rng.standard_normal(nb) + 1j * rng.standard_normal(nb)
+    alpha = [rng.standard_normal((nb, nb)) + 1j * rng.standard_normal((nb, nb)) for _ in o.pairs]
+    got = lz.get_perturb_averages_q(R1, alpha, True)
+    ref = oq.perturb_averages_qspace(e["X_q"], e["Y_q"], e["w_q"], rho, R1, alpha, e["T"], True, iq,
+                                     o.pairs, o.symmetries, o.valid)
+    return [(got[0], ref[0]), *zip(got[1], ref[1])]
+
+
+@pytest.mark.parametrize("what", ["X", "Y", "XY", "X element", "Y element", "XY element"])
+@pytest.mark.parametrize("weight,size", [(0.0, 1e3), (0.0, 1e6), (0.0, 1e8), (1e-40, 1e6),
+                                         (1e-24, 1e6), (1e-12, 1e3), (1.0, 1e3), (1.0, 1e6)])
+@pytest.mark.parametrize("nb", [5, 20])
+def test_bloch_space_outlier(gpu_lib, what, weight, size, nb):
+    """The same in Bloch space, against the oracle: N <= 300 float64 terms, 1e-13 of the
+    largest entry of a block (tests/test_gpu_qspace_digits.py); an element of one q-point
+    takes nothing from the blocks of the others."""
+    from tdscha_gb300.synthetic import make_qspace_ensemble
+    e = make_qspace_ensemble((3, 1, 1), nb, 300, seed=nb, T=250.0, dispersion=0.3, rho_sigma=0.2)
+    at = (1, 37, 3) if "element" in what else (slice(None), 37)
+    for k in "XY":
+        if k in what.split()[0]:
+            e[k + "_q"] = e[k + "_q"].copy()
+            e[k + "_q"][at] *= size
+    rho = e["rho"].copy()
+    rho[37] *= weight
+    for a, b in _bloch_averages(e, rho, 1):
+        assert np.abs(a - b).max() <= 1e-12 * np.abs(b).max()
+
+
+@pytest.mark.parametrize("what", ["real", "noise"])
+@pytest.mark.parametrize("scale", [2.0 ** -40, 1.0, 2.0 ** 40])
+@pytest.mark.parametrize("iq", [0, 1])
+def test_bloch_space_at_gamma(gpu_lib, what, scale, iq):
+    """Imaginary parts at Gamma that are zero, or rounding noise over 40 decades, in
+    ensembles of small and of large numbers.  Tolerance as above."""
+    from tdscha_gb300.synthetic import make_qspace_ensemble
+    e = make_qspace_ensemble((3, 1, 1), 5, 300, seed=3, T=250.0, dispersion=0.3, rho_sigma=0.2)
+    rng = np.random.default_rng(4)
+    for k in ("X_q", "Y_q"):
+        e[k] = scale * e[k]
+        re = e[k][0].real
+        e[k][0] = re + (1j * re * 10.0 ** rng.uniform(-57, -17, re.shape) if what == "noise" else 0)
+    for a, b in _bloch_averages(e, e["rho"], iq):
+        assert np.abs(a - b).max() <= 1e-12 * np.abs(b).max()
