@@ -276,10 +276,10 @@ int psi_finalize64(tdscha_ctx *c, const double *gpart, int nsplit, long sstride,
                    long lda, const double *fpart, int nfchunk, cudaStream_t st);
 // the two halves of psi_finalize64: hs and fs of images j0 .. j0 + nj - 1 (the
 // partials of image j0 first; with fY != nullptr they are G_js without its factors
-// fY[a] fY[b]), then f and d2v from all of them
+// fY[a] fY[b]), then f and d2v from all of them (NaN where *failed is set, if given)
 int psi_hsum64(tdscha_ctx *c, const double *gpart, int nsplit, long sstride, long jstride, long lda,
                const double *fpart, int nfchunk, const double *fY, int j0, int nj, cudaStream_t st);
-int psi_reduce64(tdscha_ctx *c, cudaStream_t st);
+int psi_reduce64(tdscha_ctx *c, const int *failed, cudaStream_t st);
 int psi_finalize32(tdscha_ctx *c, const float *gpart, int nsplit, long sstride, long jstride,
                    long lda, const float *fpart, int nfchunk, double *f_out, double *d2v_out,
                    cudaStream_t st);

@@ -272,7 +272,8 @@ struct DgArgs {
     const int *bmap;
     long nitems;
     int Mp;
-    int *err;
+    int *err;              // failure code, for the host
+    int *failed;           // set with it, for the kernels that end the call (or null)
     long long budget;
     // stage A
     const double *dt, *gt, *vs, *vt;
@@ -827,7 +828,10 @@ __global__ void __launch_bounds__(DgShape<kMode>::threads, 1) k_dg_gemm(const Dg
         }
         if (fail_code) *abort = 1;
     }
-    if (fail_code && lane == 0) *(volatile int *)args.err = 10 + fail_code;
+    if (fail_code && lane == 0) {
+        *(volatile int *)args.err = 10 + fail_code;
+        if (args.failed) *(volatile int *)args.failed = 1;
+    }
     tc_fence_before();
     __syncthreads();
     if (warp == kEpi + 1) {

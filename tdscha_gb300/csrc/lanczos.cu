@@ -2233,9 +2233,10 @@ extern "C" int tdscha_lanczos_run_batch(tdscha_run *runs, int n_runs) {
             double *sh = r.kind == 0 ? ((tdscha_ctx *)r.ctx)->stat_host : ((tdscha_qctx *)r.ctx)->stat_host;
             int e = read_back_steps(hd, sd, sh, r.capacity, next[i], k, streams[i], r.hist,
                                     r.start_step, &r.steps_done, &r.converged, &stop);
-            if (e == TDSCHA_OK)
-                e = r.kind == 0 ? mixed_check_error((tdscha_ctx *)r.ctx)
-                                : qdigits_check_error((tdscha_qctx *)r.ctx);
+            // a wait that gave up outranks what its NaN results gave
+            const int w = r.kind == 0 ? mixed_check_error((tdscha_ctx *)r.ctx)
+                                      : qdigits_check_error((tdscha_qctx *)r.ctx);
+            if (w != TDSCHA_OK) e = w;
             if (e != TDSCHA_OK) { fail(i, e); continue; }
             next[i] = k + 1;
             if (stop || done[i] >= r.n_iter) active[i] = false;

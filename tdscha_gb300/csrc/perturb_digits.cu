@@ -275,12 +275,14 @@ __device__ __forceinline__ double dg_y1(const DgSource &c, const double *__restr
 // the exponent above the row's maximum, and the two vectors of the row scalars.
 // Also clears the image's maxima of alpha, beta and the force weights.  With many
 // images rows M and M + 1 are those two vectors, digits of rows `image` of the tiles vb.
+// failed: the call's failure flag, cleared by its first pass (null in the others).
 __global__ void __launch_bounds__(128) k_dg_y1(const DgSources src, const double *__restrict__ fY,
                                                const int *__restrict__ ecol, int M, int Mp,
                                                __half *__restrict__ yb, int *__restrict__ et,
                                                double *__restrict__ vs, double *__restrict__ vt,
                                                __half *__restrict__ vb, int *__restrict__ etv,
-                                               unsigned long long *__restrict__ absmax) {
+                                               unsigned long long *__restrict__ absmax,
+                                               int *__restrict__ failed) {
     pdl_enter();
     extern __shared__ double yrow[];     // M
     __shared__ int sh[4];
@@ -333,6 +335,7 @@ __global__ void __launch_bounds__(128) k_dg_y1(const DgSources src, const double
         vt[img * Mp + n] = vec(n, false);
         if (n == 0)
             for (int k = 0; k < 4; ++k) absmax[4 * img + k] = 0ULL;
+        if (n == 0 && img == 0 && failed) *failed = 0;
     }
 }
 
@@ -596,13 +599,15 @@ __device__ __forceinline__ double dg_split_sum(const double *__restrict__ p, int
 // 32 x 32 tiles, each element summed over the splits once.  kRows = 2 and four groups
 // of threads, each with every fourth split, where slabs of 8 rows would leave SMs idle:
 // an addition takes a warp 64 cycles and the loads wait for one another (32 splits of
-// M=48: 11.4 us with the slabs of 8, 6.9 so).
+// M=48: 11.4 us with the slabs of 8, 6.9 so).  After a wait that gave up the results are
+// NaN: calls on device pointers report it that way (and in tdscha_ctx_sync).
 template <int kRows, int kGroups>
 __global__ void __launch_bounds__(32 * kRows * kGroups) k_dg_final(
     const double *__restrict__ gpart, int nsplit, long stride, int M, int Mp,
     const double *__restrict__ fpart, int nfc, const double *__restrict__ fY, double inv,
-    double *__restrict__ f, double *__restrict__ d2v) {
+    const int *__restrict__ failed, double *__restrict__ f, double *__restrict__ d2v) {
     pdl_enter();
+    if (*failed) inv = __longlong_as_double(0x7ff8000000000000LL);
     gpart += blockIdx.y * (long)Mp * Mp;
     fpart += blockIdx.y * (long)nfc * M;
     f += blockIdx.y * (long)M;
@@ -677,6 +682,7 @@ struct DigitStore {
     __half *xa = nullptr, *xb = nullptr, *yb = nullptr, *wa = nullptr;
     int *ec = nullptr, *eb = nullptr, *er = nullptr, *et = nullptr, *ew = nullptr;
     int *err = nullptr;          // bounded-wait failure code (pinned host memory)
+    int *failed = nullptr;       // whether one gave up in this call
     long long budget = kDefaultBudget;
 };
 
@@ -766,6 +772,7 @@ int digits_prepare(tdscha_ctx *c) {
         {(void **)&x->eb, 2 * i4 * Mp, false},
         // zero from the start: maxima, and the rows of padding modes
         {(void **)&x->absmax, u8 * 4 * cap, true},
+        {(void **)&x->failed, i4, true},
         {(void **)&x->etv, one * i4 * 2 * kGN, true},
         {(void **)&x->ewf, one * i4 * kGM, true},
         {(void **)&x->vb, one * 2 * (size_t)x->nkbM * kCall * kGB, true},
@@ -867,9 +874,9 @@ int digits_check_error(tdscha_ctx *c) {
 }
 
 // Stages A and B for nimg perturbations: split-K partials of every image's H in
-// x->gpart, force partials in x->fpart.
+// x->gpart, force partials in x->fpart.  first: the call's first pass.
 static int digits_contract(tdscha_ctx *c, int nimg, const DgSources &src, int apply_d4,
-                           int *nsplit, cudaStream_t st) {
+                           bool first, int *nsplit, cudaStream_t st) {
     DigitStore *x = c->dg;
     const int M = c->M, Mp = x->Mp;
     const long R = c->Nrows;
@@ -877,7 +884,7 @@ static int digits_contract(tdscha_ctx *c, int nimg, const DgSources &src, int ap
         ProfScope ps(c, 5, st);
         TDS_CUDA(launch_pdl(k_dg_y1, dim3(x->many ? M + 2 : M, nimg), 128, sizeof(double) * M, st,
                             src, (const double *)c->fY, (const int *)x->eb, M, Mp, x->yb, x->et,
-                            x->vs, x->vt, x->vb, x->etv, x->absmax));
+                            x->vs, x->vt, x->vb, x->etv, x->absmax, first ? x->failed : nullptr));
         if (x->many) {
             // s and t of all images: [x; g] times their vectors
             DgArgs g{};
@@ -890,6 +897,7 @@ static int digits_contract(tdscha_ctx *c, int nimg, const DgSources &src, int ap
             g.nitems = g.nat;
             g.bmap = x->bmap;
             g.err = x->err;
+            g.failed = x->failed;
             g.budget = x->budget;
             g.et = x->etv;
             g.er = x->er;
@@ -923,6 +931,7 @@ static int digits_contract(tdscha_ctx *c, int nimg, const DgSources &src, int ap
     ga.nitems = (long)ga.nat * ga.nbt;
     ga.Mp = Mp;
     ga.err = x->err;
+    ga.failed = x->failed;
     ga.budget = x->budget;
     ga.dt = x->dt;
     ga.gt = x->gt;
@@ -980,6 +989,7 @@ static int digits_contract(tdscha_ctx *c, int nimg, const DgSources &src, int ap
     gb.nitems = (long)nat * x->nct * *nsplit;
     gb.Mp = Mp;
     gb.err = x->err;
+    gb.failed = x->failed;
     gb.budget = x->budget;
     gb.ec = x->ec;
     gb.ew = x->ew;
@@ -1024,7 +1034,7 @@ static int digits_averages(tdscha_ctx *c, int nimg, const DgSources &src, int ap
     DigitStore *x = c->dg;
     const int M = c->M, Mp = x->Mp;
     int ns = 0;
-    TDS_TRY(digits_contract(c, nimg, src, apply_d4, &ns, st));
+    TDS_TRY(digits_contract(c, nimg, src, apply_d4, true, &ns, st));
     ProfScope ps(c, 4, st);
     const int nt = ceil_div(M, 32), nat = ceil_div((long)nimg * Mp, kGM);
     const int pairs = nt * (nt + 1) / 2;
@@ -1032,7 +1042,8 @@ static int digits_averages(tdscha_ctx *c, int nimg, const DgSources &src, int ap
     TDS_CUDA(launch_pdl(small ? k_dg_final<2, 4> : k_dg_final<8, 1>,
                         dim3((small ? 16 : 4) * pairs, nimg), 256, 0, st, (const double *)x->gpart, ns,
                         (long)nat * kGM * Mp, M, Mp, (const double *)x->fpart, x->nfc,
-                        (const double *)c->fY, 1.0 / (c->sum_rho * c->S), f, d2v));
+                        (const double *)c->fY, 1.0 / (c->sum_rho * c->S), (const int *)x->failed, f,
+                        d2v));
     return TDSCHA_OK;
 }
 
@@ -1054,12 +1065,12 @@ int perturb_digits(tdscha_ctx *c, int apply_d4, cudaStream_t st) {
         DgSource s = dg_matrix(DG_MATRIX, c->Y1all + j0 * MM, c->vsv + (long)(J + j0) * M, MM);
         s.rstride = M;
         s.S = c->vsv + (long)j0 * M;
-        TDS_TRY(digits_contract(c, nj, {{s}, 1}, apply_d4, &ns, st));
+        TDS_TRY(digits_contract(c, nj, {{s}, 1}, apply_d4, j0 == 0, &ns, st));
         const int nat = ceil_div((long)nj * Mp, kGM);
         TDS_TRY(psi_hsum64(c, x->gpart, ns, (long)nat * kGM * Mp, (long)Mp * Mp, Mp, x->fpart,
                            x->many ? 1 : x->nfc, c->fY, j0, nj, st));
     }
-    return psi_reduce64(c, st);
+    return psi_reduce64(c, x->failed, st);
 }
 
 int digits_from_matrix(tdscha_ctx *c, int apply_d4, const double *R1, const double *Y1, double *f,

@@ -173,10 +173,13 @@ __global__ void k_psi_sandwich(const int *__restrict__ sr_idx, const double *__r
     }
 }
 
-// d2v[a][b] = -inv sum_j tj[j][a][b], f[a] = inv sum_j tf[j][a], in image order.
+// d2v[a][b] = -inv sum_j tj[j][a][b], f[a] = inv sum_j tf[j][a], in image order; NaN where
+// *failed is set (failed may be null).
 __global__ void k_psi_jsum(const double *__restrict__ tj, const double *__restrict__ tf, int J,
-                           int M, double inv, double *__restrict__ f, double *__restrict__ d2v) {
+                           int M, double inv, const int *__restrict__ failed,
+                           double *__restrict__ f, double *__restrict__ d2v) {
     pdl_enter();
+    if (failed && *failed) inv = __longlong_as_double(0x7ff8000000000000LL);
     const long MM = (long)M * M;
     for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < MM; e += (long)gridDim.x * blockDim.x) {
         d2v[e] = -split_sum(tj + e, J, MM) * inv;
@@ -438,7 +441,7 @@ int psi_hsum64(tdscha_ctx *c, const double *gpart, int nsplit, long sstride, lon
     return TDSCHA_OK;
 }
 
-int psi_reduce64(tdscha_ctx *c, cudaStream_t st) {
+int psi_reduce64(tdscha_ctx *c, const int *failed, cudaStream_t st) {
     const int M = c->M, J = c->J;
     const size_t JMM = (size_t)J * M * M, JM = (size_t)J * M;
     double *hs = c->hs, *tj = hs + JMM, *fs = tj + JMM, *tf = fs + JM;
@@ -446,7 +449,7 @@ int psi_reduce64(tdscha_ctx *c, cudaStream_t st) {
     TDS_CUDA(launch_pdl(k_psi_sandwich, grid_for((long)JMM), 256, 0, st, c->sr_idx, c->sr_val, hs, fs, J,
                         M, c->maxdeg, tj, tf));
     TDS_CUDA(launch_pdl(k_psi_jsum, std::max(1, ceil_div((long)M * M, 64)), 64, 0, st, tj, tf, J, M,
-                        1.0 / (c->sum_rho * c->S), c->f, c->d2v));
+                        1.0 / (c->sum_rho * c->S), failed, c->f, c->d2v));
     return TDSCHA_OK;
 }
 
@@ -454,7 +457,7 @@ int psi_finalize64(tdscha_ctx *c, const double *gpart, int nsplit, long sstride,
                    long lda, const double *fpart, int nfchunk, cudaStream_t st) {
     TDS_TRY(psi_hsum64(c, gpart, nsplit, sstride, jstride, lda, fpart, nfchunk, nullptr, 0,
                        c->J, st));
-    return psi_reduce64(c, st);
+    return psi_reduce64(c, nullptr, st);
 }
 
 int psi_finalize32(tdscha_ctx *c, const float *gpart, int nsplit, long sstride, long jstride,

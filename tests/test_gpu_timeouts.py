@@ -58,3 +58,44 @@ def test_averages(gpu_lib, monkeypatch, M, N, S, precision):
     ctx = nat.Context(*args)
     right(_call(ctx, R1, Y1, precision))
     ctx.close()
+
+
+@pytest.mark.parametrize("M,N,S", [(48, 5000, 1), (129, 9000, 1), (24, 400, 48), (189, 2000, 8)])
+def test_device_pointers_get_nan(gpu_lib, monkeypatch, M, N, S):
+    """A call on device pointers returns before its kernels have run: after a wait that gave
+    up every result is NaN, and tdscha_ctx_sync says so once."""
+    import torch
+    ens = make_ensemble(M, N, seed=M + S, n_syms=S)
+    tables = ((ens["symmetries"], ens["degenerate_space"], ens["sym_block_id"]) if S > 1
+              else oracle.identity_symmetries(M))
+    monkeypatch.setenv("TDSCHA_WAIT_BUDGET_CYCLES", "0")
+    ctx = nat.Context(ens["X"], ens["Y"], ens["w"], ens["rho"], ens["T"], *tables)
+    monkeypatch.delenv("TDSCHA_WAIT_BUDGET_CYCLES")
+    R1 = torch.tensor(random_R1(M, 1), device="cuda")
+    Y1 = torch.tensor(random_sym(M, 2, scale=1e-3), device="cuda")
+    f, d2v = torch.zeros_like(R1), torch.zeros_like(Y1)
+    st = torch.cuda.current_stream().cuda_stream
+    nat.check(nat.load().tdscha_perturb_averages(ctx.handle, R1.data_ptr(), Y1.data_ptr(), 1,
+                                                 nat.PREC_FP64, f.data_ptr(), d2v.data_ptr(), 1, st))
+    with pytest.raises(nat.TdschaError) as e:
+        nat.check(nat.load().tdscha_ctx_sync(ctx.handle, st))
+    assert e.value.code == nat.ERR_TIMEOUT
+    assert torch.isnan(f).all() and torch.isnan(d2v).all()
+    nat.check(nat.load().tdscha_ctx_sync(ctx.handle, st))
+    ctx.close()
+
+
+@pytest.mark.parametrize("batch", [False, True])
+def test_run_reports_the_wait(gpu_lib, monkeypatch, batch):
+    """A run whose averages are NaN after such a wait reports the wait, not the NaN."""
+    from tdscha_gb300.DynamicalLanczos import Lanczos
+    from tdscha_gb300.batch import run_batch
+    M, N = 70, 4000
+    ens = make_ensemble(M, N, seed=1)
+    lanc = Lanczos.from_arrays(ens["X"], ens["Y"], ens["w"], ens["rho"], ens["T"], use_wigner=True)
+    lanc.init(use_symmetries=False)
+    lanc.prepare_perturbation(random_R1(M, 1), masses_exp=0)
+    monkeypatch.setenv("TDSCHA_WAIT_BUDGET_CYCLES", "0")
+    with pytest.raises(nat.TdschaError) as e:
+        run_batch([lanc], 4) if batch else lanc.run_FT(4, verbose=False)
+    assert e.value.code == nat.ERR_TIMEOUT
