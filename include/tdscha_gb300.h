@@ -354,6 +354,12 @@ int tdscha_qperturb_averages(tdscha_qctx *ctx, const double *R1, const double *a
 /* apply_full_L (QSpaceLanczos.py:941-961): device psi_in / psi_out of psi_size complex. */
 int tdscha_qapply_full_L(tdscha_qctx *ctx, const double *psi_in, double *psi_out, void *stream);
 
+/* Synchronise stream and report asynchronous failures, as tdscha_ctx_sync does: after
+ * tdscha_qapply_full_L, tdscha_qkpm_run and tdscha_qperturb_averages with device pointers,
+ * which return before their kernels run.  A bounded wait that gave up leaves NaN in the
+ * results of its call and is reported once. */
+int tdscha_qctx_sync(tdscha_qctx *ctx, void *stream);
+
 /*
  * Precision of the q-space averages (no counterpart in the reference, whose
  * Julia kernel is float64): TDSCHA_PREC_FP64 (default) or TDSCHA_PREC_MIXED,

@@ -161,10 +161,12 @@ class QSpaceKPM(QSpaceLanczos):
         work = torch.empty_like(A)
         mom = torch.from_numpy(np.ascontiguousarray(moments)).to(dev)
         swapped = nat.ctypes.c_int(0)
+        st = torch.cuda.current_stream().cuda_stream
         nat.check(nat.load().tdscha_qkpm_run(
             ctx.handle, A.data_ptr(), B.data_ptr(), work.data_ptr(), int(n_from),
             int(self.kpm_n_moments), float(self.kpm_rescale_a), float(self.kpm_rescale_b),
-            mom.data_ptr(), nat.ctypes.byref(swapped), torch.cuda.current_stream().cuda_stream))
+            mom.data_ptr(), nat.ctypes.byref(swapped), st))
+        nat.check(nat.load().tdscha_qctx_sync(ctx.handle, st))
         moments[:] = mom.cpu().numpy()
         if swapped.value:
             A, B = B, A

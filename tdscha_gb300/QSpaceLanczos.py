@@ -434,6 +434,7 @@ class QSpaceLanczos(Lanczos):
         out = torch.empty_like(psi)
         st = torch.cuda.current_stream().cuda_stream
         nat.check(nat.load().tdscha_qapply_full_L(ctx.handle, psi.data_ptr(), out.data_ptr(), st))
+        nat.check(nat.load().tdscha_qctx_sync(ctx.handle, st))
         return out.cpu().numpy()
 
     # ------------------------------------------------------- perturbations

@@ -31,7 +31,7 @@ EXPORTS = [
     "tdscha_mlp_num_params", "tdscha_mlp_set_params", "tdscha_mlp_get_params",
     "tdscha_mlp_forward", "tdscha_mlp_loss_grad", "tdscha_mlp_train_step",
     "tdscha_release_cached_memory", "tdscha_ctx_layout", "tdscha_ctx_tuning",
-    "tdscha_qctx_set_precision", "tdscha_ctx_set_basis_ld",
+    "tdscha_qctx_set_precision", "tdscha_ctx_set_basis_ld", "tdscha_qctx_sync",
 ]
 
 
@@ -95,6 +95,7 @@ def load():
     lib.tdscha_ctx_layout.argtypes = [_vp, _i, ctypes.POINTER(ctypes.c_longlong)]
     lib.tdscha_ctx_tuning.argtypes = [_vp, _i, _i, _d]
     lib.tdscha_qctx_set_precision.argtypes = [_vp, _c_int]
+    lib.tdscha_qctx_sync.argtypes = [_vp, _vp]
     lib.tdscha_release_cached_memory.argtypes = [_vp]
     lib.tdscha_static_hessian_expand.argtypes = [_vp, _vp, _vp, _vp]
     lib.tdscha_lanczos_run_hostbuf.argtypes = [_vp, _d, _d, _c_int, _c_int, _c_int, _c_int, _c_int,

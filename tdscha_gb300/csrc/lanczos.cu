@@ -2143,7 +2143,9 @@ extern "C" int tdscha_qlanczos_run(tdscha_qctx *ctx, double *basis_Q, double *ba
         set_error("qlanczos_run: %s", cudaGetErrorString(cudaGetLastError()));
         rc = TDSCHA_ERR_CUDA;
     }
-    return rc == TDSCHA_OK ? qdigits_check_error(ctx) : rc;
+    // a wait that gave up outranks what its NaN results gave
+    const int wrc = qdigits_check_error(ctx);
+    return wrc == TDSCHA_OK ? rc : wrc;
 }
 
 // Many independent runs together (real-space and q-space contexts mixed): each

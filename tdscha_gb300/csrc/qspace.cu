@@ -818,3 +818,11 @@ extern "C" int tdscha_qctx_set_precision(tdscha_qctx *ctx, int precision) {
     if (change && ctx->n_pairs > 0) TDS_TRY(qdigits_set_pert(ctx));
     return TDSCHA_OK;
 }
+
+extern "C" int tdscha_qctx_sync(tdscha_qctx *ctx, void *stream) {
+    set_error("");
+    if (!ctx) { set_error("qctx_sync: null context"); return TDSCHA_ERR_ARG; }
+    cudaError_t e = cudaStreamSynchronize((cudaStream_t)stream);
+    if (e != cudaSuccess) { set_error("qctx_sync: %s", cudaGetErrorString(e)); return TDSCHA_ERR_CUDA; }
+    return qdigits_check_error(ctx);
+}

@@ -42,7 +42,9 @@ struct QDigitStore {
     double *x = nullptr, *g = nullptr, *u = nullptr, *y = nullptr, *qp = nullptr;
     __half *xa = nullptr, *xb = nullptr, *yb = nullptr;
     int *ec = nullptr, *er = nullptr, *ecb = nullptr, *et = nullptr, *cofs = nullptr,
-        *wtop = nullptr, *err = nullptr;
+        *wtop = nullptr;
+    int *failed = nullptr;        // whether a bounded wait gave up in this call
+    int *err = nullptr;           // its code, until it has been reported (pinned host memory)
     int2 *erb = nullptr;          // a row's scales in y and in u, [q][Rp]
     double *rowc = nullptr;       // 8 doubles a row
     // per perturbation
@@ -241,7 +243,7 @@ __global__ void __launch_bounds__(32) k_qd_alpha(const QAlpha src, const int *__
                                                  const int *__restrict__ ec, int nb, int G, int nrt,
                                                  __half *__restrict__ yb, int *__restrict__ et,
                                                  int *__restrict__ cofs,
-                                                 int *__restrict__ wtop) {
+                                                 int *__restrict__ wtop, int *__restrict__ failed) {
     __shared__ long long s[64];
     const int nr = 2 * nb, lane = threadIdx.x, grp = blockIdx.y / G, k0 = blockIdx.y % G * nr;
     const int q = qpartner[blockIdx.y], row = k0 + blockIdx.x, n = blockIdx.x >> 1;
@@ -281,6 +283,7 @@ __global__ void __launch_bounds__(32) k_qd_alpha(const QAlpha src, const int *__
         for (int d = 0; d < kCall; ++d)
             *reinterpret_cast<uint4 *>(out + d * kGB + sw_place(row, lane)) = w[d];
     }
+    if (blockIdx.x == 0 && blockIdx.y == 0 && lane == 31) *failed = 0;
     // (there are no more pairs than q-points)
     if (blockIdx.x == 0 && (int)blockIdx.y < src.n_pairs && lane < 3) wtop[4 * blockIdx.y + lane] = INT_MIN;
     if (lane == 0) {
@@ -494,11 +497,11 @@ __global__ void __launch_bounds__(128) k_qd_wbuild(
 // The real products of the tiles to complex blocks, and f: H[row][col] of pair p and
 // split s at gpart[((s n_pairs + p) 128 + row) ld + col].  Eight lanes an element, each
 // every eighth split.  After a wait that gave up the results are NaN: calls that do not
-// return to the host report it that way.
+// return to the host report it that way (and in tdscha_qctx_sync).
 __global__ void __launch_bounds__(128) k_qd_final(const double *__restrict__ gpart, int ns, int nb,
                                                   int n_pairs, int nbq,
                                                   const double2 *__restrict__ fpart, int nff,
-                                                  double inv_norm, const int *__restrict__ err,
+                                                  double inv_norm, const int *__restrict__ failed,
                                                   double2 *__restrict__ f, double2 *__restrict__ d2v) {
     const int nr = 2 * nb, ld = nbq * kGN, uc = nbq == 1 ? nr : kGN;
     const long n = (long)n_pairs * nb * nb, e = blockIdx.x * 16L + (threadIdx.x >> 3);
@@ -533,7 +536,7 @@ __global__ void __launch_bounds__(128) k_qd_final(const double *__restrict__ gpa
         re += __shfl_xor_sync(0xffffffffu, re, o);
         im += __shfl_xor_sync(0xffffffffu, im, o);
     }
-    if (*err) inv_norm = __longlong_as_double(0x7ff8000000000000LL);
+    if (*failed) inv_norm = __longlong_as_double(0x7ff8000000000000LL);
     if (out && k0 == 0) *out = make_double2(re * inv_norm, im * inv_norm);
 }
 
@@ -544,6 +547,7 @@ void qdigits_release(tdscha_qctx *c) {
     if (!c->qd) return;
     cached_free(c->qd->slab);
     cached_free(c->qd->pslab);
+    if (c->qd->err) cudaFreeHost(c->qd->err);
     delete c->qd;
     c->qd = nullptr;
 }
@@ -608,7 +612,7 @@ static int qdigits_prepare(tdscha_qctx *c) {
         {(void **)&x->ecb, sizeof(int) * (size_t)n_q * x->nbq * kGN},
         {(void **)&x->et, sizeof(int) * x->ngrp * 64},
         {(void **)&x->cofs, sizeof(int) * x->ngrp * 64},
-        {(void **)&x->err, sizeof(int)},
+        {(void **)&x->failed, sizeof(int)},
         {(void **)&fl, sizeof(float) * kFlushes * kRes},
         {(void **)&x->yb, (size_t)x->ngrp * kCall * kGB},
     };
@@ -619,6 +623,8 @@ static int qdigits_prepare(tdscha_qctx *c) {
         return TDSCHA_OK;
     }
     c->qd = x;
+    TDS_CUDA(cudaMallocHost((void **)&x->err, sizeof(int)));
+    *x->err = 0;
     place(parts, x->slab);
     uint8_t *z = reinterpret_cast<uint8_t *>(x->ec);
     TDS_CUDA(cudaMemsetAsync(z, 0, (uint8_t *)x->slab + total - z, 0));
@@ -693,12 +699,11 @@ int qdigits_set_pert(tdscha_qctx *c) {
 
 bool qdigits_ready(const tdscha_qctx *c) { return c->qd && c->qd->n_pairs > 0; }
 
+// After the stream has been waited for
 int qdigits_check_error(tdscha_qctx *c) {
-    if (!c->qd) return TDSCHA_OK;
-    int v = 0;
-    TDS_CUDA(cudaMemcpy(&v, c->qd->err, sizeof(int), cudaMemcpyDeviceToHost));
-    if (!v) return TDSCHA_OK;
-    TDS_CUDA(cudaMemset(c->qd->err, 0, sizeof(int)));
+    if (!c->qd || !*(volatile int *)c->qd->err) return TDSCHA_OK;
+    const int v = *(volatile int *)c->qd->err;
+    *(volatile int *)c->qd->err = 0;
     set_error("tensor-core pipeline: a bounded wait expired (code %d)", v);
     return TDSCHA_ERR_TIMEOUT;
 }
@@ -713,7 +718,7 @@ int qdigits_perturb(tdscha_qctx *c, int apply_d4, const double *psi, cudaStream_
     double2 *rowc = reinterpret_cast<double2 *>(x->rowc), *fpart = reinterpret_cast<double2 *>(x->fpart);
     TDS_CUDA(launch_pdl(k_qd_alpha, dim3(x->nr, n_q), 32, 0, st, src, (const int *)c->qpair,
                         (const int *)c->qrole, (const int *)c->qpartner, (const int *)x->ec, nb, x->G,
-                        (int)x->nrt, x->yb, x->et, x->cofs, x->wtop));
+                        (int)x->nrt, x->yb, x->et, x->cofs, x->wtop, x->failed));
     DgArgs a{};
     a.a = x->xa;
     a.b = x->yb;
@@ -728,6 +733,7 @@ int qdigits_perturb(tdscha_qctx *c, int apply_d4, const double *psi, cudaStream_
     a.cofs = x->cofs;
     a.nr = x->nr;
     a.err = x->err;
+    a.failed = x->failed;
     a.budget = x->budget;
     a.dt = x->x;
     a.gt = x->g;
@@ -762,6 +768,7 @@ int qdigits_perturb(tdscha_qctx *c, int apply_d4, const double *psi, cudaStream_
     b.Mp = x->nbq * kGN;
     b.M = x->nbq * kGN;
     b.err = x->err;
+    b.failed = x->failed;
     b.budget = x->budget;
     b.ec = x->ecb;
     b.ew = x->ew;
@@ -773,7 +780,7 @@ int qdigits_perturb(tdscha_qctx *c, int apply_d4, const double *psi, cudaStream_
     const long n = (long)x->n_pairs * nb * nb + nb;
     TDS_CUDA(launch_pdl(k_qd_final, ceil_div(n, 16), 128, 0, st, (const double *)x->gpart, x->ns, nb,
                         x->n_pairs, x->nbq, (const double2 *)fpart, x->nfc,
-                        1.0 / (c->sum_rho * c->S), (const int *)x->err, c->f, c->d2v));
+                        1.0 / (c->sum_rho * c->S), (const int *)x->failed, c->f, c->d2v));
     return TDSCHA_OK;
 }
 

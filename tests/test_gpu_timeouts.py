@@ -99,3 +99,46 @@ def test_run_reports_the_wait(gpu_lib, monkeypatch, batch):
     with pytest.raises(nat.TdschaError) as e:
         run_batch([lanc], 4) if batch else lanc.run_FT(4, verbose=False)
     assert e.value.code == nat.ERR_TIMEOUT
+
+
+@pytest.mark.parametrize("call", ["averages", "averages on device pointers", "apply", "run", "batch",
+                                  "moments"])
+def test_bloch_space(gpu_lib, monkeypatch, call):
+    """Every way into the Bloch-space averages reports the wait, once, and leaves nothing of
+    it to the next call."""
+    import torch
+    from tdscha_gb300.batch import run_batch
+    from tdscha_gb300.QSpaceKPM import QSpaceKPM
+    from tdscha_gb300.synthetic import make_qspace_ensemble
+    e = make_qspace_ensemble((4, 2, 1), 12, 9000, seed=2, dispersion=0.2)
+    ql = QSpaceKPM.from_arrays(e["X_q"], e["Y_q"], e["w_q"], e["rho"], e["T"], q_points=e["q"])
+    ql.init(use_symmetries=False)
+    ql.prepare_mode_q(1, 2)
+    rng = np.random.default_rng(1)
+    R1 = rng.standard_normal(12) + 0j
+    alpha = [rng.standard_normal((12, 12)) + 0j for _ in ql.unique_pairs]
+    monkeypatch.setenv("TDSCHA_WAIT_BUDGET_CYCLES", "0")
+    ctx = ql._qcontext()
+    st = torch.cuda.current_stream().cuda_stream
+    if call == "averages on device pointers":
+        a, b = (torch.tensor(v, device="cuda") for v in (R1, np.stack(alpha)))
+        f, d2v = torch.zeros_like(a), torch.zeros_like(b)
+        nat.check(nat.load().tdscha_qperturb_averages(ctx.handle, a.data_ptr(), b.data_ptr(), 1,
+                                                      f.data_ptr(), d2v.data_ptr(), 1, st))
+    with pytest.raises(nat.TdschaError) as err:
+        if call == "averages":
+            ql.get_perturb_averages_q(R1, alpha)
+        elif call == "apply":
+            ql.apply_full_L()
+        elif call == "run":
+            ql.run_FT(3, verbose=False)
+        elif call == "batch":
+            run_batch([ql], 3)
+        elif call == "moments":
+            ql.run_KPM(8, lambda_min=0.0, lambda_max=1e-4, verbose=False)
+        else:
+            nat.check(nat.load().tdscha_qctx_sync(ctx.handle, st))
+    assert err.value.code == nat.ERR_TIMEOUT
+    nat.check(nat.load().tdscha_qctx_sync(ctx.handle, st))
+    if call == "averages on device pointers":
+        assert torch.isnan(f.real).all() and torch.isnan(d2v.real).all()
