@@ -69,7 +69,10 @@ int tdscha_get_perturb_average_sym(int M, int N, const double *X, const double *
  * rows and two-limb fp16 operands used by TDSCHA_PREC_MIXED.  with_mixed = 0:
  * float64 storage only; 1: both; 2: the mixed operands only (4-byte storage),
  * the float64 image rows released once the operands are built, so that
- * TDSCHA_PREC_FP64 calls on this context return TDSCHA_ERR_STATE.  Replaces
+ * TDSCHA_PREC_FP64 calls on this context return TDSCHA_ERR_STATE.  The operands of the
+ * float64 tensor-core path are made with the context where with_mixed = 0, and at the
+ * first TDSCHA_PREC_FP64 call where it is 1 (which allocates; inside a stream capture the
+ * CUDA cores serve the call instead).  Replaces
  * the state the reference keeps in `Lanczos`
  * (Modules/DynamicalLanczos.py:183-505, :694-871) and re-sends to the C
  * module on every call.  Host pointers.

@@ -150,6 +150,7 @@ struct tdscha_ctx {
     int nblk_dot = 0;
     tdscha::MixedStore mx;
     tdscha::DigitStore *dg = nullptr;   // float64 averages by digit products (null: CUDA cores)
+    bool dg_pending = false;            // not yet prepared (digits_first_use)
     // diagnostics: CUDA-event pairs per kernel id while profiling is on
     int prof = 0;
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> prof_ev[8];
@@ -204,6 +205,8 @@ int perturb_fp64(tdscha_ctx *c, int apply_d4, cudaStream_t st);
 int alloc_fp64_scratch(tdscha_ctx *c);
 // perturb_digits.cu: the float64 averages by exact digit products on the tensor cores
 int digits_prepare(tdscha_ctx *c);
+// At the start of a float64 call: prepares what the creation of a mixed context left
+int digits_first_use(tdscha_ctx *c, cudaStream_t st);
 void digits_release(tdscha_ctx *c);
 int digits_check_error(tdscha_ctx *c);
 int perturb_digits(tdscha_ctx *c, int apply_d4, cudaStream_t st);

@@ -424,7 +424,10 @@ images_done:
     CUC(cudaMemset(c->scal, 0, sizeof(double) * 64));
     CUC(cudaMallocHost((void **)&c->host_pinned, sizeof(double) * 64));
     TRYC(build_pair_coeffs(c));
-    if (with_mixed != 2) TRYC(digits_prepare(c));
+    // mixed contexts may never see a float64 call, and their own operands come first where
+    // memory is short: digits at the first such call (M=573, N=50000: 2.3 GB and 1.2 of 5.5 ms)
+    c->dg_pending = with_mixed == 1;
+    if (with_mixed == 0) TRYC(digits_prepare(c));
     if (!c->dg) TRYC(alloc_fp64_scratch(c));
     if (with_mixed) TRYC(mixed_prepare(c));
     CUC(cudaDeviceSynchronize());
@@ -531,6 +534,7 @@ extern "C" int tdscha_perturb_averages(tdscha_ctx *ctx, const double *R1, const 
         for (long k = 0; k < (long)M * M; ++k)
             if (!std::isfinite(Y1[k])) { set_error("perturb_averages: non-finite Y1"); return TDSCHA_ERR_NAN; }
     }
+    if (precision == TDSCHA_PREC_FP64) TDS_TRY(digits_first_use(ctx, st));
     // the tensor-core paths read and write device arrays in place: R1 and Y1 are
     // read by their first kernels, f_out and d2v_out written by their last
     if (device_ptrs && precision == TDSCHA_PREC_FP64 && digits_single(ctx))

@@ -280,6 +280,7 @@ int apply_full_L_dev(tdscha_ctx *c, const double *psi_in, double *psi_out, int t
     int M = c->M;
     long H = c->H;
     int with_anh = !c->ignore_v3;
+    if (with_anh && precision == TDSCHA_PREC_FP64) TDS_TRY(digits_first_use(c, st));
     if (with_anh) {
         if (precision == TDSCHA_PREC_MIXED && c->with_mixed && !c->use_wigner) {
             // the tensor-core path reads Y1 and R1 straight from psi while it
@@ -332,6 +333,7 @@ static bool pair_apply_enabled() {
 int apply_full_L_pair_dev(tdscha_ctx *c, const double *q, const double *p, double *Lq,
                           double *pL, int precision, cudaStream_t st) {
     const bool both = pair_apply_enabled() && !c->use_wigner && !c->ignore_v3 && c->tr_ntrans == 0;
+    if (both && precision == TDSCHA_PREC_FP64) TDS_TRY(digits_first_use(c, st));
     const bool mixed = precision == TDSCHA_PREC_MIXED && c->with_mixed && c->f2;
     const bool digits = precision == TDSCHA_PREC_FP64 && digits_batch(c) >= 2;
     if (!both || !(mixed || digits)) {

@@ -865,6 +865,17 @@ int digits_prepare(tdscha_ctx *c) {
     return TDSCHA_OK;
 }
 
+// Outside of stream captures, where nothing may be allocated (a call in one takes the CUDA
+// cores and leaves the digits to a later call)
+int digits_first_use(tdscha_ctx *c, cudaStream_t st) {
+    if (!c->dg_pending) return TDSCHA_OK;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    TDS_CUDA(cudaStreamIsCapturing(st, &cap));
+    if (cap != cudaStreamCaptureStatusNone) return TDSCHA_OK;
+    c->dg_pending = false;
+    return digits_prepare(c);
+}
+
 int digits_check_error(tdscha_ctx *c) {
     if (!c->dg || !*(volatile int *)c->dg->err) return TDSCHA_OK;
     const int v = *(volatile int *)c->dg->err;

@@ -198,6 +198,7 @@ extern "C" int tdscha_static_L(tdscha_ctx *ctx, int nvec, const double *psi_in, 
     const int harm = what & 1, anh = (what >> 1) & 1;
     const int nbu = std::max(1, std::min(ceil_div((long)M * M, 256), 4096));
     const int nba = std::max(1, std::min(ceil_div(Ps, 256), 4096));
+    if (anh && precision == TDSCHA_PREC_FP64) TDS_TRY(digits_first_use(ctx, st));
     const int batch = anh && precision == TDSCHA_PREC_FP64 ? digits_batch(ctx) : 0;
     // float64 averages of many vectors together: one launch per kernel for all
     for (int v = 0; batch > 0 && v < nvec; v += batch) {
