@@ -156,20 +156,30 @@ __device__ __forceinline__ void digit_norms(const uint4 (&w)[kRes], int c, float
     }
 }
 
-// out[L - 3][digit]: largest norm (squared) over the accumulations of L = 3 +
-// blockIdx.y blocks of any row; nrm[tile][block][digit][rows], thread = row.
+// out[L - 3][digit]: largest norm (squared) of any row over any L = 3 + blockIdx.y blocks
+// that follow one another (a split of the contraction may start at any block);
+// nrm[tile][block][digit][rows], thread = row, kWindowStarts first blocks a block.  The sums
+// are whole numbers up to 9 2^20, exact in fp32.
+constexpr int kWindowStarts = 32;
 static __global__ void k_dg_windows(const float *__restrict__ nrm, int nkb, float *__restrict__ out) {
-    const float *p = nrm + blockIdx.x * (long)nkb * kRes * blockDim.x + threadIdx.x;
-    const int L = kFlushMin + blockIdx.y;
-    float mx[kRes] = {};
-    for (int kb = 0; kb < nkb; kb += L) {
-        float s[kRes] = {};
-        for (int k = kb; k < min(nkb, kb + L); ++k)
+    const int L = kFlushMin + blockIdx.y, s0 = blockIdx.z * kWindowStarts,
+              s1 = min(s0 + kWindowStarts, max(1, nkb - L + 1));
+    if (s0 >= s1) return;
+    const long step = (long)kRes * blockDim.x;
+    const float *p = nrm + (blockIdx.x * (long)nkb + s0) * step + threadIdx.x, *q = p;
+    float s[kRes] = {}, mx[kRes];
+    for (int k = s0; k < min(nkb, s0 + L); ++k, q += step)
 #pragma unroll
-            for (int d = 0; d < kRes; ++d) s[d] += p[((long)k * kRes + d) * blockDim.x];
+        for (int d = 0; d < kRes; ++d) s[d] += q[d * blockDim.x];
 #pragma unroll
-        for (int d = 0; d < kRes; ++d) mx[d] = fmaxf(mx[d], s[d]);
-    }
+    for (int d = 0; d < kRes; ++d) mx[d] = s[d];
+#pragma unroll 4
+    for (int k = s0 + 1; k < s1; ++k, p += step, q += step)
+#pragma unroll
+        for (int d = 0; d < kRes; ++d) {
+            s[d] += q[d * blockDim.x] - p[d * blockDim.x];
+            mx[d] = fmaxf(mx[d], s[d]);
+        }
 #pragma unroll
     for (int d = 0; d < kRes; ++d) {
 #pragma unroll
@@ -178,6 +188,12 @@ static __global__ void k_dg_windows(const float *__restrict__ nrm, int nkb, floa
         if ((threadIdx.x & 31) == 0)
             atomicMax(reinterpret_cast<int *>(out + blockIdx.y * kRes + d), __float_as_int(mx[d]));
     }
+}
+
+// (nkb <= 65535 kWindowStarts, over a hundred million rows)
+inline cudaError_t dg_windows(const float *nrm, int tiles, int rows, int nkb, float *out, cudaStream_t st) {
+    k_dg_windows<<<dim3(tiles, kFlushes, ceil_div(nkb, kWindowStarts)), rows, 0, st>>>(nrm, nkb, out);
+    return cudaGetLastError();
 }
 
 // The longest accumulation (K blocks) that keeps orders 0..4 below 2^24 for any

@@ -835,12 +835,10 @@ int digits_prepare(tdscha_ctx *c) {
     float *nrm = reinterpret_cast<float *>(x->wa);
     k_dg_xa<<<dim3((unsigned)nrt, x->nkbM), 256>>>(c->D, x->ec, x->er, R, M, x->nkbM, x->xa, nrm);
     TDS_CHECK_LAUNCH();
-    k_dg_windows<<<dim3((unsigned)nrt, kFlushes), kGM>>>(nrm, x->nkbM, fl);
-    TDS_CHECK_LAUNCH();
+    TDS_CUDA(dg_windows(nrm, (int)nrt, kGM, x->nkbM, fl, 0));
     k_dg_xb<<<dim3((unsigned)x->nkbR, x->nct), 256>>>(x->dt, x->ec, x->er, Mp, x->nkbR, x->xb, nrm);
     TDS_CHECK_LAUNCH();
-    k_dg_windows<<<dim3(x->nct, kFlushes), kGN>>>(nrm, (int)x->nkbR, fl + kFlushes * kRes);
-    TDS_CHECK_LAUNCH();
+    TDS_CUDA(dg_windows(nrm, x->nct, kGN, (int)x->nkbR, fl + kFlushes * kRes, 0));
     if (x->many) {
         __half *ga = x->xa + kRes * elems, *gb = x->xb + kRes * elems;
         k_dg_ga<<<dim3((unsigned)nrt, x->nkbM), 256>>>(x->gt, ecg, erg, M, Mp, x->nkbM, ga);

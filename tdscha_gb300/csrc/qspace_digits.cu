@@ -645,8 +645,7 @@ static int qdigits_prepare(tdscha_qctx *c) {
     k_qd_xb<<<dim3((unsigned)x->nkb, n_q * x->nbq), 256>>>(x->y, x->u, x->ecb, x->erb, nr, x->nbq,
                                                            x->nrt, x->nkb, x->xb, nrm);
     TDS_CHECK_LAUNCH();
-    k_dg_windows<<<dim3(n_q * x->nbq, kFlushes), kGN>>>(nrm, (int)x->nkb, fl);
-    TDS_CHECK_LAUNCH();
+    TDS_CUDA(dg_windows(nrm, n_q * x->nbq, kGN, (int)x->nkb, fl, 0));
     float h_fl[kFlushes * kRes];
     TDS_CUDA(cudaMemcpy(h_fl, fl, sizeof(h_fl), cudaMemcpyDeviceToHost));
     x->flush = digits_flush(h_fl);
