@@ -131,12 +131,6 @@ __device__ __forceinline__ double pow2(int e) {
     return __longlong_as_double((long long)(e < -1022 ? 0 : min(e + 1023, 2047)) << 52);
 }
 
-// What a configuration's element counts for in the scale of its column: its exponent, less
-// what its weight is below the largest one (exponent rtop); INT_MIN of nothing.
-__device__ __forceinline__ int dg_weighted_exp(double x, double rho, int rtop) {
-    return x != 0 && rho != 0 ? exp_above(x) + min(0, exp_above(rho) - rtop) : INT_MIN;
-}
-
 // Sums of the squares of each digit over the 64 elements of a block's row, from
 // the eight lanes that hold it: nrm[digit * rows + row].
 __device__ __forceinline__ void digit_norms(const uint4 (&w)[kRes], int c, float *__restrict__ nrm,

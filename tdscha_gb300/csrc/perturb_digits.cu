@@ -83,15 +83,28 @@ __global__ void __launch_bounds__(128) k_dg_colexp(const double *__restrict__ D,
                                                    const double *__restrict__ rho, int rho_div, int rtop,
                                                    long R, int M, int Mp, long per,
                                                    int *__restrict__ ec) {
+    __shared__ int less[128];      // what 128 rows' elements count for beside their exponents
     const int m = blockIdx.x * 128 + threadIdx.x;
-    if (m >= M) return;
-    const double *a = blockIdx.z ? F : D;
+    const double *a = (blockIdx.z ? F : D) + min(m, M - 1);
     const long r0 = blockIdx.y * per, r1 = min(R, r0 + per);
     int e = INT_MIN;
-#pragma unroll 4
-    for (long r = r0; r < r1; ++r)
-        e = max(e, dg_weighted_exp(a[r * M + m], rho[rho_div == 1 ? r : r / rho_div], rtop));
-    atomicMax(ec + blockIdx.z * Mp + m, e);
+    for (long c0 = r0; c0 < r1; c0 += 128) {
+        const int n = (int)min(128L, r1 - c0);
+        const long r = c0 + threadIdx.x;
+        __syncthreads();
+        if (r < r1) {
+            const double w = rho[rho_div == 1 ? r : r / rho_div];
+            less[threadIdx.x] = w != 0 ? min(0, exp_above(w) - rtop) : INT_MIN / 2;
+        }
+        __syncthreads();
+#pragma unroll 8
+        for (int k = 0; k < n; ++k) {
+            const double x = a[(c0 + k) * M];
+            const int v = exp_above(x) + less[k];
+            e = max(e, x != 0 ? v : INT_MIN);
+        }
+    }
+    if (m < M && e > INT_MIN / 4) atomicMax(ec + blockIdx.z * Mp + m, e);
 }
 
 // From there: g's scales from y's, and 0 of a column without an element; eb has kZeroExp
@@ -135,22 +148,25 @@ __global__ void k_dg_cols(const double *__restrict__ D, const double *__restrict
     }
 }
 
-// er[r]: exponent above the maximum over the modes of |x| 2^-ec (kZeroExp for a zero row)
-__global__ void k_dg_rowexp(const double *__restrict__ dt, const int *__restrict__ ec, int M,
-                            int Mp, int *__restrict__ er) {
+// er[r], er[Rp + r]: exponents above the maxima over the modes of |x| 2^-ec and |g| 2^-ec
+// (kZeroExp for a row of zeros)
+__global__ void k_dg_rowexp(const double *__restrict__ dt, const double *__restrict__ gt,
+                            const int *__restrict__ ec, int M, int Mp, int *__restrict__ er) {
     __shared__ int sh[8][128];
     const long rt = blockIdx.x;
-    const int row = threadIdx.x, g = threadIdx.y;
+    const int row = threadIdx.x, g = threadIdx.y, *e0 = ec + blockIdx.y * Mp;
+    const double *a = (blockIdx.y ? gt : dt) + rt * Mp * 128 + row;
     int e = INT_MIN;
+#pragma unroll 4
     for (int m = g; m < M; m += 8) {
-        const double d = dt[(rt * Mp + m) * 128 + row];
-        if (d != 0) e = max(e, exp_above(d) - ec[m]);
+        const double d = a[m * 128L];
+        if (d != 0) e = max(e, exp_above(d) - e0[m]);
     }
     sh[g][row] = e;
     __syncthreads();
     if (g == 0) {
         for (int k = 1; k < 8; ++k) e = max(e, sh[k][row]);
-        er[rt * 128 + row] = e == INT_MIN ? kZeroExp : e;
+        er[(blockIdx.y * (long)gridDim.x + rt) * 128 + row] = e == INT_MIN ? kZeroExp : e;
     }
 }
 
@@ -827,9 +843,7 @@ int digits_prepare(tdscha_ctx *c) {
     k_dg_cols<<<dim3((unsigned)nrt, Mp / 32), dim3(32, 8)>>>(c->D, c->F, c->fY, R, M, Mp, x->dt,
                                                               x->gt);
     TDS_CHECK_LAUNCH();
-    k_dg_rowexp<<<(unsigned)nrt, dim3(128, 8)>>>(x->dt, x->ec, M, Mp, x->er);
-    TDS_CHECK_LAUNCH();
-    k_dg_rowexp<<<(unsigned)nrt, dim3(128, 8)>>>(x->gt, ecg, M, Mp, erg);
+    k_dg_rowexp<<<dim3((unsigned)nrt, 2), dim3(128, 8)>>>(x->dt, x->gt, x->ec, M, Mp, x->er);
     TDS_CHECK_LAUNCH();
     // the digit norms pass through the W digits' space, which is zeroed again
     float *nrm = reinterpret_cast<float *>(x->wa);

@@ -91,6 +91,12 @@ __global__ void __launch_bounds__(256) k_qd_cols(const double *__restrict__ Xr,
     }
 }
 
+// What a configuration's element counts for in the scale of its column: its exponent, less
+// what its weight is below the largest one (exponent rtop); INT_MIN of nothing.
+__device__ __forceinline__ int dg_weighted_exp(double x, double rho, int rtop) {
+    return x != 0 && rho != 0 ? exp_above(x) + min(0, exp_above(rho) - rtop) : INT_MIN;
+}
+
 // Scales of the columns, their largest weighted exponents (dg_weighted_exp): of x in ec, of y
 // and u as the tiles [y | u] have them in ecb.  A column without an element (the imaginary
 // parts at Gamma, masked modes) has kZeroExp, which leaves it out of the rows' scales of A_q
