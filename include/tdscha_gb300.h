@@ -217,6 +217,24 @@ int tdscha_ctx_profile_read(tdscha_ctx *ctx, int kernel_id, double *total_ms, in
 int tdscha_ctx_layout(tdscha_ctx *ctx, int *images_on_perturbation, long long *ensemble_rows);
 
 /*
+ * Which kernels serve the context's float64 averages (no counterpart in the reference):
+ * exact digit products on the tensor cores, or, where their operands (44 bytes an element
+ * of X and what W and the partial sums take, see TDSCHA_PREC_FP64) would not fit, float64
+ * on the CUDA cores, about 30 times slower at M=573, N=50000.  They do not fit where they
+ * take more than 4 GB and more than a quarter of the device memory that is free or idle in
+ * the library's cache, where they cannot be allocated, above 25600 modes, and with
+ * TDSCHA_FP64_DIGITS=0 in the environment when they are made.  PENDING: not chosen yet (a
+ * context with with_mixed = 1 before its first float64 call; a Bloch-space context before
+ * its first tdscha_qctx_set_pert in float64).  NONE: with_mixed = 2.
+ */
+#define TDSCHA_FP64_CUDA_CORES 0
+#define TDSCHA_FP64_TENSOR_CORES 1
+#define TDSCHA_FP64_PENDING 2
+#define TDSCHA_FP64_NONE 3
+int tdscha_ctx_fp64_path(tdscha_ctx *ctx, int *path);
+int tdscha_qctx_fp64_path(tdscha_qctx *ctx, int *path);
+
+/*
  * The tensor-core shapes the autotuner chose for a context created with the
  * mixed path (no counterpart in the reference).  At creation the context
  * times one mixed application for each candidate -- stage A with two

@@ -14,6 +14,7 @@ LIB_PATH = os.path.join(HERE, "libtdscha_gb300.so")
 OK = 0
 ERR_ARG, ERR_CUDA, ERR_NAN, ERR_STATE, ERR_TIMEOUT = -1, -2, -3, -4, -5
 PREC_FP64, PREC_MIXED = 0, 1
+FP64_PATHS = ("CUDA cores", "tensor cores", "pending", "none")
 
 # every symbol the public header declares
 EXPORTS = [
@@ -32,6 +33,7 @@ EXPORTS = [
     "tdscha_mlp_forward", "tdscha_mlp_loss_grad", "tdscha_mlp_train_step",
     "tdscha_release_cached_memory", "tdscha_ctx_layout", "tdscha_ctx_tuning",
     "tdscha_qctx_set_precision", "tdscha_ctx_set_basis_ld", "tdscha_qctx_sync",
+    "tdscha_ctx_fp64_path", "tdscha_qctx_fp64_path",
 ]
 
 
@@ -96,6 +98,8 @@ def load():
     lib.tdscha_ctx_tuning.argtypes = [_vp, _i, _i, _d]
     lib.tdscha_qctx_set_precision.argtypes = [_vp, _c_int]
     lib.tdscha_qctx_sync.argtypes = [_vp, _vp]
+    lib.tdscha_ctx_fp64_path.argtypes = [_vp, _i]
+    lib.tdscha_qctx_fp64_path.argtypes = [_vp, _i]
     lib.tdscha_release_cached_memory.argtypes = [_vp]
     lib.tdscha_static_hessian_expand.argtypes = [_vp, _vp, _vp, _vp]
     lib.tdscha_lanczos_run_hostbuf.argtypes = [_vp, _d, _d, _c_int, _c_int, _c_int, _c_int, _c_int,
@@ -219,6 +223,12 @@ class Context:
                                        ctypes.byref(ms)))
         return a.value, n.value, ms.value
 
+    def fp64_path(self):
+        """Which kernels serve float64 averages: one of FP64_PATHS."""
+        path = ctypes.c_int(0)
+        check(load().tdscha_ctx_fp64_path(self.handle, ctypes.byref(path)))
+        return FP64_PATHS[path.value]
+
     def basis_ld(self):
         """Row stride used for Lanczos basis buffers: P rounded up to 32 doubles
         (256-byte rows, so that the re-biorthogonalisation reads element pairs)."""
@@ -322,6 +332,12 @@ class QContext:
         if getattr(self, "_precision", None) != code:
             check(load().tdscha_qctx_set_precision(self.handle, code))
             self._precision = code
+
+    def fp64_path(self):
+        """Which kernels serve float64 averages: one of FP64_PATHS."""
+        path = ctypes.c_int(0)
+        check(load().tdscha_qctx_fp64_path(self.handle, ctypes.byref(path)))
+        return FP64_PATHS[path.value]
 
     def set_pert(self, iq_pert, q_pair_map, ignore_harmonic=False, ignore_v3=False,
                  ignore_v4=False):

@@ -257,6 +257,7 @@ int q_apply_full_L_dev(tdscha_qctx *c, const double *psi_in, double *psi_out, cu
 void qdigits_release(tdscha_qctx *c);
 int qdigits_set_pert(tdscha_qctx *c);
 bool qdigits_ready(const tdscha_qctx *c);
+int qdigits_path(const tdscha_qctx *c);
 int qdigits_perturb(tdscha_qctx *c, int apply_d4, const double *psi, cudaStream_t st);
 int qdigits_check_error(tdscha_qctx *c);
 // preprocess.cu
@@ -301,6 +302,10 @@ inline int ceil_div(long a, long b) { return (int)((a + b - 1) / b); }
 // callers free after synchronising.
 cudaError_t cached_malloc(void **p, size_t bytes);
 void cached_free(void *p);
+// Whether a path that the library can do without may take this much device memory: up to
+// 4 GB always, above that a quarter of what is free or idle in the cache (an allocation
+// that needs the idle blocks gets them).
+bool memory_to_spare(size_t bytes);
 // frees a block at once (cudaFree), whether it came from cached_malloc or not
 void release_block(void *p);
 template <typename T>

@@ -163,6 +163,21 @@ cudaError_t tdscha::cached_malloc(void **p, size_t bytes) {
     return e;
 }
 
+bool tdscha::memory_to_spare(size_t bytes) {
+    if (bytes <= (size_t(4) << 30)) return true;
+    size_t fr = 0, all = 0, idle = 0;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaMemGetInfo(&fr, &all) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    BlockCache &bc = block_cache();
+    std::lock_guard<std::mutex> lock(bc.mu);
+    for (const BlockCache::Idle &b : bc.order)
+        if (b.dev == dev) idle += b.bytes;
+    return bytes <= (fr + idle) / 4;
+}
+
 void tdscha::cached_free(void *p) {
     if (!p) return;
     BlockCache &bc = block_cache();
@@ -622,6 +637,15 @@ extern "C" int tdscha_ctx_layout(tdscha_ctx *ctx, int *images_on_perturbation,
     }
     *images_on_perturbation = ctx->J;
     *ensemble_rows = ctx->Nrows;
+    return TDSCHA_OK;
+}
+
+extern "C" int tdscha_ctx_fp64_path(tdscha_ctx *ctx, int *path) {
+    set_error("");
+    if (!ctx || !path) { set_error("ctx_fp64_path: null pointer"); return TDSCHA_ERR_ARG; }
+    *path = ctx->dg ? TDSCHA_FP64_TENSOR_CORES
+            : !ctx->D ? TDSCHA_FP64_NONE
+            : ctx->dg_pending ? TDSCHA_FP64_PENDING : TDSCHA_FP64_CUDA_CORES;
     return TDSCHA_OK;
 }
 

@@ -806,16 +806,7 @@ int digits_prepare(tdscha_ctx *c) {
         if (p.zero && !zero0) zero0 = total;
         total += (p.bytes + 1023) & ~size_t(1023);
     }
-    // a quarter of the free memory at most (asked for only where it can matter)
-    if (total > (size_t(4) << 30)) {
-        size_t fr = 0, all = 0;
-        if (cudaMemGetInfo(&fr, &all) != cudaSuccess || total > fr / 4) {
-            cudaGetLastError();
-            delete x;
-            return TDSCHA_OK;
-        }
-    }
-    if (cached_malloc(&x->slab, total) != cudaSuccess) {
+    if (!memory_to_spare(total) || cached_malloc(&x->slab, total) != cudaSuccess) {
         cudaGetLastError();
         delete x;
         return TDSCHA_OK;

@@ -826,3 +826,10 @@ extern "C" int tdscha_qctx_sync(tdscha_qctx *ctx, void *stream) {
     if (e != cudaSuccess) { set_error("qctx_sync: %s", cudaGetErrorString(e)); return TDSCHA_ERR_CUDA; }
     return qdigits_check_error(ctx);
 }
+
+extern "C" int tdscha_qctx_fp64_path(tdscha_qctx *ctx, int *path) {
+    set_error("");
+    if (!ctx || !path) { set_error("qctx_fp64_path: null pointer"); return TDSCHA_ERR_ARG; }
+    *path = qdigits_path(ctx);
+    return TDSCHA_OK;
+}

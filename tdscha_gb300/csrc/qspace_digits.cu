@@ -558,16 +558,6 @@ void qdigits_release(tdscha_qctx *c) {
     c->qd = nullptr;
 }
 
-static bool fits(size_t bytes) {
-    if (bytes <= (size_t(4) << 30)) return true;
-    size_t fr = 0, all = 0;
-    if (cudaMemGetInfo(&fr, &all) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    return bytes <= fr / 4;
-}
-
 struct QPart {
     void **p;
     size_t bytes;
@@ -623,7 +613,7 @@ static int qdigits_prepare(tdscha_qctx *c) {
         {(void **)&x->yb, (size_t)x->ngrp * kCall * kGB},
     };
     const size_t total = place(parts, nullptr);
-    if (!fits(total) || cached_malloc(&x->slab, total) != cudaSuccess) {
+    if (!memory_to_spare(total) || cached_malloc(&x->slab, total) != cudaSuccess) {
         cudaGetLastError();
         delete x;
         return TDSCHA_OK;
@@ -689,7 +679,7 @@ int qdigits_set_pert(tdscha_qctx *c) {
     cached_free(x->pslab);
     x->pslab = nullptr;
     const size_t total = place(parts, nullptr);
-    if (!fits(total) || cached_malloc(&x->pslab, total) != cudaSuccess) {
+    if (!memory_to_spare(total) || cached_malloc(&x->pslab, total) != cudaSuccess) {
         cudaGetLastError();
         x->pslab = nullptr;
         x->n_pairs = 0;         // this perturbation on the CUDA cores
@@ -703,6 +693,11 @@ int qdigits_set_pert(tdscha_qctx *c) {
 }
 
 bool qdigits_ready(const tdscha_qctx *c) { return c->qd && c->qd->n_pairs > 0; }
+
+int qdigits_path(const tdscha_qctx *c) {
+    if (c->n_pairs == 0 || c->precision == TDSCHA_PREC_MIXED) return TDSCHA_FP64_PENDING;
+    return qdigits_ready(c) ? TDSCHA_FP64_TENSOR_CORES : TDSCHA_FP64_CUDA_CORES;
+}
 
 // After the stream has been waited for
 int qdigits_check_error(tdscha_qctx *c) {
