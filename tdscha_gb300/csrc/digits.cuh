@@ -131,6 +131,14 @@ __device__ __forceinline__ double pow2(int e) {
     return __longlong_as_double((long long)(e < -1022 ? 0 : min(e + 1023, 2047)) << 52);
 }
 
+// What a configuration's elements count for in the scales of their columns beside their
+// exponents: what its weight is below the largest one (exponent rtop), if that is much.
+// With every weight counted, ordinary configurations would lie outside by a bit or two.
+__device__ __forceinline__ int dg_weight_exp(double rho, int rtop) {
+    const int e = exp_above(rho) - rtop;
+    return rho == 0 ? INT_MIN / 2 : e < -8 ? e : 0;
+}
+
 // Sums of the squares of each digit over the 64 elements of a block's row, from
 // the eight lanes that hold it: nrm[digit * rows + row].
 __device__ __forceinline__ void digit_norms(const uint4 (&w)[kRes], int c, float *__restrict__ nrm,

@@ -16,37 +16,41 @@
 //
 // Digits: 7 of the resident operand (55 bits under the largest element of its
 // row), 8 of the operand made per call (62 bits), products of order 0..7 (35 of
-// 56).  What is left out is below 2^-64 of the product of the two row maxima;
-// the float64 sums this replaces round every partial sum at 2^-53.
+// 56).  Before the sums an element of the resident operand is rounded by up to 2^-56
+// of its row's largest, one of the per-call operand by 2^-63.  Left out are the products
+// of order 8 and above: six pairs of digits, up to 2^14 in units of 2^-77 each, 2^-60.4 of
+// the product of the two rows' largest elements for every element of the sum.  Both are
+// relative to the largest elements of the rows, not to the result; the float64
+// sums this replaces round every partial sum at 2^-53 of itself.
 //
 // Length of an accumulation: three K blocks (192 elements) keep orders 0..4 exact
 // for any input (5 * 192 products of 2^14 stay below 2^24).  The digits of real
 // numbers are far from their limits, so the longest accumulation is chosen per
 // ensemble by a bound that holds for every perturbation: by Cauchy and Schwarz the
 // order-o sum is at most sum_i |d_i| 128 sqrt(K) with |d_i| the largest 2-norm of
-// digit i over K elements of any row, measured when the context is made
-// (digits_flush).  Gaussian displacements allow five to seven blocks.  Orders 5..7
-// could round, by 2^-53 of the row maxima's product or less, only where the
+// digit i over any K consecutive elements of any row, measured when the operands are
+// made (k_dg_windows, digits_flush).  Gaussian displacements allow five to seven blocks.
+// Orders 5..7 could round, by 2^-53 of the row maxima's product or less, only where the
 // digits of two rows agree in sign and size over a whole accumulation.
 //
 // Error (2-norm, against 113-bit arithmetic) of f and d2v, these kernels | those
-// of perturb_fp64.cu: M=573 N=2000 6.9e-16 7.0e-16 | 1.3e-15 1.2e-15; with Y1 over
-// six decades 7.9e-16 7.7e-16 | 1.4e-15 1.2e-15; M=192 N=3000 1.5e-15 1.5e-15 |
-// 1.7e-15 1.6e-15; M=24 N=400 48 images 1.3e-15 5.3e-16 | 3.1e-15 5.6e-16.
-// One call: M=573 N=50000 57.1 -> 1.71 ms; M=189 N=10000 48 images 62.8 -> 2.10 ms;
+// of perturb_fp64.cu: M=573 N=2000 6.5e-16 6.9e-16 | 1.3e-15 1.2e-15; with Y1 over
+// six decades 7.8e-16 7.6e-16 | 1.4e-15 1.2e-15; M=192 N=3000 1.4e-15 1.5e-15 |
+// 1.7e-15 1.6e-15; M=24 N=400 48 images 1.2e-15 5.4e-16 | 3.1e-15 5.6e-16.
+// One call: M=573 N=50000 57.1 -> 1.71 ms; M=189 N=10000 48 images 62.8 -> 2.09 ms;
 // M=97 N=4999 554 -> 66 us; M=21 N=1000 245 -> 34 us.
 //
 // Scales: a mode's is the largest exponent of its elements, each less what its
-// configuration's weight is below the largest weight; a configuration's is the exponent
-// above its largest element in those units.  Both are powers of two and both operands of
-// stage B are without the configuration's: W's rows carry it instead.  So a configuration
-// that the weights take out, or nearly so, costs the others nothing, however far out it
-// lies, and loses itself at most as many bits as its weight is smaller (a scale of a
-// configuration is never further above 1 than that).  With the columns' maxima over all
-// configurations as the only scales one outlier of weight 0, 1e6 times the others, took 20
-// bits from all of them: errors of d2v of 2e-11 (and 2e-9 at 1e8).  The mean exponent of a
-// mode's elements as its scale leaves a mode of rounding noise over many decades, as
-// symmetry makes them, to set the scales of the configurations.
+// configuration's weight is below the largest weight (dg_weight_exp); a configuration's is
+// the exponent above its largest element in those units.  Both are powers of two, and stage
+// B's X is without the configuration's: W carries it instead.  So a configuration that the
+// weights take out, or nearly so, costs the others nothing, however far out it lies, and
+// loses itself at most as many bits as its weight is smaller (a configuration's scale is
+// never further above 1 than that).  With the columns' maxima over all configurations as the
+// only scales one outlier of weight 0, 1e6 times the others, took 20 bits from all of them:
+// errors of d2v of 2e-11 (and 2e-9 at 1e8).  The mean exponent of a mode's elements as its
+// scale leaves a mode of rounding noise over many decades, as symmetry makes them, to set
+// the scales of the configurations.
 //
 // Form of the contractions, with g = y / f_Y (= f_psi y) so that both operands
 // of the second stage come from x and g alone (u = f_Y x, y = f_Y g):
@@ -93,8 +97,7 @@ __global__ void __launch_bounds__(128) k_dg_colexp(const double *__restrict__ D,
         const long r = c0 + threadIdx.x;
         __syncthreads();
         if (r < r1) {
-            const double w = rho[rho_div == 1 ? r : r / rho_div];
-            less[threadIdx.x] = w != 0 ? min(0, exp_above(w) - rtop) : INT_MIN / 2;
+            less[threadIdx.x] = dg_weight_exp(rho[rho_div == 1 ? r : r / rho_div], rtop);
         }
         __syncthreads();
 #pragma unroll 8
@@ -513,7 +516,7 @@ __global__ void __launch_bounds__(256) k_dg_wbuild(
 // their own with the rows that the blocks blockIdx.y == modes / 32 build in wf: digits
 // of the weights of x (rows 0 .. 63: images) and of g (rows 64 .. 127); as two float64
 // products an element they were half of this kernel's work.  M=189, N=10000, 48 images:
-// 781 us with the forces and every image its own pass over x and g, 376 so.
+// 781 us with the forces and every image its own pass over x and g, 364 so.
 constexpr int kWImages = 8;
 __global__ void __launch_bounds__(256) k_dg_wimages(
     const double *__restrict__ dt, const double *__restrict__ gt,

@@ -25,6 +25,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
+#include <cstring>
 #include <vector>
 
 #include "digits.cuh"
@@ -46,6 +47,7 @@ struct QDigitStore {
     int *failed = nullptr;        // whether a bounded wait gave up in this call
     int *err = nullptr;           // its code, until it has been reported (pinned host memory)
     int2 *erb = nullptr;          // a row's scales in y and in u, [q][Rp]
+    int *rowfar = nullptr, anyfar = 0;
     double *rowc = nullptr;       // 8 doubles a row
     // per perturbation
     uint32_t abytes = 0;          // of a digit of a W block: rows up to a multiple of eight
@@ -91,13 +93,7 @@ __global__ void __launch_bounds__(256) k_qd_cols(const double *__restrict__ Xr,
     }
 }
 
-// What a configuration's element counts for in the scale of its column: its exponent, less
-// what its weight is below the largest one (exponent rtop); INT_MIN of nothing.
-__device__ __forceinline__ int dg_weighted_exp(double x, double rho, int rtop) {
-    return x != 0 && rho != 0 ? exp_above(x) + min(0, exp_above(rho) - rtop) : INT_MIN;
-}
-
-// Scales of the columns, their largest weighted exponents (dg_weighted_exp): of x in ec, of y
+// Scales of the columns, their largest weighted exponents (dg_weight_exp): of x in ec, of y
 // and u as the tiles [y | u] have them in ecb.  A column without an element (the imaginary
 // parts at Gamma, masked modes) has kZeroExp, which leaves it out of the rows' scales of A_q
 // and of W's bounds.
@@ -113,10 +109,11 @@ __global__ void __launch_bounds__(128) k_qd_colscale(const double *__restrict__ 
     for (long rt = 0; rt < nrt; ++rt) {
         const long o = (((long)q * nrt + rt) * nr + c) * 128 + threadIdx.x, r = rt * 128 + threadIdx.x;
         if (r >= R) break;
-        const double w = rho[(unsigned)r / (unsigned)S];
-        e[0] = max(e[0], dg_weighted_exp(x[o], w, rtop));
-        e[1] = max(e[1], dg_weighted_exp(y[o], w, rtop));
-        e[2] = max(e[2], dg_weighted_exp(u[o], w, rtop));
+        const int less = dg_weight_exp(rho[(unsigned)r / (unsigned)S], rtop);
+        const double v[3] = {x[o], y[o], u[o]};
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+            if (v[k] != 0) e[k] = max(e[k], exp_above(v[k]) + less);
     }
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -127,16 +124,17 @@ __global__ void __launch_bounds__(128) k_qd_colscale(const double *__restrict__ 
     if (threadIdx.x >= 3) return;
     const int k = threadIdx.x;
     int top = max(max(sh[0][k], sh[1][k]), max(sh[2][k], sh[3][k]));
-    if (top == INT_MIN) top = kZeroExp;
+    if (top < INT_MIN / 4) top = kZeroExp;
     if (k == 0) ec[q / G * 64 + q % G * nr + c] = top;
     else ecb[(long)q * nbq * kGN + (k == 1 ? c : nbq == 1 ? nr + c : kGN + c)] = top;
 }
 
-// erb[q][r]: exponents above the largest |y| 2^-ecb and |u| 2^-ecb of a row
+// erb[q][r]: exponents above |y| 2^-ecb and |u| 2^-ecb of a row; rowfar[r]: one is above 0
 __global__ void __launch_bounds__(128) k_qd_rowscale(const double *__restrict__ y,
                                                      const double *__restrict__ u,
                                                      const int *__restrict__ ecb, int nr, int nbq,
-                                                     int2 *__restrict__ erb) {
+                                                     int2 *__restrict__ erb, int *__restrict__ rowfar,
+                                                     int *__restrict__ anyfar) {
     const int q = blockIdx.y, *e = ecb + (long)q * nbq * kGN;
     const long t = (long)q * gridDim.x + blockIdx.x;
     int ey = INT_MIN, eu = INT_MIN;
@@ -146,7 +144,13 @@ __global__ void __launch_bounds__(128) k_qd_rowscale(const double *__restrict__ 
         if (a != 0) ey = max(ey, exp_above(a) - e[c]);
         if (b != 0) eu = max(eu, exp_above(b) - e[nbq == 1 ? nr + c : kGN + c]);
     }
-    erb[t * 128 + threadIdx.x] = make_int2(ey == INT_MIN ? kZeroExp : ey, eu == INT_MIN ? kZeroExp : eu);
+    // An ordinary row stays at the columns' scales: with its own, up to 2^3 larger, its first
+    // digits would be, and accumulations shorter (4x4x2 grid, 5 bands, N=5000 140 us a call
+    // with them, 132 so).
+    auto scale = [](int e) { return e == INT_MIN ? kZeroExp : e <= 0 && e >= -3 ? 0 : e; };
+    const int2 e2 = make_int2(scale(ey), scale(eu));
+    erb[t * 128 + threadIdx.x] = e2;
+    if (max(e2.x, e2.y) > 0) rowfar[blockIdx.x * 128L + threadIdx.x] = *anyfar = 1;
 }
 
 // er[group][r]: exponent above the largest |x| 2^-ec of a row
@@ -289,9 +293,10 @@ __global__ void __launch_bounds__(32) k_qd_alpha(const QAlpha src, const int *__
         for (int d = 0; d < kCall; ++d)
             *reinterpret_cast<uint4 *>(out + d * kGB + sw_place(row, lane)) = w[d];
     }
-    if (blockIdx.x == 0 && blockIdx.y == 0 && lane == 31) *failed = 0;
+    if (blockIdx.x == 0 && blockIdx.y == 0 && lane >= 30) wtop[lane - 30] = INT_MIN;
+    if (blockIdx.x == 0 && blockIdx.y == 0 && lane == 29) *failed = 0;
     // (there are no more pairs than q-points)
-    if (blockIdx.x == 0 && (int)blockIdx.y < src.n_pairs && lane < 3) wtop[4 * blockIdx.y + lane] = INT_MIN;
+    if (blockIdx.x == 0 && (int)blockIdx.y < src.n_pairs && lane < 3) wtop[4 + 4 * blockIdx.y + lane] = INT_MIN;
     if (lane == 0) {
         et[grp * 64 + row] = e;
         cofs[grp * 64 + row] =
@@ -301,9 +306,13 @@ __global__ void __launch_bounds__(32) k_qd_alpha(const QAlpha src, const int *__
 
 // Row weights (k_q_rows of qspace.cu): 64 rows a block, four threads a row, each a
 // quarter of the sums (with one thread a row its loads took 13 us at 2000 rows).
-// Rows past the end get zeros.  wtop, of each pair (q1, q2): the largest exponents of
-// w_cross with its row's scales in u of q1 and y of q2, of w_cross with those in y of q1
-// and u of q2, and of w_diag with those in u of both; kBadExp of one that is not finite.
+// Rows past the end get zeros.  wtop: the largest exponents of w_cross and w_diag over the
+// rows whose own scales are at most 1 everywhere; and of each pair (q1, q2), from 4 + 4 pair
+// on, over the others (rowfar), of w_cross with the row's scales in u of q1 and y of q2, of
+// w_cross with those in y of q1 and u of q2, and of w_diag with those in u of both.  An
+// ensemble without such rows takes the form without (kFar; with it 2 to 4 us of 85 with 36
+// pairs).  kBadExp of one that is not finite.
+template <bool kFar>
 __global__ void __launch_bounds__(256) k_qd_rows(const double *__restrict__ qp, int ngrp,
                                                  const double *__restrict__ u,
                                                  const double *__restrict__ y,
@@ -311,11 +320,12 @@ __global__ void __launch_bounds__(256) k_qd_rows(const double *__restrict__ qp, 
                                                  const double *__restrict__ rho, int S, long R,
                                                  long nrt, int nb, int iq_pert, int apply_d4,
                                                  const int2 *__restrict__ erb,
+                                                 const int *__restrict__ rowfar,
                                                  const int *__restrict__ pair_q, int n_pairs,
                                                  double2 *__restrict__ rowc,
                                                  int *__restrict__ wtop) {
     __shared__ double sum[8][4][64];
-    __shared__ int we[2][64];      // exponents of w_cross, w_diag
+    __shared__ int we[2][kFar ? 64 : 1];      // exponents of w_cross, w_diag of the rows far out
     const int part = threadIdx.x >> 6, i = threadIdx.x & 63;
     const long r = blockIdx.x * 64L + i;
     pdl_enter();
@@ -341,7 +351,9 @@ __global__ void __launch_bounds__(256) k_qd_rows(const double *__restrict__ qp, 
 #pragma unroll
     for (int k = 0; k < 8; ++k) sum[k][part][i] = s[k];
     __syncthreads();
+    if (!kFar && threadIdx.x >= 64) return;
     if (threadIdx.x < 64) {
+        const int far = kFar ? rowfar[r] : 0;
         double2 w[4] = {};
         if (r < R) {
 #pragma unroll
@@ -361,10 +373,14 @@ __global__ void __launch_bounds__(256) k_qd_rows(const double *__restrict__ qp, 
             const unsigned long long a =
                 max((unsigned long long)__double_as_longlong(w[2 + k].x) & 0x7fffffffffffffffULL,
                     (unsigned long long)__double_as_longlong(w[2 + k].y) & 0x7fffffffffffffffULL);
-            we[k][i] = a >= 0x7ff0000000000000ULL ? kBadExp
-                       : a ? exp_above(__longlong_as_double((long long)a)) : INT_MIN;
+            const int e = a >= 0x7ff0000000000000ULL ? kBadExp
+                          : a ? exp_above(__longlong_as_double((long long)a)) : INT_MIN;
+            if (kFar) we[k][i] = far ? e : INT_MIN;
+            const int m = __reduce_max_sync(0xffffffffu, far ? INT_MIN : e);
+            if ((threadIdx.x & 31) == 0) atomicMax(wtop + k, m);
         }
     }
+    if (!kFar) return;
     __syncthreads();
     const int lane = threadIdx.x & 31;
     for (int p = threadIdx.x >> 5; p < n_pairs; p += 8) {
@@ -383,7 +399,7 @@ __global__ void __launch_bounds__(256) k_qd_rows(const double *__restrict__ qp, 
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
             const int e = __reduce_max_sync(0xffffffffu, top[k]);
-            if (lane == k) atomicMax(wtop + 4 * p + k, e);
+            if (lane == k) atomicMax(wtop + 4 + 4 * p + k, e);
         }
     }
 }
@@ -391,7 +407,8 @@ __global__ void __launch_bounds__(256) k_qd_rows(const double *__restrict__ qp, 
 // Digits of the rows [A1 | A2] of pair blockIdx.y over a group of K blocks: thread =
 // (band, eight rows), which makes four rows of digits; with few bands several K blocks
 // side by side.  The scales are bounds from those of the weights and of the columns; a
-// row's own scale goes into the shift that cuts the digits.  blockIdx.y == n_pairs: the partial f of the group's rows.
+// row's own scale goes into the shift that cuts the digits.  blockIdx.y == n_pairs: the
+// partial f of the group's rows.
 __global__ void __launch_bounds__(128) k_qd_wbuild(
     const double *__restrict__ u, const double *__restrict__ y, const double2 *__restrict__ rowc,
     const int *__restrict__ wtop, const int *__restrict__ ecb, const int2 *__restrict__ erb,
@@ -403,8 +420,10 @@ __global__ void __launch_bounds__(128) k_qd_wbuild(
     const int wide = max(1, 16 / nb);            // K blocks side by side
     const long kb0 = blockIdx.x * (long)per, kb1 = min(nkb, kb0 + per);
     const bool force = p == n_pairs;
-    pdl_enter();
+    // (what does not change between calls is read ahead)
     const int q1 = force ? iq_pert : pair_q[2 * p];
+    const int2 *es2 = erb + (force ? 0 : pair_q[2 * p + 1]) * nrt * 128;
+    pdl_enter();
     if (force) {
         for (int n0 = 0; n0 < nb; n0 += 16) {
             const int n = n0 + (nb < 16 ? m % nb : m);
@@ -441,8 +460,8 @@ __global__ void __launch_bounds__(128) k_qd_wbuild(
         }
         return;
     }
-    const int *wt = wtop + 4 * p;
-    const int2 *es2 = erb + pair_q[2 * p + 1] * nrt * 128;
+    const int *wt = wtop + 4 + 4 * p;
+    const int w0 = max(wtop[0], wt[0]), w1 = max(wtop[0], wt[1]), w2 = max(wtop[1], wt[2]);
     uint8_t *out = reinterpret_cast<uint8_t *>(wa) + p * nkb * kCall * (long)abytes;
     for (int n0 = 0; n0 < nb; n0 += 16) {
         const int n = n0 + (nb < 16 ? m % nb : m);
@@ -451,8 +470,8 @@ __global__ void __launch_bounds__(128) k_qd_wbuild(
         const int ym = max(ey[0], ey[1]), um = max(eu[0], eu[1]);
         // real and imaginary part: two products each, and two of them in A2
         auto bound = [](int a, int e) { return a == INT_MIN ? INT_MIN : a + e; };
-        const int b1 = bound(wt[0], um), b2 = max(bound(wt[1], ym), bound(wt[2], um));
-        const bool bad1 = wt[0] == kBadExp, bad2 = wt[1] == kBadExp || wt[2] == kBadExp;
+        const int b1 = bound(w0, um), b2 = max(bound(w1, ym), bound(w2, um));
+        const bool bad1 = w0 == kBadExp, bad2 = w1 == kBadExp || w2 == kBadExp;
         const int e1 = bad1 ? kBadExp : b1 == INT_MIN ? 0 : b1 + 1;
         const int e2 = bad2 ? kBadExp : b2 == INT_MIN ? 0 : b2 + 2;
         if (blockIdx.x == 0 && c == 0) {
@@ -469,19 +488,20 @@ __global__ void __launch_bounds__(128) k_qd_wbuild(
 #pragma unroll
             for (int k = 0; k < 8; k += 2) {
                 const double2 vur = ur[k / 2], vui = ur[64 + k / 2], vyr = yr[k / 2], vyi = yr[64 + k / 2];
+                const int4 es = *reinterpret_cast<const int4 *>(es2 + r0 + k);    // of two rows
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const double pu = h ? vur.y : vur.x, pv = h ? vui.y : vui.x;
                     const double py = h ? vyr.y : vyr.x, pz = h ? vyi.y : vyi.x;
                     const double2 wc = rowc[4 * (r0 + k + h) + 2], wd = rowc[4 * (r0 + k + h) + 3];
-                    const int2 es = es2[r0 + k + h];
+                    const int sy = h ? es.z : es.x, su = h ? es.w : es.y;
                     const double xr = fma(wc.y, pv, -wc.x * pu), xi = fma(-wc.x, pv, -wc.y * pu);
                     const double zr = fma(wd.y, pv, fma(-wd.x, pu, fma(wc.y, pz, -wc.x * py)));
                     const double zi = fma(-wd.x, pv, fma(-wd.y, pu, fma(-wc.x, pz, -wc.y * py)));
-                    a1r[k + h] = bad1 ? 0 : fixed_point(xr, 62 - e1 + es.x);
-                    a1i[k + h] = bad1 ? 0 : fixed_point(xi, 62 - e1 + es.x);
-                    a2r[k + h] = bad2 ? 0 : fixed_point(zr, 62 - e2 + es.y);
-                    a2i[k + h] = bad2 ? 0 : fixed_point(zi, 62 - e2 + es.y);
+                    a1r[k + h] = bad1 ? 0 : fixed_point(xr, 62 - e1 + sy);
+                    a1i[k + h] = bad1 ? 0 : fixed_point(xi, 62 - e1 + sy);
+                    a2r[k + h] = bad2 ? 0 : fixed_point(zr, 62 - e2 + su);
+                    a2i[k + h] = bad2 ? 0 : fixed_point(zi, 62 - e2 + su);
                 }
             }
             uint8_t *blk = out + kb * kCall * (long)abytes;
@@ -602,14 +622,15 @@ static int qdigits_prepare(tdscha_qctx *c) {
         {(void **)&x->er, sizeof(int) * x->ngrp * x->Rp},
         {(void **)&nrm, sizeof(float) * kRes * (size_t)n_q * x->nbq * kGN * x->nkb},
         {(void **)&x->erb, sizeof(int2) * rows},
-        {(void **)&x->wtop, sizeof(int) * 4 * n_q},
-        // zero from the start: exponents of padding columns, rows of padding bands
+        {(void **)&x->wtop, sizeof(int) * 4 * (n_q + 1)},
+        // zero from the start: flags, exponents of padding columns, rows of padding bands
+        {(void **)&x->rowfar, sizeof(int) * x->Rp},
         {(void **)&x->ec, sizeof(int) * x->ngrp * 64},
         {(void **)&x->ecb, sizeof(int) * (size_t)n_q * x->nbq * kGN},
         {(void **)&x->et, sizeof(int) * x->ngrp * 64},
         {(void **)&x->cofs, sizeof(int) * x->ngrp * 64},
         {(void **)&x->failed, sizeof(int)},
-        {(void **)&fl, sizeof(float) * kFlushes * kRes},
+        {(void **)&fl, sizeof(float) * (kFlushes * kRes + 1)},
         {(void **)&x->yb, (size_t)x->ngrp * kCall * kGB},
     };
     const size_t total = place(parts, nullptr);
@@ -622,7 +643,7 @@ static int qdigits_prepare(tdscha_qctx *c) {
     TDS_CUDA(cudaMallocHost((void **)&x->err, sizeof(int)));
     *x->err = 0;
     place(parts, x->slab);
-    uint8_t *z = reinterpret_cast<uint8_t *>(x->ec);
+    uint8_t *z = reinterpret_cast<uint8_t *>(x->rowfar);
     TDS_CUDA(cudaMemsetAsync(z, 0, (uint8_t *)x->slab + total - z, 0));
     const dim3 gt((unsigned)x->nrt, n_q);
     k_qd_cols<<<gt, 256>>>((const double *)c->Xr, (const double *)c->Yr, c->fY, c->fpsi, c->L, nb,
@@ -631,7 +652,8 @@ static int qdigits_prepare(tdscha_qctx *c) {
     k_qd_colscale<<<dim3(nr, n_q), 128>>>(x->x, x->y, x->u, c->rho, c->S, c->rho_top, c->R, x->nrt, nr,
                                           x->nbq, x->G, x->ec, x->ecb);
     TDS_CHECK_LAUNCH();
-    k_qd_rowscale<<<gt, 128>>>(x->y, x->u, x->ecb, nr, x->nbq, x->erb);
+    k_qd_rowscale<<<gt, 128>>>(x->y, x->u, x->ecb, nr, x->nbq, x->erb, x->rowfar,
+                               reinterpret_cast<int *>(fl) + kFlushes * kRes);
     TDS_CHECK_LAUNCH();
     const dim3 gg((unsigned)x->nrt, x->ngrp);
     k_qd_rowexp<<<gg, 128>>>(x->x, x->ec, nr, x->G, n_q, x->er);
@@ -642,9 +664,10 @@ static int qdigits_prepare(tdscha_qctx *c) {
                                                            x->nrt, x->nkb, x->xb, nrm);
     TDS_CHECK_LAUNCH();
     TDS_CUDA(dg_windows(nrm, n_q * x->nbq, kGN, (int)x->nkb, fl, 0));
-    float h_fl[kFlushes * kRes];
+    float h_fl[kFlushes * kRes + 1];
     TDS_CUDA(cudaMemcpy(h_fl, fl, sizeof(h_fl), cudaMemcpyDeviceToHost));
     x->flush = digits_flush(h_fl);
+    std::memcpy(&x->anyfar, h_fl + kFlushes * kRes, sizeof(int));
     TDS_CUDA((dg_setup<DG_QDOTS, true>()));
     TDS_CUDA((dg_setup<DG_PARTS, true>()));
     return TDSCHA_OK;
@@ -743,10 +766,10 @@ int qdigits_perturb(tdscha_qctx *c, int apply_d4, const double *psi, cudaStream_
     a.R = c->R;
     a.M = live;
     TDS_CUDA((dg_launch<DG_QDOTS, true>(a, x->nsm, st)));
-    TDS_CUDA(launch_pdl(k_qd_rows, (unsigned)x->nkb, 256, 0, st, (const double *)x->qp, x->ngrp,
+    TDS_CUDA(launch_pdl(x->anyfar ? k_qd_rows<true> : k_qd_rows<false>, (unsigned)x->nkb, 256, 0, st, (const double *)x->qp, x->ngrp,
                         (const double *)x->u, (const double *)x->y, R1, (const double *)c->rho, c->S,
                         c->R, x->nrt, nb, c->iq_pert, apply_d4, (const int2 *)x->erb,
-                        (const int *)c->pair_q, x->n_pairs, rowc, x->wtop));
+                        (const int *)x->rowfar, (const int *)c->pair_q, x->n_pairs, rowc, x->wtop));
     TDS_CUDA(launch_pdl(k_qd_wbuild, dim3(x->nfc, x->n_pairs + 1), 128, 0, st, (const double *)x->u,
                         (const double *)x->y, (const double2 *)rowc,
                         (const int *)x->wtop, (const int *)x->ecb, (const int2 *)x->erb,
