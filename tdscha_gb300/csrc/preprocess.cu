@@ -124,53 +124,93 @@ __global__ void k_prologue(const double *__restrict__ a, long n, int K, int widt
     }
 }
 
-// Scales of the columns of a'.  A row's scale is the exponent above its largest
-// |a'| 2^-ec, so any ec keeps the digits in range; what counts is that it makes the columns
-// alike.  Every row is a result of its own here, so ec is the mean over blocks of rows of the
-// largest exponent of a block: an outlier moves it by its block's share only, and a column
-// of rounding noise over many decades counts by its largest elements.
-//
-// stat[k], stat[K + k]: sum over the blocks of `per` rows of the largest exponent of
-// a s - sub (or of a, without sub) in column k, and the number of blocks that have one
-__global__ void __launch_bounds__(128) k_dg_colstat(const double *__restrict__ a, long rows, int K, long per,
-                                                    double s, const double *__restrict__ sub,
-                                                    unsigned long long *__restrict__ stat) {
-    const int k = blockIdx.x * 128 + threadIdx.x;
-    if (k >= K) return;
-    const long r0 = blockIdx.y * per, r1 = min(rows, r0 + per);
-    const double m = sub ? -sub[k] : 0.0;
-    int e = INT_MIN;
-#pragma unroll 8
-    for (long r = r0; r < r1; ++r) {
-        double v = a[r * K + k];
+// Scales of the columns of a' = (a s - sub) mul, taken into mul2 = mul 2^-ec.  A row's scale
+// is the exponent above its largest |a'| 2^-ec, so any ec keeps the digits in range; what
+// counts is that it makes the columns alike.  Every row is a result of its own here, so ec is
+// the mean of the largest exponents of 16 groups of up to 32 rows spread over all: an outlier
+// moves it by its group's share only, and a column of rounding noise over many decades counts
+// by its largest elements.  Columns without an element in these rows are searched through;
+// one without any gets kZeroExp, which leaves it out of B's scales.
+// Block: 8 columns, 128 rows at a time: a warp's float64 operation takes 64 cycles, so the
+// 512 rows are spread over many warps of many blocks.
+__global__ void __launch_bounds__(1024) k_dg_colscale(const double *__restrict__ a, long rows, int K,
+                                                      double s, const double *__restrict__ sub,
+                                                      const double *__restrict__ mul,
+                                                      double *__restrict__ mul2, int *__restrict__ ec) {
+    pdl_enter();
+    __shared__ int sh[32][8];
+    const int cc = threadIdx.x & 7, slot = threadIdx.x >> 3, warp = threadIdx.x >> 5,
+              k = blockIdx.x * 8 + cc;
+    const bool in = k < K;
+    const double m = in && sub ? -sub[k] : 0.0;
+    auto exponent = [&](double v) {
         if (sub) v = fma(v, s, m);
-        if (v != 0 && isfinite(v)) e = max(e, exp_above(v));
+        return v != 0 && isfinite(v) ? exp_above(v) : INT_MIN;
+    };
+    // over the 32 threads of a warp that have a column in common
+    auto warp_max = [](int e) {
+        e = max(e, __shfl_xor_sync(0xffffffffu, e, 8));
+        return max(e, __shfl_xor_sync(0xffffffffu, e, 16));
+    };
+    const int group = slot >> 3;                  // two warps
+    const long r0 = rows * group / 16, r1 = min(r0 + 32, rows * (group + 1) / 16);
+    int e = INT_MIN;
+    double v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const long r = r0 + (slot & 7) + 8 * i;
+        // (NaN counts as nothing, also with a mean taken off)
+        v[i] = in && r < r1 ? a[r * K + k] : __longlong_as_double(0x7ff8000000000000LL);
     }
-    if (e == INT_MIN) return;
-    atomicAdd(stat + k, (unsigned long long)(long long)e);
-    atomicAdd(stat + K + k, 1ULL);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) e = max(e, exponent(v[i]));
+    e = warp_max(e);
+    if ((threadIdx.x & 31) < 8) sh[warp][cc] = e;
+    __syncthreads();
+    int sum = 0, n = 0;
+    for (int q = 0; q < 32; q += 2) {
+        e = max(sh[q][cc], sh[q + 1][cc]);
+        if (e != INT_MIN) {
+            sum += e;
+            ++n;
+        }
+    }
+    if (__syncthreads_or(in && n == 0 && rows > 512)) {
+        e = INT_MIN;
+        if (in)
+#pragma unroll 8
+            for (long r = slot; r < rows; r += 128) e = max(e, exponent(a[r * K + k]));
+        e = warp_max(e);
+        if ((threadIdx.x & 31) < 8) sh[warp][cc] = e;
+        __syncthreads();
+        if (n == 0) {
+            for (int q = 0; q < 32; ++q) e = max(e, sh[q][cc]);
+            if (e != INT_MIN) {
+                sum = e;
+                n = 1;
+            }
+        }
+    }
+    if (!in || slot) return;
+    const double f = mul[k];
+    int out = kZeroExp;
+    if (n) {
+        // (rounded, ties upwards; with a mean taken off, s is in what was looked at.  Within
+        // what mul2 can hold.)
+        const int t = 2 * sum + n, ef = exp_above(f);
+        out = (t - (t < 0 ? 2 * n - 1 : 0)) / (2 * n) + ef - 1 + (sub ? 0 : exp_above(s) - 1);
+        out = min(max(out, ef - 1000), ef + 1000);
+    }
+    ec[k] = out;
+    mul2[k] = n ? ldexp(f, -out) : 0.0;
 }
 
-// ec[k]: the mean, and the exponents of mul[k] and of s where they multiply what was
-// counted; kZeroExp of a column without an element, which leaves it out of B's scales
-__global__ void k_dg_colscale(const unsigned long long *__restrict__ stat, int K, double s,
-                              const double *__restrict__ mul, int *__restrict__ ec) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= K) return;
-    const long long n = (long long)stat[K + k], t = 2 * (long long)stat[k] + n;
-    // rounded, ties upwards
-    ec[k] = n == 0 ? kZeroExp : (int)((t - (t < 0 ? 2 * n - 1 : 0)) / (2 * n)) + exp_above(mul[k]) + exp_above(s) - 2;
-}
-
-// Digits of the rows a' of k_prologue (real data), one warp per row, and the exponent
-// above each row's largest |a'| 2^-ec.  Rows past n (of the last tile) are zero.
-__global__ void __launch_bounds__(256) k_dg_slice_rows(const double *__restrict__ a, long n, int K,
-                                                       int nkb, double s,
-                                                       const double *__restrict__ sub,
-                                                       const double *__restrict__ mul,
-                                                       const int *__restrict__ ec,
-                                                       __half *__restrict__ out,
-                                                       int *__restrict__ er) {
+// Digits of the rows a' 2^-ec of k_prologue (real data), one warp per row, and the
+// exponent above each row's maximum.  Rows past n (of the last tile) are zero.
+__device__ __forceinline__ void dg_slice_rows(const double *__restrict__ a, long n, int K, int nkb, double s,
+                                              const double *__restrict__ sub,
+                                              const double *__restrict__ mul, __half *__restrict__ out,
+                                              int *__restrict__ er) {
     const long r = blockIdx.x * 8L + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     const double *p = a + r * K;
@@ -183,7 +223,7 @@ __global__ void __launch_bounds__(256) k_dg_slice_rows(const double *__restrict_
     if (r < n)
         for (int k = lane; k < K; k += 32) {
             const double v = value(k);
-            if (v != 0) e = max(e, isfinite(v) ? exp_above(v) - ec[k] : kBadExp);
+            if (v != 0) e = max(e, isfinite(v) ? exp_above(v) : kBadExp);
         }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, o));
@@ -197,7 +237,7 @@ __global__ void __launch_bounds__(256) k_dg_slice_rows(const double *__restrict_
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             const int m = ch * 8 + k;
-            q[k] = m < K && !bad ? fixed_point(value(m), 55 - ec[m] - e) : 0;
+            q[k] = m < K && !bad ? fixed_point(value(m), 55 - e) : 0;
         }
         uint4 w[kRes];
         digits8<kRes>(q, w);
@@ -208,14 +248,11 @@ __global__ void __launch_bounds__(256) k_dg_slice_rows(const double *__restrict_
     }
 }
 
-// Digits of the columns of b 2^ec (K x n): block = column (up to a multiple of 64, the
-// padding zero)
-__global__ void __launch_bounds__(128) k_dg_slice_cols(const double *__restrict__ b,
-                                                       const int *__restrict__ ec, int K, int n,
-                                                       int nkb, __half *__restrict__ out,
-                                                       int *__restrict__ et) {
-    __shared__ int sh[4];
-    const int c = blockIdx.x;
+// Digits of column c of b 2^ec (K x n), or of a column of padding, by a block
+__device__ __forceinline__ void dg_slice_col(int c, const double *__restrict__ b,
+                                             const int *__restrict__ ec, int K, int n, int nkb,
+                                             __half *__restrict__ out, int *__restrict__ et) {
+    __shared__ int sh[8];
     int e = INT_MIN;
     if (c < n)
         for (int k = threadIdx.x; k < K; k += blockDim.x) {
@@ -226,7 +263,8 @@ __global__ void __launch_bounds__(128) k_dg_slice_cols(const double *__restrict_
     for (int o = 16; o > 0; o >>= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, o));
     if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = e;
     __syncthreads();
-    e = max(max(sh[0], sh[1]), max(sh[2], sh[3]));
+#pragma unroll
+    for (int k = 0; k < 8; ++k) e = max(e, sh[k]);
     if (e == INT_MIN) e = 0;
     const bool bad = e >= kBadExp / 2 || c >= n;
     if (threadIdx.x == 0) et[c] = e;
@@ -247,6 +285,22 @@ __global__ void __launch_bounds__(128) k_dg_slice_cols(const double *__restrict_
     }
 }
 
+// Both in one launch: eight rows a block, then the columns (up to a multiple of 64, or none)
+__global__ void __launch_bounds__(256) k_dg_slice(const double *__restrict__ a, long rows, int row_blocks,
+                                                  int K, int nkb, double s,
+                                                  const double *__restrict__ sub,
+                                                  const double *__restrict__ mul,
+                                                  __half *__restrict__ outa, int *__restrict__ er,
+                                                  const double *__restrict__ b,
+                                                  const int *__restrict__ ec, int n,
+                                                  __half *__restrict__ outb, int *__restrict__ et) {
+    pdl_enter();
+    if ((int)blockIdx.x < row_blocks)
+        dg_slice_rows(a, rows, K, nkb, s, sub, mul, outa, er);
+    else
+        dg_slice_col(blockIdx.x - row_blocks, b, ec, K, n, nkb, outb, et);
+}
+
 // C (rows x n) = A' B by digit products: A' the rows of k_prologue, B K x n.  The
 // digits of 2^16 rows at a time (14 bytes an element) beside those of B.  The columns of A'
 // (coordinates) have scales of their own, which B's rows carry: atoms of unequal mass have
@@ -255,7 +309,7 @@ struct DigitProduct {
     void *slab = nullptr;
     __half *a = nullptr, *b = nullptr;
     int *er = nullptr, *et = nullptr, *ec = nullptr, *err = nullptr;
-    unsigned long long *stat = nullptr;
+    double *mul2 = nullptr;
     int K = 0, n = 0, nkb = 0, nbt = 0, nsm = 1;
     long chunk = 0;
     long long budget = kDefaultBudget;
@@ -277,8 +331,8 @@ struct DigitProduct {
         auto pad = [](size_t x) { return (x + 1023) & ~size_t(1023); };
         const size_t ba = (size_t)chunk * nkb * kGK * 2 * kRes, bb = (size_t)nbt * nkb * kCall * kGB,
                      be = pad(sizeof(int) * chunk), bt = pad(sizeof(int) * nbt * kGN),
-                     bs = pad(sizeof(*stat) * 2 * K), bc = pad(sizeof(int) * K);
-        if (cached_malloc(&slab, ba + bb + be + bt + bs + bc + 1024) != cudaSuccess) {
+                     bc = pad(sizeof(int) * K), bm = pad(sizeof(double) * K);
+        if (cached_malloc(&slab, ba + bb + be + bt + bc + bm + 1024) != cudaSuccess) {
             cudaGetLastError();
             slab = nullptr;
             return false;
@@ -288,9 +342,9 @@ struct DigitProduct {
         b = reinterpret_cast<__half *>(p + ba);
         er = reinterpret_cast<int *>(p + ba + bb);
         et = reinterpret_cast<int *>(p + ba + bb + be);
-        stat = reinterpret_cast<unsigned long long *>(p + ba + bb + be + bt);
-        ec = reinterpret_cast<int *>(p + ba + bb + be + bt + bs);
-        err = reinterpret_cast<int *>(p + ba + bb + be + bt + bs + bc);
+        ec = reinterpret_cast<int *>(p + ba + bb + be + bt);
+        mul2 = reinterpret_cast<double *>(p + ba + bb + be + bt + bc);
+        err = reinterpret_cast<int *>(p + ba + bb + be + bt + bc + bm);
         return true;
     }
 
@@ -302,22 +356,13 @@ struct DigitProduct {
 
     int product(const double *A, long rows, double s, const double *sub, const double *mul,
                 const double *B, double *C) {
-        // rows a block walks one after the other: 64, fewer where there would be less than
-        // 64 blocks, more where the grid would not hold them
-        const long per = std::max(std::min<long>(64, std::max<long>(4, rows / 64)), (rows + 65534) / 65535);
-        TDS_CUDA(cudaMemsetAsync(stat, 0, sizeof(*stat) * 2 * K, 0));
-        k_dg_colstat<<<dim3(ceil_div(K, 128), ceil_div(rows, per)), 128>>>(A, rows, K, per, s, sub, stat);
-        TDS_CHECK_LAUNCH();
-        // (with a mean taken off, s is in what was counted)
-        k_dg_colscale<<<ceil_div(K, 128), 128>>>(stat, K, sub ? 1.0 : s, mul, ec);
-        TDS_CHECK_LAUNCH();
-        k_dg_slice_cols<<<nbt * kGN, 128>>>(B, ec, K, n, nkb, b, et);
-        TDS_CHECK_LAUNCH();
+        const cudaStream_t st = 0;
+        TDS_CUDA(launch_pdl(k_dg_colscale, ceil_div(K, 8), 1024, 0, st, A, rows, K, s, sub, mul, mul2, ec));
         for (long r0 = 0; r0 < rows; r0 += chunk) {
             const long nr = std::min(chunk, rows - r0), nrp = (nr + kGM - 1) / kGM * kGM;
-            k_dg_slice_rows<<<(unsigned)(nrp / 8), 256>>>(A + r0 * K, nr, K, nkb, s, sub, mul, ec, a,
-                                                                er);
-            TDS_CHECK_LAUNCH();
+            const int rb = (int)(nrp / 8);
+            TDS_CUDA(launch_pdl(k_dg_slice, rb + (r0 ? 0 : nbt * kGN), 256, 0, st, A + r0 * K, nr, rb, K, nkb, s,
+                                sub, (const double *)mul2, a, er, B, (const int *)ec, n, b, et));
             DgArgs g{};
             g.a = a;
             g.b = b;
@@ -333,7 +378,7 @@ struct DigitProduct {
             g.R = nr;
             g.M = n;
             g.out = C + r0 * n;
-            TDS_CUDA((dg_launch<DG_STORE, false>(g, nsm, (cudaStream_t)0)));
+            TDS_CUDA((dg_launch<DG_STORE, false>(g, nsm, st)));
         }
         return TDSCHA_OK;
     }
