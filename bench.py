@@ -423,6 +423,8 @@ def run_ours(args):
         static = static_leg(lib, nat, ctx, M, S * N, dev,
                             lambda: nat.Context(ens["X"], ens["Y"], ens["w"], ens["rho"],
                                                 ens["T"], syms, spaces, bid, with_mixed=False))
+    # float64 stages as exact digit products: 35 of their products are one of the algorithm's
+    digits = prec_name == "fp64" and ctx.fp64_path() == "tensor cores"
     ctx.close()
     R = N * S
     flops_app = 4.0 * R * M * M          # two GEMM stages of 2 R M^2 each
@@ -433,10 +435,11 @@ def run_ours(args):
     pk_path = os.path.join(ROOT, "MEASURED_PEAKS.json")
     if os.path.exists(pk_path):
         peaks = json.load(open(pk_path))
-    # the mixed bi-Lanczos step runs L q and L^T p as one two-perturbation call
-    # (one launch of each GEMM stage for both); the profiled run made
+    # on the tensor cores a bi-Lanczos step runs L q and L^T p as one two-perturbation
+    # call (one launch of each GEMM stage for both); the profiled run made
     # 2 n_run applications
-    pair = prec_name == "mixed" and os.environ.get("TDSCHA_PAIR_APPLY", "1") != "0"
+    pair = ((prec_name == "mixed" or digits) and
+            os.environ.get("TDSCHA_PAIR_APPLY", "1") != "0")
     ppl = 2 if pair else 1                  # perturbations per GEMM-stage launch
     if kid is not None:
         tot_ms, cnt = kern[kid]
@@ -444,12 +447,14 @@ def run_ours(args):
         if kid in (0, 3):
             work = 2.0 * R * M * M * ppl     # flops per launch of one GEMM stage
             achieved = work / per_launch_s / 1e12
-            if prec_name == "fp64":
+            if prec_name == "fp64" and not digits:
                 peak, src = 1.25, "nominal GB300 FP64 1.25 TFLOP/s (not in MEASURED_PEAKS.json)"
             else:
                 peak = peaks.get("bf16_tflops", 1900.0)
                 src = "of measured bf16_tflops" if "bf16_tflops" in peaks else "of fallback"
-            roof = {"bound": "tensor" if prec_name == "mixed" else "fp64", "kernel": KERNEL_NAMES[kid],
+                if digits:
+                    peak, src = peak / 35, src + " / 35 digit products"
+            roof = {"bound": "tensor" if prec_name == "mixed" or digits else "fp64", "kernel": KERNEL_NAMES[kid],
                     "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                     "frac": achieved / peak, "traffic": None, "peak_source": src,
                     "avg_launch_ms": tot_ms / cnt}
@@ -879,14 +884,19 @@ def qspace_leg(qname, K, W, dev, peaks, with_cpu=True):
     # d2v two FMAs per block element per row
     flops = R * (8.0 * n_q * nb * nb + 16.0 * L) + R * n_pairs * nb * nb * 16.0
     achieved = flops / app_s / 1e12
+    bound, peak, src = "fp64", 1.25, "nominal GB300 FP64 (not in MEASURED_PEAKS.json)"
+    if ctx.fp64_path() == "tensor cores":
+        # exact digit products, 35 to one of the algorithm's (on tiles of 128 x 64, of
+        # which n_b x n_b blocks fill a part)
+        bound, peak = "tensor", peaks.get("bf16_tflops", 1900.0) / 35
+        src = ("of measured bf16_tflops" if "bf16_tflops" in peaks else "of fallback") + " / 35 digit products"
     out_d = {"workload": qname, "dims": list(spec["dims"]), "n_bands": nb, "N": N,
              "n_pairs": n_pairs, "psi_size": P,
              "lanczos_steps_per_s": steps_s,
              "lanczos": "Hermitian, Gram-Schmidt against all stored vectors (reference default)",
              "application_ms": app_s * 1e3,
-             "roofline": {"bound": "fp64", "achieved": achieved, "peak": 1.25, "unit": "TFLOP/s",
-                          "frac": achieved / 1.25,
-                          "peak_source": "nominal GB300 FP64 (not in MEASURED_PEAKS.json)",
+             "roofline": {"bound": bound, "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
+                          "frac": achieved / peak, "peak_source": src,
                           "flops_per_application": flops},
              "ensemble_bytes": 2 * e["X_q"].nbytes}
     # the same operator with fp32 averages on the CUDA cores (precision mixed)

@@ -34,8 +34,18 @@ extern "C" {
 #define TDSCHA_ERR_STATE (-4)    /* call not valid in the context's state       */
 #define TDSCHA_ERR_TIMEOUT (-5)  /* a bounded device wait gave up               */
 
-/* precision of the perturbation averages */
-#define TDSCHA_PREC_FP64 0       /* float64 on the CUDA cores                   */
+/* precision of the perturbation averages
+ *
+ * TDSCHA_PREC_FP64: float64 data and results.  The contractions run as exact digit
+ * products on the tensor cores (on the CUDA cores where tdscha_ctx_fp64_path says so):
+ * an element enters as a fixed-point number with 55 bits (ensemble) or 62 bits
+ * (perturbation, weighted configurations) under the largest one of its row, after
+ * power-of-two scales of the modes and of the configurations; the sums of the digits are
+ * exact and rounded once.  Over a whole array, or a row of it, errors are those of float64
+ * sums or smaller.  An element far below the others of its configuration in these units is
+ * held with fewer bits than float64 has, so that an entry to which only such elements
+ * contribute has that error relative to the larger entries beside it. */
+#define TDSCHA_PREC_FP64 0       /* float64                                     */
 #define TDSCHA_PREC_MIXED 1      /* two-limb fp16 operands, three tensor-core products per K step, fp32 accumulate */
 
 typedef struct tdscha_ctx tdscha_ctx;

@@ -435,8 +435,8 @@ __global__ void __launch_bounds__(128) k_dg_rows(const double *__restrict__ qp,
 // Exponent above |w| of a mode of an image, kBadExp where that is not finite: am, the
 // image's maxima of the rows' weights with their scales, times the scales of the mode in
 // g and x (an element is below its row's and its column's scale).  Whole numbers only: every
-// row of a W block asks for it, and four float64 operations each were 6 of the 250 us of
-// 24 vectors at M=60, N=5000.
+// row of a W block asks for it (24 vectors at M=60, N=5000: 248 us with four float64
+// operations each, 237 so).
 __device__ __forceinline__ int dg_wexp(const unsigned long long *__restrict__ am, int ex, int eg) {
     constexpr unsigned long long kInf = 0x7ff0000000000000ULL;
     const unsigned long long a = am[0], b = am[1];

@@ -20,8 +20,8 @@
 // elements; a configuration has one for y and one for u of each q-point, the exponent above its largest
 // element there.  The rows of [f2 | u2] are without it and those of A1 and A2 carry it.
 //
-// Measured (averages, one call): 4x4x4 grid, 12 bands, N=10000 2479 -> 530 us
-// (row dots 216, W 132, d2v 146 of them).
+// Measured (averages, one call): 4x4x4 grid, 12 bands, N=10000 2479 -> 526 us
+// (row dots 224, W 134, d2v 143 in a launch list).
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
