@@ -626,13 +626,13 @@ __global__ void __launch_bounds__(32 * kRows * kGroups) k_dg_final(
     const double *__restrict__ fpart, int nfc, const double *__restrict__ fY, double inv,
     const int *__restrict__ failed, double *__restrict__ f, double *__restrict__ d2v) {
     pdl_enter();
-    if (*failed) inv = __longlong_as_double(0x7ff8000000000000LL);
     gpart += blockIdx.y * (long)Mp * Mp;
     fpart += blockIdx.y * (long)nfc * M;
     f += blockIdx.y * (long)M;
     d2v += blockIdx.y * (long)M * M;
     constexpr int kSlabs = 32 / kRows;
     constexpr int kThreads = 32 * kRows;
+    const double kNaN = __longlong_as_double(0x7ff8000000000000LL);
     __shared__ double tr[kGroups][32][kRows + 1], red[kGroups][kRows][33];
     const int nt = (M + 31) / 32, slab = blockIdx.x % kSlabs;
     const int group = threadIdx.x / kThreads, t = threadIdx.x % kThreads;
@@ -659,7 +659,11 @@ __global__ void __launch_bounds__(32 * kRows * kGroups) k_dg_final(
     if (group == 0 && in) {
         for (int k = 1; k < kGroups; ++k) h += red[k][ty][tx];
         for (int k = 0; k < kGroups; ++k) h += tr[k][tx][ty];
-        const double v = -(h * fY[a]) * fY[b] * inv;
+        // (the flag beside these: read ahead of the sums it made them 10 us longer at M=24,
+        // N=50000, and 3 us between them and here)
+        const bool bad = *failed;
+        double v = -(h * fY[a]) * fY[b] * inv;
+        if (bad) v = kNaN;
         d2v[(long)a * M + b] = v;
         if (A != B) d2v[(long)b * M + a] = v;
     }
@@ -674,7 +678,7 @@ __global__ void __launch_bounds__(32 * kRows * kGroups) k_dg_final(
         if (threadIdx.x < 32 && e < M) {
             acc = 0;
             for (int k = 0; k < kGroups * kRows; ++k) acc += red[k / kRows][k % kRows][tx];
-            f[e] = acc * inv;
+            f[e] = *failed ? kNaN : acc * inv;
         }
     }
 }
@@ -783,6 +787,7 @@ int digits_prepare(tdscha_ctx *c) {
         // (the column parts of small tiles are at most as many as there are SMs)
         {(void **)&x->qp, d * 4 * std::max((size_t)x->nct * cap, (size_t)(x->nsm / nrt)) * R, false},
         {(void **)&x->abcc, d * 4 * (size_t)cap * x->Rp, false},
+        {(void **)&x->failed, i4, false},
         {(void **)&x->gpart, gbytes, false},
         {(void **)&x->fpart, d * (size_t)cap * x->nfc * M, false},
         {(void **)&x->fo, c->J == 1 ? d * cap * M : 0, false},
@@ -791,7 +796,6 @@ int digits_prepare(tdscha_ctx *c) {
         {(void **)&x->eb, 2 * i4 * Mp, false},
         // zero from the start: maxima, and the rows of padding modes
         {(void **)&x->absmax, u8 * 4 * cap, true},
-        {(void **)&x->failed, i4, true},
         {(void **)&x->etv, one * i4 * 2 * kGN, true},
         {(void **)&x->ewf, one * i4 * kGM, true},
         {(void **)&x->vb, one * 2 * (size_t)x->nkbM * kCall * kGB, true},

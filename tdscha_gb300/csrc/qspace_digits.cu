@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(128) k_qd_rowscale(const double *__restrict__ 
     }
     // An ordinary row stays at the columns' scales: with its own, up to 2^3 larger, its first
     // digits would be, and accumulations shorter (4x4x2 grid, 5 bands, N=5000 140 us a call
-    // with them, 132 so).
+    // with them, 132 so; in real space, with more columns to a row, own scales cost nothing).
     auto scale = [](int e) { return e == INT_MIN ? kZeroExp : e <= 0 && e >= -3 ? 0 : e; };
     const int2 e2 = make_int2(scale(ey), scale(eu));
     erb[t * 128 + threadIdx.x] = e2;
@@ -629,7 +629,6 @@ static int qdigits_prepare(tdscha_qctx *c) {
         {(void **)&x->ecb, sizeof(int) * (size_t)n_q * x->nbq * kGN},
         {(void **)&x->et, sizeof(int) * x->ngrp * 64},
         {(void **)&x->cofs, sizeof(int) * x->ngrp * 64},
-        {(void **)&x->failed, sizeof(int)},
         {(void **)&fl, sizeof(float) * (kFlushes * kRes + 1)},
         {(void **)&x->yb, (size_t)x->ngrp * kCall * kGB},
     };
@@ -692,6 +691,7 @@ int qdigits_set_pert(tdscha_qctx *c) {
     std::vector<int> bmap(x->n_pairs);
     for (int p = 0; p < x->n_pairs; ++p) bmap[p] = pq[2 * p + 1] * x->nbq;
     const std::vector<QPart> parts = {
+        {(void **)&x->failed, sizeof(int)},
         {(void **)&x->gpart, sizeof(double) * (size_t)x->ns * x->n_pairs * kGM * x->nbq * kGN},
         {(void **)&x->fpart, sizeof(double) * 2 * x->nfc * c->nb},
         {(void **)&x->ew, sizeof(int) * x->n_pairs * kGM},

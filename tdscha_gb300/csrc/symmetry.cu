@@ -179,11 +179,13 @@ __global__ void k_psi_jsum(const double *__restrict__ tj, const double *__restri
                            int M, double inv, const int *__restrict__ failed,
                            double *__restrict__ f, double *__restrict__ d2v) {
     pdl_enter();
-    if (failed && *failed) inv = __longlong_as_double(0x7ff8000000000000LL);
     const long MM = (long)M * M;
+    const double kNaN = __longlong_as_double(0x7ff8000000000000LL);
     for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < MM; e += (long)gridDim.x * blockDim.x) {
-        d2v[e] = -split_sum(tj + e, J, MM) * inv;
-        if (e < M) f[e] = split_sum(tf + e, J, (long)M) * inv;
+        const double d = -split_sum(tj + e, J, MM) * inv;
+        const bool bad = failed && *failed;       // (read ahead it holds the sums' loads up)
+        d2v[e] = bad ? kNaN : d;
+        if (e < M) f[e] = bad ? kNaN : split_sum(tf + e, J, (long)M) * inv;
     }
 }
 
