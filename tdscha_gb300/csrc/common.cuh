@@ -306,6 +306,10 @@ void cached_free(void *p);
 // 4 GB always, above that a quarter of what is free or idle in the cache (an allocation
 // that needs the idle blocks gets them).
 bool memory_to_spare(size_t bytes);
+// A word of pinned host memory (zero) that every device can write, and its return; from one
+// page for the process (pinning memory takes 0.1 ms), null if there is none to be had
+int *flag_alloc();
+void flag_free(int *p);
 // frees a block at once (cudaFree), whether it came from cached_malloc or not
 void release_block(void *p);
 template <typename T>

@@ -163,6 +163,43 @@ cudaError_t tdscha::cached_malloc(void **p, size_t bytes) {
     return e;
 }
 
+namespace {
+// 64 bytes a flag, so that no two share a line; pages of 64, kept for the process
+struct FlagPool {
+    std::mutex mu;
+    std::list<int *> idle;
+};
+FlagPool &flag_pool() {
+    static FlagPool *fp = new FlagPool();
+    return *fp;
+}
+}  // namespace
+
+int *tdscha::flag_alloc() {
+    constexpr int kFlags = 64, kInts = 16;
+    FlagPool &fp = flag_pool();
+    std::lock_guard<std::mutex> lock(fp.mu);
+    if (fp.idle.empty()) {
+        int *page = nullptr;
+        if (cudaHostAlloc((void **)&page, sizeof(int) * kFlags * kInts, cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        for (int k = 0; k < kFlags; ++k) fp.idle.push_back(page + k * kInts);
+    }
+    int *p = fp.idle.front();
+    fp.idle.pop_front();
+    *p = 0;
+    return p;
+}
+
+void tdscha::flag_free(int *p) {
+    if (!p) return;
+    FlagPool &fp = flag_pool();
+    std::lock_guard<std::mutex> lock(fp.mu);
+    fp.idle.push_back(p);
+}
+
 bool tdscha::memory_to_spare(size_t bytes) {
     if (bytes <= (size_t(4) << 30)) return true;
     size_t fr = 0, all = 0, idle = 0;

@@ -573,7 +573,7 @@ void qdigits_release(tdscha_qctx *c) {
     if (!c->qd) return;
     cached_free(c->qd->slab);
     cached_free(c->qd->pslab);
-    if (c->qd->err) cudaFreeHost(c->qd->err);
+    flag_free(c->qd->err);
     delete c->qd;
     c->qd = nullptr;
 }
@@ -633,14 +633,14 @@ static int qdigits_prepare(tdscha_qctx *c) {
         {(void **)&x->yb, (size_t)x->ngrp * kCall * kGB},
     };
     const size_t total = place(parts, nullptr);
-    if (!memory_to_spare(total) || cached_malloc(&x->slab, total) != cudaSuccess) {
+    x->err = flag_alloc();
+    if (!x->err || !memory_to_spare(total) || cached_malloc(&x->slab, total) != cudaSuccess) {
         cudaGetLastError();
+        flag_free(x->err);
         delete x;
         return TDSCHA_OK;
     }
     c->qd = x;
-    TDS_CUDA(cudaMallocHost((void **)&x->err, sizeof(int)));
-    *x->err = 0;
     place(parts, x->slab);
     uint8_t *z = reinterpret_cast<uint8_t *>(x->rowfar);
     TDS_CUDA(cudaMemsetAsync(z, 0, (uint8_t *)x->slab + total - z, 0));
